@@ -22,6 +22,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/fz_b200.h"
@@ -96,16 +97,19 @@ __device__ __forceinline__ double chain_tmid(double t0, double dz, double tm0, d
 //
 // L lanes per column: 32 (a warp) or 16 (two columns per warp: each lane
 // holds six elements, and every per-column scalar of the chain costs half
-// the warp instructions).  At most 128 registers a thread (four blocks, 16
-// warps per SM): the chain is bound by dependent FP64 latency, so resident
-// warps count more than the few spilled values.
+// the warp instructions).  What bounds it: full batches the FP64 work of the
+// Saha factors and of some 3.8 GET_RHO iterations per solve, five solves a
+// height; small batches the latency of that dependent chain.  Pg and 1/Pg of
+// a step's last stage serve the next step's first one, and d ln Pg is formed
+// as rho / Pg g dz without a division.  65,536 columns of 128 heights: 66.1
+// -> 43.4 ms with the 7-operation electron sum (get_rho_warp); one column on
+// precomputed factors 0.67 -> 0.44 ms, with the tensor-core group sum.
 //
 // PRE: the Saha factors of every temperature sample come precomputed from
 // k_saha (rows sa of the columns [c0, c0 + cn) of the list), and the chain
 // keeps only what is sequential: the GET_RHO iterations and the RK4 steps --
 // half the latency of a column's chain, the form for small batches (an
-// inversion's tail); on full batches the Saha work fills the stalls of the
-// GET_RHO iterations and the plain form is faster.  gate > 0: run only when
+// inversion's tail).  gate > 0: run only when
 // the column count is at most gate; gate < 0: only when it is above -gate (a
 // captured launch over a device-side count takes the form that suits it).
 template <bool HE, int L, bool PRE>
@@ -132,10 +136,12 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
   const int col = list ? list[g] : g;
   const int nsamp = HE ? 2 * nz - 1 : nz;
   const double2* rows = PRE ? sa + (size_t)(g - first) * nsamp * 96 : nullptr;
-  const unsigned hyd = saha_hyd<L>(K, lane);
   const float* m = model + (size_t)col * 13 * nz;
   float* mo = mout + (size_t)col * 13 * nz;
   double2* ch = chem + (size_t)col * nz;
+  // PRE: the next sample's row, loaded one or two GET_RHO solves before it is taken
+  double2 nx[NS];
+  if (PRE) saha_load<L>(nx, rows, lane);
   if (mo != m)
     for (int i = lane; i < 13 * nz; i += L) mo[i] = m[i];
   __syncwarp(group_mask<L>());
@@ -147,16 +153,19 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
     double nelec = 0.0;
     WarpSahaT<L> w;
     for (int k = 0; k < nz; ++k) {
-      if (PRE)
-        saha_load(w, (double)mget(m, nz, 0, k), hyd, rows + (size_t)k * 96, lane);
-      else
+      if (PRE) {
+        saha_take<L>(w, (double)mget(m, nz, 0, k), nx, K);
+        if (k + 1 < nz) saha_load<L>(nx, rows + (size_t)(k + 1) * 96, lane);
+      } else {
         saha_prepare(w, (double)mget(m, nz, 0, k), K, tb, lane);
-      const RhoOut r = get_rho_warp(w, ab, (double)mget(m, nz, 1, k), nelec, K, lane);
+      }
+      const double pg = (double)mget(m, nz, 1, k), ipg = rcp_d(pg);
+      const RhoOut r = get_rho_warp(w, ab, pg, nelec, K, lane);
       st |= r.status;
       if (lane == 0) {
         mo[2 * nz + k] = (float)r.dens;
         mo[3 * nz + k] = (float)r.pelec;
-        mo[4 * nz + k] = (float)r.molecw;
+        mo[4 * nz + k] = (float)rho_molecw(r, w.kt, ipg);
         ch[k] = make_double2(r.nhyd, nelec);
       }
     }
@@ -169,19 +178,24 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
     // stages need T(k+1) (stage 1), the linear midpoint (stages 2, 3) and
     // T(k) (stage 4 and the final GET_RHO), and T(k) is the next step's T(k+1).
     WarpSahaT<L> w;
-    if (PRE)
-      saha_load(w, (double)mget(m, nz, 0, top), hyd, rows, lane);
-    else
+    if (PRE) {
+      saha_take<L>(w, (double)mget(m, nz, 0, top), nx, K);
+      if (top > 0) saha_load<L>(nx, rows + 96, lane);
+    } else {
       saha_prepare(w, (double)mget(m, nz, 0, top), K, tb, lane);
+    }
+    // Pg at the height the step starts from and its reciprocal, kept from
+    // the previous step's last stage
+    double pg0 = exp_any(u0, K.exp2_32), ipg0 = rcp_d(pg0);
     {
-      const RhoOut r = get_rho_warp(w, ab, exp(u0), nelec, K, lane);
+      const RhoOut r = get_rho_warp(w, ab, pg0, nelec, K, lane);
       st |= r.status;
       if (lane == 0) {
         const float pel = (float)r.pelec;
-        mo[1 * nz + top] = (float)exp(u0);
+        mo[1 * nz + top] = (float)pg0;
         mo[2 * nz + top] = (float)r.dens;
         mo[3 * nz + top] = pel;
-        mo[4 * nz + top] = (float)r.molecw;
+        mo[4 * nz + top] = (float)rho_molecw(r, w.kt, ipg0);
         ch[top] = make_double2(r.nhyd, (double)pel / KBOL / (double)mget(m, nz, 0, top));
       }
     }
@@ -190,39 +204,55 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
       const double t1 = t0 + dz;
       const double tm0 = (double)mget(m, nz, 0, k + 1), tm1 = (double)mget(m, nz, 0, k);
       const double tmid = chain_tmid(t0, dz, tm0, tm1);
-      const double2* srow = PRE ? rows + (size_t)(2 * (nz - 2 - k) + 1) * 96 : nullptr;   // the midpoint's row, then T(k)'s
-      double kk[4] = {0.0, 0.0, 0.0, 0.0};
-      double u1 = 0.0;
+      // d ln Pg of a stage: -MOLECW m_u g / (k T) dz = -(rho / Pg) g dz
+      const double mgdz = -GRAV * dz;
+      double u1 = 0.0, ksum = 0.0, y = u0, pg = pg0, ipg = ipg0;
 #pragma unroll 1
       for (int stg = 0; stg < 5; ++stg) {
-        if (stg == 1 || stg == 3) {
-          if (PRE)
-            saha_load(w, stg == 1 ? tmid : tm1, hyd, stg == 1 ? srow : srow + 96, lane);
-          else
-            saha_prepare(w, stg == 1 ? tmid : tm1, K, tb, lane);
+        if (stg > 0) {
+          pg = exp_any(y, K.exp2_32);
+          ipg = rcp_d(pg);
         }
-        const double tem = stg == 0 ? tm0 : (stg < 3 ? tmid : tm1);
-        const double y = stg == 0 ? u0 : (stg == 1 ? u0 + kk[0] / 2.0 : (stg == 2 ? u0 + kk[1] / 2.0 : (stg == 3 ? u0 + kk[2] : u1)));
-        const RhoOut q = get_rho_warp(w, ab, exp(y), nelec, K, lane);
+        if (stg == 1 || stg == 3) {
+          if (PRE) {
+            // sample 2 (nz-2-k) + 1 is this step's midpoint, the next one T(k)
+            saha_take<L>(w, stg == 1 ? tmid : tm1, nx, K);
+            const int nxt = 2 * (nz - 2 - k) + (stg == 1 ? 2 : 3);
+            if (nxt < nsamp) saha_load<L>(nx, rows + (size_t)nxt * 96, lane);
+          } else {
+            saha_prepare(w, stg == 1 ? tmid : tm1, K, tb, lane);
+          }
+        }
+        const RhoOut q = get_rho_warp(w, ab, pg, nelec, K, lane);
         st |= q.status;
         if (stg < 4) {
-          const double d = (-q.molecw * MAMU * GRAV / (KBOL * tem)) * dz;
-          kk[0] = stg == 0 ? d : kk[0];
-          kk[1] = stg == 1 ? d : kk[1];
-          kk[2] = stg == 2 ? d : kk[2];
-          kk[3] = stg == 3 ? d : kk[3];
-          if (stg == 3) u1 = u0 + 1.0 / 6.0 * (kk[0] + 2.0 * kk[1] + 2.0 * kk[2] + kk[3]);
+          const double d = (q.dens * mgdz) * ipg;
+          if (stg == 0) {
+            ksum = d;
+            y = fma(0.5, d, u0);
+          } else if (stg == 1) {
+            ksum = fma(2.0, d, ksum);
+            y = fma(0.5, d, u0);
+          } else if (stg == 2) {
+            ksum = fma(2.0, d, ksum);
+            y = u0 + d;
+          } else {
+            u1 = fma(1.0 / 6.0, ksum + d, u0);
+            y = u1;
+          }
         } else if (lane == 0) {
           const float pel = (float)q.pelec;
-          mo[1 * nz + k] = (float)exp(u1);
+          mo[1 * nz + k] = (float)pg;
           mo[2 * nz + k] = (float)q.dens;
           mo[3 * nz + k] = pel;
-          mo[4 * nz + k] = (float)q.molecw;
+          mo[4 * nz + k] = (float)rho_molecw(q, w.kt, ipg);
           // FORWARD1D uses NELEC = PEL/KBOL/TEM from the REAL*4 model (src/forward.f90:900)
           ch[k] = make_double2(q.nhyd, (double)pel / KBOL / tm1);
         }
       }
       u0 = u1;
+      pg0 = pg;
+      ipg0 = ipg;
       t0 = t1;
     }
   }
@@ -235,20 +265,24 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
 // height and, with HE, the RK4 midpoint temperature of each step --
 // functions of the model alone -- so this half of the chemistry's FP64 work
 // leaves the sequential chain and runs with every (sample, element slot) in
-// parallel, one CTA per column.  Row s of the i-th column of the chunk:
-// sa[(i * nsamp + s) * 96 + slot] = (a1, a2) of the slot's element; samples
-// (HE) 0 = T(top), 2j+1 = the midpoint of step j (height nz-2-j) and 2j+2 =
-// T(nz-2-j); without HE, s = T(s).  A warp takes one sample at a time, lane
-// l the slots l, l + 32 and l + 64 (its elements fixed for the whole
-// column, so their table lines stay in L1); gridDim.y CTAs share a column's
-// samples (small batches: latency).  gate > 0: run only when the column
-// count is at most gate.
+// parallel.  Row s of the i-th column of the chunk: sa[(i * nsamp + s) * 96 +
+// slot] = (a2, c) of the slot's element; samples (HE) 0 = T(top), 2j+1 = the
+// midpoint of step j (height nz-2-j) and 2j+2 = T(nz-2-j); without HE, s =
+// T(s).  A thread keeps one element slot for all its samples: the
+// coefficients of the slot's three active partition-function pieces stay in
+// registers, reloaded only when a sample leaves the temperature interval they
+// hold for, so a sample costs its arithmetic (some 50 FP64 operations) and
+// one 16-byte store: 0.67 -> 0.19 ms on 504 columns of 256 samples against a
+// lane that reads its pieces again for every sample.  gridDim.y CTAs share a
+// column's samples (small batches: latency).  gate > 0: run only when the column count is at most gate.
+constexpr int SAHA_GROUPS = 4;   // samples a CTA takes at once, 96 threads each
 __host__ __device__ inline size_t saha_smem(int nz) {
   return (size_t)(2 * nz - 1) * (sizeof(double) + sizeof(SahaT)) + (size_t)2 * nz * sizeof(double);
 }
 
 template <bool HE>
-__global__ void __launch_bounds__(256) k_saha(const Consts* __restrict__ Kg, const PFTable* __restrict__ tb,
+__global__ void __launch_bounds__(96 * SAHA_GROUPS) k_saha(const Consts* __restrict__ Kg,
+                                              const PFTable* __restrict__ tb,
                                               int ncol, int nz, const float* __restrict__ model,
                                               double2* __restrict__ sa, int c0, int cn,
                                               const int* __restrict__ list, const int* __restrict__ nlist,
@@ -293,20 +327,64 @@ __global__ void __launch_bounds__(256) k_saha(const Consts* __restrict__ Kg, con
     for (int k = threadIdx.x; k < nz; k += blockDim.x) ts[k] = (double)mget(m, nz, 0, k);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nsamp; i += blockDim.x) tt[i] = saha_t(ts[i], K);
+  const int grp = threadIdx.x / 96, slot = threadIdx.x - 96 * grp;
+  const int s0 = SAHA_GROUPS * (int)blockIdx.y, sstep = SAHA_GROUPS * (int)gridDim.y;
+  // the terms of this CTA's samples: [s0 + i sstep, + SAHA_GROUPS)
+  for (int i = threadIdx.x; i < nsamp; i += blockDim.x)
+    if ((i - s0) % sstep >= 0 && (i - s0) % sstep < SAHA_GROUPS) tt[i] = saha_t(ts[i], K);
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int e0 = K.lane_elem[lane], e1 = K.lane_elem[lane + 32], e2 = K.lane_elem[lane + 64];
-  double2* out = sa + (size_t)blockIdx.x * nsamp * 96;
-  const int wstride = (blockDim.x >> 5) * gridDim.y;
-  for (int smp = (threadIdx.x >> 5) + blockIdx.y * (blockDim.x >> 5); smp < nsamp; smp += wstride) {
-    const double T = ts[smp];
-    const SahaT t = tt[smp];
-    double2* o = out + (size_t)smp * 96;
-    o[lane] = saha_elem<true>(e0, T, t, K, tb);
-    o[lane + 32] = saha_elem<false>(e1, T, t, K, tb);
-    o[lane + 64] = saha_elem<false>(e2, T, t, K, tb);
+  const int el = K.lane_elem[slot], e = el < 0 ? 0 : el;
+  const double x1 = K.csaha2 * fz_tab_xi[e], x2 = K.csaha2 * fz_tab_xii[e];
+  double2* out = sa + (size_t)blockIdx.x * nsamp * 96 + slot;
+  double c[3][6], bc[3], lo = 0.0, hi = 0.0;   // the active pieces and the open interval of T they hold for
+  int form[3], var[3];
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    form[s] = 0;
+    var[s] = 0;
+    bc[s] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) c[s][i] = 0.0;
   }
+  auto sample = [&](auto expf, int smp) {
+    const SahaT& t = tt[smp];
+    const double T = t.var[0];
+    if (!(T > lo && T < hi)) {
+      lo = -1.0e300;
+      hi = 1.0e300;
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        const int nv = tb->nv[e][s];
+        int act = 0;
+#pragma unroll
+        for (int i = 1; i < FZ_PF_MAXV; ++i) {
+          if (i >= nv) continue;
+          const double th = __ldg(&tb->p[e][s][i].th);
+          if (piece_on(__ldg(&tb->p[e][s][i].cond), th, T)) act = i;
+          if (th <= T) lo = fmax(lo, th);   // T = th holds for this sample alone: lo = T fails the next test
+          if (th >= T) hi = fmin(hi, th);
+        }
+        const PFPiece* p = &tb->p[e][s][act];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) c[s][i] = __ldg(&p->c[i]);
+        form[s] = __ldg(&p->form);
+        var[s] = __ldg(&p->var);
+        bc[s] = __ldg(form[s] == 1 ? &p->base : &p->clamp);
+      }
+    }
+    constexpr bool EXPF = decltype(expf)::value;
+    double u[3];
+#pragma unroll
+    for (int s = 0; s < 3; ++s) u[s] = piece_value<EXPF>(c[s], t.var[var[s]], form[s], bc[s], K.exp2_32);
+    const double e1 = exp_tab(cut650(__dmul_rn(x1, t.it)), K.exp2_32);
+    const double e2 = exp_tab(cut650(__dmul_rn(x2, t.it)), K.exp2_32);
+    const double2 f = saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
+    out[(size_t)smp * 96] = el >= 0 ? f : make_double2(0.0, 0.0);
+  };
+  if (slot < 32)   // a warp of its own: the slots whose elements may hold an exponential
+    for (int smp = s0 + grp; smp < nsamp; smp += sstep) sample(std::true_type{}, smp);
+  else
+    for (int smp = s0 + grp; smp < nsamp; smp += sstep) sample(std::false_type{}, smp);
 }
 
 // HE anchored at the height of least |log tau5| of the input model
@@ -349,16 +427,17 @@ __global__ void __launch_bounds__(128) k_chain_med(const Consts* __restrict__ Kg
   saha_prepare(w, tz, K, tb, lane);
   double nelec_down;
   {
-    const RhoOut r = get_rho_warp(w, ab, exp(ua), nelec, K, lane);
+    const double pg = exp_any(ua, K.exp2_32);
+    const RhoOut r = get_rho_warp(w, ab, pg, nelec, K, lane);
     st |= r.status;
     nelec_down = r.pelec / KBOL / tz;
     __syncwarp();
     if (lane == 0) {
       const float pel = (float)r.pelec;
-      mo[1 * nz + iz] = (float)exp(ua);
+      mo[1 * nz + iz] = (float)pg;
       mo[2 * nz + iz] = (float)r.dens;
       mo[3 * nz + iz] = pel;
-      mo[4 * nz + iz] = (float)r.molecw;
+      mo[4 * nz + iz] = (float)rho_molecw(r, w.kt, rcp_d(pg));
       ch[iz] = make_double2(r.nhyd, (double)pel / KBOL / tz);
     }
   }
@@ -373,20 +452,20 @@ __global__ void __launch_bounds__(128) k_chain_med(const Consts* __restrict__ Kg
 #pragma unroll 1
     for (int stg = 0; stg < 5; ++stg) {
       if (stg == 1 || stg == 3) saha_prepare(w, stg == 1 ? tmid : tm1, K, tb, lane);
-      const double tem = stg == 0 ? tm0 : (stg < 3 ? tmid : tm1);
       const double y = stg == 0 ? u0 : (stg == 1 ? u0 + kk[0] / 2.0 : (stg == 2 ? u0 + kk[1] / 2.0 : (stg == 3 ? u0 + kk[2] : u1)));
-      const RhoOut q = get_rho_warp(w, ab, exp(y), nelec, K, lane);
+      const double pg = exp_any(y, K.exp2_32), ipg = rcp_d(pg);
+      const RhoOut q = get_rho_warp(w, ab, pg, nelec, K, lane);
       st |= q.status;
       if (stg < 4) {
-        const double d = (-q.molecw * MAMU * GRAV / (KBOL * tem)) * dz;
+        const double d = (q.dens * (-GRAV * dz)) * ipg;   // as k_chain
         kk[stg] = d;
         if (stg == 3) u1 = u0 + 1.0 / 6.0 * (kk[0] + 2.0 * kk[1] + 2.0 * kk[2] + kk[3]);
       } else if (lane == 0) {
         const float pel = (float)q.pelec;
-        mo[1 * nz + kt] = (float)exp(u1);
+        mo[1 * nz + kt] = (float)pg;
         mo[2 * nz + kt] = (float)q.dens;
         mo[3 * nz + kt] = pel;
-        mo[4 * nz + kt] = (float)q.molecw;
+        mo[4 * nz + kt] = (float)rho_molecw(q, w.kt, ipg);
         ch[kt] = make_double2(q.nhyd, (double)pel / KBOL / tm1);
       }
     }
@@ -1584,7 +1663,8 @@ const double kXII[FZ_NELEM] = {
 #include "fz_xii.inc"
 };
 
-void host_consts(Consts& K) {
+// False if a value piece carries a condition that piece_on does not know.
+bool host_consts(Consts& K) {
   K.csaha1 = std::pow(HPLA, 3.0) / std::pow(2.0 * DPI * MELE * KBOL, 3.0 / 2.0);
   K.csaha2 = EVOLT / KBOL;
   K.rbohr = std::pow(HPLA, 2.0) / (4.0 * std::pow(DPI, 2.0) * MELE * std::pow(QELE, 2.0));
@@ -1595,19 +1675,25 @@ void host_consts(Consts& K) {
     K.deno_sa = K.deno_sa + K.ab10[i];
   }
   for (int i = 0; i < FZ_NELEM; ++i) K.deno_sam = K.deno_sam + MAMU * kMatom[i] * K.ab10[i];
-  // lane/slot assignment of the elements: exponential-form elements first
-  std::vector<int> order;
+  for (int j = 0; j < 32; ++j) K.exp2_32[j] = std::exp2(j / 32.0);
+  // lane/slot assignment of the elements: hydrogen, then the exponential-form elements
+  std::vector<int> order(1, 0);
   PFTable* t = new PFTable;
   fzh_pf_table(t);
   for (int pass = 0; pass < 2; ++pass)
-    for (int e = 0; e < FZ_NELEM; ++e) {
+    for (int e = 1; e < FZ_NELEM; ++e) {
       bool ex = false;
       for (int s = 0; s < 3; ++s)
         for (int i = 0; i < t->nv[e][s]; ++i) ex = ex || t->p[e][s][i].form == 1;
       if (ex == (pass == 0)) order.push_back(e);
     }
+  bool known = true;
+  for (int e = 0; e < FZ_NELEM; ++e)
+    for (int s = 0; s < 3; ++s)
+      for (int i = 1; i < t->nv[e][s]; ++i) known = known && (t->p[e][s][i].cond == 1 || t->p[e][s][i].cond == 2);
   delete t;
   for (int i = 0; i < 96; ++i) K.lane_elem[i] = i < (int)order.size() ? order[i] : -1;
+  return known;
 }
 
 // Wavelength-only factors of OPAC_CONTINUUM at lambda0 [A], src/cont_opacity.f90:48-357.
@@ -2043,10 +2129,10 @@ void launch_k_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, in
     ProfScope ps(c, 13, s, list ? 0 : cn);
     const dim3 gs((unsigned)cn, cn <= c->nsm ? 4u : 1u);
     if (hydrostatic)
-      k_saha<true><<<gs, 256, ssm, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, 0, cn, list, nlist,
+      k_saha<true><<<gs, 96 * SAHA_GROUPS, ssm, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, 0, cn, list, nlist,
                                         gate);
     else
-      k_saha<false><<<gs, 256, ssm, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, 0, cn, list, nlist,
+      k_saha<false><<<gs, 96 * SAHA_GROUPS, ssm, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, 0, cn, list, nlist,
                                          gate);
   }
   ProfScope ps(c, 14, s, list ? 0 : cn);
@@ -3540,7 +3626,10 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
   DevParams& P = c->hp;
   std::memset(&P, 0, sizeof(P));
   Consts K;
-  host_consts(K);
+  if (!host_consts(K)) {
+    delete c;
+    return FZ_ERR_STATE;
+  }
   int numw = 0, nlu = 0, ncomp = 0;
   std::vector<LamP> lam;
   std::vector<double> lam_l;

@@ -24,8 +24,10 @@ struct Consts {
   double ab10[FZ_NELEM];   // 10**(ABUND-12)
   // element handled by lane l in slot j of the warp chemistry: lane_elem[32*j+l]
   // (-1 = idle).  Slot 0 holds every element whose partition function has an
-  // exponential piece, so slots 1 and 2 never evaluate one.
+  // exponential piece, so slots 1 and 2 never evaluate one; hydrogen is first
+  // (lane 0, slot 0 for every L).
   int lane_elem[96];
+  double exp2_32[32];   // 2^(j/32), exp_tab's table
 };
 
 constexpr double DPI = 3.141592653589793238462643;
@@ -66,34 +68,6 @@ __device__ __forceinline__ double horner6(const double* c, double x) {
   return r;
 }
 
-// U of one (element, stage) without divergent branches: the active piece
-// (the last whose condition holds) is selected by predication, then one
-// Horner evaluation and one exponential (used only by exp forms).
-template <bool EXPF>
-__device__ __forceinline__ double pf_stage(const PFTable* __restrict__ tb, int e, int s, double T,
-                                           const double var[3]) {
-  const int nv = tb->nv[e][s];
-  int act = 0;
-#pragma unroll
-  for (int i = 1; i < FZ_PF_MAXV; ++i) {
-    const int cond = __ldg(&tb->p[e][s][i].cond);
-    const double th = __ldg(&tb->p[e][s][i].th);
-    const bool ok = (cond == 1 && T > th) || (cond == 2 && T < th) || (cond == 3 && T <= th) || (cond == 4 && T >= th);
-    act = (i < nv && ok) ? i : act;
-  }
-  const PFPiece* p = &tb->p[e][s][act];
-  double c[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) c[i] = __ldg(&p->c[i]);
-  const int form = __ldg(&p->form), v = __ldg(&p->var);
-  const double x = v == 0 ? var[0] : (v == 1 ? var[1] : var[2]);
-  const double h = horner6(c, x);
-  double u = h;
-  if (EXPF) u = form == 1 ? __ldg(&p->base) + exp(h) : u;
-  u = form == 2 ? fmax(__ldg(&p->clamp), h) : u;
-  return nv > 0 ? u : 0.0;
-}
-
 // U_I, U_II, U_III of element zn (1-based), src/atom_database.f90:121-1035
 // (generated piece table; branchy, used outside the warp chemistry).
 __device__ __forceinline__ double pf_vpiece(const fz_pf_vpiece& p, const double var[3]) {
@@ -115,28 +89,63 @@ __device__ __forceinline__ void partition_u(int zn, double T, const double var[3
   }
 }
 
-// 1/y to ~1 ulp: hardware approximation refined by two Newton steps.
+// 1/y to ~1 ulp: the hardware approximation (relative error below 1e-6)
+// corrected by one third-order (Halley) step, whose own error is its cube:
+// three FMAs, one fewer in number and in the dependent chain than two Newton
+// steps (measured over 2^20 values of 400 binades: at most 2.3e-16).
 __device__ __forceinline__ double rcp_d(double y) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
-  double e = fma(-y, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-y, r, 1.0);
-  return fma(r, e, r);
+  const double e = fma(-y, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// exp(x) to ~1 ulp by the table method (Tang, ACM TOMS 15, 1989): x =
+// n ln2/32 + r, exp(x) = 2^(n/32) (1 + r + ... + r^6/720), the 32 fractional
+// powers of two from a table (in shared memory).  11 FP64 operations, for
+// |x| <= 700 (NaN gives NaN); larger |x| is cut to the range the exponent
+// field holds.
+__device__ __forceinline__ double exp_tab(double x, const double* __restrict__ tab) {
+  const double MAGIC = 6755399441055744.0;              // 1.5 * 2^52: the sum's low word is the rounded integer
+  const double INV = 46.16624130844683;                 // 32 / ln 2
+  const double LHI = 0.021660849390173098;              // ln 2 / 32, its low 20 bits zero: n LHI is exact
+  const double LLO = 2.325192846878874e-12;             // ln 2 / 32 - LHI
+  const double t = fma(x, INV, MAGIC);
+  const int n = __double2loint(t);
+  const double nd = t - MAGIC;
+  const double r = fma(nd, -LLO, fma(nd, -LHI, x));
+  double q = fma(r, 1.0 / 720.0, 1.0 / 120.0);
+  q = fma(r, q, 1.0 / 24.0);
+  q = fma(r, q, 1.0 / 6.0);
+  q = fma(r, q, 0.5);
+  q = fma(__dmul_rn(r, r), q, r);
+  const double s = tab[n & 31];
+  const double v = fma(s, q, s);
+  const int m = min(max(n >> 5, -1020), 1020);
+  return __hiloint2double(__double2hiint(v) + (m << 20), __double2loint(v));
+}
+
+// exp(x) of any x: the table method inside its range, exp() outside (the
+// high word orders the magnitudes; infinities and NaN take exp()).
+__device__ __forceinline__ double exp_any(double x, const double* __restrict__ tab) {
+  return (__double2hiint(x) & 0x7fffffff) < 0x4085e000 ? exp_tab(x, tab) : exp(x);
 }
 
 // --------------------------------------------------------- warp chemistry
 // One column's chemistry on a group of L lanes (L = 32: a warp; L = 16: a
 // half-warp, two columns per warp), lanes over the elements: the element of
 // lane l in slot j is lane_elem[L*j + l], NS = 96 / L slots per lane.  The
-// exponential-form elements come first in lane_elem, so only the first
-// 32 / L slots of a lane (the first 32 of the 96) evaluate an exponential.
+// exponential-form elements come first in lane_elem (after hydrogen), so
+// only the first 32 / L slots of a lane (the first 32 of the 96) evaluate an
+// exponential.
+//
+// An element's Saha factors enter GET_RHO as alpha_II and the product
+// alpha_I alpha_II (a2 and c): see get_rho_warp.
 template <int L>
 struct WarpSahaT {
   static constexpr int NS = 96 / L;
-  double T;
-  double a1[NS], a2[NS];
-  unsigned hyd;   // bit j: the lane's slot j holds hydrogen
+  double T, kt, idkt;   // T, k T, 1 / (DENO_SA k T)
+  double a2[NS], c[NS];
 };
 using WarpSaha = WarpSahaT<32>;
 
@@ -146,99 +155,122 @@ __device__ __forceinline__ double clamp650(double e) {
   return e;
 }
 
+// The same limits by the magnitude's high word (no FP64 compare).
+__device__ __forceinline__ double cut650(double e) {
+  return (__double2hiint(e) & 0x7fffffff) < 0x40845000 ? e : copysign(650.0, e);
+}
+
 // The temperature terms the Saha factors of every element share: 1/T,
-// T^(-3/2) x CSAHA1 and the partition functions' variables (T, T/1000,
+// T^(-3/2) x CSAHA1 / 2 and the partition functions' variables (T, T/1000,
 // log(5040/T)).
 struct SahaT {
-  double it, lamelec, var[3];
+  double it, hl, var[3];
 };
 
 __device__ __forceinline__ SahaT saha_t(double T, const Consts& K) {
   SahaT t;
   t.it = rcp_d(T);
-  t.lamelec = K.csaha1 * (t.it * sqrt(t.it));   // T^(-3/2)
+  t.hl = __dmul_rn(0.5 * K.csaha1, __dmul_rn(t.it, sqrt(t.it)));
   t.var[0] = T;
   t.var[1] = 1.0e-3 * T;
   t.var[2] = log(5040.0 / T);
   return t;
 }
 
-// The Saha factors (a1, a2) of element el (-1: an idle slot, (0, 0)) at
-// temperature T (SHORT_PRE_ION_CALC_TEMPRHO, src/chemical_equilibrium.f90:
-// 1601-1652).  EXPF: the element's partition-function pieces may hold an
-// exponential (every such element sits in the first 32 slots).
+// The condition of a value piece on T: the generated table holds none
+// (piece 0), T > th (1) and T < th (2) only (checked when a context is made).
+__device__ __forceinline__ bool piece_on(int cond, double th, double T) { return cond == 1 ? T > th : T < th; }
+
+// (alpha_II, alpha_I alpha_II) of one element from its partition functions
+// and the two Boltzmann factors (SHORT_PRE_ION_CALC_TEMPRHO,
+// src/chemical_equilibrium.f90:1601-1652: alpha_I = U_I / (2 U_II) lambda e1,
+// alpha_II = U_II / (2 U_III) lambda e2; U_II cancels in the product, so one
+// reciprocal serves both).  Products only, rounded one by one, so that every
+// kernel that forms them gets the same bits.
+__device__ __forceinline__ double2 saha_factors(double u0, double u1, double u2, double e1, double e2, double hl) {
+  const double w = __dmul_rn(__dmul_rn(hl, rcp_d(u2)), e2);
+  return make_double2(__dmul_rn(u1, w), __dmul_rn(__dmul_rn(__dmul_rn(u0, hl), e1), w));
+}
+
+// U of a value piece at its variable (Horner, then the piece's form).
 template <bool EXPF>
-__device__ __forceinline__ double2 saha_elem(int el, double T, const SahaT& t, const Consts& K,
-                                             const PFTable* __restrict__ tb) {
+__device__ __forceinline__ double piece_value(const double c[6], double x, int form, double bc,
+                                              const double* __restrict__ tab) {
+  const double h = horner6(c, x);
+  double u = h;
+  if (EXPF && form == 1) u = bc + exp_tab(h, tab);
+  if (form == 2 && h < bc) u = bc;
+  return u;
+}
+
+// The Saha factors of element el (-1: an idle slot, zeros) at one
+// temperature.  EXPF: the element's pieces may hold an exponential.
+template <bool EXPF>
+__device__ __forceinline__ double2 saha_elem(int el, const SahaT& t, const Consts& K, const PFTable* __restrict__ tb) {
   const int e = el < 0 ? 0 : el;
-  const double u0 = pf_stage<EXPF>(tb, e, 0, T, t.var);
-  const double u1 = pf_stage<EXPF>(tb, e, 1, T, t.var);
-  const double u2 = pf_stage<EXPF>(tb, e, 2, T, t.var);
-  const double e1 = exp(clamp650(K.csaha2 * fz_tab_xi[e] * t.it));
-  const double e2 = exp(clamp650(K.csaha2 * fz_tab_xii[e] * t.it));
-  return make_double2(el >= 0 ? (u0 * (0.5 * rcp_d(u1))) * t.lamelec * e1 : 0.0,
-                      el >= 0 ? (u1 * (0.5 * rcp_d(u2))) * t.lamelec * e2 : 0.0);
-}
-
-// Bit j of the lane's hydrogen mask: its slot j holds hydrogen.
-template <int L>
-__device__ __forceinline__ unsigned saha_hyd(const Consts& K, int lane) {
-  unsigned h = 0u;
+  const double T = t.var[0];
+  double u[3];
 #pragma unroll
-  for (int j = 0; j < WarpSahaT<L>::NS; ++j)
-    if (K.lane_elem[L * j + lane] == 0) h |= 1u << j;
-  return h;
+  for (int s = 0; s < 3; ++s) {
+    const int nv = tb->nv[e][s];
+    int act = 0;
+#pragma unroll
+    for (int i = 1; i < FZ_PF_MAXV; ++i)
+      if (i < nv && piece_on(__ldg(&tb->p[e][s][i].cond), __ldg(&tb->p[e][s][i].th), T)) act = i;
+    const PFPiece* p = &tb->p[e][s][act];
+    double c[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) c[i] = __ldg(&p->c[i]);
+    const int form = __ldg(&p->form), v = __ldg(&p->var);
+    const double bc = __ldg(form == 1 ? &p->base : &p->clamp);
+    u[s] = piece_value<EXPF>(c, v == 0 ? t.var[0] : (v == 1 ? t.var[1] : t.var[2]), form, bc, K.exp2_32);
+  }
+  const double e1 = exp_tab(cut650(__dmul_rn(K.csaha2 * fz_tab_xi[e], t.it)), K.exp2_32);
+  const double e2 = exp_tab(cut650(__dmul_rn(K.csaha2 * fz_tab_xii[e], t.it)), K.exp2_32);
+  const double2 f = saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
+  return el >= 0 ? f : make_double2(0.0, 0.0);
 }
 
-// Per-lane Saha factors of the lane's elements at temperature T
-// (SHORT_PRE_ION_CALC_TEMPRHO, src/chemical_equilibrium.f90:1601-1652): the
-// arithmetic of saha_t + saha_elem written inline (so the chain's register
-// allocation stays as it was), bit for bit the same values.
+// The scalars of GET_RHO that depend on the temperature alone.
+template <int L>
+__device__ __forceinline__ void saha_scalars(WarpSahaT<L>& w, double T, const Consts& K) {
+  w.T = T;
+  w.kt = __dmul_rn(KBOL, T);
+  w.idkt = rcp_d(__dmul_rn(K.deno_sa, w.kt));
+}
+
+// Per-lane Saha factors of the lane's elements at temperature T.
 template <int L>
 __device__ __forceinline__ void saha_prepare(WarpSahaT<L>& w, double T, const Consts& K,
                                              const PFTable* __restrict__ tb, int lane) {
   constexpr int NS = WarpSahaT<L>::NS;
-  constexpr int NEXP = 32 / L;   // the lane's slots among the first 32 (the 23 exponential-form elements)
-  w.T = T;
-  w.hyd = 0u;
-  const double it = rcp_d(T);
-  const double lamelec = K.csaha1 * (it * sqrt(it));   // T^(-3/2)
-  const double var[3] = {T, 1.0e-3 * T, log(5040.0 / T)};
+  constexpr int NEXP = 32 / L;   // the lane's slots among the first 32
+  saha_scalars(w, T, K);
+  const SahaT t = saha_t(T, K);
 #pragma unroll
   for (int j = 0; j < NS; ++j) {
     const int el = K.lane_elem[L * j + lane];
-    const int e = el < 0 ? 0 : el;
-    double u0, u1, u2;
-    if (j < NEXP) {
-      u0 = pf_stage<true>(tb, e, 0, T, var);
-      u1 = pf_stage<true>(tb, e, 1, T, var);
-      u2 = pf_stage<true>(tb, e, 2, T, var);
-    } else {
-      u0 = pf_stage<false>(tb, e, 0, T, var);
-      u1 = pf_stage<false>(tb, e, 1, T, var);
-      u2 = pf_stage<false>(tb, e, 2, T, var);
-    }
-    const double e1 = exp(clamp650(K.csaha2 * fz_tab_xi[e] * it));
-    const double e2 = exp(clamp650(K.csaha2 * fz_tab_xii[e] * it));
-    if (el == 0) w.hyd |= 1u << j;
-    w.a1[j] = el >= 0 ? (u0 * (0.5 * rcp_d(u1))) * lamelec * e1 : 0.0;
-    w.a2[j] = el >= 0 ? (u1 * (0.5 * rcp_d(u2))) * lamelec * e2 : 0.0;
+    const double2 f = j < NEXP ? saha_elem<true>(el, t, K, tb) : saha_elem<false>(el, t, K, tb);
+    w.a2[j] = f.x;
+    w.c[j] = f.y;
   }
 }
 
-
 // The lane's Saha factors of one temperature sample from a precomputed row
-// (96 slots of (a1, a2) in slot order, k_saha).
+// (96 slots of (a2, c) in slot order, k_saha).
 template <int L>
-__device__ __forceinline__ void saha_load(WarpSahaT<L>& w, double T, unsigned hyd, const double2* __restrict__ row,
-                                          int lane) {
-  w.T = T;
-  w.hyd = hyd;
+__device__ __forceinline__ void saha_load(double2 (&f)[WarpSahaT<L>::NS], const double2* __restrict__ row, int lane) {
+#pragma unroll
+  for (int j = 0; j < WarpSahaT<L>::NS; ++j) f[j] = __ldcs(row + L * j + lane);
+}
+template <int L>
+__device__ __forceinline__ void saha_take(WarpSahaT<L>& w, double T, const double2 (&f)[WarpSahaT<L>::NS],
+                                          const Consts& K) {
+  saha_scalars(w, T, K);
 #pragma unroll
   for (int j = 0; j < WarpSahaT<L>::NS; ++j) {
-    const double2 a = __ldcs(row + L * j + lane);
-    w.a1[j] = a.x;
-    w.a2[j] = a.y;
+    w.a2[j] = f[j].x;
+    w.c[j] = f[j].y;
   }
 }
 
@@ -248,10 +280,28 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;   // xor butterfly: bit-identical in every lane
 }
 
-// Sum over the L lanes of a group (xor butterfly within the group; mask:
-// the group's lanes).
+// One FP64 tensor-core product D = A B (8x4 by 4x8): a lane holds A(lane/4,
+// lane%4) and B(lane%4, lane/4) and gets D(lane/4, 2 (lane%4) + {0, 1}).
+__device__ __forceinline__ void dmma(double a, double b, double& d0, double& d1) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+      : "=d"(d0), "=d"(d1)
+      : "d"(a), "d"(b), "d"(0.0));
+}
+
+// Sum over the L lanes of a group, the same bits in each of them.  L = 32:
+// two tensor-core products with ones (the 8 sums of 4 lanes, two of them to
+// each lane; their pair's sum; the sum of the 4 pairs), 69 cycles of latency
+// against 195 for five shuffle levels -- this form serves the small batches,
+// which wait for their chains.  L = 16 serves full batches, where a product's
+// 16 FP64 pipe cycles would cost more than the shuffles.
 template <int L>
 __device__ __forceinline__ double group_sum(double v, unsigned mask) {
+  if (L == 32) {
+    double d0, d1;
+    dmma(1.0, v, d0, d1);
+    dmma(d0 + d1, 1.0, d0, d1);
+    return d0;
+  }
 #pragma unroll
   for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
   return v;
@@ -264,9 +314,14 @@ __device__ __forceinline__ unsigned group_mask() {
 }
 
 struct RhoOut {
-  double nhyd, pelec, dens, molecw;
+  double nhyd, pelec, dens;
   int status;
 };
+
+// MOLECW of a GET_RHO result at gas pressure PG (ipg = 1/PG).
+__device__ __forceinline__ double rho_molecw(const RhoOut& r, double kt, double ipg) {
+  return ((r.dens * kt) * (1.0 / MAMU)) * ipg;
+}
 
 // GET_RHO, src/chemical_equilibrium.f90:165-278.  All lanes of the group
 // call it with the same arguments; nelec (the warm-start chain) is updated in
@@ -274,8 +329,11 @@ struct RhoOut {
 // (:1659-1701), NELEC_EST = N_H+ - N_H- + sum_{Z>1} (N_II + N_III), is
 // evaluated per element as ab*(1+y)/(1+y+xy) (hydrogen: ab*(1-xy)/(1+y+xy))
 // with x = ne*alpha_I, y = ne*alpha_II: algebraically the reference's three
-// quotients, one division instead of five.  ab[j] = 10**(ABUND-12) of the
-// lane's elements (0 past element 92).
+// quotients.  With a2 = alpha_II and c = alpha_I alpha_II that is two FMAs
+// for numerator and denominator, one reciprocal (three FMAs), a product and
+// the accumulating FMA: 7 FP64 operations an element and iteration (12 with
+// x, y and two Newton steps).  ab[j] = 10**(ABUND-12) of the lane's elements
+// (0 past element 92); hydrogen is lane 0's slot 0.
 template <int L>
 __device__ __forceinline__ RhoOut get_rho_warp(const WarpSahaT<L>& w, const double ab[WarpSahaT<L>::NS], double PG,
                                                double& nelec, const Consts& K, int lane) {
@@ -290,23 +348,27 @@ __device__ __forceinline__ RhoOut get_rho_warp(const WarpSahaT<L>& w, const doub
   if (pelec > PG) nelec = (PG * 0.5) / (KBOL * T);
   int iter = 1;
   double nnew = nelec, nold = nelec;
-  const double kt = KBOL * T, idkt = rcp_d(K.deno_sa * KBOL * T);
+  const double kt = w.kt, idkt = w.idkt;
   bool go = true;
   while (go) {
     nold = nnew;
-    nhyd = (PG - nnew * kt) * idkt;
-    const double ne = nnew;
-    double s = 0.0;
+    nhyd = fma(-nnew, kt, PG) * idkt;
+    const double ne = nnew, ne2 = ne * ne;
+    double s0 = 0.0, s1 = 0.0;
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
-      const double x = ne * w.a1[j], y = ne * w.a2[j];
-      const double xy = x * y;
-      const double num = ((w.hyd >> j) & 1u) ? (1.0 - xy) : (1.0 + y);   // hydrogen: N_H+ - N_H-
-      s = fma(ab[j] * num, rcp_d(1.0 + y + xy), s);
+      double num = fma(ne, w.a2[j], 1.0);
+      const double den = fma(ne2, w.c[j], num);
+      if (j == 0 && lane == 0) num = fma(-ne2, w.c[j], 1.0);   // hydrogen: N_H+ - N_H-
+      if (j & 1)
+        s1 = fma(ab[j] * num, rcp_d(den), s1);
+      else
+        s0 = fma(ab[j] * num, rcp_d(den), s0);
     }
-    s = group_sum<L>(s, mask);
-    const double est = nhyd * s;
-    nnew = (fmax(est, 0.0) + nold) * 0.5;
+    const double s = group_sum<L>(s0 + s1, mask);
+    // (max(EST, 0) + NOLD) / 2 with EST = nhyd s (a NaN estimate counts as 0)
+    const double half = 0.5 * nold, v = fma(0.5 * nhyd, s, half);
+    nnew = v > half ? v : half;
     iter = iter + 1;
     // ERROR = |(NEW-OLD)/NEW| > 1e-4, ITER <= 100, NHYD >= 0
     go = fabs(nnew - nold) > 1.0e-4 * fabs(nnew) && iter <= 100 && nhyd >= 0.0;
@@ -314,9 +376,8 @@ __device__ __forceinline__ RhoOut get_rho_warp(const WarpSahaT<L>& w, const doub
   r.status = 0;
   if (iter >= 100 || nhyd < 0.0) r.status = 1;
   nelec = nnew;
-  nhyd = (PG - nelec * KBOL * T) * idkt;
-  r.dens = nhyd * K.deno_sam + nelec * MELE;
-  r.molecw = ((r.dens * KBOL * T) * (1.0 / MAMU)) * rcp_d(PG);
+  nhyd = fma(-nelec, kt, PG) * idkt;
+  r.dens = fma(nhyd, K.deno_sam, nelec * MELE);
   if (nhyd != nhyd || nnew != nnew) r.status = 2;
   if (nelec < 0.0 || nhyd <= 0.0) r.status = 1;
   r.nhyd = nhyd;

@@ -80,13 +80,22 @@ __device__ __forceinline__ void copy_to_shared(T* dst, const T* src) {
 }
 
 // ----------------------------------------------------------------- k_chain
-// The temperature at the midpoint of an RK4 step of dz from height t0 (the
-// linear interpolation of RK4_LOG, src/hydrostatic_tools.f90:377), written
-// once for k_chain and k_saha so both round alike.
-__device__ __forceinline__ double chain_tmid(double t0, double dz, double tm0, double tm1) {
-  const double it1 = t0 + dz / 2.0;
-  return tm0 / dz * (t0 + dz - it1) + tm1 / dz * (it1 - t0);
+// The temperature at the midpoint of an RK4 step: RK4_LOG's linear
+// interpolation at t0 + dz/2 (src/hydrostatic_tools.f90:377) is the mean of
+// the two heights' temperatures (NaN for dz = 0, where the interpolation
+// divides by it).
+__device__ __forceinline__ double chain_tmid(double dz, double tm0, double tm1) {
+  return dz != 0.0 ? 0.5 * (tm0 + tm1) : __longlong_as_double(0x7ff8000000000000ll);
 }
+
+// 16 bytes from device to shared memory in the background; a thread reads
+// what it copied itself after cp_wait.
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // One warp per column walks the heights sequentially: the GET_RHO warm-start
 // chain (NELEC of one call seeds the next, src/forward.f90:914) and, in
@@ -101,19 +110,24 @@ __device__ __forceinline__ double chain_tmid(double t0, double dz, double tm0, d
 // Saha factors and of some 3.8 GET_RHO iterations per solve, five solves a
 // height; small batches the latency of that dependent chain.  Pg and 1/Pg of
 // a step's last stage serve the next step's first one, and d ln Pg is formed
-// as rho / Pg g dz without a division.  65,536 columns of 128 heights: 66.1
-// -> 43.4 ms with the 7-operation electron sum (get_rho_warp); one column on
-// precomputed factors 0.67 -> 0.44 ms, with the tensor-core group sum.
+// as rho / Pg g dz without a division.
 //
 // PRE: the Saha factors of every temperature sample come precomputed from
 // k_saha (rows sa of the columns [c0, c0 + cn) of the list), and the chain
-// keeps only what is sequential: the GET_RHO iterations and the RK4 steps --
-// half the latency of a column's chain, the form for small batches (an
-// inversion's tail).  gate > 0: run only when
-// the column count is at most gate; gate < 0: only when it is above -gate (a
-// captured launch over a device-side count takes the form that suits it).
+// keeps only what is sequential: the GET_RHO iterations and the RK4 steps.
+// 65,536 columns of 128 heights: 66.1 ms with the factors computed inside by
+// the 12-operation electron sum, 43.4 with the 7-operation one (get_rho_warp),
+// 12.4 (k_saha) + 15.4 with k_saha's rows, which cross device memory twice
+// (392 KB a column) behind the arithmetic of both kernels.  One column 0.67 ->
+// 0.44 ms.  96 registers, five CTAs an SM (20 warps; with 16 lanes 128
+// registers and four CTAs measure 16.1).  Without PRE the factors are computed
+// in place: the form of the allocation-free entry point, and of a context
+// without memory for rows.  gate > 0: run only when the column count is at
+// most gate; gate < 0: only when it is above -gate (a captured launch over a
+// device-side count takes the lanes that suit it).
+constexpr int CHAIN_PRE_CTAS = 5;
 template <bool HE, int L, bool PRE>
-__global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg, const PFTable* __restrict__ tb, int ncol,
+__global__ void __launch_bounds__(128, PRE ? CHAIN_PRE_CTAS : 4) k_chain(const Consts* __restrict__ Kg, const PFTable* __restrict__ tb, int ncol,
                                                int nz, const float* model, float* mout, double2* __restrict__ chem,
                                                int* __restrict__ status, const int* __restrict__ list = nullptr,
                                                const int* __restrict__ nlist = nullptr,
@@ -139,9 +153,27 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
   const float* m = model + (size_t)col * 13 * nz;
   float* mo = mout + (size_t)col * 13 * nz;
   double2* ch = chem + (size_t)col * nz;
-  // PRE: the next sample's row, loaded one or two GET_RHO solves before it is taken
-  double2 nx[NS];
-  if (PRE) saha_load<L>(nx, rows, lane);
+  // PRE: the next sample's row, on its way to shared memory one or two
+  // GET_RHO solves before it is taken (no registers held by the prefetch)
+  __shared__ double2 rowbuf[PRE ? NS * 128 : 1];
+  double2* nx = rowbuf + (PRE ? threadIdx.x : 0);
+  const double2* src = rows + lane;
+  auto fetch = [&](int smp) {
+    if (!PRE) return;
+#pragma unroll
+    for (int j = 0; j < NS; ++j) cp16(nx + 128 * j, src + (size_t)smp * 96 + L * j);
+  };
+  auto take = [&](WarpSahaT<L>& w, double T) {
+    saha_scalars(w, T, K);
+    cp_wait();
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+      const double2 f = nx[128 * j];
+      w.a2[j] = f.x;
+      w.c[j] = f.y;
+    }
+  };
+  fetch(0);
   if (mo != m)
     for (int i = lane; i < 13 * nz; i += L) mo[i] = m[i];
   __syncwarp(group_mask<L>());
@@ -154,8 +186,8 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
     WarpSahaT<L> w;
     for (int k = 0; k < nz; ++k) {
       if (PRE) {
-        saha_take<L>(w, (double)mget(m, nz, 0, k), nx, K);
-        if (k + 1 < nz) saha_load<L>(nx, rows + (size_t)(k + 1) * 96, lane);
+        take(w, (double)mget(m, nz, 0, k));
+        if (k + 1 < nz) fetch(k + 1);
       } else {
         saha_prepare(w, (double)mget(m, nz, 0, k), K, tb, lane);
       }
@@ -172,15 +204,14 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
   } else {
     const int top = nz - 1;
     double nelec = (double)mget(m, nz, 3, top) / KBOL / (double)mget(m, nz, 0, top);
-    double t0 = (double)mget(m, nz, 12, top) * 1000.0 * 100.0;
     double u0 = log((double)mget(m, nz, 1, top));
     // One Saha buffer serves the whole integration: within a step the RK4
     // stages need T(k+1) (stage 1), the linear midpoint (stages 2, 3) and
     // T(k) (stage 4 and the final GET_RHO), and T(k) is the next step's T(k+1).
     WarpSahaT<L> w;
     if (PRE) {
-      saha_take<L>(w, (double)mget(m, nz, 0, top), nx, K);
-      if (top > 0) saha_load<L>(nx, rows + 96, lane);
+      take(w, (double)mget(m, nz, 0, top));
+      fetch(1);
     } else {
       saha_prepare(w, (double)mget(m, nz, 0, top), K, tb, lane);
     }
@@ -201,9 +232,8 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
     }
     for (int k = nz - 2; k >= 0; --k) {
       const double dz = ((double)mget(m, nz, 12, k) - (double)mget(m, nz, 12, k + 1)) * 1000.0 * 100.0;
-      const double t1 = t0 + dz;
       const double tm0 = (double)mget(m, nz, 0, k + 1), tm1 = (double)mget(m, nz, 0, k);
-      const double tmid = chain_tmid(t0, dz, tm0, tm1);
+      const double tmid = chain_tmid(dz, tm0, tm1);
       // d ln Pg of a stage: -MOLECW m_u g / (k T) dz = -(rho / Pg) g dz
       const double mgdz = -GRAV * dz;
       double u1 = 0.0, ksum = 0.0, y = u0, pg = pg0, ipg = ipg0;
@@ -216,9 +246,9 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
         if (stg == 1 || stg == 3) {
           if (PRE) {
             // sample 2 (nz-2-k) + 1 is this step's midpoint, the next one T(k)
-            saha_take<L>(w, stg == 1 ? tmid : tm1, nx, K);
+            take(w, stg == 1 ? tmid : tm1);
             const int nxt = 2 * (nz - 2 - k) + (stg == 1 ? 2 : 3);
-            if (nxt < nsamp) saha_load<L>(nx, rows + (size_t)nxt * 96, lane);
+            if (nxt < nsamp) fetch(nxt);
           } else {
             saha_prepare(w, stg == 1 ? tmid : tm1, K, tb, lane);
           }
@@ -253,7 +283,6 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
       u0 = u1;
       pg0 = pg;
       ipg0 = ipg;
-      t0 = t1;
     }
   }
   if (lane == 0 && status) status[col] = st;
@@ -268,123 +297,120 @@ __global__ void __launch_bounds__(128, 4) k_chain(const Consts* __restrict__ Kg,
 // parallel.  Row s of the i-th column of the chunk: sa[(i * nsamp + s) * 96 +
 // slot] = (a2, c) of the slot's element; samples (HE) 0 = T(top), 2j+1 = the
 // midpoint of step j (height nz-2-j) and 2j+2 = T(nz-2-j); without HE, s =
-// T(s).  A thread keeps one element slot for all its samples: the
-// coefficients of the slot's three active partition-function pieces stay in
-// registers, reloaded only when a sample leaves the temperature interval they
-// hold for, so a sample costs its arithmetic (some 50 FP64 operations) and
-// one 16-byte store: 0.67 -> 0.19 ms on 504 columns of 256 samples against a
-// lane that reads its pieces again for every sample.  gridDim.y CTAs share a
-// column's samples (small batches: latency).  gate > 0: run only when the column count is at most gate.
-constexpr int SAHA_GROUPS = 4;   // samples a CTA takes at once, 96 threads each
-__host__ __device__ inline size_t saha_smem(int nz) {
-  return (size_t)(2 * nz - 1) * (sizeof(double) + sizeof(SahaT)) + (size_t)2 * nz * sizeof(double);
-}
+// T(s).
+//
+// A warp takes one third of the slots of spt <= 64 samples of a column, and
+// shares nothing with its neighbours: a lane first forms the terms of its
+// samples (1/T, T^(-3/2), the logarithm), then the warp walks the samples
+// with the coefficients of the lane's three active partition-function pieces
+// in registers, reloaded only when a sample leaves the temperature interval
+// they hold for.  A sample then costs its arithmetic (some 50 FP64
+// operations, 80 in the third with exponential pieces) and a 16-byte store:
+// 504 columns of 256 samples 0.67 -> 0.15 ms against a warp that read its
+// pieces again for every sample, 65,536 x 255 in 12.4 ms.  What bounds it: FP64
+// (44 % of the pipe) and the dependent operations of a sample at 20 warps per
+// SM; two samples at a time on 16 warps measure the same, 24 warps spill
+// (16.8 ms).  CTAs that shared a column's terms waited on their barrier (16.4).
+constexpr int SAHA_SPT = 64;   // samples a warp takes at most
+constexpr int SAHA_CTAS = 5;   // per SM
 
 template <bool HE>
-__global__ void __launch_bounds__(96 * SAHA_GROUPS) k_saha(const Consts* __restrict__ Kg,
-                                              const PFTable* __restrict__ tb,
-                                              int ncol, int nz, const float* __restrict__ model,
-                                              double2* __restrict__ sa, int c0, int cn,
-                                              const int* __restrict__ list, const int* __restrict__ nlist,
-                                              int gate) {
-  extern __shared__ double sm_saha[];
+__global__ void __launch_bounds__(128, SAHA_CTAS) k_saha(const Consts* __restrict__ Kg, const PFTable* __restrict__ tb,
+                                                 int ncol, int nz, const float* __restrict__ model,
+                                                 double2* __restrict__ sa, int c0, int cn, int spt,
+                                                 const int* __restrict__ list, const int* __restrict__ nlist) {
   __shared__ Consts K;
+  __shared__ SahaT terms[4][SAHA_SPT];
   const int count = list ? *nlist : ncol;
-  if (gate > 0 && count > gate) return;
-  const int g = c0 + (int)blockIdx.x;
-  if ((int)blockIdx.x >= cn || g >= count) return;
-  copy_to_shared(&K, Kg);
-  const int col = list ? list[g] : g;
-  const float* m = model + (size_t)col * 13 * nz;
+  const int cend = min(cn, count - c0);
   const int nsamp = HE ? 2 * nz - 1 : nz;
-  double* ts = sm_saha;                                        // the samples' temperatures
-  SahaT* tt = reinterpret_cast<SahaT*>(sm_saha + nsamp);       // and their shared terms
-  double* dzs = sm_saha + nsamp + nsamp * (sizeof(SahaT) / sizeof(double));   // HE: dz of step j
-  double* t0s = dzs + nz;                                                     // and its start height
-  if (HE) {
-    const int top = nz - 1;
-    for (int j = threadIdx.x; j < nz - 1; j += blockDim.x) {
-      const int k = nz - 2 - j;
-      dzs[j] = ((double)mget(m, nz, 12, k) - (double)mget(m, nz, 12, k + 1)) * 1000.0 * 100.0;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {   // the integration's own running height, added in its order
-      double t0 = (double)mget(m, nz, 12, top) * 1000.0 * 100.0;
-      for (int j = 0; j < nz - 1; ++j) {
-        t0s[j] = t0;
-        t0 = t0 + dzs[j];
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) ts[0] = (double)mget(m, nz, 0, top);
-    for (int j = threadIdx.x; j < nz - 1; j += blockDim.x) {
-      const int k = nz - 2 - j;
-      const double tm0 = (double)mget(m, nz, 0, k + 1), tm1 = (double)mget(m, nz, 0, k);
-      ts[2 * j + 1] = chain_tmid(t0s[j], dzs[j], tm0, tm1);
-      ts[2 * j + 2] = tm1;
-    }
-  } else {
-    for (int k = threadIdx.x; k < nz; k += blockDim.x) ts[k] = (double)mget(m, nz, 0, k);
-  }
+  const int nblk = (nsamp + spt - 1) / spt;
+  const long long ntask = (long long)max(cend, 0) * 3 * nblk;
+  if ((long long)blockIdx.x * 4 >= ntask) return;
+  copy_to_shared(&K, Kg);
   __syncthreads();
-  const int grp = threadIdx.x / 96, slot = threadIdx.x - 96 * grp;
-  const int s0 = SAHA_GROUPS * (int)blockIdx.y, sstep = SAHA_GROUPS * (int)gridDim.y;
-  // the terms of this CTA's samples: [s0 + i sstep, + SAHA_GROUPS)
-  for (int i = threadIdx.x; i < nsamp; i += blockDim.x)
-    if ((i - s0) % sstep >= 0 && (i - s0) % sstep < SAHA_GROUPS) tt[i] = saha_t(ts[i], K);
-  __syncthreads();
-  const int el = K.lane_elem[slot], e = el < 0 ? 0 : el;
-  const double x1 = K.csaha2 * fz_tab_xi[e], x2 = K.csaha2 * fz_tab_xii[e];
-  double2* out = sa + (size_t)blockIdx.x * nsamp * 96 + slot;
-  double c[3][6], bc[3], lo = 0.0, hi = 0.0;   // the active pieces and the open interval of T they hold for
-  int form[3], var[3];
-#pragma unroll
-  for (int s = 0; s < 3; ++s) {
-    form[s] = 0;
-    var[s] = 0;
-    bc[s] = 0.0;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) c[s][i] = 0.0;
-  }
-  auto sample = [&](auto expf, int smp) {
-    const SahaT& t = tt[smp];
-    const double T = t.var[0];
-    if (!(T > lo && T < hi)) {
-      lo = -1.0e300;
-      hi = 1.0e300;
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const int nv = tb->nv[e][s];
-        int act = 0;
-#pragma unroll
-        for (int i = 1; i < FZ_PF_MAXV; ++i) {
-          if (i >= nv) continue;
-          const double th = __ldg(&tb->p[e][s][i].th);
-          if (piece_on(__ldg(&tb->p[e][s][i].cond), th, T)) act = i;
-          if (th <= T) lo = fmax(lo, th);   // T = th holds for this sample alone: lo = T fails the next test
-          if (th >= T) hi = fmin(hi, th);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  SahaT* tt = terms[wid];
+  for (long long task = (long long)blockIdx.x * 4 + wid; task < ntask; task += (long long)gridDim.x * 4) {
+    const int third = (int)(task % 3);
+    const long long cb = task / 3;
+    const int ci = (int)(cb / nblk), s0 = (int)(cb % nblk) * spt;
+    const int n = min(spt, nsamp - s0);
+    const int col = list ? list[c0 + ci] : c0 + ci;
+    const float* m = model + (size_t)col * 13 * nz;
+    __syncwarp();   // the previous task's terms no longer read
+    for (int i = lane; i < n; i += 32) {
+      const int s = s0 + i;
+      double T;
+      if (HE) {
+        const int k = nz - 1 - (s + 1) / 2;   // the height the sample's step ends at (s = 0: the top)
+        T = (double)mget(m, nz, 0, k);
+        if (s & 1) {
+          const double dz = (double)mget(m, nz, 12, k) - (double)mget(m, nz, 12, k + 1);
+          T = chain_tmid(dz, (double)mget(m, nz, 0, k + 1), T);
         }
-        const PFPiece* p = &tb->p[e][s][act];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) c[s][i] = __ldg(&p->c[i]);
-        form[s] = __ldg(&p->form);
-        var[s] = __ldg(&p->var);
-        bc[s] = __ldg(form[s] == 1 ? &p->base : &p->clamp);
+      } else {
+        T = (double)mget(m, nz, 0, s);
       }
+      tt[i] = saha_t(T, K);
     }
-    constexpr bool EXPF = decltype(expf)::value;
-    double u[3];
+    __syncwarp();
+    const int slot = 32 * third + lane;
+    const int el = K.lane_elem[slot], e = el < 0 ? 0 : el;
+    const double x1 = K.csaha2 * fz_tab_xi[e], x2 = K.csaha2 * fz_tab_xii[e];
+    double2* out = sa + ((size_t)ci * nsamp + s0) * 96 + slot;
+    double c[3][6], bc[3], lo = 0.0, hi = 0.0;   // the active pieces and the open interval of T they hold for
+    int var[3];
+    bool expo[3];
 #pragma unroll
-    for (int s = 0; s < 3; ++s) u[s] = piece_value<EXPF>(c[s], t.var[var[s]], form[s], bc[s], K.exp2_32);
-    const double e1 = exp_tab(cut650(__dmul_rn(x1, t.it)), K.exp2_32);
-    const double e2 = exp_tab(cut650(__dmul_rn(x2, t.it)), K.exp2_32);
-    const double2 f = saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
-    out[(size_t)smp * 96] = el >= 0 ? f : make_double2(0.0, 0.0);
-  };
-  if (slot < 32)   // a warp of its own: the slots whose elements may hold an exponential
-    for (int smp = s0 + grp; smp < nsamp; smp += sstep) sample(std::true_type{}, smp);
-  else
-    for (int smp = s0 + grp; smp < nsamp; smp += sstep) sample(std::false_type{}, smp);
+    for (int s = 0; s < 3; ++s) {
+      expo[s] = false;
+      var[s] = 0;
+      bc[s] = 0.0;
+#pragma unroll
+      for (int i = 0; i < 6; ++i) c[s][i] = 0.0;
+    }
+    auto sample = [&](auto expf, int i) {
+      const SahaT& t = tt[i];
+      const double T = t.var[0];
+      if (!(T > lo && T < hi)) {
+        lo = -1.0e300;
+        hi = 1.0e300;
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          const int nv = tb->nv[e][s];
+          int act = 0;
+#pragma unroll
+          for (int q = 1; q < FZ_PF_MAXV; ++q) {
+            if (q >= nv) continue;
+            const double th = __ldg(&tb->p[e][s][q].th);
+            if (piece_on(__ldg(&tb->p[e][s][q].cond), th, T)) act = q;
+            if (th <= T) lo = fmax(lo, th);   // T = th holds for this sample alone: lo = T fails the next test
+            if (th >= T) hi = fmin(hi, th);
+          }
+          const PFPiece* p = &tb->p[e][s][act];
+#pragma unroll
+          for (int q = 0; q < 6; ++q) c[s][q] = __ldg(&p->c[q]);
+          const int form = __ldg(&p->form);
+          expo[s] = form == 1;
+          var[s] = __ldg(&p->var);
+          bc[s] = piece_bc(form, __ldg(&p->base), __ldg(&p->clamp));
+        }
+      }
+      constexpr bool EXPF = decltype(expf)::value;
+      double u[3];
+#pragma unroll
+      for (int s = 0; s < 3; ++s) u[s] = piece_value<EXPF>(c[s], t.var[var[s]], expo[s], bc[s], K.exp2_32);
+      const double e1 = exp_tab<false>(cut650(__dmul_rn(x1, t.it)), K.exp2_32);
+      const double e2 = exp_tab<false>(cut650(__dmul_rn(x2, t.it)), K.exp2_32);
+      const double2 f = saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
+      out[(size_t)i * 96] = f;
+    };
+    if (third == 0)
+      for (int i = 0; i < n; ++i) sample(std::true_type{}, i);
+    else
+      for (int i = 0; i < n; ++i) sample(std::false_type{}, i);
+  }
 }
 
 // HE anchored at the height of least |log tau5| of the input model
@@ -442,11 +468,10 @@ __global__ void __launch_bounds__(128) k_chain_med(const Consts* __restrict__ Kg
     }
   }
   // the Saha buffer holds T(kf) when a step from kf to kt starts
-  auto step = [&](int kf, int kt, double& t0, double& u0) {
+  auto step = [&](int kf, int kt, double& u0) {
     const double dz = ((double)mget(m, nz, 12, kt) - (double)mget(m, nz, 12, kf)) * 1000.0 * 100.0;
     const double tm0 = (double)mget(m, nz, 0, kf), tm1 = (double)mget(m, nz, 0, kt);
-    const double it1 = t0 + dz / 2.0;
-    const double tmid = tm0 / dz * (t0 + dz - it1) + tm1 / dz * (it1 - t0);
+    const double tmid = chain_tmid(dz, tm0, tm1);
     double kk[4] = {0.0, 0.0, 0.0, 0.0};
     double u1 = 0.0;
 #pragma unroll 1
@@ -470,16 +495,14 @@ __global__ void __launch_bounds__(128) k_chain_med(const Consts* __restrict__ Kg
       }
     }
     u0 = u1;
-    t0 = t0 + dz;
   };
-  double t0 = (double)mget(m, nz, 12, iz) * 1000.0 * 100.0, u0 = ua;
-  for (int k = iz + 1; k < nz; ++k) step(k - 1, k, t0, u0);
+  double u0 = ua;
+  for (int k = iz + 1; k < nz; ++k) step(k - 1, k, u0);
   if (iz > 0) {
-    t0 = (double)mget(m, nz, 12, iz) * 1000.0 * 100.0;
     u0 = ua;
     nelec = nelec_down;
     saha_prepare(w, tz, K, tb, lane);
-    for (int k = iz - 1; k >= 0; --k) step(k + 1, k, t0, u0);
+    for (int k = iz - 1; k >= 0; --k) step(k + 1, k, u0);
   }
   if (lane == 0 && status) status[col] = st;
 }
@@ -1913,8 +1936,8 @@ struct fz_ctx {
   // scratch (grown on demand): per (column, height) nH, ne and the opacity slab
   float* d_slab = nullptr;
   double2* d_chem = nullptr;
-  double2* d_saha = nullptr;   // k_saha's rows of a chunk of columns
-  size_t saha_bytes = 0;
+  double2* d_saha = nullptr;   // k_saha's rows of a chunk of saha_cols columns (saha_want asked for)
+  int saha_cols = 0, saha_want = 0;
   size_t scratch_cols = 0;
   // staging for the host-buffer API
   float* d_model = nullptr;
@@ -2002,11 +2025,19 @@ int cuda_fail(cudaError_t e) {
     if (_rc) return _rc;                      \
   } while (0)
 
-// k_chain takes precomputed Saha factors (k_saha) for batches of at most
-// SAHA_MAX_COLS columns: the rows of that many columns.
-constexpr int SAHA_MAX_COLS = 1024;
+// k_chain runs on precomputed Saha factors (k_saha's rows), in chunks of at
+// most SAHA_CHUNK_SM columns per SM (a full wave of 16-lane chains: 20 warps of
+// two columns) whose rows stay within SAHA_MAX_BYTES.
+constexpr int SAHA_CHUNK_SM = 40;
+constexpr size_t SAHA_MAX_BYTES = (size_t)5 << 29;
+// Listed batches (an inversion pool's occupied slots, counted on the device)
+// of at most this many columns take a warp per column.
+constexpr int CHAIN_LIST_32 = 1024;
 size_t saha_row_bytes(const fz_ctx* c) { return (size_t)(2 * c->nz - 1) * 96 * sizeof(double2); }
-int saha_chunk_cols(int ncol) { return std::min(ncol, SAHA_MAX_COLS); }
+int saha_chunk_cols(const fz_ctx* c, int ncol) {
+  const size_t cap = std::max<size_t>(1, SAHA_MAX_BYTES / saha_row_bytes(c));
+  return (int)std::min<size_t>(std::min(ncol, SAHA_CHUNK_SM * c->nsm), cap);
+}
 
 int ensure_scratch(fz_ctx* c, int ncol) {
   if ((size_t)ncol > c->scratch_cols) {
@@ -2019,19 +2050,21 @@ int ensure_scratch(fz_ctx* c, int ncol) {
     FZ_CK(cudaMalloc(&c->d_chem, (size_t)ncol * c->nz * sizeof(double2)));
     c->scratch_cols = ncol;
   }
-  const size_t sb = (size_t)saha_chunk_cols(ncol) * saha_row_bytes(c);
-  if (sb > c->saha_bytes) {
+  const int want = saha_chunk_cols(c, ncol);
+  if (want > c->saha_want) {
     cudaFree(c->d_saha);
     c->d_saha = nullptr;
-    c->saha_bytes = 0;
-    FZ_CK(cudaMalloc(&c->d_saha, sb));
-    c->saha_bytes = sb;
-    // k_saha's shared memory (the samples' temperatures and terms) above the
-    // default 48 KB for tall columns; set here, before any stream capture
-    const size_t ssm = saha_smem(c->nz);
-    if (ssm > 48 * 1024 && ssm <= 200 * 1024) {
-      FZ_CK(cudaFuncSetAttribute(k_saha<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
-      FZ_CK(cudaFuncSetAttribute(k_saha<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
+    c->saha_cols = 0;
+    c->saha_want = want;
+    // without the memory for a whole chunk, smaller ones; without any, the
+    // chain computes its own factors
+    for (int n = want; n > 0 && !c->d_saha; n = n > 64 ? n / 2 : 0) {
+      if (cudaMalloc(&c->d_saha, (size_t)n * saha_row_bytes(c)) == cudaSuccess) {
+        c->saha_cols = n;
+      } else {
+        c->d_saha = nullptr;
+        cudaGetLastError();
+      }
     }
   }
   return 0;
@@ -2088,61 +2121,53 @@ void launch_k_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, in
     k_chain_med<<<g, 128, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem, d_status);
     return;
   }
-  if (lanes != 16 && lanes != 32) lanes = ncol >= 16 * c->nsm ? 16 : 32;
+  const bool autol = lanes != 16 && lanes != 32;
+  if (autol) lanes = ncol >= 16 * c->nsm ? 16 : 32;
   const int nsamp = hydrostatic ? 2 * c->nz - 1 : c->nz;
-  // the precomputed form when the context's rows hold the batch's first
-  // SAHA_MAX_COLS columns and k_saha's shared memory fits; a batch of known
-  // size takes one form, a listed batch (count on the device) launches both,
-  // each gated by the count
-  const int per = saha_chunk_cols(ncol);
-  const size_t ssm = saha_smem(c->nz);
-  pre = pre && c->d_saha && (size_t)per * nsamp * 96 * sizeof(double2) <= c->saha_bytes && ssm <= 200 * 1024;
-  const bool plain = !pre || list || ncol > SAHA_MAX_COLS;
-  const bool fast = pre && (list || ncol <= SAHA_MAX_COLS);
-  const int gate = list ? SAHA_MAX_COLS : 0;
-  if (plain) {
-    ProfScope ps(c, 0, s, ncol);
-    const size_t threads = (size_t)ncol * lanes;
-    const dim3 gc((unsigned)((threads + wpb * 32 - 1) / (wpb * 32)));
-    const int pg = fast ? -gate : 0;
-    if (lanes == 16) {
-      if (hydrostatic)
-        k_chain<true, 16, false><<<gc, wpb * 32, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem,
-                                                         d_status, list, nlist, nullptr, 0, 0, pg);
-      else
-        k_chain<false, 16, false><<<gc, wpb * 32, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem,
-                                                          d_status, list, nlist, nullptr, 0, 0, pg);
-    } else {
-      if (hydrostatic)
-        k_chain<true, 32, false><<<gc, wpb * 32, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem,
-                                                         d_status, list, nlist, nullptr, 0, 0, pg);
-      else
-        k_chain<false, 32, false><<<gc, wpb * 32, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem,
-                                                          d_status, list, nlist, nullptr, 0, 0, pg);
-    }
-  }
-  if (!fast) return;
-  // the small-batch form: every column's Saha rows (split over a few CTAs a
-  // column, for latency), then the chains on them, always 32 lanes a column
-  const int cn = per;
-  {
-    ProfScope ps(c, 13, s, list ? 0 : cn);
-    const dim3 gs((unsigned)cn, cn <= c->nsm ? 4u : 1u);
+  pre = pre && c->saha_cols > 0;
+  auto chain = [&](auto he, auto lc, auto pc, int c0, int cn, int gate) {
+    constexpr bool HE = decltype(he)::value, PRE = decltype(pc)::value;
+    constexpr int L = decltype(lc)::value;
+    ProfScope ps(c, PRE ? 14 : 0, s, PRE && list ? 0 : cn);
+    const unsigned gc = (unsigned)(((size_t)cn * L + wpb * 32 - 1) / (wpb * 32));
+    k_chain<HE, L, PRE><<<gc, wpb * 32, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem, d_status,
+                                                list, nlist, PRE ? c->d_saha : nullptr, c0, cn, gate);
+  };
+  auto chain_l = [&](auto pc, int l, int c0, int cn, int gate) {
+    using C16 = std::integral_constant<int, 16>;
+    using C32 = std::integral_constant<int, 32>;
     if (hydrostatic)
-      k_saha<true><<<gs, 96 * SAHA_GROUPS, ssm, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, 0, cn, list, nlist,
-                                        gate);
+      l == 16 ? chain(std::true_type{}, C16{}, pc, c0, cn, gate) : chain(std::true_type{}, C32{}, pc, c0, cn, gate);
     else
-      k_saha<false><<<gs, 96 * SAHA_GROUPS, ssm, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, 0, cn, list, nlist,
-                                         gate);
+      l == 16 ? chain(std::false_type{}, C16{}, pc, c0, cn, gate) : chain(std::false_type{}, C32{}, pc, c0, cn, gate);
+  };
+  if (!pre) {
+    chain_l(std::false_type{}, lanes, 0, ncol, 0);
+    return;
   }
-  ProfScope ps(c, 14, s, list ? 0 : cn);
-  const dim3 gc((unsigned)(((size_t)cn * 32 + wpb * 32 - 1) / (wpb * 32)));
-  if (hydrostatic)
-    k_chain<true, 32, true><<<gc, wpb * 32, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem,
-                                                    d_status, list, nlist, c->d_saha, 0, cn, gate);
-  else
-    k_chain<false, 32, true><<<gc, wpb * 32, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem,
-                                                     d_status, list, nlist, c->d_saha, 0, cn, gate);
+  // a listed batch's first chunk launches both forms, each gated by the count
+  const int gate = list && autol && lanes == 16 ? CHAIN_LIST_32 : 0;
+  const int per = std::min(c->saha_cols, ncol);
+  for (int c0 = 0; c0 < ncol; c0 += per) {
+    const int cn = std::min(per, ncol - c0);
+    {
+      // every column's rows (few columns: several CTAs a column, for latency)
+      ProfScope ps(c, 13, s, list ? 0 : cn);
+      // fewer samples a warp while the batch has fewer warps' work than the SMs hold
+      const int nblk0 = (nsamp + SAHA_SPT - 1) / SAHA_SPT;
+      const int spt = cn * nblk0 * 3 >= 8 * c->nsm ? SAHA_SPT : (cn * nblk0 * 3 >= 2 * c->nsm ? SAHA_SPT / 4 : 8);
+      const long long tasks = (long long)cn * 3 * ((nsamp + spt - 1) / spt);
+      const unsigned gs = (unsigned)std::min<long long>((tasks + 3) / 4, (long long)c->nsm * SAHA_CTAS * 2);
+      if (hydrostatic)
+        k_saha<true><<<gs, 128, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, c0, cn, spt, list,
+                                        nlist);
+      else
+        k_saha<false><<<gs, 128, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, c0, cn, spt, list,
+                                         nlist);
+    }
+    if (gate && c0 == 0) chain_l(std::true_type{}, 32, 0, std::min(cn, gate), gate);
+    chain_l(std::true_type{}, lanes, c0, cn, -gate);
+  }
 }
 
 // The LSF pass over nrows rows of numw values (no-op without a valid LSF).

@@ -100,35 +100,38 @@ __device__ __forceinline__ double rcp_d(double y) {
   return fma(r, fma(e, e, e), r);
 }
 
+// exp_tab's constants, read as operands from the constant bank: 1.5 * 2^52
+// (the sum's low word is the rounded integer), 32 / ln 2, ln 2 / 32 in two
+// parts (the first with its low 20 bits zero, so n times it is exact), 1/6!,
+// 1/5!, 1/4!, 1/3!.
+__constant__ double EXP_C[8] = {6755399441055744.0, 46.16624130844683, -0.021660849390173098, -2.325192846878874e-12,
+                                1.0 / 720.0, 1.0 / 120.0, 1.0 / 24.0, 1.0 / 6.0};
+
 // exp(x) to ~1 ulp by the table method (Tang, ACM TOMS 15, 1989): x =
 // n ln2/32 + r, exp(x) = 2^(n/32) (1 + r + ... + r^6/720), the 32 fractional
 // powers of two from a table (in shared memory).  11 FP64 operations, for
-// |x| <= 700 (NaN gives NaN); larger |x| is cut to the range the exponent
-// field holds.
+// |x| <= 700 (NaN gives NaN); with CUT, larger |x| ends at 2^+-1020.
+template <bool CUT>
 __device__ __forceinline__ double exp_tab(double x, const double* __restrict__ tab) {
-  const double MAGIC = 6755399441055744.0;              // 1.5 * 2^52: the sum's low word is the rounded integer
-  const double INV = 46.16624130844683;                 // 32 / ln 2
-  const double LHI = 0.021660849390173098;              // ln 2 / 32, its low 20 bits zero: n LHI is exact
-  const double LLO = 2.325192846878874e-12;             // ln 2 / 32 - LHI
-  const double t = fma(x, INV, MAGIC);
+  const double t = fma(x, EXP_C[1], EXP_C[0]);
   const int n = __double2loint(t);
-  const double nd = t - MAGIC;
-  const double r = fma(nd, -LLO, fma(nd, -LHI, x));
-  double q = fma(r, 1.0 / 720.0, 1.0 / 120.0);
-  q = fma(r, q, 1.0 / 24.0);
-  q = fma(r, q, 1.0 / 6.0);
+  const double nd = t - EXP_C[0];
+  const double r = fma(nd, EXP_C[3], fma(nd, EXP_C[2], x));
+  double q = fma(r, EXP_C[4], EXP_C[5]);
+  q = fma(r, q, EXP_C[6]);
+  q = fma(r, q, EXP_C[7]);
   q = fma(r, q, 0.5);
   q = fma(__dmul_rn(r, r), q, r);
   const double s = tab[n & 31];
   const double v = fma(s, q, s);
-  const int m = min(max(n >> 5, -1020), 1020);
+  const int m = CUT ? min(max(n >> 5, -1020), 1020) : n >> 5;
   return __hiloint2double(__double2hiint(v) + (m << 20), __double2loint(v));
 }
 
 // exp(x) of any x: the table method inside its range, exp() outside (the
 // high word orders the magnitudes; infinities and NaN take exp()).
 __device__ __forceinline__ double exp_any(double x, const double* __restrict__ tab) {
-  return (__double2hiint(x) & 0x7fffffff) < 0x4085e000 ? exp_tab(x, tab) : exp(x);
+  return (__double2hiint(x) & 0x7fffffff) < 0x4085e000 ? exp_tab<false>(x, tab) : exp(x);
 }
 
 // --------------------------------------------------------- warp chemistry
@@ -192,19 +195,23 @@ __device__ __forceinline__ double2 saha_factors(double u0, double u1, double u2,
   return make_double2(__dmul_rn(u1, w), __dmul_rn(__dmul_rn(__dmul_rn(u0, hl), e1), w));
 }
 
-// U of a value piece at its variable (Horner, then the piece's form).
-template <bool EXPF>
-__device__ __forceinline__ double piece_value(const double c[6], double x, int form, double bc,
-                                              const double* __restrict__ tab) {
-  const double h = horner6(c, x);
-  double u = h;
-  if (EXPF && form == 1) u = bc + exp_tab(h, tab);
-  if (form == 2 && h < bc) u = bc;
-  return u;
+// The bound of a value piece's second form: the base of base + exp(h), the
+// lower limit of max(clamp, h), and a limit that never holds for h alone.
+__device__ __forceinline__ double piece_bc(int form, double base, double clamp) {
+  return form == 1 ? base : (form == 2 ? clamp : -1.0e300);
 }
 
-// The Saha factors of element el (-1: an idle slot, zeros) at one
-// temperature.  EXPF: the element's pieces may hold an exponential.
+// U of a value piece at its variable x (Horner, then the piece's form).
+template <bool EXPF>
+__device__ __forceinline__ double piece_value(const double c[6], double x, bool expo, double bc,
+                                              const double* __restrict__ tab) {
+  const double h = horner6(c, x);
+  if (EXPF && expo) return bc + exp_tab<true>(h, tab);
+  return h < bc ? bc : h;
+}
+
+// The Saha factors of element el at one temperature (an idle slot, -1, gets
+// hydrogen's: its abundance is 0).  EXPF: the element's pieces may hold an exponential.
 template <bool EXPF>
 __device__ __forceinline__ double2 saha_elem(int el, const SahaT& t, const Consts& K, const PFTable* __restrict__ tb) {
   const int e = el < 0 ? 0 : el;
@@ -222,13 +229,12 @@ __device__ __forceinline__ double2 saha_elem(int el, const SahaT& t, const Const
 #pragma unroll
     for (int i = 0; i < 6; ++i) c[i] = __ldg(&p->c[i]);
     const int form = __ldg(&p->form), v = __ldg(&p->var);
-    const double bc = __ldg(form == 1 ? &p->base : &p->clamp);
-    u[s] = piece_value<EXPF>(c, v == 0 ? t.var[0] : (v == 1 ? t.var[1] : t.var[2]), form, bc, K.exp2_32);
+    u[s] = piece_value<EXPF>(c, v == 0 ? t.var[0] : (v == 1 ? t.var[1] : t.var[2]), form == 1,
+                             piece_bc(form, __ldg(&p->base), __ldg(&p->clamp)), K.exp2_32);
   }
-  const double e1 = exp_tab(cut650(__dmul_rn(K.csaha2 * fz_tab_xi[e], t.it)), K.exp2_32);
-  const double e2 = exp_tab(cut650(__dmul_rn(K.csaha2 * fz_tab_xii[e], t.it)), K.exp2_32);
-  const double2 f = saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
-  return el >= 0 ? f : make_double2(0.0, 0.0);
+  const double e1 = exp_tab<false>(cut650(__dmul_rn(K.csaha2 * fz_tab_xi[e], t.it)), K.exp2_32);
+  const double e2 = exp_tab<false>(cut650(__dmul_rn(K.csaha2 * fz_tab_xii[e], t.it)), K.exp2_32);
+  return saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
 }
 
 // The scalars of GET_RHO that depend on the temperature alone.
@@ -253,24 +259,6 @@ __device__ __forceinline__ void saha_prepare(WarpSahaT<L>& w, double T, const Co
     const double2 f = j < NEXP ? saha_elem<true>(el, t, K, tb) : saha_elem<false>(el, t, K, tb);
     w.a2[j] = f.x;
     w.c[j] = f.y;
-  }
-}
-
-// The lane's Saha factors of one temperature sample from a precomputed row
-// (96 slots of (a2, c) in slot order, k_saha).
-template <int L>
-__device__ __forceinline__ void saha_load(double2 (&f)[WarpSahaT<L>::NS], const double2* __restrict__ row, int lane) {
-#pragma unroll
-  for (int j = 0; j < WarpSahaT<L>::NS; ++j) f[j] = __ldcs(row + L * j + lane);
-}
-template <int L>
-__device__ __forceinline__ void saha_take(WarpSahaT<L>& w, double T, const double2 (&f)[WarpSahaT<L>::NS],
-                                          const Consts& K) {
-  saha_scalars(w, T, K);
-#pragma unroll
-  for (int j = 0; j < WarpSahaT<L>::NS; ++j) {
-    w.a2[j] = f[j].x;
-    w.c[j] = f[j].y;
   }
 }
 

@@ -12,12 +12,14 @@ def _ctx(fz, nz):
 
 
 @pytest.mark.parametrize("he", [False, True])
-@pytest.mark.parametrize("nz,ncol", [(2, 1), (3, 5), (33, 148), (33, 149), (128, 3)])
+@pytest.mark.parametrize("nz,ncol", [(2, 1), (3, 5), (33, 99), (33, 149), (128, 3), (3, 2367), (3, 2368), (3, 5921)])
 def test_precomputed_factors_equal_the_chains_own(fz, nz, ncol, he):
     """fz_forward_device_static computes the Saha factors inside the chain,
     fz_forward_device takes k_saha's rows: the same bits.  Temperatures reach
     from 1,500 K to 45,000 K, through every piece of the partition functions,
-    and a column at a piece's own threshold (6,000 K) everywhere."""
+    and a column at a piece's own threshold (6,000 K) everywhere.  2,368
+    columns is where the chain changes from 32 to 16 lanes, 5,921 the first size of two
+    chunks of rows."""
     import torch
     ctx = _ctx(fz, nz)
     m = fz.atmos.make_columns(ncol, nz, seed=5)

@@ -2025,6 +2025,11 @@ int cuda_fail(cudaError_t e) {
     if (_rc) return _rc;                      \
   } while (0)
 
+// cudaMemcpy from pageable memory returns once the data is staged, before it
+// has arrived; the context's stream does not wait for the legacy stream it
+// travels on.  To be called between such copies and a launch that reads them.
+int copies_done() { return cuda_fail(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 // k_chain runs on precomputed Saha factors (k_saha's rows), in chunks of at
 // most SAHA_CHUNK_SM columns per SM (a full wave of 16-lane chains: 20 warps of
 // two columns) whose rows stay within SAHA_MAX_BYTES.
@@ -2648,6 +2653,7 @@ int lm_conf(fz_ctx* c, int npix, const fz_lm_opts* o, LMConf& C) {
       c->nhss_host.clear();
       FZ_CK(cudaMalloc(&c->d_nhss, hbig.size() * sizeof(double)));
       FZ_CK(cudaMemcpy(c->d_nhss, hbig.data(), hbig.size() * sizeof(double), cudaMemcpyHostToDevice));
+      FZ_CK_RC(copies_done());
       c->nhss_host = hbig;
     }
     C.d_hss = c->d_nhss;
@@ -3356,6 +3362,7 @@ static int lsf_install(fz_ctx* c, int region, std::vector<double>& yk) {
   FZ_CK(cudaStreamSynchronize(c->stream));
   if (!c->d_lsf) FZ_CK(cudaMalloc(&c->d_lsf, (size_t)c->numw * sizeof(double)));
   FZ_CK(cudaMemcpy(c->d_lsf, c->lsf.yk.data(), (size_t)c->numw * sizeof(double), cudaMemcpyHostToDevice));
+  FZ_CK_RC(copies_done());
   c->lsf.on = false;
   for (int r = 0; r < c->nreg; ++r) c->lsf.on = c->lsf.on || c->lsf.valid[r];
   return valid;
@@ -3764,6 +3771,7 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
     std::memcpy(c->gain.data(), gain, 4 * numw * sizeof(float));
     if ((rc = cuda_fail(cudaMemcpy(c->d_gain, gain, 4 * numw * sizeof(float), cudaMemcpyHostToDevice))))
       return fail(rc);
+    if ((rc = copies_done())) return fail(rc);
   } else {
     double* d_l = nullptr;
     int* d_st = nullptr;
@@ -3773,6 +3781,7 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
       return fail(rc);
     }
     cudaMemcpy(d_l, lam_l.data(), numw * sizeof(double), cudaMemcpyHostToDevice);
+    copies_done();
     k_gain<<<1, 256, FZ_HSRA_LEN * nreg * sizeof(double), c->stream>>>(c->d_params, c->d_consts, c->d_pf, d_l,
                                                                         c->d_gain, d_st);
     rc = cuda_fail(cudaGetLastError());
@@ -4023,6 +4032,7 @@ int fz_rf_nodes(fz_ctx* c, const int* nodes) {
     FZ_CK(cudaMemcpy(c->d_nnorm, nrm.data(), np * sizeof(double), cudaMemcpyHostToDevice));
     c->nhss_host.clear();
   }
+  FZ_CK_RC(copies_done());
   c->rf = rf;
   const size_t sms = rf_smem(c);
   int maxsm = 0;
@@ -4469,6 +4479,7 @@ static int lm_perturbation_host(fz_ctx* c, int npix, int np, int nfreq, const do
       const size_t nj = (size_t)npix * np * nfreq;
       if ((rc = cuda_fail(cudaMalloc(&d_j64, nj * sizeof(double))))) break;
       rc = cuda_fail(cudaMemcpy(d_j64, jac64, nj * sizeof(double), cudaMemcpyHostToDevice));
+      if (!rc) rc = copies_done();
       if (!rc) {
         k_f64_to_f32<<<(int)std::min<size_t>((nj + 255) / 256, (size_t)c->nsm * 16), 256, 0, c->stream>>>(
             nj, d_j64, L.jacb);
@@ -4479,6 +4490,7 @@ static int lm_perturbation_host(fz_ctx* c, int npix, int np, int nfreq, const do
     }
     cudaMemcpy(L.diff, diff, (size_t)npix * nfreq * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(d_w, ones.data(), nfreq * sizeof(double), cudaMemcpyHostToDevice);
+    if ((rc = copies_done())) break;
     if (big) {
       const int nb = (np + GT_M - 1) / GT_M;
       if ((rc = cuda_fail(cudaFuncSetAttribute(k_lm_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -4692,6 +4704,7 @@ int fz_lm_rearange(fz_ctx* c, int npix, float* models, const double* delta, int 
   if (!rc) rc = cuda_fail(cudaMalloc(&dd, db));
   if (!rc) rc = cuda_fail(cudaMemcpy(dm, models, mb, cudaMemcpyHostToDevice));
   if (!rc) rc = cuda_fail(cudaMemcpy(dd, delta, db, cudaMemcpyHostToDevice));
+  if (!rc) rc = copies_done();
   if (!rc) rc = fz_lm_rearange_device(c, npix, dm, dd, node_expansion, c->stream);
   if (!rc) rc = cuda_fail(cudaStreamSynchronize(c->stream));
   if (!rc) rc = cuda_fail(cudaMemcpy(models, dm, mb, cudaMemcpyDeviceToHost));

@@ -802,9 +802,9 @@ int fz_mlp_set_params(fz_mlp* p, const float* host) {
   size_t o = 0;
   for (int l = 0; l < p->nl; ++l) {
     const size_t nw = (size_t)p->dim[l] * p->dim[l + 1];
-    MLP_CK(cudaMemcpy(p->W[l], host + o, nw * sizeof(float), cudaMemcpyHostToDevice));
+    MLP_CK(cudaMemcpyAsync(p->W[l], host + o, nw * sizeof(float), cudaMemcpyHostToDevice, p->stream));
     o += nw;
-    MLP_CK(cudaMemcpy(p->b[l], host + o, p->dim[l + 1] * sizeof(float), cudaMemcpyHostToDevice));
+    MLP_CK(cudaMemcpyAsync(p->b[l], host + o, p->dim[l + 1] * sizeof(float), cudaMemcpyHostToDevice, p->stream));
     o += p->dim[l + 1];
     k_to_bf16<<<grid1(nw), 256, 0, p->stream>>>(nw, p->W[l], p->Wb[l]);
   }
@@ -890,7 +890,8 @@ int fz_mlp_set_loss_weights(fz_mlp* p, const float* w, int n) {
   for (int j = 0; j < n; ++j)
     if (!(w[j] >= 0.0f) || !std::isfinite(w[j])) return FZ_ERR_ARG;
   if (!p->d_lw) MLP_CK(cudaMalloc(&p->d_lw, (size_t)n * sizeof(float)));
-  MLP_CK(cudaMemcpy(p->d_lw, w, (size_t)n * sizeof(float), cudaMemcpyHostToDevice));
+  MLP_CK(cudaMemcpyAsync(p->d_lw, w, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, p->stream));
+  MLP_CK(cudaStreamSynchronize(p->stream));
   return 0;
 }
 

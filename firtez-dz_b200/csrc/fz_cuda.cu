@@ -49,8 +49,7 @@ struct DevParams {
   int lu_nc[MAXLU], lu_c0[MAXLU];
   int lu_nt[MAXLU][3];      // components per type: sigma_red, pi, sigma_blue
   float lu_duv[MAXLU];      // -1e3 lambda0 / c: d u / d v_z = lu_duv / Doppler width [mA]
-  float comp_shift[MAXCOMP], comp_str[MAXCOMP];
-  int comp_type[MAXCOMP];
+  float2 comp[MAXCOMP];     // (shift [mA/G], strength) of each component
 };
 
 // Per-wavelength constants.
@@ -584,104 +583,107 @@ __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, 
 }
 
 // ----------------------------------------------------------------- k_synth
-// One height of OLD_ANALYTICAL_SOLVER (src/rtesolver.f90:163-187): I_k =
-// (1 - O) S e0 + O I_{k-1}, om0 = 1 - O(1,1).
-__device__ __forceinline__ void rte_step(const float O[16], float om0, float S, float& I0, float& I1, float& I2,
-                                         float& I3) {
-  const float n0 = fmaf(om0, S, fmaf(O[0], I0, fmaf(O[1], I1, fmaf(O[2], I2, O[3] * I3))));
-  const float n1 = fmaf(-O[4], S, fmaf(O[4], I0, fmaf(O[5], I1, fmaf(O[6], I2, O[7] * I3))));
-  const float n2 = fmaf(-O[8], S, fmaf(O[8], I0, fmaf(O[9], I1, fmaf(O[10], I2, O[11] * I3))));
-  const float n3 = fmaf(-O[12], S, fmaf(O[12], I0, fmaf(O[13], I1, fmaf(O[14], I2, O[15] * I3))));
-  I0 = n0;
-  I1 = n1;
-  I2 = n2;
-  I3 = n3;
+// The optical depth at 5000 A between two heights from their slab rows (KC5
+// and rho) and z [km], each product and sum rounded on its own, so that every
+// kernel adds the same increments.
+__device__ __forceinline__ double tau_inc(const float* r0, const float* r1, float z1, float z0) {
+  const float a = __fadd_rn(__fmul_rn(r0[2], r0[3]), __fmul_rn(r1[2], r1[3])) / 2.0f;
+  return __dmul_rn((double)a, ((double)z1 - (double)z0) * 1000.0 * 100.0);
+}
+
+// log tau5 from the top, src/forward.f90:1000-1006 (REAL*4 accumulation), by
+// one warp: the layers' increments by its lanes, the running sum by lane 0,
+// the logarithms by its lanes again.  The increments and sums take the place
+// of the staged rows' KC5 and rho, which nothing else reads.
+__device__ __forceinline__ void log_tau5_warp(float* sm, int sw, int nz, float* mo, int lane) {
+  for (int k0 = 0; k0 < nz - 1; k0 += 32) {
+    const int k = k0 + lane;
+    double inc = 0.0;
+    if (k < nz - 1) {
+      inc = tau_inc(sm + k * sw, sm + (k + 1) * sw, mo[12 * nz + k + 1], mo[12 * nz + k]);
+    }
+    __syncwarp();
+    if (k < nz - 1) *reinterpret_cast<double*>(sm + k * sw + 2) = inc;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    float t = 1e-9f;
+    sm[(nz - 1) * sw + 2] = t;
+    for (int k = nz - 2; k >= 0; --k) {
+      t = (float)((double)t + *reinterpret_cast<const double*>(sm + k * sw + 2));
+      sm[k * sw + 2] = t;
+    }
+  }
+  __syncwarp();
+  for (int k = lane; k < nz; k += 32) mo[11 * nz + k] = log10f(sm[k * sw + 2]);
+}
+
+// Sum of a line's components c .. e - 1 of one type: H and F weighted by
+// their strengths, at u = shift (B idd) + x0 idd.
+__device__ __forceinline__ void voigt_sum(const DevParams& P, int c, int e, float a, float bi, float xi, float& h,
+                                          float& f) {
+  h = 0.f;
+  f = 0.f;
+  for (; c < e; ++c) {
+    const float2 cc = P.comp[c];
+    const VoigtW w = voigt_w(a, fmaf(cc.x, bi, xi));
+    const float k = cc.y * w.id;
+    h = fmaf(w.h, k, h);
+    f = fmaf(w.f, k, f);
+  }
 }
 
 // The synthesis of column col from its slab staged in shared memory (sm),
-// one thread per wavelength l.
+// one thread per wavelength l.  What bounds it: FP32 issue -- 38 FMA-pipe
+// operations a Zeeman component (voigt_w) and some 130 for the Planck
+// function, the operator and the formal-solution step of a layer.  65,536
+// columns of 128 heights and 224 wavelengths: 61.1 ms with the operator's 16
+// elements formed from CUDA's sinh, sin and exp, 37.9 with rte_layer, at half
+// the error against 64 bits (relative 6.4e-7 -> 2.9e-7).
 __device__ __forceinline__ void synth_column(const DevParams& P, const LamP* __restrict__ lam,
-                                             const float* __restrict__ gain, const float* sm, int col,
+                                             const float* __restrict__ gain, float* sm, int col,
                                              double* __restrict__ syn, float* mout, int* __restrict__ status) {
   const int nz = P.nz, sw = P.sw;
   const int l = threadIdx.x;
+  // the last warp, whose lines mostly have the fewest components
+  if (l >= (int)blockDim.x - 32) log_tau5_warp(sm, sw, nz, mout + (size_t)col * 13 * nz, l & 31);
   if (l >= P.numw) return;
-  if (l == 0) {
-    // log tau5 from the top, src/forward.f90:1000-1006 (REAL*4 accumulation)
-    float* mo = mout + (size_t)col * 13 * nz;
-    float tau = 1e-9f;
-    mo[11 * nz + nz - 1] = log10f(tau);
-    for (int k = nz - 2; k >= 0; --k) {
-      const float a = (sm[k * sw + 2] * sm[k * sw + 3] + sm[(k + 1) * sw + 2] * sm[(k + 1) * sw + 3]) / 2.0f;
-      const double b = ((double)mo[12 * nz + k + 1] - (double)mo[12 * nz + k]) * 1000.0 * 100.0;
-      tau = (float)((double)tau + (double)a * b);
-      mo[11 * nz + k] = log10f(tau);
-    }
-  }
   const LamP lp = lam[l];
   const int r = lp.reg;
   const int nb = P.reg_nb[r], lb = P.reg_lb[r];
   const int goff = slab_geo(P.nreg), loff = slab_line(P.nreg);
   float I0 = 0.f, I1 = 0.f, I2 = 0.f, I3 = 0.f;
-  int bad = 0;
+  bool bad = false;
   for (int k = 0; k < nz; ++k) {
     const float* row = sm + k * sw;
-    const float T = row[0];
-    const float S = lp.c1 / expm1f(lp.c2 / T);
+    const float S = planck(lp.c1, lp.c2, row[0]);
     if (k == 0 || row[1] != 0.0f) {   // SET_BOUNDARY, src/rtesolver.f90:1134-1147
       I0 = S;
       I1 = I2 = I3 = 0.f;
       continue;
     }
-    const float g1 = row[goff], g2 = row[goff + 1], g3 = row[goff + 2], g4 = row[goff + 3], g5 = row[goff + 4],
-                B = row[goff + 5];
-    float tI = row[4 + r], tQ = 0.f, tU = 0.f, tV = 0.f, rQ = 0.f, rU = 0.f, rV = 0.f;
+    const float B = row[goff + 5];
+    float tI = row[4 + r], hQ = 0.f, hV = 0.f, fQ = 0.f, fV = 0.f;
     for (int b = 0; b < nb; ++b) {
       const float* q = row + loff + 4 * (lb + b);
       const float kldz = q[0], a = q[1], idd = q[2];
-      const float x0 = lp.wave + q[3];
-      float h0 = 0.f, h1 = 0.f, h2 = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;
+      const float xi = (lp.wave + q[3]) * idd, bi = B * idd;
       // components are stored sigma_red (dM=-1), pi, sigma_blue (dM=+1)
-      int c = P.lu_c0[lb + b];
+      const int c = P.lu_c0[lb + b];
       const int e0 = c + P.lu_nt[lb + b][0], e1 = e0 + P.lu_nt[lb + b][1], e2 = e1 + P.lu_nt[lb + b][2];
-      for (; c < e0; ++c) {
-        float h, f;
-        voigt_f32(a, fmaf(P.comp_shift[c], B, x0) * idd, h, f);
-        h0 = fmaf(P.comp_str[c], h, h0);
-        f0 = fmaf(P.comp_str[c], f, f0);
-      }
-      for (; c < e1; ++c) {
-        float h, f;
-        voigt_f32(a, fmaf(P.comp_shift[c], B, x0) * idd, h, f);
-        h1 = fmaf(P.comp_str[c], h, h1);
-        f1 = fmaf(P.comp_str[c], f, f1);
-      }
-      for (; c < e2; ++c) {
-        float h, f;
-        voigt_f32(a, fmaf(P.comp_shift[c], B, x0) * idd, h, f);
-        h2 = fmaf(P.comp_str[c], h, h2);
-        f2 = fmaf(P.comp_str[c], f, f2);
-      }
+      float h0, h1, h2, f0, f1, f2;
+      voigt_sum(P, c, e0, a, bi, xi, h0, f0);
+      voigt_sum(P, e0, e1, a, bi, xi, h1, f1);
+      voigt_sum(P, e1, e2, a, bi, xi, h2, f2);
       const float hs = h0 + h2, fs = f0 + f2;
-      const float hl = 0.5f * h1 - 0.25f * hs, fl = 0.5f * f1 - 0.25f * fs;
-      tI = fmaf(kldz, g1 * hs + g2 * h1, tI);
-      tQ = fmaf(kldz, g3 * hl, tQ);
-      tU = fmaf(kldz, g4 * hl, tU);
-      tV = fmaf(kldz, g5 * (h0 - h2), tV);
-      rQ = fmaf(kldz, g3 * fl, rQ);
-      rU = fmaf(kldz, g4 * fl, rU);
-      rV = fmaf(kldz, g5 * (f0 - f2), rV);
+      tI = fmaf(kldz, fmaf(row[goff], hs, row[goff + 1] * h1), tI);
+      hQ = fmaf(kldz, fmaf(0.5f, h1, -0.25f * hs), hQ);
+      fQ = fmaf(kldz, fmaf(0.5f, f1, -0.25f * fs), fQ);
+      hV = fmaf(kldz, h0 - h2, hV);
+      fV = fmaf(kldz, f0 - f2, fV);
     }
-    float O[16], om0 = 0.0f;
-    if (!(isfinite(tI) && isfinite(tQ) && isfinite(tU) && isfinite(tV) && isfinite(rQ) && isfinite(rU) &&
-          isfinite(rV))) {
-      bad = 1;   // the reference replaces a non-finite matrix by the identity
-#pragma unroll
-      for (int i = 0; i < 16; ++i) O[i] = (i % 5 == 0) ? 1.f : 0.f;
-    } else {
-      evol_f32(tI, tQ, tU, tV, rQ, rU, rV, O, om0);
-    }
-    rte_step(O, om0, S, I0, I1, I2, I3);
+    const float g3 = row[goff + 2], g4 = row[goff + 3], g5 = row[goff + 4];
+    bad |= rte_layer(tI, g3 * hQ, g4 * hQ, g5 * hV, g3 * fQ, g4 * fQ, g5 * fV, S, I0, I1, I2, I3);
   }
   // CALCULATE_EQUIVALENT_SYN1D: x GAIN, Stokes-major
   const int nw = P.numw;
@@ -690,7 +692,7 @@ __device__ __forceinline__ void synth_column(const DevParams& P, const LamP* __r
   o[1 * nw + l] = (double)I1 * (double)gain[4 * l + 1];
   o[2 * nw + l] = (double)I2 * (double)gain[4 * l + 2];
   o[3 * nw + l] = (double)I3 * (double)gain[4 * l + 3];
-  if (!(isfinite(I0) && isfinite(I1) && isfinite(I2) && isfinite(I3))) bad = 1;
+  if (!(isfinite(I0) && isfinite(I1) && isfinite(I2) && isfinite(I3))) bad = true;
   if (status && __any_sync(__activemask(), bad) && (l & 31) == 0) atomicOr(&status[col], FZ_NAN);
 }
 
@@ -717,7 +719,7 @@ __global__ void __launch_bounds__(MAXNUMW) k_synth(const DevParams* __restrict__
     const int n4 = nz * sw / 4;
     for (int i = threadIdx.x; i < n4; i += blockDim.x) sm_synth4[i] = __ldg(src + i);
     __syncthreads();
-    synth_column(P, lam, gain, reinterpret_cast<const float*>(sm_synth4), col, syn, mout, status);
+    synth_column(P, lam, gain, reinterpret_cast<float*>(sm_synth4), col, syn, mout, status);
   }
 }
 
@@ -1004,18 +1006,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
   __syncthreads();
   const int l = threadIdx.x;
   const bool active = l < P.numw;
-  if (l == 0) {
-    // log tau5, src/forward.f90:1000-1006 (as k_synth)
-    float* mo = mout + (size_t)col * 13 * nz;
-    float tau = 1e-9f;
-    mo[11 * nz + nz - 1] = log10f(tau);
-    for (int k = nz - 2; k >= 0; --k) {
-      const float a = (sm[k * sw + 2] * sm[k * sw + 3] + sm[(k + 1) * sw + 2] * sm[(k + 1) * sw + 3]) / 2.0f;
-      const double b = ((double)mo[12 * nz + k + 1] - (double)mo[12 * nz + k]) * 1000.0 * 100.0;
-      tau = (float)((double)tau + (double)a * b);
-      mo[11 * nz + k] = log10f(tau);
-    }
-  }
+  if (l >= nthr - 32) log_tau5_warp(sm, sw, nz, mout + (size_t)col * 13 * nz, l & 31);
   const LamP lp = lam[active ? l : 0];
   const int r = lp.reg;
   const int nb = P.reg_nb[r], lb = P.reg_lb[r];
@@ -1070,7 +1061,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
         for (int t = 0; t < 3; ++t) {
           const int e = c + P.lu_nt[lb][t];
           for (; c < e; ++c) {
-            const float shf = P.comp_shift[c], st = P.comp_str[c];
+            const float shf = P.comp[c].x, st = P.comp[c].y;
             const float u = fmaf(shf, B, x0) * idd;
             float h, f;
             voigt_f32(a, u, h, f);
@@ -1269,7 +1260,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
       for (int t = 0; t < 3; ++t) {
         const int e = c + P.lu_nt[lb + b][t];
         for (; c < e; ++c) {
-          const float shf = P.comp_shift[c], st = P.comp_str[c];
+          const float shf = P.comp[c].x, st = P.comp[c].y;
           const float u = fmaf(shf, B, x0) * idd;
           float h, f;
           voigt_f32(a, u, h, f);
@@ -2772,20 +2763,9 @@ __global__ void k_rte(int ncol, int nz, int nw, const float* __restrict__ eta, c
     const double dz = 1e5 * fabs(k == nz - 1 ? zz[k] - zz[k - 1] : zz[k + 1] - zz[k]);
     const float* e = eta + ((size_t)col * nz + k) * 7 * nw + l;
     float t[7];
-    bool fin = true;
 #pragma unroll
-    for (int i = 0; i < 7; ++i) {
-      t[i] = (float)((double)e[(size_t)i * nw] * dz);
-      fin = fin && isfinite(t[i]);
-    }
-    float O[16], om0 = 0.0f;
-    if (!fin) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) O[i] = (i % 5 == 0) ? 1.f : 0.f;
-    } else {
-      evol_f32(t[0], t[1], t[2], t[3], t[4], t[5], t[6], O, om0);
-    }
-    rte_step(O, om0, S, I0, I1, I2, I3);
+    for (int i = 0; i < 7; ++i) t[i] = (float)((double)e[(size_t)i * nw] * dz);
+    rte_layer(t[0], t[1], t[2], t[3], t[4], t[5], t[6], S, I0, I1, I2, I3);
   }
   double* o = out + ((size_t)col * nw + l) * 4;
   o[0] = I0;
@@ -2813,9 +2793,7 @@ __global__ void k_tau5(int ncol, int nz, int sw, const float* __restrict__ slab,
   float tau = 1e-9f;
   mo[11 * nz + nz - 1] = log10f(tau);
   for (int k = nz - 2; k >= 0; --k) {
-    const float a = (sm[k * sw + 2] * sm[k * sw + 3] + sm[(k + 1) * sw + 2] * sm[(k + 1) * sw + 3]) / 2.0f;
-    const double b = ((double)mo[12 * nz + k + 1] - (double)mo[12 * nz + k]) * 1000.0 * 100.0;
-    tau = (float)((double)tau + (double)a * b);
+    tau = (float)((double)tau + tau_inc(sm + k * sw, sm + (k + 1) * sw, mo[12 * nz + k + 1], mo[12 * nz + k]));
     mo[11 * nz + k] = log10f(tau);
   }
 }
@@ -3696,17 +3674,24 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
       int at = ncomp;
       // group by type (ZEEMAN_COMP order kept within a type); components of
       // zero strength (the M = 0 -> 0 pi component of a Delta J = 0 line) add
-      // exactly nothing to any sum and are left out
+      // exactly nothing to any sum and are left out; those of one type at the
+      // same shift (levels of equal Lande factors) are one component of their
+      // summed strength: every sum over them is linear in it
       for (int t = -1; t <= 1; ++t) {
-        P.lu_nt[nlu][t + 1] = 0;
-        for (int i = 0; i < n; ++i)
-          if (ty[i] == t && stg[i] != 0.0) {
-            P.comp_shift[at] = (float)sh[i];
-            P.comp_str[at] = (float)stg[i];
-            P.comp_type[at] = t;
-            ++at;
-            ++P.lu_nt[nlu][t + 1];
+        const int t0 = at;
+        std::vector<double> str;
+        for (int i = 0; i < n; ++i) {
+          if (ty[i] != t || stg[i] == 0.0) continue;
+          int j = t0;
+          while (j < at && P.comp[j].x != (float)sh[i]) ++j;
+          if (j == at) {
+            P.comp[at++].x = (float)sh[i];
+            str.push_back(0.0);
           }
+          str[j - t0] += stg[i];
+        }
+        for (int j = t0; j < at; ++j) P.comp[j].y = (float)str[j - t0];
+        P.lu_nt[nlu][t + 1] = at - t0;
       }
       P.lu_nc[nlu] = at - ncomp;
       ncomp = at;

@@ -463,40 +463,202 @@ __device__ __forceinline__ double get_damping(const LineP& L, double nh, double 
 // with w = P(z)/Q(z) at z = a - i|v|.  P (degree 6) and Q (monic, degree 7)
 // have real coefficients, so each is reduced modulo the real quadratic
 // (z^2 - 2 Re z z + |z|^2) that z solves (Knuth, TAOCP vol. 2, 4.6.4):
-// 2 FMA per degree instead of a complex multiply-add.  The quotient is
-// P conj(Q') sc / |Q'|^2 with Q' = Q sc, sc = 1 / max(|Re Q|, |Im Q|), so
-// |Q'|^2 lies in [1, 2] whatever the size of Q (an error in sc cancels);
-// its reciprocals are the approximate ones (a few ulp in all, far inside
-// the approximation's own error) and no compare or select is needed.
-__device__ __forceinline__ void voigt_f32(float a, float u, float& H, float& F) {
-  const float A0 = 122.607931777104326f, A1 = 214.382388694706425f, A2 = 181.928533092181549f,
-              A3 = 93.155580458138441f, A4 = 30.180142196210589f, A5 = 5.912626209773153f,
-              A6 = .564189583562615f, B0 = 122.60793177387535f, B1 = 352.730625110963558f,
-              B2 = 457.334478783897737f, B3 = 348.703917719495792f, B4 = 170.354001821091472f,
-              B5 = 53.992906912940207f, B6 = 10.479857114260399f;
-  const float v = fabsf(u);
-  const float x = a, y = -v;
-  const float r = 2.0f * x, s = fmaf(x, x, v * v);
+// 2 FMA per degree instead of a complex multiply-add.  Real coefficients also
+// make w(conj z) = conj w(z), so z = a - i v gives F with its sign and no
+// absolute value.  With P = p1 z + p0, Q = q1 z + q0:
+//   H = ((p1 a + p0)(q1 a + q0) + p1 q1 v^2) / |Q|^2,  F = v (p0 q1 - p1 q0) / |Q|^2
+// (the quotient by the approximate reciprocal, a few ulp in all, far inside
+// the approximation's own error).  Every coefficient carries a factor 2^-62:
+// |Q|^2 then stays in range up to |z| = 2e5 and no scaling is computed.
+// 38 FMA-pipe operations and one reciprocal a component with its two sums;
+// the form with a scaled denominator and Smith's signs took some 50.
+__device__ __forceinline__ float rcp_a(float y) {   // 1/y, approximate (1 ulp)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return r;
+}
+struct VoigtW {
+  float h, f, id;   // H = h id, F = f id
+};
+__device__ __forceinline__ VoigtW voigt_w(float a, float u) {
+  const float K = 2.168404344971009e-19f;   // 2^-62
+  const float A0 = 122.607931777104326f * K, A1 = 214.382388694706425f * K, A2 = 181.928533092181549f * K,
+              A3 = 93.155580458138441f * K, A4 = 30.180142196210589f * K, A5 = 5.912626209773153f * K,
+              A6 = .564189583562615f * K, B0 = 122.60793177387535f * K, B1 = 352.730625110963558f * K,
+              B2 = 457.334478783897737f * K, B3 = 348.703917719495792f * K, B4 = 170.354001821091472f * K,
+              B5 = 53.992906912940207f * K, B6 = 10.479857114260399f * K;
+  const float uu = u * u, r = a + a, s = fmaf(a, a, uu);
   float p1 = A6, p0 = A5, t;
 #define FZ_KSTEP(C, hi, lo) \
   t = hi;                   \
   hi = fmaf(r, t, lo);      \
   lo = fmaf(-s, t, (C));
   FZ_KSTEP(A4, p1, p0) FZ_KSTEP(A3, p1, p0) FZ_KSTEP(A2, p1, p0) FZ_KSTEP(A1, p1, p0) FZ_KSTEP(A0, p1, p0)
-  float q1 = 1.0f, q0 = B6;
+  float q1 = K, q0 = B6;
   FZ_KSTEP(B5, q1, q0) FZ_KSTEP(B4, q1, q0) FZ_KSTEP(B3, q1, q0) FZ_KSTEP(B2, q1, q0) FZ_KSTEP(B1, q1, q0)
   FZ_KSTEP(B0, q1, q0)
 #undef FZ_KSTEP
-  // P = p1 z + p0, Q = q1 z + q0
-  const float nr = fmaf(p1, x, p0), ni = p1 * y;
-  const float dr = fmaf(q1, x, q0), di = q1 * y;
-  const float sc = __fdividef(1.0f, fmaxf(fabsf(dr), fabsf(di)));
-  const float dr1 = dr * sc, di1 = di * sc;
-  const float k = sc * __fdividef(1.0f, fmaf(dr1, dr1, di1 * di1));
-  const float wr = fmaf(nr, dr1, ni * di1) * k;
-  const float wi = fmaf(ni, dr1, -(nr * di1)) * k;
-  H = wr;
-  F = (u < 0.0f) ? -wi : wi;
+  const float nr = fmaf(p1, a, p0), dr = fmaf(q1, a, q0), y = q1 * uu;
+  VoigtW w;
+  w.id = rcp_a(fmaf(q1, y, dr * dr));
+  w.h = fmaf(p1, y, nr * dr);
+  w.f = u * fmaf(p0, q1, -(p1 * q0));
+  return w;
+}
+__device__ __forceinline__ void voigt_f32(float a, float u, float& H, float& F) {
+  const VoigtW w = voigt_w(a, u);
+  H = w.h * w.id;
+  F = w.f * w.id;
+}
+
+// ------------------------------------- FP32 formal solution of one layer
+// e^x = S (1 + p) with S a power of two: the reduction by ln 2 in two parts
+// and p = e^r - 1 on |r| <= ln2/2 (weighted least-maximum fit of degree 6,
+// relative error 1.7e-8), so that e^x and e^x - 1 both come without
+// cancellation.  S is cut to 2^-126 .. 2^127; NaN gives NaN.
+struct ExpF {
+  float S, p;
+  __device__ __forceinline__ float exp() const { return fmaf(S, p, S); }
+  __device__ __forceinline__ float expm1() const { return fmaf(S, p, S - 1.0f); }
+};
+__device__ __forceinline__ ExpF exp_parts(float x) {
+  const float MAGIC = 12582912.0f;   // 1.5 * 2^23
+  const float t = fmaf(x, 1.4426950408889634f, MAGIC), n = t - MAGIC;
+  const float r = fmaf(n, -1.428606765330187e-06f, fmaf(n, -0.693145751953125f, x));
+  float q = fmaf(r, 0.00138825155f, 0.00836653821f);
+  q = fmaf(r, q, 0.0416672006f);
+  q = fmaf(r, q, 0.166665435f);
+  q = fmaf(r, q, 0.49999997f);
+  ExpF e;
+  e.p = fmaf(r * r, q, r);
+  const int i = min(max(__float_as_int(t) - 0x4b400000, -126), 127);
+  e.S = __int_as_float((i + 127) << 23);
+  return e;
+}
+
+// 1/sqrt(y), approximate.
+__device__ __forceinline__ float rsqrt_a(float y) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return r;
+}
+
+// c1 / (e^(c2/T) - 1), each quotient corrected by its remainder.
+__device__ __forceinline__ float planck(float c1, float c2, float T) {
+  const float rt = rcp_a(T);
+  const float q0 = c2 * rt;
+  const float m = exp_parts(fmaf(fmaf(-q0, T, c2), rt, q0)).expm1();
+  const float rm = rcp_a(m);
+  const float s0 = c1 * rm;
+  return fmaf(fmaf(-s0, m, c1), rm, s0);
+}
+
+// The evolution operator of one layer (src/rtesolver.f90:269-473) from its
+// optical-depth increments t = eta dz, written on three scalar functions of
+// d = |eta|^2 - |rho|^2 and e = eta.rho (x = lambda_1 dz, y = lambda_2 dz with
+// sign(x y) = sign(e), x^2 - y^2 = d, x y = e, theta = x^2 + y^2):
+//   O = e^-tI { (1 + am) 1 - al X - be Y + ga M }
+//   am = (cosh x + cos y) / 2 - 1,  al = (x sinh x + y sin y) / theta,
+//   be = (x sin y - y sinh x) / theta,  ga = (cosh x - cos y) / theta,
+// where X has the elements of (eta, rho), Y those of (-rho, eta) and M is the
+// reference's M4 before its factor 2/theta.
+struct EvolABG {
+  float am, al, be, ga;
+};
+
+// The four functions.  They are entire in d and e^2: where both are below
+// 1/4 (a layer of optical depth up to about 1/2: most of an atmosphere) their
+// series have no quotient by theta and no root; above, from the roots, with
+// the reference's clamp of cosh and sinh at 2^53 (-> 1e15, :464-465).
+__device__ __forceinline__ EvolABG evol_abg(float d, float e) {
+  EvolABG o;
+  if (fmaxf(fabsf(d), fabsf(e)) <= 0.25f) {
+    const float e2 = e * e, d2 = d * d;
+    const float f1 = d2 + e2, f2 = fmaf(2.0f, e2, d2), f3 = d * f2;
+    const float g3 = d * fmaf(3.0f, e2, d2), h4 = fmaf(f2, f2, -2.0f * (e2 * e2));
+    o.al = fmaf(f3, 1.0f / 5040.0f, fmaf(f1, 1.0f / 120.0f, fmaf(d, 1.0f / 6.0f, 1.0f)));
+    o.be = -e * fmaf(f3, 1.0f / 362880.0f, fmaf(f1, 1.0f / 5040.0f, fmaf(d, 1.0f / 120.0f, 1.0f / 6.0f)));
+    o.ga = fmaf(f3, 1.0f / 40320.0f, fmaf(f1, 1.0f / 720.0f, fmaf(d, 1.0f / 24.0f, 0.5f)));
+    o.am = fmaf(h4, 1.0f / 80640.0f, fmaf(g3, 1.0f / 1440.0f, fmaf(f2, 1.0f / 48.0f, 0.25f * d)));
+    return o;
+  }
+  // R = theta / 2 and 1/R, then the larger root and its reciprocal (one
+  // Newton step each: about 1 ulp)
+  const float z = fmaf(0.25f * d, d, e * e);
+  float g = rsqrt_a(z);
+  g = fmaf(0.5f * g, fmaf(-z * g, g, 1.0f), g);
+  const float w = fmaf(z, g, 0.5f * fabsf(d));
+  float k = rsqrt_a(w);
+  k = fmaf(0.5f * k, fmaf(-w * k, k, 1.0f), k);
+  const float big = w * k, small = e * k;
+  const float x = d >= 0.0f ? big : small, y = d >= 0.0f ? small : big;
+  // sinh x and sinh^2(x/2) from e^(x/2) - 1
+  const ExpF ex = exp_parts(0.5f * x);
+  const float t = ex.expm1(), v = ex.exp();
+  float ri = rcp_a(v);
+  ri = fmaf(ri, fmaf(-v, ri, 1.0f), ri);
+  const float tr = t * ri, s2 = t + tr;   // 2 sinh(x/2)
+  float a = 0.25f * (s2 * s2), sh = s2 * fmaf(0.5f * t, tr, 1.0f);
+  // sin y and sin^2(y/2) from the half angle modulo pi (either sign of both
+  // factors gives the same products)
+  const float hy = 0.5f * y;
+  float sn, cs;
+  if (fabsf(hy) < 3.0e4f) {
+    const float n = rintf(hy * 0.3183098861837907f);
+    const float r = fmaf(n, -1.50995803e-07f, fmaf(n, -0.000967502594f, fmaf(n, -3.140625f, hy)));
+    const float ss = r * r;
+    sn = fmaf(r * ss, fmaf(ss, fmaf(ss, fmaf(ss, 2.60576121e-06f, -0.00019809595f), 0.00833306648f), -0.166666597f), r);
+    cs = fmaf(ss, fmaf(ss, fmaf(ss, fmaf(ss, fmaf(ss, -2.60769184e-07f, 2.47618755e-05f), -0.00138884038f), 0.0416666418f), -0.5f), 1.0f);
+  } else {
+    sn = sinf(hy);
+    cs = cosf(hy);
+  }
+  const float b = sn * sn, sy = 2.0f * (sn * cs);
+  float q = a + b;
+  o.am = a - b;
+  if (fabsf(x) >= 37.42994775f) {   // cosh, sinh >= 2^53 in float64
+    const float c2 = fmaf(-2.0f, b, 1.0f);
+    sh = copysignf(1e15f, x);
+    o.am = 0.5f * (1e15f + c2) - 1.0f;
+    q = 0.5f * (1e15f - c2);
+  }
+  const float it = 0.5f * g;
+  o.al = fmaf(x, sh, y * sy) * it;
+  o.be = fmaf(x, sy, -(y * sh)) * it;
+  o.ga = q * g;
+  return o;
+}
+
+// One height of OLD_ANALYTICAL_SOLVER (src/rtesolver.f90:163-187), I <- (1 - O)
+// S e0 + O I, applied as I + O (I - S e0) + S e0 row by row without forming O:
+// the operator's vectors are al eta - be rho and al rho + be eta, and 1 - O(1,1)
+// comes without cancellation from e^-tI - 1.  A non-finite matrix counts as
+// the identity (returns true), as in the reference.
+__device__ __forceinline__ bool rte_layer(float tI, float tQ, float tU, float tV, float rQ, float rU, float rV,
+                                          float S, float& I0, float& I1, float& I2, float& I3) {
+  const float eta2 = fmaf(tV, tV, fmaf(tU, tU, tQ * tQ)), rho2 = fmaf(rV, rV, fmaf(rU, rU, rQ * rQ));
+  if (!(fabsf(tI + (eta2 + rho2)) < 3.0e38f)) return true;
+  const float e = fmaf(tV, rV, fmaf(tU, rU, tQ * rQ));
+  const EvolABG f = evol_abg(eta2 - rho2, e);
+  const ExpF ex = exp_parts(-tI);
+  const float E = ex.exp(), gh = f.ga * (0.5f * (eta2 + rho2));
+  const float om0 = -fmaf(E, f.am + gh, ex.expm1());
+  const float uQ = fmaf(f.al, tQ, -(f.be * rQ)), uU = fmaf(f.al, tU, -(f.be * rU)), uV = fmaf(f.al, tV, -(f.be * rV));
+  const float vQ = fmaf(f.al, rQ, f.be * tQ), vU = fmaf(f.al, rU, f.be * tU), vV = fmaf(f.al, rV, f.be * tV);
+  const float cQ = f.ga * fmaf(tU, rV, -(tV * rU)), cU = f.ga * fmaf(tV, rQ, -(tQ * rV)),
+              cV = f.ga * fmaf(tQ, rU, -(tU * rQ));
+  const float w0 = I0 - S;
+  const float ge = f.ga * fmaf(tV, I3, fmaf(tU, I2, tQ * I1)), gr = f.ga * fmaf(rV, I3, fmaf(rU, I2, rQ * I1));
+  const float dg = (1.0f - gh) + f.am;
+  const float n0 = fmaf(uV - cV, I3, fmaf(uU - cU, I2, (uQ - cQ) * I1));
+  const float n1 = fmaf(rQ, gr, fmaf(tQ, ge, fmaf(vV, I2, fmaf(-vU, I3, fmaf(dg, I1, -((uQ + cQ) * w0))))));
+  const float n2 = fmaf(rU, gr, fmaf(tU, ge, fmaf(vQ, I3, fmaf(-vV, I1, fmaf(dg, I2, -((uU + cU) * w0))))));
+  const float n3 = fmaf(rV, gr, fmaf(tV, ge, fmaf(vU, I1, fmaf(-vQ, I2, fmaf(dg, I3, -((uV + cV) * w0))))));
+  I0 = fmaf(-E, n0, fmaf(-om0, w0, I0));
+  I1 = E * n1;
+  I2 = E * n2;
+  I3 = E * n3;
+  return false;
 }
 
 // Evolution operator O of one layer from its optical-depth increments
@@ -598,13 +760,6 @@ __device__ __forceinline__ void evol_matrix(const EvolCore& c, float tI, float t
   O[7] = eS * m2_42 + eH * m3_42 + eQ * m4_42;
   O[14] = -eS * m2_43 - eH * m3_43 + eQ * m4_43;
   O[11] = eS * m2_43 + eH * m3_43 + eQ * m4_43;
-}
-
-__device__ __forceinline__ void evol_f32(float tI, float tQ, float tU, float tV, float rQ, float rU, float rV,
-                                         float O[16], float& om0) {
-  EvolCore c;
-  evol_core(tI, tQ, tU, tV, rQ, rU, rV, c);
-  evol_matrix(c, tI, tQ, tU, tV, rQ, rU, rV, O, om0);
 }
 
 }  // namespace fzd

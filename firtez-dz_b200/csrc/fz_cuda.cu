@@ -17,17 +17,20 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <new>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "../../include/fz_b200.h"
 #include "fz_host.h"
 #include "fz_physics.cuh"
+#include "fz_layer2.cuh"
 #include "fz_rf.cuh"
 
 using namespace fzd;
@@ -49,7 +52,7 @@ struct DevParams {
   int lu_nc[MAXLU], lu_c0[MAXLU];
   int lu_nt[MAXLU][3];      // components per type: sigma_red, pi, sigma_blue
   float lu_duv[MAXLU];      // -1e3 lambda0 / c: d u / d v_z = lu_duv / Doppler width [mA]
-  float2 comp[MAXCOMP];     // (shift [mA/G], strength) of each component
+  float4 comp[MAXCOMP];     // (shift [mA/G], shift, strength, strength) of each component
 };
 
 // Per-wavelength constants.
@@ -60,14 +63,23 @@ struct LamP {
   int reg;
 };
 
-// slab row layout: T, boundary flag, KC5 (REAL), rho (REAL), kc*dz per
-// region, 6 field-geometry factors, 4 floats per used line
+// A thread's wavelengths in k_synth: two neighbours l0, l0 + 1 of one region
+// (n = 2), the last of an odd region (n = 1, both halves the same), or none.
+struct PairP {
+  float wave[2], c1[2], c2[2];   // as LamP
+  int reg, l0, n, pad;
+};
+
+// slab row layout: T, boundary flag, KC5 (REAL), rho (REAL), 4 floats per used
+// line, 6 field-geometry factors, kc*dz per region (rows, lines and factors
+// start on 16 bytes)
 __host__ __device__ inline int slab_w(int nreg, int nlu) {
   const int w = 4 + nreg + 6 + 4 * nlu;
   return (w + 3) & ~3;
 }
-__host__ __device__ inline int slab_geo(int nreg) { return 4 + nreg; }
-__host__ __device__ inline int slab_line(int nreg) { return 4 + nreg + 6; }
+constexpr int SLAB_LINE = 4;
+__host__ __device__ inline int slab_geo(int nlu) { return 4 + 4 * nlu; }
+__host__ __device__ inline int slab_kc(int nlu) { return 4 + 4 * nlu + 6; }
 
 __device__ __forceinline__ float mget(const float* m, int nz, int p, int k) { return m[p * nz + k]; }
 
@@ -542,7 +554,7 @@ __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, 
     row[1] = (kc5 < KC5THRESHOLD) ? 0.0f : 1.0f;
     row[2] = (float)kc5;
     row[3] = mget(m, nz, 2, k);
-    for (int r = 0; r < P.nreg; ++r) row[4 + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
+    for (int r = 0; r < P.nreg; ++r) row[slab_kc(P.nlu) + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
     // field geometry, src/absorption_matrix.f90:919-991
     {
       const double x = mget(m, nz, 5, k), y = mget(m, nz, 6, k), z = mget(m, nz, 7, k);
@@ -558,7 +570,7 @@ __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, 
         c2p = (x2 - y2) / (x2 + y2);
         s2p = 2. * x * y / (x2 + y2);
       }
-      float* g = row + slab_geo(P.nreg);
+      float* g = row + slab_geo(P.nlu);
       g[0] = (float)(0.25 * cgf);
       g[1] = (float)(0.5 * sgf);
       g[2] = (float)(sgf * c2p);
@@ -573,7 +585,7 @@ __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, 
       const double damp = get_damping(L, nhyd, T);
       const double dldop = 1e3 * (sqrt(L.vdk * T) * L.l0 / LIGHT);
       const double dlv = -1e3 * L.l0 * vz / LIGHT;
-      float* q = row + slab_line(P.nreg) + 4 * b;
+      float* q = row + SLAB_LINE + 4 * b;
       q[0] = (float)(klin * dz);
       q[1] = (float)damp;
       q[2] = (float)(1.0 / dldop);
@@ -618,108 +630,166 @@ __device__ __forceinline__ void log_tau5_warp(float* sm, int sw, int nz, float* 
   for (int k = lane; k < nz; k += 32) mo[11 * nz + k] = log10f(sm[k * sw + 2]);
 }
 
-// Sum of a line's components c .. e - 1 of one type: H and F weighted by
-// their strengths, at u = shift (B idd) + x0 idd.
-__device__ __forceinline__ void voigt_sum(const DevParams& P, int c, int e, float a, float bi, float xi, float& h,
-                                          float& f) {
-  h = 0.f;
-  f = 0.f;
+// What k_synth reads of DevParams, in shared memory.
+struct SynthP {
+  alignas(16) int c[MAXLU][4];   // ends of a line's sigma_red, pi, sigma_blue components
+  float4 comp[MAXCOMP];
+  int nlu, nb[MAXREG], lb[MAXREG];
+};
+__device__ __forceinline__ void synth_params(SynthP& s, const DevParams* __restrict__ P) {
+  const int t = threadIdx.x;
+  if (t == 0) s.nlu = P->nlu;
+  if (t < MAXREG) {
+    s.nb[t] = P->reg_nb[t];
+    s.lb[t] = P->reg_lb[t];
+  }
+  int n = 0;
+  for (int b = 0; b < P->nlu; ++b) n = P->lu_c0[b] + P->lu_nc[b];
+  for (int b = t; b < P->nlu; b += blockDim.x) {
+    int e = P->lu_c0[b];
+    s.c[b][0] = e;
+    for (int q = 0; q < 3; ++q) s.c[b][q + 1] = e += P->lu_nt[b][q];
+  }
+  for (int i = t; i < n; i += blockDim.x) s.comp[i] = P->comp[i];
+}
+
+// Sum of a line's components c .. e - 1 of one type at two wavelengths: H and F
+// weighted by their strengths, at u = shift (B idd) + x0 idd.
+__device__ __forceinline__ void voigt_sum2(const SynthP& P, int c, int e, const VoigtA& A, F2 bi, F2 xi, F2& h,
+                                           F2& f) {
+  h = f2(0.f);
+  f = h;
+#pragma unroll 2
   for (; c < e; ++c) {
-    const float2 cc = P.comp[c];
-    const VoigtW w = voigt_w(a, fmaf(cc.x, bi, xi));
-    const float k = cc.y * w.id;
-    h = fmaf(w.h, k, h);
-    f = fmaf(w.f, k, f);
+    const ulonglong2 cc = *reinterpret_cast<const ulonglong2*>(&P.comp[c]);
+    F2 wh, wf, k;
+    voigt_w2(A, fma2(F2{cc.x}, bi, xi), wh, wf, k);
+    k = F2{cc.y} * k;
+    h = fma2(wh, k, h);
+    f = fma2(wf, k, f);
   }
 }
 
-// The synthesis of column col from its slab staged in shared memory (sm),
-// one thread per wavelength l.  What bounds it: FP32 issue -- 38 FMA-pipe
-// operations a Zeeman component (voigt_w) and some 130 for the Planck
-// function, the operator and the formal-solution step of a layer.  65,536
-// columns of 128 heights and 224 wavelengths: 61.1 ms with the operator's 16
-// elements formed from CUDA's sinh, sin and exp, 37.9 with rte_layer, at half
-// the error against 64 bits (relative 6.4e-7 -> 2.9e-7).
-__device__ __forceinline__ void synth_column(const DevParams& P, const LamP* __restrict__ lam,
-                                             const float* __restrict__ gain, float* sm, int col,
-                                             double* __restrict__ syn, float* mout, int* __restrict__ status) {
-  const int nz = P.nz, sw = P.sw;
-  const int l = threadIdx.x;
-  // the last warp, whose lines mostly have the fewest components
-  if (l >= (int)blockDim.x - 32) log_tau5_warp(sm, sw, nz, mout + (size_t)col * 13 * nz, l & 31);
-  if (l >= P.numw) return;
-  const LamP lp = lam[l];
-  const int r = lp.reg;
-  const int nb = P.reg_nb[r], lb = P.reg_lb[r];
-  const int goff = slab_geo(P.nreg), loff = slab_line(P.nreg);
-  float I0 = 0.f, I1 = 0.f, I2 = 0.f, I3 = 0.f;
+// The layer of slab row `row` at a thread's two wavelengths.  Returns true if
+// one of its matrices is not finite.
+__device__ __forceinline__ bool synth_layer(const SynthP& P, const PairP& pr, const float* row, Layer2& L) {
+  const int nb = P.nb[pr.reg], lb = P.lb[pr.reg];
+  const float* geo = row + slab_geo(P.nlu);
+  const float4 ga = *reinterpret_cast<const float4*>(geo);          // 0.25 cgf, 0.5 sgf, sgf c2p, sgf s2p
+  const float2 gb = *reinterpret_cast<const float2*>(geo + 4);      // 0.5 cosg, B
+  F2 tI = f2(geo[6 + pr.reg]), hQ = f2(0.f), hV = hQ, fQ = hQ, fV = hQ;
+  for (int b = 0; b < nb; ++b) {
+    const float4 q = *reinterpret_cast<const float4*>(row + SLAB_LINE + 4 * (lb + b));   // KLIN dz, a, 1/Doppler, shift
+    const VoigtA A = voigt_a(q.y);
+    const F2 idd = f2(q.z), kldz = f2(q.x), bi = f2(gb.y * q.z);
+    const F2 xi = (f2(pr.wave[0], pr.wave[1]) + f2(q.w)) * idd;
+    // components are stored sigma_red (dM=-1), pi, sigma_blue (dM=+1)
+    const int4 c = *reinterpret_cast<const int4*>(P.c[lb + b]);
+    F2 h0, h1, h2, f0, f1, f2_;
+    voigt_sum2(P, c.x, c.y, A, bi, xi, h0, f0);
+    voigt_sum2(P, c.y, c.z, A, bi, xi, h1, f1);
+    voigt_sum2(P, c.z, c.w, A, bi, xi, h2, f2_);
+    const F2 hs = h0 + h2, fs = f0 + f2_;
+    tI = fma2(kldz, fma2(f2(ga.x), hs, f2(ga.y) * h1), tI);
+    hQ = fma2(kldz, fma2(f2(0.5f), h1, f2(-0.25f) * hs), hQ);
+    fQ = fma2(kldz, fma2(f2(0.5f), f1, f2(-0.25f) * fs), fQ);
+    hV = fma2(kldz, h0 - h2, hV);
+    fV = fma2(kldz, f0 - f2_, fV);
+  }
+  const F2 g3 = f2(ga.z), g4 = f2(ga.w), g5 = f2(gb.x);
+  L.t[0] = g3 * hQ;
+  L.t[1] = g4 * hQ;
+  L.t[2] = g5 * hV;
+  L.r[0] = g3 * fQ;
+  L.r[1] = g4 * fQ;
+  L.r[2] = g5 * fV;
+  return layer_set(L, tI);
+}
+
+__device__ __forceinline__ F2 synth_planck(const PairP& pr, float T) {
+  return planck2(f2(pr.c1[0], pr.c1[1]), f2(pr.c2[0], pr.c2[1]), f2(T), f2(rcp_a(T)));
+}
+
+// CALCULATE_EQUIVALENT_SYN1D: x GAIN, Stokes-major.  Returns true if a value is
+// not finite.
+__device__ __forceinline__ bool synth_store(const PairP& pr, const F2 I[4], const float* __restrict__ gain, int nw,
+                                            double* __restrict__ o) {
   bool bad = false;
-  for (int k = 0; k < nz; ++k) {
-    const float* row = sm + k * sw;
-    const float S = planck(lp.c1, lp.c2, row[0]);
-    if (k == 0 || row[1] != 0.0f) {   // SET_BOUNDARY, src/rtesolver.f90:1134-1147
-      I0 = S;
-      I1 = I2 = I3 = 0.f;
-      continue;
-    }
-    const float B = row[goff + 5];
-    float tI = row[4 + r], hQ = 0.f, hV = 0.f, fQ = 0.f, fV = 0.f;
-    for (int b = 0; b < nb; ++b) {
-      const float* q = row + loff + 4 * (lb + b);
-      const float kldz = q[0], a = q[1], idd = q[2];
-      const float xi = (lp.wave + q[3]) * idd, bi = B * idd;
-      // components are stored sigma_red (dM=-1), pi, sigma_blue (dM=+1)
-      const int c = P.lu_c0[lb + b];
-      const int e0 = c + P.lu_nt[lb + b][0], e1 = e0 + P.lu_nt[lb + b][1], e2 = e1 + P.lu_nt[lb + b][2];
-      float h0, h1, h2, f0, f1, f2;
-      voigt_sum(P, c, e0, a, bi, xi, h0, f0);
-      voigt_sum(P, e0, e1, a, bi, xi, h1, f1);
-      voigt_sum(P, e1, e2, a, bi, xi, h2, f2);
-      const float hs = h0 + h2, fs = f0 + f2;
-      tI = fmaf(kldz, fmaf(row[goff], hs, row[goff + 1] * h1), tI);
-      hQ = fmaf(kldz, fmaf(0.5f, h1, -0.25f * hs), hQ);
-      fQ = fmaf(kldz, fmaf(0.5f, f1, -0.25f * fs), fQ);
-      hV = fmaf(kldz, h0 - h2, hV);
-      fV = fmaf(kldz, f0 - f2, fV);
-    }
-    const float g3 = row[goff + 2], g4 = row[goff + 3], g5 = row[goff + 4];
-    bad |= rte_layer(tI, g3 * hQ, g4 * hQ, g5 * hV, g3 * fQ, g4 * fQ, g5 * fV, S, I0, I1, I2, I3);
+  o += pr.l0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    float a, b;
+    f2_get(I[c], a, b);
+    o[(size_t)c * nw] = (double)a * (double)gain[4 * pr.l0 + c];
+    if (pr.n > 1) o[(size_t)c * nw + 1] = (double)b * (double)gain[4 * pr.l0 + 4 + c];
+    if (!(isfinite(a) && isfinite(b))) bad = true;
   }
-  // CALCULATE_EQUIVALENT_SYN1D: x GAIN, Stokes-major
-  const int nw = P.numw;
-  double* o = syn + (size_t)col * 4 * nw;
-  o[0 * nw + l] = (double)I0 * (double)gain[4 * l + 0];
-  o[1 * nw + l] = (double)I1 * (double)gain[4 * l + 1];
-  o[2 * nw + l] = (double)I2 * (double)gain[4 * l + 2];
-  o[3 * nw + l] = (double)I3 * (double)gain[4 * l + 3];
-  if (!(isfinite(I0) && isfinite(I1) && isfinite(I2) && isfinite(I3))) bad = true;
-  if (status && __any_sync(__activemask(), bad) && (l & 31) == 0) atomicOr(&status[col], FZ_NAN);
+  return bad;
 }
 
-// One CTA per column, one thread per wavelength, FP32: the Stokes synthesis
-// of the column's slab.  With a list, the CTAs walk list[0, *nlist) (the
-// occupied slots of an inversion pool) with a grid stride.
-__global__ void __launch_bounds__(MAXNUMW) k_synth(const DevParams* __restrict__ Pg, const LamP* __restrict__ lam,
-                                                   const float* __restrict__ gain, int ncol,
-                                                   const float* __restrict__ slab, double* __restrict__ syn,
-                                                   float* mout, int* __restrict__ status,
-                                                   const int* __restrict__ list = nullptr,
-                                                   const int* __restrict__ nlist = nullptr) {
+// One CTA per column, FP32, two wavelengths per thread: the Stokes synthesis of
+// the column's slab, staged in shared memory; with a list, the CTAs walk
+// list[0, *nlist) (the occupied slots of an inversion pool) with a grid
+// stride.  npt table entries (whole warps, the costly ones first) cover the
+// wavelengths; a warp takes the next 32 entries not yet taken and walks the
+// heights, so a CTA of few warps evens out regions of many and of few Zeeman
+// components.  What bounds it: the FP32 pipe (68 % active; an isolated voigt_w2
+// loop reaches 89 %) -- 38 operations a component and some 130 for the Planck
+// function, the operator and the formal-solution step of a layer, at each
+// wavelength.  65,536 columns of 128 heights, two lines of 112 wavelengths: 61.1
+// ms with the operator's 16 elements formed from CUDA's sinh, sin and exp, 37.9
+// with rte_layer one wavelength a thread, 34.4 with two; four lines on 4,087
+// columns of 160 heights 12.3, 7.4, 6.3.  The error against 64 bits halved
+// (relative 6.4e-7 -> 2.9e-7).
+__global__ void __launch_bounds__(256, 2) k_synth(
+    const DevParams* __restrict__ Pg, const PairP* __restrict__ pairs, int npt, const float* __restrict__ gain, int ncol,
+    const float* __restrict__ slab, double* __restrict__ syn, float* mout, int* __restrict__ status,
+    const int* __restrict__ list = nullptr, const int* __restrict__ nlist = nullptr) {
   extern __shared__ float4 sm_synth4[];
-  __shared__ DevParams P;
+  __shared__ SynthP P;
+  __shared__ int next;
   const int count = list ? *nlist : ncol;
   if ((int)blockIdx.x >= count) return;
-  copy_to_shared(&P, Pg);
-  const int nz = Pg->nz, sw = Pg->sw;
+  synth_params(P, Pg);
+  const int nz = Pg->nz, sw = Pg->sw, nw = Pg->numw;
+  const int n4 = nz * sw / 4, lane = threadIdx.x & 31;
+  float* sm = reinterpret_cast<float*>(sm_synth4);
   for (int idx = blockIdx.x; idx < count; idx += gridDim.x) {
     const int col = list ? list[idx] : idx;
     __syncthreads();   // P in place; the previous column's slab no longer read
-    // stage the column's slab (nz*sw floats, 16-byte rows) in shared memory
     const float4* src = reinterpret_cast<const float4*>(slab + (size_t)col * nz * sw);
-    const int n4 = nz * sw / 4;
     for (int i = threadIdx.x; i < n4; i += blockDim.x) sm_synth4[i] = __ldg(src + i);
+    if (threadIdx.x == 0) next = 0;
     __syncthreads();
-    synth_column(P, lam, gain, reinterpret_cast<float*>(sm_synth4), col, syn, mout, status);
+    if (threadIdx.x >= blockDim.x - 32) log_tau5_warp(sm, sw, nz, mout + (size_t)col * 13 * nz, lane);
+    double* o = syn + (size_t)col * 4 * nw;
+    bool bad = false;
+    while (true) {
+      int w = 0;
+      if (lane == 0) w = atomicAdd(&next, 32);
+      w = __shfl_sync(0xffffffffu, w, 0);
+      if (w >= npt) break;
+      const PairP pr = pairs[w + lane];
+      if (pr.n > 0) {
+        F2 I[4] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
+        Layer2 L;
+        for (int k = 0; k < nz; ++k) {
+          const float* row = sm + k * sw;
+          const float2 tf = *reinterpret_cast<const float2*>(row);
+          L.S = synth_planck(pr, tf.x);
+          if (k == 0 || tf.y != 0.0f) {   // SET_BOUNDARY, src/rtesolver.f90:1134-1147
+            I[0] = L.S;
+            I[1] = I[2] = I[3] = f2(0.f);
+            continue;
+          }
+          bad |= synth_layer(P, pr, row, L);
+          layer_apply(L, I);
+        }
+        bad |= synth_store(pr, I, gain, nw, o);
+      }
+      __syncwarp();
+    }
+    if (status && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&status[col], FZ_NAN);
   }
 }
 
@@ -839,7 +909,7 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
         c2p = xm / xp;
         s2p = 2. * x * y / xp;
       }
-      float* g = row + slab_geo(nreg);
+      float* g = row + slab_geo(nlu);
       g[0] = (float)(0.25 * cgf);
       g[1] = (float)(0.5 * sgf);
       g[2] = (float)(sgf * c2p);
@@ -868,7 +938,7 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
       row[rf_he(nreg, nlu) + 1] = pgk;
     }
     for (int r = 0; r < nreg; ++r) {
-      row[4 + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
+      row[slab_kc(nlu) + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
       double dt, dp;
       cont_der(T, nelec, nhyd, P.cont[r], cd, dt, dp);
       row[rf_dkc(nreg, nlu) + 2 * r] = (float)(dt * dz);
@@ -880,7 +950,7 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
       const double damp = get_damping(L, nhyd, T);
       const double dldop = 1e3 * (sqrt(L.vdk * T) * L.l0 / LIGHT);
       const double dlv = -1e3 * L.l0 * (double)mget(m, nz, 10, k) / LIGHT;
-      float* q = row + slab_line(nreg) + 4 * b;
+      float* q = row + SLAB_LINE + 4 * b;
       q[0] = (float)(klin * dz);
       q[1] = (float)damp;
       q[2] = (float)(1.0 / dldop);
@@ -1010,7 +1080,8 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
   const LamP lp = lam[active ? l : 0];
   const int r = lp.reg;
   const int nb = P.reg_nb[r], lb = P.reg_lb[r];
-  const int goff = slab_geo(nreg), loff = slab_line(nreg);
+  const int goff = slab_geo(nlu), kcoff = slab_kc(nlu);
+  constexpr int loff = SLAB_LINE;
   const int dkoff = rf_dkc(nreg, nlu) + 2 * r, dloff = rf_dline(nreg, nlu), dgoff = rf_dgeo(nreg, nlu);
   const int dboff = rf_db(nreg, nlu), heoff = rf_he(nreg, nlu);
   float I0 = 0.f, I1 = 0.f, I2 = 0.f, I3 = 0.f;
@@ -1061,7 +1132,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
         for (int t = 0; t < 3; ++t) {
           const int e = c + P.lu_nt[lb][t];
           for (; c < e; ++c) {
-            const float shf = P.comp[c].x, st = P.comp[c].y;
+            const float shf = P.comp[c].x, st = P.comp[c].z;
             const float u = fmaf(shf, B, x0) * idd;
             float h, f;
             voigt_f32(a, u, h, f);
@@ -1088,7 +1159,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
       sts4(su + 3 * nthr, avu[0], avu[1], avu[2], cau[0]);
       sts4(su + 4 * nthr, cau[1], cau[2], avs[0], avs[1]);
       sts4(su + 5 * nthr, avs[2], cas[0], cas[1], cas[2]);
-      float tI = row[4 + r], tQ, tU, tV, rQ, rU, rV;
+      float tI = row[kcoff + r], tQ, tU, tV, rQ, rU, rV;
       {
         const float hs = hh[0] + hh[2], fs = ff[0] + ff[2];
         const float hl = 0.5f * hh[1] - 0.25f * hs, fl = 0.5f * ff[1] - 0.25f * fs;
@@ -1240,7 +1311,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
       I3 = n3;
       continue;
     }
-    float tI = row[4 + r], tQ = 0.f, tU = 0.f, tV = 0.f, rQ = 0.f, rU = 0.f, rV = 0.f;
+    float tI = row[kcoff + r], tQ = 0.f, tU = 0.f, tV = 0.f, rQ = 0.f, rU = 0.f, rV = 0.f;
     float dtau[NSLOT][7];
 #pragma unroll
     for (int p = 0; p < NSLOT; ++p)
@@ -1260,7 +1331,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
       for (int t = 0; t < 3; ++t) {
         const int e = c + P.lu_nt[lb + b][t];
         for (; c < e; ++c) {
-          const float shf = P.comp[c].x, st = P.comp[c].y;
+          const float shf = P.comp[c].x, st = P.comp[c].z;
           const float u = fmaf(shf, B, x0) * idd;
           float h, f;
           voigt_f32(a, u, h, f);
@@ -1710,6 +1781,56 @@ bool host_consts(Consts& K) {
   return known;
 }
 
+// k_synth's threads: the regions' wavelengths in pairs, either one region after
+// the other or each region from a warp boundary, whichever costs fewer
+// operations (a warp that holds two regions runs the components of both); the
+// costly warps first (even: all cost the same).
+std::vector<PairP> synth_pairs(const DevParams& P, const std::vector<LamP>& lam, bool& even) {
+  std::vector<PairP> best;
+  double cost = 0.0;
+  for (int pad = 0; pad < 2; ++pad) {
+    std::vector<PairP> v;
+    const PairP none{};
+    for (int r = 0; r < P.nreg; ++r) {
+      while (pad && v.size() % 32) v.push_back(none);
+      for (int j = 0; j < P.reg_nw[r]; j += 2) {
+        PairP p{};
+        p.reg = r;
+        p.l0 = P.reg_p0[r] + j;
+        p.n = std::min(2, P.reg_nw[r] - j);
+        for (int i = 0; i < 2; ++i) {
+          const LamP& l = lam[p.l0 + (i < p.n ? i : 0)];
+          p.wave[i] = l.wave;
+          p.c1[i] = l.c1;
+          p.c2[i] = l.c2;
+        }
+        v.push_back(p);
+      }
+    }
+    while (v.size() % 32) v.push_back(none);
+    std::vector<std::pair<double, size_t>> warps;   // (- cost, first entry)
+    double c = 0.0;
+    for (size_t w = 0; w < v.size(); w += 32) {
+      bool has[MAXREG] = {};
+      for (size_t i = w; i < w + 32; ++i)
+        if (v[i].n) has[v[i].reg] = true;
+      double cw = 130.0;
+      for (int r = 0; r < P.nreg; ++r)
+        for (int b = 0; has[r] && b < P.reg_nb[r]; ++b) cw += 38.0 * P.lu_nc[P.reg_lb[r] + b];
+      warps.push_back({-cw, w});
+      c += cw;
+    }
+    if (best.empty() || c < cost) {
+      best.clear();
+      std::sort(warps.begin(), warps.end());
+      for (const auto& w : warps) best.insert(best.end(), v.begin() + w.second, v.begin() + w.second + 32);
+      even = warps.front().first == warps.back().first;
+      cost = c;
+    }
+  }
+  return best;
+}
+
 // Wavelength-only factors of OPAC_CONTINUUM at lambda0 [A], src/cont_opacity.f90:48-357.
 ContP host_cont(double l0) {
   static const double A1[6] = {0, 2483.346, -3449.889, 2200.04, -696.271, 88.283};
@@ -1923,6 +2044,9 @@ struct fz_ctx {
   size_t smooth_len = 0;
   size_t oscr_len = 0;
   LamP* d_lam = nullptr;
+  PairP* d_pairs = nullptr;   // npt entries: k_synth's wavelengths by thread
+  int npt = 0;
+  bool pairs_even = false;     // its warps of equal cost
   float* d_gain = nullptr;
   // scratch (grown on demand): per (column, height) nH, ne and the opacity slab
   float* d_slab = nullptr;
@@ -2189,6 +2313,23 @@ int launch_lsf(fz_ctx* c, T* d_data, long long nrows, int rows_per_col, cudaStre
   return cuda_fail(cudaGetLastError());
 }
 
+// k_synth over the slabs of ncol columns (or the listed ones).  Threads of a CTA:
+// where the table's warps cost alike, all of them (up to 256); where they do
+// not, 128 for batches that leave the SMs waiting on a few columns' chains and
+// 64 above, where two warps of changing entries fill the SMs evenly (two lines
+// of 112 wavelengths, 128 heights, ms with 64 and 128: 444 columns 0.40 and
+// 0.36, 592 0.404 and 0.410, 2,048 1.16 and 1.24; one blended region of 500,
+// 504 columns of 256 heights with 64, 128, 256: 2.52, 2.24, 2.10).
+void launch_synth(fz_ctx* c, int ncol, const float* slab, double* d_syn, float* d_mout, int* d_status, cudaStream_t s,
+                  const int* list = nullptr, const int* nlist = nullptr) {
+  ProfScope ps(c, 2, s, ncol);
+  const int threads = std::min(c->npt, c->pairs_even ? 256 : (ncol < 4 * c->nsm ? 128 : 64));
+  // listed: a grid of 32 CTAs per SM walks the list
+  const int grid = list ? std::min(ncol, c->nsm * 32) : ncol;
+  k_synth<<<grid, threads, (size_t)c->nz * c->sw * sizeof(float), s>>>(c->d_params, c->d_pairs, c->npt, c->d_gain, ncol,
+                                                                      slab, d_syn, d_mout, d_status, list, nlist);
+}
+
 // The synthesis of ncol columns, or with a list of the columns list[0,
 // *nlist) among ncol slots (an inversion pool's occupied slots; the count
 // read on the device, so that a captured graph replays for any count).
@@ -2207,15 +2348,7 @@ int launch_forward(fz_ctx* c, int ncol, const float* d_model, int hydrostatic, d
     k_opac<<<blocks, 256, 0, s>>>(c->d_params, c->d_consts, ncol, d_mout, c->d_chem, c->d_slab, list, nlist);
   }
   FZ_CK(cudaGetLastError());
-  const int threads = (c->numw + 31) & ~31;
-  const size_t sms = (size_t)c->nz * c->sw * sizeof(float);
-  {
-    ProfScope ps(c, 2, s, ncol);
-    // listed: a grid of 32 CTAs per SM walks the list
-    const int grid = list ? std::min(ncol, c->nsm * 32) : ncol;
-    k_synth<<<grid, threads, sms, s>>>(c->d_params, c->d_lam, c->d_gain, ncol, c->d_slab, d_syn, d_mout, d_status,
-                                       list, nlist);
-  }
+  launch_synth(c, ncol, c->d_slab, d_syn, d_mout, d_status, s, list, nlist);
   FZ_CK(cudaGetLastError());
   return launch_lsf<double>(c, d_syn, (long long)ncol * 4, 4, s, list, nlist);
 }
@@ -3685,12 +3818,13 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
           int j = t0;
           while (j < at && P.comp[j].x != (float)sh[i]) ++j;
           if (j == at) {
-            P.comp[at++].x = (float)sh[i];
+            P.comp[at].x = P.comp[at].y = (float)sh[i];
+            ++at;
             str.push_back(0.0);
           }
           str[j - t0] += stg[i];
         }
-        for (int j = t0; j < at; ++j) P.comp[j].y = (float)str[j - t0];
+        for (int j = t0; j < at; ++j) P.comp[j].z = P.comp[j].w = (float)str[j - t0];
         P.lu_nt[nlu][t + 1] = at - t0;
       }
       P.lu_nc[nlu] = at - ncomp;
@@ -3749,6 +3883,11 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
   if ((rc = cuda_fail(cudaMalloc(&c->d_gain, 4 * numw * sizeof(float))))) return fail(rc);
   if ((rc = cuda_fail(cudaMemcpy(c->d_params, &P, sizeof(P), cudaMemcpyHostToDevice)))) return fail(rc);
   if ((rc = cuda_fail(cudaMemcpy(c->d_consts, &K, sizeof(K), cudaMemcpyHostToDevice)))) return fail(rc);
+  const std::vector<PairP> pairs = synth_pairs(P, lam, c->pairs_even);
+  c->npt = (int)pairs.size();
+  if ((rc = cuda_fail(cudaMalloc(&c->d_pairs, pairs.size() * sizeof(PairP))))) return fail(rc);
+  if ((rc = cuda_fail(cudaMemcpy(c->d_pairs, pairs.data(), pairs.size() * sizeof(PairP), cudaMemcpyHostToDevice))))
+    return fail(rc);
   if ((rc = cuda_fail(cudaMemcpy(c->d_lam, lam.data(), numw * sizeof(LamP), cudaMemcpyHostToDevice))))
     return fail(rc);
   c->gain.assign(4 * numw, 0.0f);
@@ -3780,10 +3919,9 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
   }
   // opt in to large dynamic shared memory for the slab staging
   const int sms = nz * c->sw * (int)sizeof(float);
-  if (sms > 48 * 1024) {
-    if ((rc = cuda_fail(cudaFuncSetAttribute(k_synth, cudaFuncAttributeMaxDynamicSharedMemorySize, sms))))
-      return fail(rc);
-  }
+  if (sms > 48 * 1024 - (int)sizeof(SynthP) - 16 &&
+      (rc = cuda_fail(cudaFuncSetAttribute(k_synth, cudaFuncAttributeMaxDynamicSharedMemorySize, sms))))
+    return fail(rc);
   *out = c;
   return 0;
 }
@@ -3872,6 +4010,7 @@ int fz_destroy(fz_ctx* c) {
                   (void*)c->inv.out, (void*)c->inv.it, (void*)c->inv.st, (void*)c->inv.fb})
     cudaFree(p);
   cudaFree(c->d_lam);
+  cudaFree(c->d_pairs);
   cudaFree(c->d_gain);
   cudaFree(c->d_slab);
   cudaFree(c->d_chem);
@@ -5039,9 +5178,7 @@ int fz_forward_device_static(fz_ctx* c, int ncol, const float* d_model, int hydr
   const int blocks = (int)std::min<size_t>((total + 255) / 256, (size_t)c->nsm * 16);
   k_opac<<<blocks, 256, 0, s>>>(c->d_params, c->d_consts, ncol, d_model_out, chem, slab);
   FZ_CK(cudaGetLastError());
-  const int threads = (c->numw + 31) & ~31;
-  const size_t sms = (size_t)c->nz * c->sw * sizeof(float);
-  k_synth<<<ncol, threads, sms, s>>>(c->d_params, c->d_lam, c->d_gain, ncol, slab, d_syn, d_model_out, d_status);
+  launch_synth(c, ncol, slab, d_syn, d_model_out, d_status, s);
   FZ_CK(cudaGetLastError());
   return launch_lsf<double>(c, d_syn, (long long)ncol * 4, 4, s);   // allocates nothing
 }

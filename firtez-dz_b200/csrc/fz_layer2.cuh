@@ -1,0 +1,279 @@
+// The formal solution of two wavelengths at once in FP32 (sm_100a): a thread's
+// two wavelengths sit in the halves of 64-bit registers, and FFMA2 (fma.rn.f32x2)
+// runs both in one issue slot at the FP32 pipe's full rate.  Measured on
+// dependent chains: 16 FMAs take 17.2 cycles of an SM sub-partition as 8
+// FFMA2, 19.3 as 16 FFMA, and with 16 integer operations beside them 19.5
+// against 28.6 -- the scalar form's other instructions cost issue slots that
+// the packed form has free.  Each half is rounded as the scalar operation is.
+#pragma once
+#include "fz_physics.cuh"
+
+namespace fzd {
+
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void f2_get(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 operator-(F2 x) {
+  float a, b;
+  f2_get(x, a, b);
+  return f2(-a, -b);
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return a + (-b); }
+__device__ __forceinline__ F2 rcp2(F2 x) {
+  float a, b;
+  f2_get(x, a, b);
+  return f2(rcp_a(a), rcp_a(b));
+}
+__device__ __forceinline__ F2 rsqrt2(F2 x) {
+  float a, b;
+  f2_get(x, a, b);
+  return f2(rsqrt_a(a), rsqrt_a(b));
+}
+
+// The terms of voigt_w that a line's components at one height share.
+struct VoigtA {
+  F2 a, r, aa;   // a, 2 a, a^2
+};
+__device__ __forceinline__ VoigtA voigt_a(float a) { return VoigtA{f2(a), f2(a + a), f2(a * a)}; }
+
+// voigt_w (fz_physics.cuh) at two arguments u.
+__device__ __forceinline__ void voigt_w2(const VoigtA& A, F2 u, F2& h, F2& f, F2& id) {
+  const float K = 2.168404344971009e-19f;   // 2^-62
+  const float A0 = 122.607931777104326f * K, A1 = 214.382388694706425f * K, A2 = 181.928533092181549f * K,
+              A3 = 93.155580458138441f * K, A4 = 30.180142196210589f * K, A5 = 5.912626209773153f * K,
+              A6 = .564189583562615f * K, B0 = 122.60793177387535f * K, B1 = 352.730625110963558f * K,
+              B2 = 457.334478783897737f * K, B3 = 348.703917719495792f * K, B4 = 170.354001821091472f * K,
+              B5 = 53.992906912940207f * K, B6 = 10.479857114260399f * K;
+  const F2 uu = u * u, ns = -(uu + A.aa);
+  F2 p1 = f2(A6), p0 = f2(A5), t;
+#define FZ_KSTEP2(C, hi, lo) \
+  t = hi;                    \
+  hi = fma2(A.r, t, lo);     \
+  lo = fma2(ns, t, f2(C));
+  FZ_KSTEP2(A4, p1, p0) FZ_KSTEP2(A3, p1, p0) FZ_KSTEP2(A2, p1, p0) FZ_KSTEP2(A1, p1, p0) FZ_KSTEP2(A0, p1, p0)
+  F2 q1 = f2(K), q0 = f2(B6);
+  FZ_KSTEP2(B5, q1, q0) FZ_KSTEP2(B4, q1, q0) FZ_KSTEP2(B3, q1, q0) FZ_KSTEP2(B2, q1, q0) FZ_KSTEP2(B1, q1, q0)
+  FZ_KSTEP2(B0, q1, q0)
+#undef FZ_KSTEP2
+  const F2 nr = fma2(p1, A.a, p0), dr = fma2(q1, A.a, q0), y = q1 * uu;
+  id = rcp2(fma2(q1, y, dr * dr));
+  h = fma2(p1, y, nr * dr);
+  f = u * fma2(p0, q1, -(p1 * q0));
+}
+
+// exp_parts at two arguments.
+struct ExpF2 {
+  F2 S, p;
+  __device__ __forceinline__ F2 exp() const { return fma2(S, p, S); }
+  __device__ __forceinline__ F2 expm1() const { return fma2(S, p, S + f2(-1.0f)); }
+};
+__device__ __forceinline__ float exp_scale(float t) {
+  const int i = min(max(__float_as_int(t) - 0x4b400000, -126), 127);
+  return __int_as_float((i + 127) << 23);
+}
+__device__ __forceinline__ ExpF2 exp_parts2(F2 x) {
+  const float MAGIC = 12582912.0f;
+  const F2 t = fma2(x, f2(1.4426950408889634f), f2(MAGIC)), n = t + f2(-MAGIC);
+  const F2 r = fma2(n, f2(-1.428606765330187e-06f), fma2(n, f2(-0.693145751953125f), x));
+  F2 q = fma2(r, f2(EXP_Q4), f2(EXP_Q3));
+  q = fma2(r, q, f2(EXP_Q2));
+  q = fma2(r, q, f2(EXP_Q1));
+  q = fma2(r, q, f2(EXP_Q0));
+  ExpF2 e;
+  e.p = fma2(r * r, q, r);
+  float t0, t1;
+  f2_get(t, t0, t1);
+  e.S = f2(exp_scale(t0), exp_scale(t1));
+  return e;
+}
+
+// planck at two wavelengths (T and 1/T approximate in both halves).
+__device__ __forceinline__ F2 planck2(F2 c1, F2 c2, F2 T, F2 rt) {
+  const F2 q0 = c2 * rt;
+  const F2 m = exp_parts2(fma2(fma2(-q0, T, c2), rt, q0)).expm1();
+  const F2 rm = rcp2(m);
+  const F2 s0 = c1 * rm;
+  return fma2(fma2(-s0, m, c1), rm, s0);
+}
+
+// evol_abg at two arguments: the series where it holds for both.
+struct EvolABG2 {
+  F2 am, al, be, ga;
+};
+__device__ __forceinline__ EvolABG2 evol_abg2(F2 d, F2 e) {
+  EvolABG2 o;
+  float d0, d1, e0, e1;
+  f2_get(d, d0, d1);
+  f2_get(e, e0, e1);
+  if (fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(e0), fabsf(e1))) <= 0.25f) {
+    const F2 ee = e * e, dd = d * d;
+    const F2 g1 = dd + ee, g2 = fma2(f2(2.0f), ee, dd), g3 = d * g2;
+    const F2 g4 = d * fma2(f2(3.0f), ee, dd), g5 = fma2(g2, g2, f2(-2.0f) * (ee * ee));
+    o.al = fma2(g3, f2(1.0f / 5040.0f), fma2(g1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
+    o.be = -e * fma2(g3, f2(1.0f / 362880.0f), fma2(g1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
+    o.ga = fma2(g3, f2(1.0f / 40320.0f), fma2(g1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
+    o.am = fma2(g5, f2(1.0f / 80640.0f), fma2(g4, f2(1.0f / 1440.0f), fma2(g2, f2(1.0f / 48.0f), f2(0.25f) * d)));
+    return o;
+  }
+  // the guards keep a half whose matrix vanishes finite beside one above the limit
+  const F2 TINY = f2(1.0e-37f), HALF = f2(0.5f);
+  const F2 z = fma2(f2(0.25f) * d, d, fma2(e, e, TINY));
+  F2 g = rsqrt2(z);
+  g = fma2(HALF * g, fma2(-z * g, g, f2(1.0f)), g);
+  const F2 ad = f2(fabsf(d0), fabsf(d1));
+  const F2 w = fma2(z, g, fma2(HALF, ad, TINY));
+  F2 k = rsqrt2(w);
+  k = fma2(HALF * k, fma2(-w * k, k, f2(1.0f)), k);
+  const F2 big = w * k, small = e * k;
+  float b0, b1, s0, s1;
+  f2_get(big, b0, b1);
+  f2_get(small, s0, s1);
+  const bool p0 = d0 >= 0.0f, p1 = d1 >= 0.0f;
+  const float x0 = p0 ? b0 : s0, x1 = p1 ? b1 : s1, y0 = p0 ? s0 : b0, y1 = p1 ? s1 : b1;
+  const F2 x = f2(x0, x1), y = f2(y0, y1);
+  const ExpF2 ex = exp_parts2(HALF * x);
+  const F2 t = ex.expm1(), v = ex.exp();
+  F2 ri = rcp2(v);
+  ri = fma2(ri, fma2(-v, ri, f2(1.0f)), ri);
+  const F2 tr = t * ri, sh2 = t + tr;
+  const F2 a = f2(0.25f) * (sh2 * sh2);
+  F2 sh = sh2 * fma2(HALF * t, tr, f2(1.0f));
+  const F2 hy = HALF * y;
+  F2 sn, cs;
+  if (fmaxf(fabsf(y0), fabsf(y1)) < 6.0e4f) {
+    float h0, h1;
+    f2_get(hy * f2(0.3183098861837907f), h0, h1);
+    const F2 n = f2(rintf(h0), rintf(h1));
+    const F2 r = fma2(n, f2(-PI_F_LO), fma2(n, f2(-PI_F_MID), fma2(n, f2(-PI_F_HI), hy)));
+    const F2 ss = r * r;
+    sn = fma2(r * ss, fma2(ss, fma2(ss, fma2(ss, f2(SIN_Q3), f2(SIN_Q2)), f2(SIN_Q1)), f2(SIN_Q0)), r);
+    cs = fma2(ss, fma2(ss, fma2(ss, fma2(ss, fma2(ss, f2(COS_Q4), f2(COS_Q3)), f2(COS_Q2)), f2(COS_Q1)), f2(COS_Q0)),
+              f2(1.0f));
+  } else {
+    sn = f2(sinf(0.5f * y0), sinf(0.5f * y1));
+    cs = f2(cosf(0.5f * y0), cosf(0.5f * y1));
+  }
+  const F2 b = sn * sn, sy = f2(2.0f) * (sn * cs);
+  F2 q = a + b;
+  o.am = a - b;
+  if (fmaxf(fabsf(x0), fabsf(x1)) >= 37.42994775f) {   // the reference's clamp, half by half
+    float am[2], qq[2], sv[2], bb[2];
+    const float xx[2] = {x0, x1};
+    f2_get(o.am, am[0], am[1]);
+    f2_get(q, qq[0], qq[1]);
+    f2_get(sh, sv[0], sv[1]);
+    f2_get(b, bb[0], bb[1]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (fabsf(xx[i]) >= 37.42994775f) {
+        const float c2 = fmaf(-2.0f, bb[i], 1.0f);
+        sv[i] = copysignf(1e15f, xx[i]);
+        am[i] = 0.5f * (1e15f + c2) - 1.0f;
+        qq[i] = 0.5f * (1e15f - c2);
+      }
+    sh = f2(sv[0], sv[1]);
+    o.am = f2(am[0], am[1]);
+    q = f2(qq[0], qq[1]);
+  }
+  const F2 it = HALF * g;
+  o.al = fma2(x, sh, y * sy) * it;
+  o.be = fma2(x, sy, -(y * sh)) * it;
+  o.ga = q * g;
+  return o;
+}
+
+// What the formal solution needs of one layer at two wavelengths (rte_layer,
+// fz_physics.cuh): I <- I - om0 w0 - E um.I, ... with w0 = I0 - S.
+struct Layer2 {
+  F2 S, om0, E, dg, ga, t[3], r[3], um[3], up[3], v[3];
+};
+constexpr int LAYER2_F2 = sizeof(Layer2) / sizeof(F2);
+
+// The layer from its optical depths (t: eta_Q, U, V; r: rho_Q, U, V); a half
+// with a non-finite matrix becomes the identity.  Returns whether one did.
+__device__ __forceinline__ bool layer_set(Layer2& L, F2 tI) {
+  const F2 eta2 = fma2(L.t[2], L.t[2], fma2(L.t[1], L.t[1], L.t[0] * L.t[0]));
+  const F2 rho2 = fma2(L.r[2], L.r[2], fma2(L.r[1], L.r[1], L.r[0] * L.r[0]));
+  const F2 er = fma2(L.t[2], L.r[2], fma2(L.t[1], L.r[1], L.t[0] * L.r[0]));
+  const F2 sum = eta2 + rho2;
+  float c0, c1;
+  f2_get(tI + sum, c0, c1);
+  const EvolABG2 f = evol_abg2(eta2 - rho2, er);
+  const ExpF2 ex = exp_parts2(-tI);
+  const F2 gh = f.ga * (f2(0.5f) * sum);
+  L.ga = f.ga;
+  L.E = ex.exp();
+  L.om0 = -fma2(L.E, f.am + gh, ex.expm1());
+  L.dg = (f2(1.0f) - gh) + f.am;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    const F2 u = fma2(f.al, L.t[i], -(f.be * L.r[i]));
+    const F2 c = f.ga * fma2(L.t[j], L.r[k], -(L.t[k] * L.r[j]));
+    L.um[i] = u - c;
+    L.up[i] = u + c;
+    L.v[i] = fma2(f.al, L.r[i], f.be * L.t[i]);
+  }
+  const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
+  if (b0 || b1) {
+    auto put = [&](F2& x, float v) {
+      float a, b;
+      f2_get(x, a, b);
+      x = f2(b0 ? v : a, b1 ? v : b);
+    };
+    put(L.om0, 0.0f);
+    put(L.E, 1.0f);
+    put(L.dg, 1.0f);
+    put(L.ga, 0.0f);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      put(L.t[i], 0.0f);
+      put(L.r[i], 0.0f);
+      put(L.um[i], 0.0f);
+      put(L.up[i], 0.0f);
+      put(L.v[i], 0.0f);
+    }
+  }
+  return b0 || b1;
+}
+
+__device__ __forceinline__ void layer_apply(const Layer2& L, F2 I[4]) {
+  const F2 w0 = I[0] - L.S;
+  const F2 ge = L.ga * fma2(L.t[2], I[3], fma2(L.t[1], I[2], L.t[0] * I[1]));
+  const F2 gr = L.ga * fma2(L.r[2], I[3], fma2(L.r[1], I[2], L.r[0] * I[1]));
+  const F2 n0 = fma2(L.um[2], I[3], fma2(L.um[1], I[2], L.um[0] * I[1]));
+  F2 n[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    n[i] = fma2(L.r[i], gr,
+                fma2(L.t[i], ge, fma2(L.v[k], I[1 + j], fma2(-L.v[j], I[1 + k], fma2(L.dg, I[1 + i], -(L.up[i] * w0))))));
+  }
+  I[0] = fma2(-L.E, n0, fma2(-L.om0, w0, I[0]));
+#pragma unroll
+  for (int i = 0; i < 3; ++i) I[1 + i] = L.E * n[i];
+}
+
+}  // namespace fzd

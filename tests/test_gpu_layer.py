@@ -72,3 +72,18 @@ def test_equal_lande_factors_share_a_component(fz, orc):
     assert np.all(st == 0)
     assert np.max(np.abs(syn[:, 0] / ref[:, 0] - 1)) < 1e-5
     assert np.max(np.abs(syn[:, 1:] - ref[:, 1:])) < 1e-6
+
+
+@pytest.mark.parametrize("n1,n2", [(1, 1), (2, 3), (63, 2), (64, 65), (130, 1), (511, 513)])
+def test_wavelength_pairs_of_any_region_sizes(fz, orc, n1, n2):
+    """Two wavelengths a thread: odd regions end in a single one, regions start
+    inside or at the start of a warp, up to the largest NUMW."""
+    lines = fz.lines_parse(fz.atmos.line_database_text())
+    reg = fz.regions_from_lines_section("1 %d -300.0 2.5\n2 %d -200.0 3.5\n" % (n1, n2), lines)
+    g, _ = orc.gain(lines, reg)
+    m = fz.atmos.make_columns(2, 12, seed=3)
+    syn, _, st = fz.Synthesis(lines, reg, nz=12, gain=g).forward(m, hydrostatic=True)
+    ref, _, _ = orc.forward(lines, reg, g, m, hydrostatic=True)
+    assert np.all(st == 0)
+    assert np.max(np.abs(syn[:, 0] / ref[:, 0] - 1)) < 1e-5
+    assert np.max(np.abs(syn[:, 1:] - ref[:, 1:])) < 1e-6

@@ -967,29 +967,6 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
   }
 }
 
-// Offset (floats, 16-byte aligned) of the per-thread sums of k_synth_rf
-// behind the slab (nz x sw), the coefficient table (nz x np) and the node
-// accumulators (np x 4 x nthr); the block's dynamic shared memory is that
-// offset plus six float4 a thread.
-__host__ __device__ __forceinline__ int rf_sums_off(int nz, int sw, int np, int nthr) {
-  return (nz * sw + nz * np + np * 4 * nthr + 3) & ~3;
-}
-
-// A thread's own float4 in shared memory, stored and loaded as volatile
-// instructions: the loads are issued where they stand, so the values are not
-// kept in registers between the store and the loads.
-__device__ __forceinline__ void sts4(float4* p, float a, float b, float c, float d) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(p))),
-               "f"(a), "f"(b), "f"(c), "f"(d));
-}
-__device__ __forceinline__ float4 lds4(const float4* p) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))));
-  return v;
-}
-
 // Linear maps from the per-type (sigma_red, pi, sigma_blue) sums of one line
 // to the seven matrix elements (eta_I,Q,U,V, rho_Q,U,V), the grouping of the
 // component accumulation of src/absorption_matrix.f90:1948-2278.
@@ -1030,12 +1007,10 @@ __device__ __forceinline__ void lmap(const Geo& g, const float h[3], const float
 // jac in the (NFREQ, 6 NZ) layout and the layer's operator to oscr
 // ((nz, 16, NUMW) per column, zero where the boundary condition is taken);
 // k_rf_prop then applies the products of the operators above each layer.
+// Regions may hold blended lines (contexts without any run k_synth_rf2).
 // MAXT: the block-size bound, 256 (two blocks per SM) up to 256
 // wavelengths, 512 (one) up to 512; both hold 128 registers a thread.
-// BLEND: regions with blended lines are present and every region runs the
-// general path below; without, only the single-line path is compiled in,
-// which keeps the general path's register demand out of the kernel.
-template <bool HE, bool FULL, int MAXT, bool BLEND>
+template <bool HE, bool FULL, int MAXT>
 __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const DevParams* __restrict__ Pg, const RFConf* __restrict__ Rg,
                                                   const LamP* __restrict__ lam, const float* __restrict__ gain,
                                                   int ncol, const float* __restrict__ slab,
@@ -1057,9 +1032,6 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
   float* sm = reinterpret_cast<float*>(sm_rf4);
   float* coef = sm + nz * sw;
   float* Dacc = coef + nz * np;
-  // the per-wavelength sums of the single-line path, six float4 a thread
-  // (vector v of thread l at sums[v * nthr + l]), after the accumulators
-  float4* sums = reinterpret_cast<float4*>(sm + rf_sums_off(nz, sw, np, nthr));
   {
     const float4* src = reinterpret_cast<const float4*>(slab + (size_t)col * nz * sw);
     const int n4 = nz * sw / 4;
@@ -1114,203 +1086,6 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
     const Geo g{row[goff], row[goff + 1], row[goff + 2], row[goff + 3], row[goff + 4]};
     const float B = row[goff + 5];
     const float halfT = 0.5f / T;
-    if (!BLEND) {
-      // One line in every region (no blends): each parameter's optical-depth
-      // derivatives are formed from the line's per-type sums when its
-      // response is taken, in a runtime loop over the parameters -- one
-      // copy of the directional derivative and of the node update, and no
-      // 6 x 7 array held across the operator algebra.  The arithmetic is
-      // that of the general path below, expression for expression.
-      const float* qq = row + loff + 4 * lb;
-      const float kldz = qq[0], a = qq[1], idd = qq[2];
-      const float x0 = lp.wave + qq[3];
-      float hh[3] = {0, 0, 0}, ff[3] = {0, 0, 0}, av[3] = {0, 0, 0}, ca[3] = {0, 0, 0};
-      float avu[3] = {0, 0, 0}, cau[3] = {0, 0, 0}, avs[3] = {0, 0, 0}, cas[3] = {0, 0, 0};
-      {
-        int c = P.lu_c0[lb];
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-          const int e = c + P.lu_nt[lb][t];
-          for (; c < e; ++c) {
-            const float shf = P.comp[c].x, st = P.comp[c].z;
-            const float u = fmaf(shf, B, x0) * idd;
-            float h, f;
-            voigt_f32(a, u, h, f);
-            const float dhv = 2.0f * fmaf(a, f, -u * h);
-            const float dha = 2.0f * (fmaf(a, h, u * f) - 0.56418958354775628f);
-            hh[t] = fmaf(st, h, hh[t]);
-            ff[t] = fmaf(st, f, ff[t]);
-            const float sv = st * dhv, sa = st * dha;
-            av[t] += sv;
-            ca[t] += sa;
-            avu[t] = fmaf(sv, u, avu[t]);
-            cau[t] = fmaf(sa, u, cau[t]);
-            avs[t] = fmaf(sv, shf, avs[t]);
-            cas[t] = fmaf(sa, shf, cas[t]);
-          }
-        }
-      }
-      // the sums wait in shared memory through the operator algebra and are
-      // read back per parameter: 24 registers fewer across the loop below
-      float4* su = sums + l;
-      sts4(su, hh[0], hh[1], hh[2], ff[0]);
-      sts4(su + nthr, ff[1], ff[2], av[0], av[1]);
-      sts4(su + 2 * nthr, av[2], ca[0], ca[1], ca[2]);
-      sts4(su + 3 * nthr, avu[0], avu[1], avu[2], cau[0]);
-      sts4(su + 4 * nthr, cau[1], cau[2], avs[0], avs[1]);
-      sts4(su + 5 * nthr, avs[2], cas[0], cas[1], cas[2]);
-      float tI = row[kcoff + r], tQ, tU, tV, rQ, rU, rV;
-      {
-        const float hs = hh[0] + hh[2], fs = ff[0] + ff[2];
-        const float hl = 0.5f * hh[1] - 0.25f * hs, fl = 0.5f * ff[1] - 0.25f * fs;
-        tI = fmaf(kldz, g.g1 * hs + g.g2 * hh[1], tI);
-        tQ = fmaf(kldz, g.g3 * hl, 0.f);
-        tU = fmaf(kldz, g.g4 * hl, 0.f);
-        tV = fmaf(kldz, g.g5 * (hh[0] - hh[2]), 0.f);
-        rQ = fmaf(kldz, g.g3 * fl, 0.f);
-        rU = fmaf(kldz, g.g4 * fl, 0.f);
-        rV = fmaf(kldz, g.g5 * (ff[0] - ff[2]), 0.f);
-      }
-      const float* dl = row + dloff + 4 * lb;
-      const float dkt = dl[0], dkp = dl[1], ddt = dl[2], ddp = dl[3];
-      float O[16], om0 = 0.0f;
-      EvolSt es;
-      const bool fin = isfinite(tI) && isfinite(tQ) && isfinite(tU) && isfinite(tV) && isfinite(rQ) &&
-                       isfinite(rU) && isfinite(rV);
-      if (!fin) {
-        bad = 1;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) O[i] = (i % 5 == 0) ? 1.f : 0.f;
-      } else {
-        evol_state(tI, tQ, tU, tV, rQ, rU, rV, O, om0, es);
-      }
-      const float n0 = fmaf(om0, S, fmaf(O[0], I0, fmaf(O[1], I1, fmaf(O[2], I2, O[3] * I3))));
-      const float n1 = fmaf(-O[4], S, fmaf(O[4], I0, fmaf(O[5], I1, fmaf(O[6], I2, O[7] * I3))));
-      const float n2 = fmaf(-O[8], S, fmaf(O[8], I0, fmaf(O[9], I1, fmaf(O[10], I2, O[11] * I3))));
-      const float n3 = fmaf(-O[12], S, fmaf(O[12], I0, fmaf(O[13], I1, fmaf(O[14], I2, O[15] * I3))));
-      // the operator products with the incoming vector (T, Pg; every
-      // parameter without HE) -- with HE the B and v_z responses use the
-      // outgoing one, switched to at p = 2
-      EvolW v;
-      if (fin) {
-        const float win[4] = {I0 - S, I1, I2, I3};
-        evol_w(es, O, win, v);
-      }
-      const float dS = lp.c1 * (q / T) * ((em1 + 1.0f) / (em1 * em1));
-      float OH[4] = {0.f, 0.f, 0.f, 0.f}, ck = 0.f, pgk = 0.f;
-      bool prop = false;
-      if (HE) {
-        ck = row[heoff];
-        pgk = row[heoff + 1];
-        prop = O[0] > 1.0e-5f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          OH[i] = prop ? O[4 * i] * H[0] + O[4 * i + 1] * H[1] + O[4 * i + 2] * H[2] + O[4 * i + 3] * H[3] : H[i];
-      }
-      const float* ckr = FULL ? nullptr : coef + k * np;
-#pragma unroll 1
-      for (int p = 0; p < NSLOT; ++p) {
-        // every parameter's optical-depth derivatives in one form:
-        //   dt = A lmap(GA, hh, ff) + B lmap(g, U, V), dt[0] += C0
-        const float4 s0 = lds4(su), s1 = lds4(su + nthr), s2 = lds4(su + 2 * nthr);
-        const float hh[3] = {s0.x, s0.y, s0.z}, ff[3] = {s0.w, s1.x, s1.y};
-        const float av[3] = {s1.z, s1.w, s2.x}, ca[3] = {s2.y, s2.z, s2.w};
-        float U[3], V[3], A, B, C0 = 0.0f;
-        Geo GA = g;
-        if (p == 0) {   // T at constant Pg: dKLIN, du/dT = -u/(2T), da/dT
-          const float4 s3 = lds4(su + 3 * nthr), s4 = lds4(su + 4 * nthr);
-          const float avu[3] = {s3.x, s3.y, s3.z}, cau[3] = {s3.w, s4.x, s4.y};
-#pragma unroll
-          for (int t = 0; t < 3; ++t) {
-            U[t] = fmaf(ca[t], ddt, -avu[t] * halfT);
-            V[t] = fmaf(av[t], ddt, cau[t] * halfT);
-          }
-          A = dkt;
-          B = kldz;
-          C0 = row[dkoff];
-        } else if (p == 1) {   // Pg at constant T: dKLIN and da/dPg
-#pragma unroll
-          for (int t = 0; t < 3; ++t) {
-            U[t] = ca[t];
-            V[t] = av[t];
-          }
-          A = dkp;
-          B = kldz * ddp;
-          C0 = row[dkoff + 1];
-        } else if (p < 5) {   // B_i: geometry factors and the shift term du/dB
-          const float4 s4 = lds4(su + 4 * nthr), s5 = lds4(su + 5 * nthr);
-          U[0] = s4.z; U[1] = s4.w; U[2] = s5.x;
-          V[0] = -s5.y; V[1] = -s5.z; V[2] = -s5.w;
-          const float* dg = row + dgoff + 5 * (p - 2);
-          GA = Geo{dg[0], dg[1], dg[2], dg[3], dg[4]};
-          A = kldz;
-          B = kldz * (idd * row[dboff + p - 2]);
-        } else {   // v_z: du/dv = lu_duv / Doppler width
-#pragma unroll
-          for (int t = 0; t < 3; ++t) {
-            U[t] = av[t];
-            V[t] = -ca[t];
-          }
-          A = 0.0f;
-          B = kldz * P.lu_duv[lb] * idd;
-        }
-        float dt[7], ta[7], tb[7];
-        lmap(GA, hh, ff, ta);
-        lmap(g, U, V, tb);
-#pragma unroll
-        for (int x = 0; x < 7; ++x) dt[x] = A != 0.0f ? fmaf(A, ta[x], B * tb[x]) : B * tb[x];
-        dt[0] = C0 + dt[0];
-        float rfp[4] = {0.f, 0.f, 0.f, 0.f};
-        if (fin) {
-          if (HE && p == 2) {
-            const float wout[4] = {n0 - S, n1, n2, n3};
-            evol_w(es, O, wout, v);
-          }
-          evol_dir(es, v, dt, rfp);
-        }
-        if (p == 0) {
-          // source-function term (1 - O) e0 dS/dT, then the HE global term
-          rfp[0] = fmaf(om0, dS, rfp[0]);
-          rfp[1] = fmaf(-O[4], dS, rfp[1]);
-          rfp[2] = fmaf(-O[8], dS, rfp[2]);
-          rfp[3] = fmaf(-O[12], dS, rfp[3]);
-          if (HE) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) rfp[i] = fmaf(ck, OH[i], rfp[i]);
-          }
-        }
-        if (HE && p == 1) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) H[i] = prop ? fmaf(rfp[i], pgk, OH[i]) : H[i];
-        }
-        if (FULL) {
-          const int nw = P.numw;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) jcol[((size_t)p * nz + k) * fstride + c * nw + l] = rfp[c];
-        } else {
-          const int j0 = C.n0[p], j1 = j0 + C.nj[p];
-          for (int j = j0; j < j1; ++j) {
-            float* d = Dacc + (j * 4) * nthr + l;
-            const float d0 = d[0], d1 = d[nthr], d2 = d[2 * nthr], d3 = d[3 * nthr];
-            const float cj = ckr[j];
-            d[0] = fmaf(cj, rfp[0], fmaf(O[0], d0, fmaf(O[1], d1, fmaf(O[2], d2, O[3] * d3))));
-            d[nthr] = fmaf(cj, rfp[1], fmaf(O[4], d0, fmaf(O[5], d1, fmaf(O[6], d2, O[7] * d3))));
-            d[2 * nthr] = fmaf(cj, rfp[2], fmaf(O[8], d0, fmaf(O[9], d1, fmaf(O[10], d2, O[11] * d3))));
-            d[3 * nthr] = fmaf(cj, rfp[3], fmaf(O[12], d0, fmaf(O[13], d1, fmaf(O[14], d2, O[15] * d3))));
-          }
-        }
-      }
-      if (FULL) {
-        const int nw = P.numw;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) ocol[((size_t)k * 16 + i) * nw + l] = O[i];
-      }
-      I0 = n0;
-      I1 = n1;
-      I2 = n2;
-      I3 = n3;
-      continue;
-    }
     float tI = row[kcoff + r], tQ = 0.f, tU = 0.f, tV = 0.f, rQ = 0.f, rU = 0.f, rV = 0.f;
     float dtau[NSLOT][7];
 #pragma unroll
@@ -1541,28 +1316,321 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
   if (status && __any_sync(__activemask(), bad) && (l & 31) == 0) atomicOr(&status[col], FZ_NAN);
 }
 
-// k_synth_rf with the block-size bound its thread count needs
-template <bool HE, bool FULL, typename... A>
-void launch_synth_rf(bool blend, int blocks, int threads, size_t sms, cudaStream_t s, A... a) {
-  if (threads <= 256) {
-    if (blend)
-      k_synth_rf<HE, FULL, 256, true><<<blocks, threads, sms, s>>>(a...);
-    else
-      k_synth_rf<HE, FULL, 256, false><<<blocks, threads, sms, s>>>(a...);
+// ------------------------------------------------------------- k_synth_rf2
+// k_synth_rf for regions of one line each, two wavelengths per thread
+// (fz_layer2.cuh).  A warp takes the next 32 entries of the pair table and
+// walks the heights with accumulators of its own in shared memory (np x 4 x
+// 32 pairs): one CTA per column, no barrier between the staging and the end.
+// Per height: the Voigt sums with their derivative sums, the layer's operator
+// with the derivatives of its scalar functions (layer_d2), the products with
+// the incoming and -- with HE -- the outgoing Stokes vector that every
+// direction shares (resp_w), then for each of the six parameters the
+// optical-depth derivatives, the response (resp_dir) and the update of the
+// parameter's nodes.  FULL as k_synth_rf.
+//
+// What bounds it: the FP32 pipe -- per height and wavelength some 52 operations a
+// Zeeman component, 100 for each Stokes vector's products, 46 a direction, 20 a
+// node -- at 8 warps per SM (two CTAs of 4 warps; 247 registers hold the sums, the
+// operator and the products, and the two wavelengths give the independent work
+// that more warps would).  2,048 columns of 128 heights, two lines of 112
+// wavelengths, 13 nodes: 11.5 ms with a directional derivative of some 250
+// operations for each parameter one wavelength a thread, 5.2 here; 77 columns 1.08
+// and 0.49; every height of 256 columns of 96 heights 1.15 and 0.57.  Error of
+// the node Jacobian against 64 bits 1.86e-5 -> 1.82e-5 of its norm.
+// vec: neighbouring wavelengths may be stored as one 8-byte word.
+__device__ __forceinline__ void rf_store(float* p, F2 x, int n, bool vec) {
+  if (vec) {
+    *reinterpret_cast<unsigned long long*>(p) = x.v;
   } else {
-    if (blend)
-      k_synth_rf<HE, FULL, 512, true><<<blocks, threads, sms, s>>>(a...);
-    else
-      k_synth_rf<HE, FULL, 512, false><<<blocks, threads, sms, s>>>(a...);
+    float a, b;
+    f2_get(x, a, b);
+    p[0] = a;
+    if (n > 1) p[1] = b;
   }
 }
 
 template <bool HE, bool FULL>
-cudaError_t set_synth_rf_attr(cudaFuncAttribute attr, int v) {
-  cudaError_t e = cudaFuncSetAttribute(k_synth_rf<HE, FULL, 256, false>, attr, v);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_rf<HE, FULL, 512, false>, attr, v);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_synth_rf<HE, FULL, 256, true>, attr, v);
-  return e == cudaSuccess ? cudaFuncSetAttribute(k_synth_rf<HE, FULL, 512, true>, attr, v) : e;
+__global__ void __launch_bounds__(128, 2) k_synth_rf2(
+    const DevParams* __restrict__ Pg, const RFConf* __restrict__ Rg, const PairP* __restrict__ pairs, int npt, bool vec,
+    const float* __restrict__ gain, const float* __restrict__ slab, const float* __restrict__ coefg,
+    double* __restrict__ syn, float* __restrict__ jac, float* __restrict__ oscr, float* mout, int* __restrict__ status,
+    const int* __restrict__ list, const int* __restrict__ nlist) {
+  if (list && (int)blockIdx.x >= *nlist) return;
+  extern __shared__ float4 sm_rf4[];
+  __shared__ SynthP P;
+  __shared__ RFConf C;
+  __shared__ float duv[MAXLU];
+  __shared__ int next;
+  __shared__ unsigned inf_mask[2];
+  synth_params(P, Pg);
+  if (!FULL) copy_to_shared(&C, Rg);
+  const int col = list ? list[blockIdx.x] : (int)blockIdx.x;
+  const int nz = Pg->nz, nreg = Pg->nreg, nlu = Pg->nlu, nw = Pg->numw, np = FULL ? 0 : Rg->np;
+  const int sw = rf_w(nreg, nlu), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  float* sm = reinterpret_cast<float*>(sm_rf4);
+  float* coef = sm + nz * sw;
+  F2* D = reinterpret_cast<F2*>(coef + ((nz * np + 3) & ~3)) + (size_t)wid * np * 4 * 32 + lane;
+  {
+    const float4* src = reinterpret_cast<const float4*>(slab + (size_t)col * nz * sw);
+    const int n4 = nz * sw / 4;
+    for (int i = threadIdx.x; i < n4; i += blockDim.x) sm_rf4[i] = __ldg(src + i);
+    if (!FULL)
+      for (int i = threadIdx.x; i < nz * np; i += blockDim.x) coef[i] = __ldg(coefg + i);
+    for (int i = threadIdx.x; i < nlu; i += blockDim.x) duv[i] = Pg->lu_duv[i];
+    if (threadIdx.x == 0) next = 0;
+    if (threadIdx.x < 2) inf_mask[threadIdx.x] = 0u;
+  }
+  __syncthreads();
+  if (threadIdx.x >= blockDim.x - 32) log_tau5_warp(sm, sw, nz, mout + (size_t)col * 13 * nz, lane);
+  const size_t nfreq = (size_t)4 * nw;
+  float* jcol = jac + (size_t)col * (FULL ? NSLOT * nz : np) * nfreq;
+  float* ocol = FULL ? oscr + (size_t)col * nz * 16 * nw : nullptr;
+  const int dgoff = rf_dgeo(nreg, nlu), dboff = rf_db(nreg, nlu), heoff = rf_he(nreg, nlu);
+  const F2 ZERO = f2(0.0f);
+  bool bad = false;
+  unsigned mask[2] = {0u, 0u};
+  while (true) {
+    int w0 = 0;
+    if (lane == 0) w0 = atomicAdd(&next, 32);
+    w0 = __shfl_sync(0xffffffffu, w0, 0);
+    if (w0 >= npt) break;
+    const PairP pr = pairs[w0 + lane];
+    if (pr.n > 0) {
+      const int r = pr.reg, lb = P.lb[r];
+      const int4 ce = *reinterpret_cast<const int4*>(P.c[lb]);
+      const float lduv = duv[lb];
+      const float* dkc = sm + rf_dkc(nreg, nlu) + 2 * r;
+      const float* dli = sm + rf_dline(nreg, nlu) + 4 * lb;
+      F2 I[4] = {ZERO, ZERO, ZERO, ZERO}, H[4] = {ZERO, ZERO, ZERO, ZERO};
+      if (!FULL)
+        for (int j = 0; j < 4 * np; ++j) D[j * 32] = ZERO;
+      for (int k = 0; k < nz; ++k) {
+        const float* row = sm + k * sw;
+        const float2 tf = *reinterpret_cast<const float2*>(row);
+        const float rt = rcp_a(tf.x);
+        // c1 / (e^q - 1), q = c2 / T, and its T derivative S (q / T) e^q / (e^q - 1)
+        const F2 c1 = f2(pr.c1[0], pr.c1[1]), c2 = f2(pr.c2[0], pr.c2[1]);
+        const F2 q0 = c2 * f2(rt), q = fma2(fma2(-q0, f2(tf.x), c2), f2(rt), q0);
+        const F2 em1 = exp_parts2(q).expm1(), rm = rcp2(em1);
+        const F2 S0 = c1 * rm, S = fma2(fma2(-S0, em1, c1), rm, S0);
+        if (k == 0 || tf.y != 0.0f) {   // SET_BOUNDARY
+          I[0] = S;
+          I[1] = I[2] = I[3] = ZERO;
+          if (FULL) {
+#pragma unroll
+            for (int p = 0; p < NSLOT; ++p)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) rf_store(jcol + ((size_t)p * nz + k) * nfreq + c * nw + pr.l0, ZERO, pr.n, vec);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) rf_store(ocol + ((size_t)k * 16 + i) * nw + pr.l0, ZERO, pr.n, vec);
+          } else {
+            for (int j = 0; j < 4 * np; ++j) D[j * 32] = ZERO;
+          }
+          continue;
+        }
+        // the line's sums per type (sigma_red, pi, sigma_blue): H, F and, with
+        // s the strength, s dH/du (av), s dH/da (ca), these times u and times
+        // the component's shift
+        const float4 ln = *reinterpret_cast<const float4*>(row + SLAB_LINE + 4 * lb);   // KLIN dz, a, 1/Doppler, shift
+        const float* geo = row + slab_geo(nlu);
+        const float4 ga = *reinterpret_cast<const float4*>(geo);
+        const float2 gb = *reinterpret_cast<const float2*>(geo + 4);
+        F2 hh[3], ff[3], av[3], ca[3], avu[3], cau[3], avs[3], cas[3];
+        {
+          const VoigtA A = voigt_a(ln.y);
+          const F2 bi = f2(gb.y * ln.z), xi = (f2(pr.wave[0], pr.wave[1]) + f2(ln.w)) * f2(ln.z);
+#pragma unroll
+          for (int t = 0; t < 3; ++t) {
+            hh[t] = ff[t] = av[t] = ca[t] = avu[t] = cau[t] = avs[t] = cas[t] = ZERO;
+            const int c1_ = t == 0 ? ce.y : (t == 1 ? ce.z : ce.w);
+            for (int c = t == 0 ? ce.x : (t == 1 ? ce.y : ce.z); c < c1_; ++c) {
+              const ulonglong2 cc = *reinterpret_cast<const ulonglong2*>(&P.comp[c]);
+              const F2 shf{cc.x}, st{cc.y}, u = fma2(shf, bi, xi);
+              F2 h, f, id;
+              voigt_w2(A, u, h, f, id);
+              const F2 sid = st * id;
+              h = h * sid;   // s H
+              f = f * sid;   // s F
+              hh[t] = hh[t] + h;
+              ff[t] = ff[t] + f;
+              // dH/du = 2 (a F - u H), dH/da = 2 (a H + u F - 1/sqrt(pi)); the
+              // factor 2 comes with the sums' use
+              const F2 sv = fma2(A.a, f, -(u * h)), sa = fma2(A.a, h, fma2(u, f, f2(-0.56418958354775628f) * st));
+              av[t] = av[t] + sv;
+              ca[t] = ca[t] + sa;
+              avu[t] = fma2(sv, u, avu[t]);
+              cau[t] = fma2(sa, u, cau[t]);
+              avs[t] = fma2(sv, shf, avs[t]);
+              cas[t] = fma2(sa, shf, cas[t]);
+            }
+          }
+        }
+        // (0.25 cgf) hs + (0.5 sgf) h_pi, the linear part hl and the circular
+        // part hd of a triple of sums
+        struct Tri {
+          F2 I, l, d;
+        };
+        auto tri = [&](F2 a, F2 b, F2 c, float g1, float g2) {
+          const F2 hs = a + c;
+          return Tri{fma2(f2(g1), hs, f2(g2) * b), fma2(f2(0.5f), b, f2(-0.25f) * hs), a - c};
+        };
+        const F2 kldz = f2(ln.x), g3 = f2(ga.z), g4 = f2(ga.w), g5 = f2(gb.x);
+        const Tri h0 = tri(hh[0], hh[1], hh[2], ga.x, ga.y), f0 = tri(ff[0], ff[1], ff[2], ga.x, ga.y);
+        LayerD2 L;
+        {
+          const F2 kh = kldz * h0.l, kf = kldz * f0.l;
+          L.t[0] = g3 * kh;
+          L.t[1] = g4 * kh;
+          L.t[2] = g5 * (kldz * h0.d);
+          L.r[0] = g3 * kf;
+          L.r[1] = g4 * kf;
+          L.r[2] = g5 * (kldz * f0.d);
+        }
+        bad |= layer_d2(L, fma2(kldz, h0.I, f2(geo[6 + r])));
+        const F2* O = L.O;
+        // I <- I + O (I - S e0) + S e0, 1 - O(1,1) without cancellation
+        const F2 win[4] = {I[0] - S, I[1], I[2], I[3]};
+        F2 n[4];
+        n[0] = fma2(O[3], win[3], fma2(O[2], win[2], fma2(O[1], win[1], fma2(-L.om0, win[0], I[0]))));
+#pragma unroll
+        for (int i = 1; i < 4; ++i)
+          n[i] = fma2(O[4 * i + 3], win[3], fma2(O[4 * i + 2], win[2], fma2(O[4 * i + 1], win[1], O[4 * i] * win[0])));
+        Resp2 R;
+        resp_w(L, win, R);
+        const float* ckr = FULL ? nullptr : coef + k * np;
+        // the response of parameter slot p into its nodes (or out, FULL)
+        auto put = [&](int p, const F2 rf[4]) {
+          if (FULL) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) rf_store(jcol + ((size_t)p * nz + k) * nfreq + c * nw + pr.l0, rf[c], pr.n, vec);
+          } else {
+            const int j0 = C.n0[p], j1 = j0 + C.nj[p];
+#pragma unroll 1
+            for (int j = j0; j < j1; ++j) {
+              F2* d = D + (size_t)j * 128;
+              const F2 d0[4] = {d[0], d[32], d[64], d[96]};
+              const F2 cj = f2(ckr[j]);
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                d[32 * i] = fma2(cj, rf[i], fma2(O[4 * i], d0[0], fma2(O[4 * i + 1], d0[1],
+                                 fma2(O[4 * i + 2], d0[2], O[4 * i + 3] * d0[3]))));
+            }
+          }
+        };
+        // optical-depth derivatives of the form a (h0, f0) + b (th, tf)
+        auto dir = [&](F2 a, F2 b, const Tri& th, const Tri& tf_, F2 c0, F2 rf[4]) {
+          const F2 l = fma2(a, h0.l, b * th.l), m = fma2(a, f0.l, b * tf_.l);
+          const F2 dt[3] = {g3 * l, g4 * l, g5 * fma2(a, h0.d, b * th.d)};
+          const F2 dr[3] = {g3 * m, g4 * m, g5 * fma2(a, f0.d, b * tf_.d)};
+          resp_dir(L, R, c0 + fma2(a, h0.I, b * th.I), dt, dr, rf);
+        };
+        const float* dl = dli + k * sw;
+        F2 rf[4];
+        // T at constant Pg: dKLIN, du/dT = -u/(2T), da/dT; the source function
+        F2 OH[4] = {ZERO, ZERO, ZERO, ZERO};
+        float pgk = 0.f;
+        bool p0 = false, p1 = false;
+        {
+          const F2 ddt = f2(2.0f * dl[2]), ht = f2(rt);   // 2 / (2 T)
+          F2 U[3], V[3];
+#pragma unroll
+          for (int t = 0; t < 3; ++t) {
+            U[t] = fma2(ca[t], ddt, -(avu[t] * ht));
+            V[t] = fma2(av[t], ddt, cau[t] * ht);
+          }
+          dir(f2(dl[0]), kldz, tri(U[0], U[1], U[2], ga.x, ga.y), tri(V[0], V[1], V[2], ga.x, ga.y), f2(dkc[k * sw]), rf);
+          const F2 dS = S * ((q * f2(rt)) * ((em1 + f2(1.0f)) * rm));
+          rf[0] = fma2(L.om0, dS, rf[0]);
+#pragma unroll
+          for (int i = 1; i < 4; ++i) rf[i] = fma2(-O[4 * i], dS, rf[i]);
+          if (HE) {
+            // the global T term of OLD_ANALYTICAL_SOLVER, skipped where O(1,1) <= 1e-5
+            const F2 ck = f2(row[heoff]);
+            pgk = row[heoff + 1];
+            float o0, o1;
+            f2_get(O[0], o0, o1);
+            p0 = o0 > 1.0e-5f;
+            p1 = o1 > 1.0e-5f;
+            mat4(O, H, OH);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float a, b, ha, hb;
+              f2_get(OH[i], a, b);
+              f2_get(H[i], ha, hb);
+              OH[i] = f2(p0 ? a : ha, p1 ? b : hb);
+              rf[i] = fma2(ck, OH[i], rf[i]);
+            }
+          }
+          put(0, rf);
+        }
+        // Pg at constant T: dKLIN and da/dPg
+        dir(f2(dl[1]), f2(ln.x * (2.0f * dl[3])), tri(ca[0], ca[1], ca[2], ga.x, ga.y), tri(av[0], av[1], av[2], ga.x, ga.y),
+            f2(dkc[k * sw + 1]), rf);
+        if (HE) {
+          const F2 pg2 = f2(p0 ? pgk : 0.0f, p1 ? pgk : 0.0f);   // where skipped H stays (OH = H there)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) H[i] = fma2(rf[i], pg2, OH[i]);
+        }
+        put(1, rf);
+        if (HE) {
+          const F2 wout[4] = {n[0] - S, n[1], n[2], n[3]};
+          resp_w(L, wout, R);
+        }
+        // B_i: the geometry factors and the shift term du/dB = shift / Doppler width
+        {
+          const Tri ts = tri(avs[0], avs[1], avs[2], ga.x, ga.y), us = tri(-cas[0], -cas[1], -cas[2], ga.x, ga.y);
+          const F2 gs[6] = {g3 * ts.l, g4 * ts.l, g5 * ts.d, g3 * us.l, g4 * us.l, g5 * us.d};
+          const F2 hs = hh[0] + hh[2];
+#pragma unroll 1
+          for (int i = 0; i < 3; ++i) {
+            const float* dg = row + dgoff + 5 * i;
+            const F2 kb = f2(2.0f * (ln.x * (ln.z * row[dboff + i])));
+            const F2 a3 = f2(ln.x * dg[2]), a4 = f2(ln.x * dg[3]), a5 = f2(ln.x * dg[4]);
+            const F2 dI = fma2(f2(ln.x * dg[0]), hs, fma2(f2(ln.x * dg[1]), hh[1], kb * ts.I));
+            const F2 dt[3] = {fma2(a3, h0.l, kb * gs[0]), fma2(a4, h0.l, kb * gs[1]), fma2(a5, h0.d, kb * gs[2])};
+            const F2 dr[3] = {fma2(a3, f0.l, kb * gs[3]), fma2(a4, f0.l, kb * gs[4]), fma2(a5, f0.d, kb * gs[5])};
+            resp_dir(L, R, dI, dt, dr, rf);
+            put(2 + i, rf);
+          }
+        }
+        // v_z: du/dv = lu_duv / Doppler width
+        dir(ZERO, f2(2.0f * (ln.x * lduv * ln.z)), tri(av[0], av[1], av[2], ga.x, ga.y),
+            tri(-ca[0], -ca[1], -ca[2], ga.x, ga.y), ZERO, rf);
+        put(5, rf);
+        if (FULL)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) rf_store(ocol + ((size_t)k * 16 + i) * nw + pr.l0, O[i], pr.n, vec);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) I[i] = n[i];
+      }
+      bad |= synth_store(pr, I, gain, nw, syn + (size_t)col * 4 * nw);
+      if (!FULL) {
+        // EQVDSYN = REAL(sum) * GAIN (src/forward.f90:614-621)
+        for (int j = 0; j < np; ++j)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int l1 = pr.l0 + (pr.n > 1);
+            const F2 v = D[(size_t)(4 * j + c) * 32] * f2(gain[4 * pr.l0 + c], gain[4 * l1 + c]);
+            rf_store(jcol + (size_t)j * nfreq + c * nw + pr.l0, v, pr.n, vec);
+            float a, b;
+            f2_get(v, a, b);
+            if (isinf(a) || isinf(b)) mask[j >> 5] |= 1u << (j & 31);
+          }
+      }
+    }
+    __syncwarp();
+  }
+  if (!FULL) {
+    // columns whose |.| sum overflows REAL*4 are zeroed (src/forward.f90:673-679)
+    if (mask[0]) atomicOr(&inf_mask[0], mask[0]);
+    if (mask[1]) atomicOr(&inf_mask[1], mask[1]);
+    __syncthreads();
+    if (inf_mask[0] | inf_mask[1])
+      for (int j = 0; j < np; ++j)
+        if (inf_mask[j >> 5] & (1u << (j & 31)))
+          for (int i = threadIdx.x; i < (int)nfreq; i += blockDim.x) jcol[(size_t)j * nfreq + i] = 0.0f;
+  }
+  if (status && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&status[col], FZ_NAN);
 }
 
 // true when some region of the context holds blended lines
@@ -2047,6 +2115,7 @@ struct fz_ctx {
   PairP* d_pairs = nullptr;   // npt entries: k_synth's wavelengths by thread
   int npt = 0;
   bool pairs_even = false;     // its warps of equal cost
+  bool pairs_vec = false;      // every entry two wavelengths from an even one, NUMW even
   float* d_gain = nullptr;
   // scratch (grown on demand): per (column, height) nH, ne and the opacity slab
   float* d_slab = nullptr;
@@ -2353,16 +2422,87 @@ int launch_forward(fz_ctx* c, int ncol, const float* d_model, int hydrostatic, d
   return launch_lsf<double>(c, d_syn, (long long)ncol * 4, 4, s, list, nlist);
 }
 
+// Shared memory of the node Jacobian's accumulation in one block of a thread
+// per wavelength (k_synth_rf, and the limit that layouts are held to).
 size_t rf_smem(const fz_ctx* c) {
-  const int threads = (c->numw + 31) & ~31;
-  return ((size_t)rf_sums_off(c->nz, rf_w(c->nreg, c->nlu), c->rf.np, threads) + (size_t)24 * threads) *
-         sizeof(float);
+  const int threads = (c->numw + 31) & ~31, np = c->rf.np;
+  const size_t base = ((size_t)c->nz * rf_w(c->nreg, c->nlu) + (size_t)c->nz * np + (size_t)np * 4 * threads + 3) & ~(size_t)3;
+  return (base + (size_t)24 * threads) * sizeof(float);
 }
 
-// the same for the FULL variant (no coefficient table or accumulators)
+// the same for the response functions at every height (no coefficient table
+// or accumulators)
 size_t rf_smem_full(const fz_ctx* c) {
   const int threads = (c->numw + 31) & ~31;
-  return ((size_t)rf_sums_off(c->nz, rf_w(c->nreg, c->nlu), 0, threads) + (size_t)24 * threads) * sizeof(float);
+  return ((((size_t)c->nz * rf_w(c->nreg, c->nlu) + 3) & ~(size_t)3) + (size_t)24 * threads) * sizeof(float);
+}
+
+// k_synth_rf2's shared memory with w warps a CTA, and its warps: up to four
+// that the SM's shared memory holds (0: not even one, k_synth_rf runs).
+size_t rf2_smem(const fz_ctx* c, bool full, int w) {
+  const int np = full ? 0 : c->rf.np;
+  return ((size_t)c->nz * rf_w(c->nreg, c->nlu) + (((size_t)c->nz * np + 3) & ~(size_t)3)) * sizeof(float) +
+         (size_t)w * np * 4 * 32 * sizeof(F2);
+}
+int rf2_warps(const fz_ctx* c, bool full) {
+  int w = std::min(4, c->npt / 32);
+  while (w > 0 && rf2_smem(c, full, w) > 220 * 1024) --w;
+  return w;
+}
+
+// The RF synthesis of the columns in c->d_rfslab: k_synth_rf2 for regions of
+// one line each, k_synth_rf where lines are blended.
+template <bool HE, bool FULL>
+void launch_synth_rf_t(fz_ctx* c, int ncol, double* d_syn, float* d_jac, float* d_oscr, float* d_mout, int* d_status,
+                       cudaStream_t s, const int* list, const int* nlist) {
+  const int w = has_blends(c) ? 0 : rf2_warps(c, FULL);
+  if (w > 0) {
+    const bool vec = c->pairs_vec && ((uintptr_t)d_jac & 7) == 0;   // d_oscr is the context's own
+    k_synth_rf2<HE, FULL><<<ncol, 32 * w, rf2_smem(c, FULL, w), s>>>(
+        c->d_params, c->d_rf, c->d_pairs, c->npt, vec, c->d_gain, c->d_rfslab, c->d_coef, d_syn, d_jac, d_oscr,
+        d_mout, d_status, list, nlist);
+    return;
+  }
+  const int threads = (c->numw + 31) & ~31;
+  const size_t sms = FULL ? rf_smem_full(c) : rf_smem(c);
+  if (threads <= 256)
+    k_synth_rf<HE, FULL, 256><<<ncol, threads, sms, s>>>(c->d_params, c->d_rf, c->d_lam, c->d_gain, ncol, c->d_rfslab,
+                                                         c->d_coef, d_syn, d_jac, d_oscr, d_mout, d_status, list, nlist);
+  else
+    k_synth_rf<HE, FULL, 512><<<ncol, threads, sms, s>>>(c->d_params, c->d_rf, c->d_lam, c->d_gain, ncol, c->d_rfslab,
+                                                         c->d_coef, d_syn, d_jac, d_oscr, d_mout, d_status, list, nlist);
+}
+template <bool FULL>
+void launch_synth_rf(fz_ctx* c, int ncol, int hydrostatic, double* d_syn, float* d_jac, float* d_oscr, float* d_mout,
+                     int* d_status, cudaStream_t s, const int* list = nullptr, const int* nlist = nullptr) {
+  ProfScope ps(c, 4, s, list ? 0 : ncol);
+  if (hydrostatic)
+    launch_synth_rf_t<true, FULL>(c, ncol, d_syn, d_jac, d_oscr, d_mout, d_status, s, list, nlist);
+  else
+    launch_synth_rf_t<false, FULL>(c, ncol, d_syn, d_jac, d_oscr, d_mout, d_status, s, list, nlist);
+}
+
+// Opt in to the dynamic shared memory that launch_synth_rf<FULL> uses (to be
+// called before any stream capture), all of the SM's unified storage as shared
+// memory so that two CTAs can be resident.
+template <bool FULL>
+int prepare_synth_rf(fz_ctx* c) {
+  auto set = [&](auto kern, size_t sms) -> int {
+    FZ_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms));
+    FZ_CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    return 0;
+  };
+  const int w = has_blends(c) ? 0 : rf2_warps(c, FULL);
+  if (w > 0) {
+    const size_t sms = rf2_smem(c, FULL, w);
+    FZ_CK_RC(set(k_synth_rf2<true, FULL>, sms));
+    return set(k_synth_rf2<false, FULL>, sms);
+  }
+  const size_t sms = FULL ? rf_smem_full(c) : rf_smem(c);
+  FZ_CK_RC(set(k_synth_rf<true, FULL, 256>, sms));
+  FZ_CK_RC(set(k_synth_rf<false, FULL, 256>, sms));
+  FZ_CK_RC(set(k_synth_rf<true, FULL, 512>, sms));
+  return set(k_synth_rf<false, FULL, 512>, sms);
 }
 
 // The response-function kernels run one thread per wavelength in blocks of
@@ -2400,15 +2540,9 @@ int ensure_rf_scratch(fz_ctx* c, int ncol) {
       FZ_CK(cudaMalloc(&c->d_oscr, nop * sizeof(float)));
       c->oscr_len = nop;
     }
-    const size_t fsm = rf_smem_full(c);
-    FZ_CK((set_synth_rf_attr<true, true>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm)));
-    FZ_CK((set_synth_rf_attr<false, true>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm)));
+    FZ_CK_RC(prepare_synth_rf<true>(c));
   } else {
-    const size_t sms = rf_smem(c);
-    if (sms > 48 * 1024) {
-      FZ_CK((set_synth_rf_attr<true, false>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms)));
-      FZ_CK((set_synth_rf_attr<false, false>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms)));
-    }
+    FZ_CK_RC(prepare_synth_rf<false>(c));
   }
   if ((size_t)ncol > c->rf_cols) {
     cudaFree(c->d_rfslab);
@@ -2468,19 +2602,7 @@ int launch_rf_stage(fz_ctx* c, int ncol, int hydrostatic, double* d_syn, float* 
     launch_opac_rf(c, ncol, d_mout, c->tune.opacrf_threads, s, list, nlist);
   }
   FZ_CK(cudaGetLastError());
-  const int threads = (c->numw + 31) & ~31;
-  const size_t sms = rf_smem(c);
-  {
-    ProfScope ps(c, 4, s, list ? 0 : ncol);
-    if (hydrostatic)
-      launch_synth_rf<true, false>(has_blends(c), ncol, threads, sms, s, c->d_params, c->d_rf, c->d_lam, c->d_gain, ncol,
-                                                         c->d_rfslab, c->d_coef, d_syn, d_jac, nullptr, d_mout,
-                                                         d_status, list, nlist);
-    else
-      launch_synth_rf<false, false>(has_blends(c), ncol, threads, sms, s, c->d_params, c->d_rf, c->d_lam, c->d_gain, ncol,
-                                                          c->d_rfslab, c->d_coef, d_syn, d_jac, nullptr, d_mout,
-                                                          d_status, list, nlist);
-  }
+  launch_synth_rf<false>(c, ncol, hydrostatic, d_syn, d_jac, nullptr, d_mout, d_status, s, list, nlist);
   FZ_CK(cudaGetLastError());
   if (c->lsf.on) {
     FZ_CK_RC(launch_lsf<double>(c, d_syn, (long long)ncol * 4, 4, s, list, nlist));
@@ -2508,18 +2630,7 @@ int launch_rf_stage_full(fz_ctx* c, int ncol, int hydrostatic, double* d_syn, fl
   }
   FZ_CK(cudaGetLastError());
   const int threads = (c->numw + 31) & ~31;
-  const size_t sms = rf_smem_full(c);
-  {
-    ProfScope ps(c, 4, s, list ? 0 : ncol);
-    if (hydrostatic)
-      launch_synth_rf<true, true>(has_blends(c), ncol, threads, sms, s, c->d_params, c->d_rf, c->d_lam, c->d_gain,
-                                  ncol, c->d_rfslab, nullptr, d_syn, c->d_rfbig, c->d_oscr, d_mout, d_status, list,
-                                  nlist);
-    else
-      launch_synth_rf<false, true>(has_blends(c), ncol, threads, sms, s, c->d_params, c->d_rf, c->d_lam, c->d_gain,
-                                   ncol, c->d_rfslab, nullptr, d_syn, c->d_rfbig, c->d_oscr, d_mout, d_status, list,
-                                   nlist);
-  }
+  launch_synth_rf<true>(c, ncol, hydrostatic, d_syn, c->d_rfbig, c->d_oscr, d_mout, d_status, s, list, nlist);
   FZ_CK(cudaGetLastError());
   {
     ProfScope ps(c, 11, s, list ? 0 : ncol);
@@ -2573,20 +2684,8 @@ int launch_forward_rf(fz_ctx* c, int ncol, const float* d_model, int hydrostatic
       FZ_CK(cudaMalloc(&c->d_oscr, need * sizeof(float)));
       c->oscr_len = need;
     }
-    const size_t sms = rf_smem_full(c);
-    FZ_CK((set_synth_rf_attr<true, true>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms)));
-    FZ_CK((set_synth_rf_attr<false, true>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms)));
-    {
-      ProfScope ps(c, 4, s, ncol);
-      if (hydrostatic)
-        launch_synth_rf<true, true>(has_blends(c), ncol, threads, sms, s, c->d_params, c->d_rf, c->d_lam, c->d_gain, ncol,
-                                                          c->d_rfslab, nullptr, d_syn, d_jac, c->d_oscr, d_mout,
-                                                          d_status, nullptr, nullptr);
-      else
-        launch_synth_rf<false, true>(has_blends(c), ncol, threads, sms, s, c->d_params, c->d_rf, c->d_lam, c->d_gain, ncol,
-                                                           c->d_rfslab, nullptr, d_syn, d_jac, c->d_oscr, d_mout,
-                                                           d_status, nullptr, nullptr);
-    }
+    FZ_CK_RC(prepare_synth_rf<true>(c));
+    launch_synth_rf<true>(c, ncol, hydrostatic, d_syn, d_jac, c->d_oscr, d_mout, d_status, s);
     FZ_CK(cudaGetLastError());
     {
       ProfScope ps(c, 11, s, ncol);
@@ -3885,6 +3984,8 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
   if ((rc = cuda_fail(cudaMemcpy(c->d_consts, &K, sizeof(K), cudaMemcpyHostToDevice)))) return fail(rc);
   const std::vector<PairP> pairs = synth_pairs(P, lam, c->pairs_even);
   c->npt = (int)pairs.size();
+  c->pairs_vec = numw % 2 == 0;
+  for (const PairP& p : pairs) c->pairs_vec = c->pairs_vec && (p.n == 0 || (p.n == 2 && p.l0 % 2 == 0));
   if ((rc = cuda_fail(cudaMalloc(&c->d_pairs, pairs.size() * sizeof(PairP))))) return fail(rc);
   if ((rc = cuda_fail(cudaMemcpy(c->d_pairs, pairs.data(), pairs.size() * sizeof(PairP), cudaMemcpyHostToDevice))))
     return fail(rc);
@@ -4165,12 +4266,7 @@ int fz_rf_nodes(fz_ctx* c, const int* nodes) {
   // shared memory; larger layouts contract the full response functions
   c->rf_full = sms > (size_t)maxsm || np > MAXNP;
   if (c->rf_full) return np;
-  FZ_CK((set_synth_rf_attr<true, false>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms)));
-  FZ_CK((set_synth_rf_attr<false, false>(cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms)));
-  // all of the SM's unified L1/shared storage as shared memory: two CTAs of
-  // ~90 KB each can then be resident
-  FZ_CK((set_synth_rf_attr<true, false>(cudaFuncAttributePreferredSharedMemoryCarveout, 100)));
-  FZ_CK((set_synth_rf_attr<false, false>(cudaFuncAttributePreferredSharedMemoryCarveout, 100)));
+  FZ_CK_RC(prepare_synth_rf<false>(c));
   return np;
 }
 

@@ -118,26 +118,17 @@ __device__ __forceinline__ F2 planck2(F2 c1, F2 c2, F2 T, F2 rt) {
   return fma2(fma2(-s0, m, c1), rm, s0);
 }
 
-// evol_abg at two arguments: the series where it holds for both.
-struct EvolABG2 {
-  F2 am, al, be, ga;
+// The functions of evol_abg from the roots, at two arguments of which one at
+// least is above the series' limit, with what their derivatives need: x, y,
+// 1/theta, sinh x, cosh x, sin y, cos y.
+struct Roots2 {
+  F2 am, al, be, ga, x, y, it, sh, ch, sy, cy;
 };
-__device__ __forceinline__ EvolABG2 evol_abg2(F2 d, F2 e) {
-  EvolABG2 o;
-  float d0, d1, e0, e1;
-  f2_get(d, d0, d1);
-  f2_get(e, e0, e1);
-  if (fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(e0), fabsf(e1))) <= 0.25f) {
-    const F2 ee = e * e, dd = d * d;
-    const F2 g1 = dd + ee, g2 = fma2(f2(2.0f), ee, dd), g3 = d * g2;
-    const F2 g4 = d * fma2(f2(3.0f), ee, dd), g5 = fma2(g2, g2, f2(-2.0f) * (ee * ee));
-    o.al = fma2(g3, f2(1.0f / 5040.0f), fma2(g1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
-    o.be = -e * fma2(g3, f2(1.0f / 362880.0f), fma2(g1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
-    o.ga = fma2(g3, f2(1.0f / 40320.0f), fma2(g1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
-    o.am = fma2(g5, f2(1.0f / 80640.0f), fma2(g4, f2(1.0f / 1440.0f), fma2(g2, f2(1.0f / 48.0f), f2(0.25f) * d)));
-    return o;
-  }
+__device__ __forceinline__ Roots2 roots2(F2 d, F2 e) {
   // the guards keep a half whose matrix vanishes finite beside one above the limit
+  float d0, d1;
+  f2_get(d, d0, d1);
+  Roots2 o;
   const F2 TINY = f2(1.0e-37f), HALF = f2(0.5f);
   const F2 z = fma2(f2(0.25f) * d, d, fma2(e, e, TINY));
   F2 g = rsqrt2(z);
@@ -178,29 +169,65 @@ __device__ __forceinline__ EvolABG2 evol_abg2(F2 d, F2 e) {
   const F2 b = sn * sn, sy = f2(2.0f) * (sn * cs);
   F2 q = a + b;
   o.am = a - b;
+  o.ch = fma2(f2(2.0f), a, f2(1.0f));
+  o.cy = fma2(f2(-2.0f), b, f2(1.0f));
   if (fmaxf(fabsf(x0), fabsf(x1)) >= 37.42994775f) {   // the reference's clamp, half by half
-    float am[2], qq[2], sv[2], bb[2];
+    float am[2], qq[2], sv[2], cv[2], bb[2];
     const float xx[2] = {x0, x1};
     f2_get(o.am, am[0], am[1]);
     f2_get(q, qq[0], qq[1]);
     f2_get(sh, sv[0], sv[1]);
+    f2_get(o.ch, cv[0], cv[1]);
     f2_get(b, bb[0], bb[1]);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
       if (fabsf(xx[i]) >= 37.42994775f) {
         const float c2 = fmaf(-2.0f, bb[i], 1.0f);
         sv[i] = copysignf(1e15f, xx[i]);
+        cv[i] = 1e15f;
         am[i] = 0.5f * (1e15f + c2) - 1.0f;
         qq[i] = 0.5f * (1e15f - c2);
       }
     sh = f2(sv[0], sv[1]);
+    o.ch = f2(cv[0], cv[1]);
     o.am = f2(am[0], am[1]);
     q = f2(qq[0], qq[1]);
   }
-  const F2 it = HALF * g;
-  o.al = fma2(x, sh, y * sy) * it;
-  o.be = fma2(x, sy, -(y * sh)) * it;
+  o.x = x;
+  o.y = y;
+  o.sh = sh;
+  o.sy = sy;
+  o.it = HALF * g;
+  o.al = fma2(x, sh, y * sy) * o.it;
+  o.be = fma2(x, sy, -(y * sh)) * o.it;
   o.ga = q * g;
+  return o;
+}
+
+// evol_abg at two arguments: the series where it holds for both.
+struct EvolABG2 {
+  F2 am, al, be, ga;
+};
+__device__ __forceinline__ EvolABG2 evol_abg2(F2 d, F2 e) {
+  EvolABG2 o;
+  float d0, d1, e0, e1;
+  f2_get(d, d0, d1);
+  f2_get(e, e0, e1);
+  if (fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(e0), fabsf(e1))) <= 0.25f) {
+    const F2 ee = e * e, dd = d * d;
+    const F2 g1 = dd + ee, g2 = fma2(f2(2.0f), ee, dd), g3 = d * g2;
+    const F2 g4 = d * fma2(f2(3.0f), ee, dd), g5 = fma2(g2, g2, f2(-2.0f) * (ee * ee));
+    o.al = fma2(g3, f2(1.0f / 5040.0f), fma2(g1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
+    o.be = -e * fma2(g3, f2(1.0f / 362880.0f), fma2(g1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
+    o.ga = fma2(g3, f2(1.0f / 40320.0f), fma2(g1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
+    o.am = fma2(g5, f2(1.0f / 80640.0f), fma2(g4, f2(1.0f / 1440.0f), fma2(g2, f2(1.0f / 48.0f), f2(0.25f) * d)));
+    return o;
+  }
+  const Roots2 R = roots2(d, e);
+  o.am = R.am;
+  o.al = R.al;
+  o.be = R.be;
+  o.ga = R.ga;
   return o;
 }
 
@@ -274,6 +301,178 @@ __device__ __forceinline__ void layer_apply(const Layer2& L, F2 I[4]) {
   I[0] = fma2(-L.E, n0, fma2(-L.om0, w0, I[0]));
 #pragma unroll
   for (int i = 0; i < 3; ++i) I[1 + i] = L.E * n[i];
+}
+
+// ------------------------------------------------ response functions
+// evol_abg2's functions and their derivatives with respect to d and e (those
+// of am are al / 4 and -be / 2).
+struct EvolD2 {
+  F2 am, al, be, ga, al_d, al_e, be_d, be_e, ga_d, ga_e;
+};
+__device__ __forceinline__ EvolD2 evol_d2(F2 d, F2 e) {
+  EvolD2 o;
+  float d0, d1, e0, e1;
+  f2_get(d, d0, d1);
+  f2_get(e, e0, e1);
+  if (fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(e0), fabsf(e1))) <= 0.25f) {
+    const F2 ee = e * e, dd = d * d;
+    const F2 s1 = dd + ee, s2 = fma2(f2(2.0f), ee, dd), s3 = d * s2;
+    const F2 s4 = d * fma2(f2(3.0f), ee, dd), s5 = fma2(s2, s2, f2(-2.0f) * (ee * ee));
+    const F2 u2 = fma2(f2(3.0f), dd, f2(2.0f) * ee);                        // d s3 / d d
+    const F2 u3 = d * fma2(f2(4.0f), dd, f2(6.0f) * ee);                    // d (d^4 + 3 d^2 e^2 + e^4) / d d
+    const F2 u4 = fma2(f2(6.0f), dd, f2(4.0f) * ee);                        // ... / d e, over e
+    o.al = fma2(s3, f2(1.0f / 5040.0f), fma2(s1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
+    o.al_d = fma2(u3, f2(1.0f / 362880.0f), fma2(u2, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 60.0f), f2(1.0f / 6.0f))));
+    o.al_e = e * fma2(u4, f2(1.0f / 362880.0f), fma2(d, f2(1.0f / 1260.0f), f2(1.0f / 60.0f)));
+    o.be = -e * fma2(s3, f2(1.0f / 362880.0f), fma2(s1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
+    o.be_d = -e * fma2(u2, f2(1.0f / 362880.0f), fma2(d, f2(1.0f / 2520.0f), f2(1.0f / 120.0f)));
+    o.be_e = -fma2(d * fma2(f2(6.0f), ee, dd), f2(1.0f / 362880.0f),
+                   fma2(fma2(f2(3.0f), ee, dd), f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
+    o.ga = fma2(s3, f2(1.0f / 40320.0f), fma2(s1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
+    o.ga_d = fma2(u3, f2(1.0f / 3628800.0f), fma2(u2, f2(1.0f / 40320.0f), fma2(d, f2(1.0f / 360.0f), f2(1.0f / 24.0f))));
+    o.ga_e = e * fma2(u4, f2(1.0f / 3628800.0f), fma2(d, f2(1.0f / 10080.0f), f2(1.0f / 360.0f)));
+    o.am = fma2(s5, f2(1.0f / 80640.0f), fma2(s4, f2(1.0f / 1440.0f), fma2(s2, f2(1.0f / 48.0f), f2(0.25f) * d)));
+    return o;
+  }
+  const Roots2 R = roots2(d, e);
+  o.am = R.am;
+  o.al = R.al;
+  o.be = R.be;
+  o.ga = R.ga;
+  // the quotient rule on (x sinh x + y sin y) / theta and its kin, with dx =
+  // (x dd / 2 + y de) / theta, dy = (x de - y dd / 2) / theta
+  const F2 x = R.x, y = R.y, it = R.it, HALF = f2(0.5f);
+  const F2 xs = x * R.sh, ys = y * R.sy, xy = fma2(x, R.sy, y * R.sh);   // x sinh x, y sin y, x sin y + y sinh x
+  const F2 xc = (x * x) * R.ch, yc = (y * y) * R.cy, ec = e * (R.ch + R.cy);
+  const F2 dit = d * it, e4 = f2(4.0f) * (e * it);
+  const F2 hit = HALF * it;
+  o.al_d = it * fma2(hit, (xs - ys) + (xc - yc), -(o.al * dit));
+  o.al_e = it * fma2(it, xy + ec, -(o.al * e4));
+  o.be_d = it * fma2(hit, xy - ec, -(o.be * dit));
+  o.be_e = it * fma2(it, (ys - xs) + (fma2(x * x, R.cy, -((y * y) * R.ch))), -(o.be * e4));
+  o.ga_d = it * fma2(hit, xs - ys, -(o.ga * dit));
+  o.ga_e = it * fma2(it, xy, -(o.ga * e4));
+  return o;
+}
+
+// A layer of the response-function kernel: its operator O and what the
+// derivatives need.
+struct LayerD2 {
+  F2 t[3], r[3], c[3], h, E, om0;   // c = eta x rho, h = (|eta|^2 + |rho|^2) / 2
+  EvolD2 f;
+  F2 O[16];
+  F2 on;   // 1; 0 in a half whose matrix is not finite (the identity there, without response)
+};
+
+__device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
+  F2 eta2 = fma2(L.t[2], L.t[2], fma2(L.t[1], L.t[1], L.t[0] * L.t[0]));
+  F2 rho2 = fma2(L.r[2], L.r[2], fma2(L.r[1], L.r[1], L.r[0] * L.r[0]));
+  F2 er = fma2(L.t[2], L.r[2], fma2(L.t[1], L.r[1], L.t[0] * L.r[0]));
+  float c0, c1;
+  f2_get(tI + (eta2 + rho2), c0, c1);
+  const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
+  L.on = f2(1.0f);
+  if (b0 || b1) {
+    auto zero = [&](F2& x) {
+      float a, b;
+      f2_get(x, a, b);
+      x = f2(b0 ? 0.0f : a, b1 ? 0.0f : b);
+    };
+    zero(tI);
+    zero(eta2);
+    zero(rho2);
+    zero(er);
+    zero(L.on);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      zero(L.t[i]);
+      zero(L.r[i]);
+    }
+  }
+  L.f = evol_d2(eta2 - rho2, er);
+  const EvolD2& f = L.f;
+  const ExpF2 ex = exp_parts2(-tI);
+  L.E = ex.exp();
+  L.h = f2(0.5f) * (eta2 + rho2);
+  const F2 gh = f.ga * L.h;
+  L.om0 = -fma2(L.E, f.am + gh, ex.expm1());
+  const F2 dg = L.E * ((f2(1.0f) - gh) + f.am), ga = L.E * f.ga;
+  L.O[0] = f2(1.0f) - L.om0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    L.c[i] = fma2(L.t[j], L.r[k], -(L.t[k] * L.r[j]));
+    const F2 u = L.E * fma2(f.al, L.t[i], -(f.be * L.r[i])), c = ga * L.c[i];
+    L.O[1 + i] = c - u;
+    L.O[4 * (1 + i)] = -(u + c);
+    L.O[5 * (1 + i)] = fma2(ga, fma2(L.t[i], L.t[i], L.r[i] * L.r[i]), dg);
+    // the pair (j, k): the symmetric part of M and the vector al rho + be eta
+    const F2 v = L.E * fma2(f.al, L.r[i], f.be * L.t[i]);
+    const F2 s = ga * fma2(L.t[j], L.t[k], L.r[j] * L.r[k]);
+    L.O[4 * (1 + j) + 1 + k] = s + v;
+    L.O[4 * (1 + k) + 1 + j] = s - v;
+  }
+  return b0 || b1;
+}
+
+__device__ __forceinline__ F2 dot3(const F2 a[3], const F2 b[3]) { return fma2(a[2], b[2], fma2(a[1], b[1], a[0] * b[0])); }
+__device__ __forceinline__ void mat4(const F2 O[16], const F2 w[4], F2 y[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) y[i] = fma2(O[4 * i], w[0], fma2(O[4 * i + 1], w[1], fma2(O[4 * i + 2], w[2], O[4 * i + 3] * w[3])));
+}
+
+// The derivative of O w for any direction of the seven optical depths, from
+// the layer and w: with dd, de the changes of d and e,
+//   dO w = Ad dd + Ae de + (r.deta - q.drho, g deta + g' drho + deta x q + drho x r) - dtI O w.
+struct Resp2 {
+  F2 Ad[4], Ae[4], q[3], r[3], g, gp, Ow[4];
+};
+__device__ __forceinline__ void resp_w(const LayerD2& L, const F2 w[4], Resp2& R) {
+  const EvolD2& f = L.f;
+  const F2 wv[3] = {w[1], w[2], w[3]};
+  const F2 ew = dot3(L.t, wv), rw = dot3(L.r, wv);
+  F2 X[4], Y[4], M[4];   // X w, Y w and M w
+  X[0] = ew;
+  Y[0] = -rw;
+  M[0] = fma2(L.h, w[0], dot3(L.c, wv));
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    X[1 + i] = fma2(L.t[i], w[0], fma2(L.r[j], wv[k], -(L.r[k] * wv[j])));
+    Y[1 + i] = fma2(-L.r[i], w[0], fma2(L.t[j], wv[k], -(L.t[k] * wv[j])));
+    M[1 + i] = fma2(L.t[i], ew, fma2(L.r[i], rw, -fma2(L.c[i], w[0], L.h * wv[i])));
+  }
+  mat4(L.O, w, R.Ow);
+  const F2 E = L.E * L.on;
+  const F2 md = E * (f2(0.25f) * f.al), me = E * (f2(-0.5f) * f.be);
+  const F2 ad = E * f.al_d, ae = E * f.al_e, bd = E * f.be_d, be = E * f.be_e, gd = E * f.ga_d, ge = E * f.ga_e;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    R.Ad[i] = fma2(gd, M[i], fma2(-bd, Y[i], fma2(-ad, X[i], md * w[i])));
+    R.Ae[i] = fma2(ge, M[i], fma2(-be, Y[i], fma2(-ae, X[i], me * w[i])));
+    R.Ow[i] = R.Ow[i] * L.on;
+  }
+  const F2 al = E * f.al, bt = E * f.be, ga = E * f.ga;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    R.q[i] = fma2(ga, Y[1 + i], -(bt * wv[i]));
+    R.r[i] = fma2(ga, X[1 + i], -(al * wv[i]));
+  }
+  R.g = fma2(ga, ew, -(al * w[0]));
+  R.gp = fma2(ga, rw, bt * w[0]);
+}
+
+__device__ __forceinline__ void resp_dir(const LayerD2& L, const Resp2& R, F2 dI, const F2 dt[3], const F2 dr[3], F2 o[4]) {
+  const F2 dd = f2(2.0f) * (dot3(L.t, dt) - dot3(L.r, dr)), de = dot3(L.r, dt) + dot3(L.t, dr);
+  o[0] = fma2(R.Ad[0], dd, fma2(R.Ae[0], de, fma2(-dI, R.Ow[0], dot3(R.r, dt) - dot3(R.q, dr))));
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    F2 v = fma2(R.g, dt[i], R.gp * dr[i]);
+    v = fma2(dt[j], R.q[k], fma2(-dt[k], R.q[j], v));
+    v = fma2(dr[j], R.r[k], fma2(-dr[k], R.r[j], v));
+    o[1 + i] = fma2(R.Ad[1 + i], dd, fma2(R.Ae[1 + i], de, fma2(-dI, R.Ow[1 + i], v)));
+  }
 }
 
 }  // namespace fzd

@@ -299,6 +299,23 @@ __global__ void __launch_bounds__(128, PRE ? CHAIN_PRE_CTAS : 4) k_chain(const C
   if (lane == 0 && status) status[col] = st;
 }
 
+// The record of element records r (n of them) that holds T, from record i on
+// (PFRecTable); T beyond all of them (or NaN) ends at one of the ends.
+__device__ __forceinline__ int rec_find(const PFRec* __restrict__ r, int n, int i, double T) {
+  while (true) {
+    const double lo = __ldg(&r[i].lo), hi = __ldg(&r[i].hi);
+    if (T > hi || (T == hi && lo < hi)) {
+      if (i == n - 1) return i;
+      ++i;
+    } else if (T < lo || (T == lo && lo < hi)) {
+      if (i == 0) return i;
+      --i;
+    } else {
+      return i;
+    }
+  }
+}
+
 // ------------------------------------------------------------------ k_saha
 // The Saha factors of every temperature sample of k_chain's integration, for
 // the listed columns [c0, c0 + cn): the samples are the model's T at each
@@ -326,7 +343,7 @@ constexpr int SAHA_SPT = 64;   // samples a warp takes at most
 constexpr int SAHA_CTAS = 5;   // per SM
 
 template <bool HE>
-__global__ void __launch_bounds__(128, SAHA_CTAS) k_saha(const Consts* __restrict__ Kg, const PFTable* __restrict__ tb,
+__global__ void __launch_bounds__(128, SAHA_CTAS) k_saha(const Consts* __restrict__ Kg, const PFRecTable* __restrict__ tb,
                                                  int ncol, int nz, const float* __restrict__ model,
                                                  double2* __restrict__ sa, int c0, int cn, int spt,
                                                  const int* __restrict__ list, const int* __restrict__ nlist) {
@@ -371,12 +388,11 @@ __global__ void __launch_bounds__(128, SAHA_CTAS) k_saha(const Consts* __restric
     const double x1 = K.csaha2 * fz_tab_xi[e], x2 = K.csaha2 * fz_tab_xii[e];
     double2* out = sa + ((size_t)ci * nsamp + s0) * 96 + slot;
     double c[3][6], bc[3], lo = 0.0, hi = 0.0;   // the active pieces and the open interval of T they hold for
-    int var[3];
-    bool expo[3];
+    int flags = 0, ir = 0;
+    const PFRec* rec = tb->r[e];
+    const int nrec = tb->n[e];
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
-      expo[s] = false;
-      var[s] = 0;
       bc[s] = 0.0;
 #pragma unroll
       for (int i = 0; i < 6; ++i) c[s][i] = 0.0;
@@ -385,33 +401,27 @@ __global__ void __launch_bounds__(128, SAHA_CTAS) k_saha(const Consts* __restric
       const SahaT& t = tt[i];
       const double T = t.var[0];
       if (!(T > lo && T < hi)) {
-        lo = -1.0e300;
-        hi = 1.0e300;
+        ir = rec_find(rec, nrec, ir, T);
+        const PFRec* p = rec + ir;
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
-          const int nv = tb->nv[e][s];
-          int act = 0;
 #pragma unroll
-          for (int q = 1; q < FZ_PF_MAXV; ++q) {
-            if (q >= nv) continue;
-            const double th = __ldg(&tb->p[e][s][q].th);
-            if (piece_on(__ldg(&tb->p[e][s][q].cond), th, T)) act = q;
-            if (th <= T) lo = fmax(lo, th);   // T = th holds for this sample alone: lo = T fails the next test
-            if (th >= T) hi = fmin(hi, th);
+          for (int q = 0; q < 6; q += 2) {
+            const double2 v = __ldg(reinterpret_cast<const double2*>(&p->c[s][q]));
+            c[s][q] = v.x;
+            c[s][q + 1] = v.y;
           }
-          const PFPiece* p = &tb->p[e][s][act];
-#pragma unroll
-          for (int q = 0; q < 6; ++q) c[s][q] = __ldg(&p->c[q]);
-          const int form = __ldg(&p->form);
-          expo[s] = form == 1;
-          var[s] = __ldg(&p->var);
-          bc[s] = piece_bc(form, __ldg(&p->base), __ldg(&p->clamp));
+          bc[s] = __ldg(&p->bc[s]);
         }
+        lo = __ldg(&p->lo);
+        hi = __ldg(&p->hi);
+        flags = __ldg(&p->flags);
       }
       constexpr bool EXPF = decltype(expf)::value;
       double u[3];
 #pragma unroll
-      for (int s = 0; s < 3; ++s) u[s] = piece_value<EXPF>(c[s], t.var[var[s]], expo[s], bc[s], K.exp2_32);
+      for (int s = 0; s < 3; ++s)
+        u[s] = piece_value<EXPF>(c[s], t.var[(flags >> (2 * s)) & 3], (flags >> (6 + s)) & 1, bc[s], K.exp2_32);
       const double e1 = exp_tab<false>(cut650(__dmul_rn(x1, t.it)), K.exp2_32);
       const double e2 = exp_tab<false>(cut650(__dmul_rn(x2, t.it)), K.exp2_32);
       const double2 f = saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
@@ -816,27 +826,154 @@ struct RFConf {
   int nj[NSLOT], n0[NSLOT];
 };
 
-// One warp per (column, height), FP64, lanes over the elements: the
-// chemistry derivatives of GET_DNHYDDTEMP at the (T, Pg, NELEC) that
-// FORWARD1D passes to it (src/forward.f90:917-918).
-__global__ void __launch_bounds__(128) k_chemder(const DevParams* __restrict__ Pg, const Consts* __restrict__ Kg,
-                                                 const PFTable* __restrict__ tb, const PFDTable* __restrict__ td,
+// The three sums of chem_der (fz_rf.cuh) for every (column, height), FP64.  A warp
+// takes hpt <= 32 heights of a column: lane h forms the terms of height h, then the
+// warp walks the heights once for each third of the element slots with the
+// lane's active value and derivative pieces in registers (reloaded when T
+// leaves the interval they hold for, as k_saha) and reduces the three values
+// over its lanes with six shuffles.  What bounds it: FP64, some 110 operations
+// an element and height (over 600 as derivatives of the reference's quotients,
+// the fixed point repeated by every lane): 2,048 columns of 128 heights 2.70 ->
+// 0.60 ms.
+struct ChemderT {
+  SahaT t;
+  double ne;
+};
+__global__ void __launch_bounds__(128, 3) k_chemder(const DevParams* __restrict__ Pg, const Consts* __restrict__ Kg,
+                                                 const PFTable* __restrict__ tb, const PFRecTable* __restrict__ tr,
                                                  int ncol, const float* __restrict__ mout,
-                                                 const double2* __restrict__ chem, double4* __restrict__ chemd,
+                                                 const double2* __restrict__ chem, double4* __restrict__ chemd, int hpt,
                                                  const int* __restrict__ list, const int* __restrict__ nlist) {
   __shared__ Consts K;
+  __shared__ ChemderT terms[4][32];
+  const int nz = Pg->nz, nblk = (nz + hpt - 1) / hpt, wpb = blockDim.x >> 5;
+  const long long ntask = (long long)(list ? *nlist : ncol) * nblk;
+  if ((long long)blockIdx.x * wpb >= ntask) return;
   copy_to_shared(&K, Kg);
   __syncthreads();
-  const int nz = Pg->nz;
-  const int lane = threadIdx.x & 31;
-  const int wpb = blockDim.x >> 5;
-  const size_t total = (size_t)(list ? *nlist : ncol) * nz;
-  for (size_t j = (size_t)blockIdx.x * wpb + (threadIdx.x >> 5); j < total; j += (size_t)gridDim.x * wpb) {
-    const int k = (int)(j % nz), col = list ? list[j / nz] : (int)(j / nz);
-    const size_t i = (size_t)col * nz + k;
-    const float* m = mout + (size_t)col * 13 * nz;
-    const ChemDer cd = chem_der_warp((double)mget(m, nz, 0, k), (double)mget(m, nz, 1, k), chem[i].y, K, tb, td, lane);
-    if (lane == 0) chemd[i] = make_double4(cd.dne_p, cd.dnh_p, cd.dne_t, cd.dnh_t);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  ChemderT* tt = terms[wid];
+  for (long long task = (long long)blockIdx.x * wpb + wid; task < ntask; task += (long long)gridDim.x * wpb) {
+    const int col = list ? list[task / nblk] : (int)(task / nblk), k0 = (int)(task % nblk) * hpt;
+    const int n = min(hpt, nz - k0);
+    __syncwarp();   // the previous task's terms no longer read
+    if (lane < n) {
+      tt[lane].t = saha_t((double)mget(mout + (size_t)col * 13 * nz, nz, 0, k0 + lane), K);
+      tt[lane].ne = chem[(size_t)col * nz + k0 + lane].y;
+    }
+    __syncwarp();
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};   // of height 8 b + lane % 8: sum lane / 8 of the three
+    auto third = [&](auto expf, int q) {
+      constexpr bool EXPF = decltype(expf)::value;
+      const int el = K.lane_elem[32 * q + lane], e = el < 0 ? 0 : el;
+      const double ab = el < 0 ? 0.0 : K.ab10[e];
+      const double x1 = K.csaha2 * fz_tab_xi[e], x2 = K.csaha2 * fz_tab_xii[e];
+      double c[3][6], d[3][6], bc[3], db[3], c5[3], lo = 0.0, hi = 0.0;
+      int flags = 0, dflags = 0, ir = 0;
+      const PFRec* rec = tr->r[e];
+      const int nrec = tr->n[e];
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        bc[s] = db[s] = c5[s] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) c[s][i] = d[s][i] = 0.0;
+      }
+      auto load = [&](double T) {
+        ir = rec_find(rec, nrec, ir, T);
+        const PFRec* p = rec + ir;
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+#pragma unroll
+          for (int i = 0; i < 6; i += 2) {
+            const double2 v = __ldg(reinterpret_cast<const double2*>(&p->c[s][i]));
+            const double2 w = __ldg(reinterpret_cast<const double2*>(&p->d[s][i]));
+            c[s][i] = v.x;
+            c[s][i + 1] = v.y;
+            d[s][i] = w.x;
+            d[s][i + 1] = w.y;
+          }
+          bc[s] = __ldg(&p->bc[s]);
+          db[s] = __ldg(&p->db[s]);
+          c5[s] = __ldg(&p->c5[s]);
+        }
+        lo = __ldg(&p->lo);
+        hi = __ldg(&p->hi);
+        flags = __ldg(&p->flags);
+        dflags = __ldg(&p->dflags);
+      };
+      auto eval = [&](int i, double v[3]) {
+        const SahaT& t = tt[i].t;
+        const double NE = tt[i].ne, it = t.it;
+        double u[3], du[3];
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          u[s] = piece_value<EXPF>(c[s], t.var[(flags >> (2 * s)) & 3], (flags >> (6 + s)) & 1, bc[s], K.exp2_32);
+          const int fl = dflags >> (10 * s);
+          double ur = u[s];
+          if (fl & 0xc0) {   // a derivative written on another value piece (U_II of tellurium)
+            const PFPiece* p = &tb->p[e][s][((fl >> 6) & 3) - 1];
+            double cr[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) cr[k] = __ldg(&p->c[k]);
+            const int form = __ldg(&p->form);
+            ur = piece_value<true>(cr, t.var[__ldg(&p->var)], form == 1, piece_bc(form, __ldg(&p->base), __ldg(&p->clamp)),
+                                   K.exp2_32);
+          }
+          double g = horner6(d[s], t.var[fl & 3]);
+          if (fl & 4) g *= -it;
+          if (fl & 8) g *= ur - db[s];
+          if (fl & 16) g *= rcp_d(ur);
+          du[s] = (fl & 32) && ur == c5[s] ? 0.0 : g;
+        }
+        const double e1 = exp_tab<false>(cut650(__dmul_rn(x1, it)), K.exp2_32);
+        const double e2 = exp_tab<false>(cut650(__dmul_rn(x2, it)), K.exp2_32);
+        const double2 f = saha_factors(u[0], u[1], u[2], e1, e2, t.hl);
+        const double it2 = it * it, dlam = -1.5 * it;
+        const double p = NE * f.x, P = (NE * NE) * f.y;
+        const double iD = rcp_d((1.0 + p) + P), w = ab * iD;
+        // d ln alpha_II / dT and d ln (alpha_I alpha_II) / dT
+        const double l2 = fma(-x2, it2, (du[1] - du[2]) + dlam);
+        const double lc = fma(-(x1 + x2), it2, fma(2.0, dlam, du[0] - du[2]));
+        if (q == 0 && lane == 0) {   // hydrogen: N_H+ - N_H- (:1841-1846)
+          v[0] = w * (1.0 - P);
+          v[1] = -(w * iD) * fma(p, 1.0 + P, 4.0 * P);
+          v[2] = -(w * iD) * fma(P * lc, 2.0 + p, (1.0 - P) * (p * l2));
+        } else {
+          const double wp = -(w * iD) * P;
+          v[0] = w * (1.0 + p);
+          v[1] = wp * (p + 2.0);
+          v[2] = wp * fma(1.0 + p, lc, -(p * l2));
+        }
+      };
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        for (int i = 8 * b; i < min(8 * b + 8, n); ++i) {
+          const double T = tt[i].t.var[0];
+          if (!(T > lo && T < hi)) load(T);
+          double v[3];
+          eval(i, v);
+          // lanes 0-7 get the first sum, 8-15 the second, 16-23 the third
+          const bool h16 = lane & 16, h8 = lane & 8;
+          double a = h16 ? v[2] : v[0], c1 = h16 ? 0.0 : v[1];
+          a += __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
+          c1 += __shfl_xor_sync(0xffffffffu, h16 ? v[1] : 0.0, 16);
+          double r = h8 ? c1 : a;
+          r += __shfl_xor_sync(0xffffffffu, h8 ? a : c1, 8);
+          r += __shfl_xor_sync(0xffffffffu, r, 4);
+          r += __shfl_xor_sync(0xffffffffu, r, 2);
+          r += __shfl_xor_sync(0xffffffffu, r, 1);
+          acc[b] += (lane & 7) == (i & 7) ? r : 0.0;
+        }
+    };
+    third(std::true_type{}, 0);
+#pragma unroll 1
+    for (int q = 1; q < 3; ++q) third(std::false_type{}, q);
+    double* out = reinterpret_cast<double*>(chemd + (size_t)col * nz + k0);
+    if (lane < 24) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        if (8 * b + (lane & 7) < n) out[4 * (8 * b + (lane & 7)) + (lane >> 3)] = acc[b];
+    }
   }
 }
 
@@ -864,13 +1001,11 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
     const double2 c = chem[i];
     const double nhyd = c.x, nelec = c.y;
     const double4 d4 = chemd[i];
-    ChemDer cd;
-    cd.dne_p = d4.x;
-    cd.dnh_p = d4.y;
-    cd.dne_t = d4.z;
-    cd.dnh_t = d4.w;
     const float Tf = mget(m, nz, 0, k);
     const double T = (double)Tf;
+    // the chemistry derivatives of GET_DNHYDDTEMP at the (T, Pg, NELEC) that
+    // FORWARD1D passes to it (src/forward.f90:917-918)
+    const ChemDer cd = chem_der(T, (double)mget(m, nz, 1, k), nelec, d4.x, d4.y, d4.z, K);
     const double dz = (k == nz - 1) ? 1e5 * fabs((double)mget(m, nz, 12, k) - (double)mget(m, nz, 12, k - 1))
                                     : 1e5 * fabs((double)mget(m, nz, 12, k + 1) - (double)mget(m, nz, 12, k));
     float* row = slab + i * sw;
@@ -2091,7 +2226,7 @@ struct fz_ctx {
   DevParams* d_params = nullptr;
   Consts* d_consts = nullptr;
   PFTable* d_pf = nullptr;
-  PFDTable* d_pfd = nullptr;
+  PFRecTable* d_pfr = nullptr;
   struct {
     int chain_warps = 4;       // k_chain warps per block
     int chain_lanes = 0;       // k_chain lanes per column: 32, 16, or 0 = by column count
@@ -2156,7 +2291,7 @@ struct fz_ctx {
   RFConf* d_rf = nullptr;
   float* d_coef = nullptr;
   float* d_rfslab = nullptr;
-  double4* d_chemd = nullptr;   // chemistry derivatives per (column, height)
+  double4* d_chemd = nullptr;   // chemistry derivative sums per (column, height): chem_der
   size_t rf_cols = 0;
   float* d_jac = nullptr;   // staging of the host-buffer API
   size_t jac_cols = 0;
@@ -2348,10 +2483,10 @@ void launch_k_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, in
       const long long tasks = (long long)cn * 3 * ((nsamp + spt - 1) / spt);
       const unsigned gs = (unsigned)std::min<long long>((tasks + 3) / 4, (long long)c->nsm * SAHA_CTAS * 2);
       if (hydrostatic)
-        k_saha<true><<<gs, 128, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, c0, cn, spt, list,
+        k_saha<true><<<gs, 128, 0, s>>>(c->d_consts, c->d_pfr, ncol, c->nz, d_model, c->d_saha, c0, cn, spt, list,
                                         nlist);
       else
-        k_saha<false><<<gs, 128, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, c->d_saha, c0, cn, spt, list,
+        k_saha<false><<<gs, 128, 0, s>>>(c->d_consts, c->d_pfr, ncol, c->nz, d_model, c->d_saha, c0, cn, spt, list,
                                          nlist);
     }
     if (gate && c0 == 0) chain_l(std::true_type{}, 32, 0, std::min(cn, gate), gate);
@@ -2568,11 +2703,13 @@ void launch_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, int*
 // (ncol bounds the grid); null: columns 0 .. ncol.
 void launch_chemder(fz_ctx* c, int ncol, const float* d_mout, int bpsm, cudaStream_t s, const int* list = nullptr,
                     const int* nlist = nullptr) {
-  const size_t cells = (size_t)ncol * c->nz;
-  size_t blocks = (cells + 3) / 4;
+  // few columns: fewer heights a warp, for latency (77 columns of 128 heights: 97
+  // us with 32, 54 with 8)
+  const int hpt = (size_t)ncol * c->nz < (size_t)32 * 8 * c->nsm ? 8 : 32;
+  size_t blocks = ((size_t)ncol * ((c->nz + hpt - 1) / hpt) + 3) / 4;
   if (bpsm > 0) blocks = std::min<size_t>(blocks, (size_t)c->nsm * bpsm);
-  k_chemder<<<(int)blocks, 128, 0, s>>>(c->d_params, c->d_consts, c->d_pf, c->d_pfd, ncol, d_mout, c->d_chem,
-                                        c->d_chemd, list, nlist);
+  k_chemder<<<(int)blocks, 128, 0, s>>>(c->d_params, c->d_consts, c->d_pf, c->d_pfr, ncol, d_mout, c->d_chem,
+                                        c->d_chemd, hpt, list, nlist);
 }
 
 void launch_opac_rf(fz_ctx* c, int ncol, const float* d_mout, int threads, cudaStream_t s, const int* list = nullptr,
@@ -3967,16 +4104,16 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
   if ((rc = cuda_fail(cudaMalloc(&c->d_params, sizeof(DevParams))))) return fail(rc);
   if ((rc = cuda_fail(cudaMalloc(&c->d_consts, sizeof(Consts))))) return fail(rc);
   if ((rc = cuda_fail(cudaMalloc(&c->d_pf, sizeof(PFTable))))) return fail(rc);
+  if ((rc = cuda_fail(cudaMalloc(&c->d_pfr, sizeof(PFRecTable))))) return fail(rc);
   {
-    std::vector<char> buf(sizeof(PFTable));
-    fzh_pf_table(reinterpret_cast<PFTable*>(buf.data()));
-    if ((rc = cuda_fail(cudaMemcpy(c->d_pf, buf.data(), sizeof(PFTable), cudaMemcpyHostToDevice)))) return fail(rc);
-  }
-  if ((rc = cuda_fail(cudaMalloc(&c->d_pfd, sizeof(PFDTable))))) return fail(rc);
-  {
-    std::vector<char> buf(sizeof(PFDTable));
-    if (fzh_pfd_table(reinterpret_cast<PFDTable*>(buf.data())) != 0) return fail(FZ_ERR_STATE);
-    if ((rc = cuda_fail(cudaMemcpy(c->d_pfd, buf.data(), sizeof(PFDTable), cudaMemcpyHostToDevice)))) return fail(rc);
+    std::vector<char> bv(sizeof(PFTable)), bd(sizeof(PFDTable)), br(sizeof(PFRecTable));
+    PFTable* v = reinterpret_cast<PFTable*>(bv.data());
+    PFDTable* d = reinterpret_cast<PFDTable*>(bd.data());
+    fzh_pf_table(v);
+    if (fzh_pfd_table(d) != 0 || fzh_pf_records(v, d, reinterpret_cast<PFRecTable*>(br.data())) != 0)
+      return fail(FZ_ERR_STATE);
+    if ((rc = cuda_fail(cudaMemcpy(c->d_pf, bv.data(), bv.size(), cudaMemcpyHostToDevice)))) return fail(rc);
+    if ((rc = cuda_fail(cudaMemcpy(c->d_pfr, br.data(), br.size(), cudaMemcpyHostToDevice)))) return fail(rc);
   }
   if ((rc = cuda_fail(cudaMalloc(&c->d_lam, numw * sizeof(LamP))))) return fail(rc);
   if ((rc = cuda_fail(cudaMalloc(&c->d_gain, 4 * numw * sizeof(float))))) return fail(rc);
@@ -4098,7 +4235,7 @@ int fz_destroy(fz_ctx* c) {
   cudaFree(c->d_params);
   cudaFree(c->d_consts);
   cudaFree(c->d_pf);
-  cudaFree(c->d_pfd);
+  cudaFree(c->d_pfr);
   cudaFree(c->d_oscr);
   cudaFree(c->d_smooth);
   cudaFree(c->d_lsf);

@@ -268,3 +268,56 @@ int fzh_pfd_table(PFDTable* t) {
     }
   return 0;
 }
+
+int fzh_pf_records(const PFTable* v, const PFDTable* d, PFRecTable* t) {
+  std::memset(t, 0, sizeof(*t));
+  for (int e = 0; e < FZ_NELEM; ++e) {
+    std::vector<double> th;
+    for (int s = 0; s < 3; ++s) {
+      for (int i = 1; i < v->nv[e][s]; ++i) th.push_back(v->p[e][s][i].th);
+      for (int i = 0; i < d->nd[e][s]; ++i)
+        if (d->d[e][s][i].cond >= 1 && d->d[e][s][i].cond <= 4) th.push_back(d->d[e][s][i].th);
+    }
+    std::sort(th.begin(), th.end());
+    th.erase(std::unique(th.begin(), th.end()), th.end());
+    const int n = 2 * (int)th.size() + 1;
+    if (n > FZ_PF_MAXREC) return -1;
+    t->n[e] = n;
+    for (int r = 0; r < n; ++r) {
+      PFRec& q = t->r[e][r];
+      const int j = r / 2;   // thresholds below an interval, or the index of a threshold
+      q.lo = r % 2 ? th[j] : (j > 0 ? th[j - 1] : -1.0e300);
+      q.hi = r % 2 ? th[j] : (j < (int)th.size() ? th[j] : 1.0e300);
+      // a temperature of the record
+      const double T = r % 2 ? th[j] : (th.empty() ? 1.0 : j == 0 ? 0.5 * th[0] : j == (int)th.size() ? 2.0 * th[j - 1] : 0.5 * (th[j - 1] + th[j]));
+      for (int s = 0; s < 3; ++s) {
+        int act = 0, dact = -1;
+        for (int i = 1; i < v->nv[e][s]; ++i) {
+          const PFPiece& p = v->p[e][s][i];
+          if (p.cond != 1 && p.cond != 2) return -1;
+          if (p.cond == 1 ? T > p.th : T < p.th) act = i;
+        }
+        for (int i = 0; i < d->nd[e][s]; ++i) {
+          const PFDPiece& p = d->d[e][s][i];
+          if (p.cond == 5 && i > 0) return -1;   // (a condition on U with another piece to fall back on)
+          if (p.cond == 0 || p.cond == 5 || (p.cond == 1 && T > p.th) || (p.cond == 2 && T < p.th) ||
+              (p.cond == 3 && T <= p.th) || (p.cond == 4 && T >= p.th))
+            dact = i;
+        }
+        const PFPiece& p = v->p[e][s][act];
+        for (int i = 0; i < 6; ++i) q.c[s][i] = p.c[i];
+        q.bc[s] = p.form == 1 ? p.base : (p.form == 2 ? p.clamp : -1.0e300);
+        q.flags |= (p.var << (2 * s)) | ((p.form == 1) << (6 + s));
+        if (dact < 0) continue;
+        const PFDPiece& g = d->d[e][s][dact];
+        for (int i = 0; i < 6; ++i) q.d[s][i] = g.c[i] * g.mult;
+        q.db[s] = g.base;
+        q.c5[s] = g.th;
+        const int other = g.ref >= 0 && g.ref != act ? g.ref + 1 : 0;
+        q.dflags |= (g.var | ((g.dx != 0) << 2) | ((g.ub != 0) << 3) | ((g.up != 0) << 4) | ((g.cond == 5) << 5) | (other << 6))
+                    << (10 * s);
+      }
+    }
+  }
+  return 0;
+}

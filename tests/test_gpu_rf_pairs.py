@@ -69,3 +69,25 @@ def test_output_at_any_word(fz):
         torch.cuda.synchronize()
         out.append(buf[off:off + n].clone())
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("scale", [0.55, 0.8, 1.0, 1.3, 1.9])
+def test_chemistry_derivatives_across_the_partition_functions(fz, orc, scale):
+    """The T response with temperatures from 2,400 to 18,000 K: every interval
+    of the partition functions' value and derivative pieces, one column at a
+    threshold of theirs (6,000 K) at every height."""
+    lines = fz.lines_parse(fz.atmos.line_database_text())
+    reg = fz.regions_from_lines_section("1 21 -215.0 21.5\n", lines)
+    g, _ = orc.gain(lines, reg)
+    nz = 33
+    m = fz.atmos.make_columns(4, nz, seed=6)
+    m[:, 0] *= np.float32(scale)
+    m[3, 0] = 6000.0
+    ctx = fz.Synthesis(lines, reg, nz=nz, gain=g)
+    nodes = {1: 3, 2: 2}
+    ctx.rf_nodes(nodes)
+    _, jac, _, st = ctx.forward_rf(m, hydrostatic=False)
+    _, ojac, _, _ = orc.forward_rf(lines, reg, g, m, nodes, hydrostatic=False)
+    assert np.all(st == 0)
+    scale_ = np.abs(ojac).max(axis=2, keepdims=True)
+    assert np.max(np.abs(jac - ojac) / np.maximum(scale_, 1e-3 * scale_.max(axis=1, keepdims=True))) < TOL

@@ -42,6 +42,7 @@ constexpr int MAXLU = 16;     // lines used by the regions (main + blends)
 constexpr int MAXCOMP = 256;  // Zeeman components of all used lines
 constexpr int MAXNUMW = 1024;
 constexpr int MAXNZ = 1024;
+constexpr int SYNTH_SMS = 148;   // B200
 
 // Per-context constants read by the kernels (global memory, one copy per ctx).
 struct DevParams {
@@ -751,19 +752,34 @@ __device__ __forceinline__ bool synth_store(const PairP& pr, const F2 I[4], cons
 // with rte_layer one wavelength a thread, 34.4 with two; four lines on 4,087
 // columns of 160 heights 12.3, 7.4, 6.3.  The error against 64 bits halved
 // (relative 6.4e-7 -> 2.9e-7).
-__global__ void __launch_bounds__(256, 2) k_synth(
+//
+// G > 1, for batches that leave the SMs waiting on a few columns' chains: G
+// groups of npt threads form the layers of G heights at once (a layer does
+// not depend on the ones below) and pass them through shared memory to the
+// first group, which applies them in order; the same operations on the same
+// values as G = 1, bit for bit (148 columns as above 174 -> 127 us with G = 4, 296
+// columns 260 -> 221 with G = 2, two CTAs per SM).  Each group starts further into
+// the table, so that a sub-partition gets costly and cheap warps alike; with G = 1
+// the CTAs beyond the first of an SM start half-way (256 columns 0.259 -> 0.257).
+// clo, chi: run only when the column count is above clo and at most chi (chi =
+// 0: any count).
+template <int G>
+__global__ void __launch_bounds__(G == 1 ? 256 : 512, G == 1 ? 2 : 1) k_synth(
     const DevParams* __restrict__ Pg, const PairP* __restrict__ pairs, int npt, const float* __restrict__ gain, int ncol,
     const float* __restrict__ slab, double* __restrict__ syn, float* mout, int* __restrict__ status,
-    const int* __restrict__ list = nullptr, const int* __restrict__ nlist = nullptr) {
+    const int* __restrict__ list = nullptr, const int* __restrict__ nlist = nullptr, int clo = 0, int chi = 0) {
   extern __shared__ float4 sm_synth4[];
   __shared__ SynthP P;
   __shared__ int next;
   const int count = list ? *nlist : ncol;
-  if ((int)blockIdx.x >= count) return;
+  if ((int)blockIdx.x >= count || count <= clo || (chi > 0 && count > chi)) return;
   synth_params(P, Pg);
   const int nz = Pg->nz, sw = Pg->sw, nw = Pg->numw;
-  const int n4 = nz * sw / 4, lane = threadIdx.x & 31;
+  const int n4 = nz * sw / 4, lane = threadIdx.x & 31, nwarp = npt >> 5;
   float* sm = reinterpret_cast<float*>(sm_synth4);
+  F2* xch = reinterpret_cast<F2*>(sm_synth4 + n4);   // G > 1: G x LAYER2_F2 x npt
+  const int grp = G > 1 ? (int)threadIdx.x / npt : 0;
+  const int rot = G > 1 ? grp * max(1, nwarp / G) : ((int)blockIdx.x / SYNTH_SMS) * (nwarp / 2);
   for (int idx = blockIdx.x; idx < count; idx += gridDim.x) {
     const int col = list ? list[idx] : idx;
     __syncthreads();   // P in place; the previous column's slab no longer read
@@ -774,33 +790,184 @@ __global__ void __launch_bounds__(256, 2) k_synth(
     if (threadIdx.x >= blockDim.x - 32) log_tau5_warp(sm, sw, nz, mout + (size_t)col * 13 * nz, lane);
     double* o = syn + (size_t)col * 4 * nw;
     bool bad = false;
-    while (true) {
-      int w = 0;
-      if (lane == 0) w = atomicAdd(&next, 32);
-      w = __shfl_sync(0xffffffffu, w, 0);
-      if (w >= npt) break;
-      const PairP pr = pairs[w + lane];
-      if (pr.n > 0) {
-        F2 I[4] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
-        Layer2 L;
-        for (int k = 0; k < nz; ++k) {
+    Layer2 L;
+    if (G == 1) {
+      while (true) {
+        int w = 0;
+        if (lane == 0) w = atomicAdd(&next, 1);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (w >= nwarp) break;
+        const PairP pr = pairs[(w + rot) % nwarp * 32 + lane];
+        if (pr.n > 0) {
+          F2 I[4] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
+          for (int k = 0; k < nz; ++k) {
+            const float* row = sm + k * sw;
+            const float2 tf = *reinterpret_cast<const float2*>(row);
+            L.S = synth_planck(pr, tf.x);
+            if (k == 0 || tf.y != 0.0f) {   // SET_BOUNDARY, src/rtesolver.f90:1134-1147
+              I[0] = L.S;
+              I[1] = I[2] = I[3] = f2(0.f);
+              continue;
+            }
+            bad |= synth_layer(P, pr, row, L);
+            layer_apply(L, I);
+          }
+          bad |= synth_store(pr, I, gain, nw, o);
+        }
+        __syncwarp();
+      }
+    } else {
+      const int t = (((int)threadIdx.x - grp * npt + 32 * rot) % npt);
+      const PairP pr = pairs[t];
+      F2 I[4] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
+      for (int k0 = 0; k0 < nz; k0 += G) {
+        const int k = k0 + grp;
+        if (k < nz && pr.n > 0) {
           const float* row = sm + k * sw;
           const float2 tf = *reinterpret_cast<const float2*>(row);
           L.S = synth_planck(pr, tf.x);
-          if (k == 0 || tf.y != 0.0f) {   // SET_BOUNDARY, src/rtesolver.f90:1134-1147
-            I[0] = L.S;
-            I[1] = I[2] = I[3] = f2(0.f);
-            continue;
+          F2* x = xch + (size_t)grp * LAYER2_F2 * npt + t;
+          if (k == 0 || tf.y != 0.0f) {
+            x[0] = L.S;
+          } else {
+            bad |= synth_layer(P, pr, row, L);
+            const F2* l = reinterpret_cast<const F2*>(&L);
+#pragma unroll
+            for (int i = 0; i < LAYER2_F2; ++i) x[(size_t)i * npt] = l[i];
           }
-          bad |= synth_layer(P, pr, row, L);
-          layer_apply(L, I);
         }
-        bad |= synth_store(pr, I, gain, nw, o);
+        __syncthreads();
+        if (grp == 0 && pr.n > 0) {
+          for (int q = 0; q < G && k0 + q < nz; ++q) {
+            const F2* x = xch + (size_t)q * LAYER2_F2 * npt + t;
+            if (k0 + q == 0 || sm[(k0 + q) * sw + 1] != 0.0f) {
+              I[0] = x[0];
+              I[1] = I[2] = I[3] = f2(0.f);
+              continue;
+            }
+            F2* l = reinterpret_cast<F2*>(&L);
+#pragma unroll
+            for (int i = 0; i < LAYER2_F2; ++i) l[i] = x[(size_t)i * npt];
+            layer_apply(L, I);
+          }
+        }
+        __syncthreads();
       }
-      __syncwarp();
+      if (grp == 0 && pr.n > 0) bad |= synth_store(pr, I, gain, nw, o);
     }
+    __syncwarp();
     if (status && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&status[col], FZ_NAN);
   }
+}
+
+// k_synth of a few columns over the whole GPU, in two launches: k_layers forms the
+// layers of hb heights of a column per CTA (a layer does not depend on the ones
+// below) in device memory, then k_layers_rte applies them in order, one warp a
+// CTA, its copies RTE_STAGES heights ahead.  The same operations on the same
+// values as k_synth, bit for bit.  What bounds it: the latency of the chain that
+// remains, some 60 FMAs a height.  One column of 128 heights, two lines of 112
+// wavelengths: 168 us with k_synth<1>, 121 with k_synth<4> on its one SM, 41 here;
+// 64 columns 172, 125, 93; above that the layers leave the L2 and k_synth wins.
+__global__ void __launch_bounds__(128, 4) k_layers(const DevParams* __restrict__ Pg, const PairP* __restrict__ pairs, int npt,
+                                                   const float* __restrict__ slab, int hb, F2* __restrict__ lay,
+                                                   int* __restrict__ status) {
+  __shared__ SynthP P;
+  const int col = blockIdx.y, nz = Pg->nz, sw = Pg->sw, lane = threadIdx.x & 31;
+  synth_params(P, Pg);
+  __syncthreads();
+  const int k0 = blockIdx.x * hb, nh = min(hb, nz - k0), nwarp = npt >> 5;
+  bool bad = false;
+  // a warp takes (height, 32 table entries) after (height, 32 table entries)
+  for (int w = threadIdx.x >> 5; w < nh * nwarp; w += blockDim.x >> 5) {
+    const int k = k0 + w / nwarp, t = 32 * (w % nwarp) + lane;
+    const PairP pr = pairs[t];
+    if (pr.n == 0) continue;
+    const float* row = slab + ((size_t)col * nz + k) * sw;
+    const float2 tf = *reinterpret_cast<const float2*>(row);
+    F2* x = lay + ((size_t)col * nz + k) * LAYER2_F2 * npt + t;
+    Layer2 L;
+    L.S = synth_planck(pr, tf.x);
+    if (k == 0 || tf.y != 0.0f) {
+      x[0] = L.S;
+      continue;
+    }
+    bad |= synth_layer(P, pr, row, L);
+    const F2* l = reinterpret_cast<const F2*>(&L);
+#pragma unroll
+    for (int i = 0; i < LAYER2_F2; ++i) x[(size_t)i * npt] = l[i];
+  }
+  __syncwarp();
+  if (status && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&status[col], FZ_NAN);
+}
+
+constexpr int RTE_STAGES = 8;
+size_t layers_rte_smem(int nz) { return (size_t)RTE_STAGES * LAYER2_F2 * 32 * sizeof(F2) + (size_t)nz * 2 * sizeof(float); }
+
+__global__ void __launch_bounds__(32) k_layers_rte(const DevParams* __restrict__ Pg, const PairP* __restrict__ pairs, int npt,
+                                                   const float* __restrict__ gain, const float* __restrict__ slab,
+                                                   const F2* __restrict__ lay, double* __restrict__ syn, float* mout,
+                                                   int* __restrict__ status) {
+  extern __shared__ float4 sm_synth4[];
+  const int col = blockIdx.y, nz = Pg->nz, sw = Pg->sw, nw = Pg->numw, lane = threadIdx.x;
+  F2* ring = reinterpret_cast<F2*>(sm_synth4);
+  float* flag = reinterpret_cast<float*>(ring + RTE_STAGES * LAYER2_F2 * 32);
+  const float* sl = slab + (size_t)col * nz * sw;
+  if ((int)blockIdx.x == npt >> 5) {   // log tau5: the rows' KC5 and rho side by side
+    for (int k = lane; k < nz; k += 32) *reinterpret_cast<float2*>(flag + 2 * k) = *reinterpret_cast<const float2*>(sl + (size_t)k * sw + 2);
+    __syncwarp();
+    log_tau5_warp(flag - 2, 2, nz, mout + (size_t)col * 13 * nz, lane);
+    return;
+  }
+  const int t = 32 * blockIdx.x + lane;
+  const PairP pr = pairs[t];
+  const F2* src = lay + (size_t)col * nz * LAYER2_F2 * npt + 32 * blockIdx.x;
+  // height k's layer of the warp's 32 entries: LAYER2_F2 rows of 256 bytes, two
+  // rows per round of 16-byte copies
+  const F2* from = src + (size_t)(lane >> 4) * npt + 2 * (lane & 15);
+  const int to = (lane >> 4) * 32 + 2 * (lane & 15);
+  auto fetch = [&](int k) {
+    if (k < nz) {
+      const F2* f = from + (size_t)k * LAYER2_F2 * npt;
+      F2* r = ring + (k % RTE_STAGES) * LAYER2_F2 * 32 + to;
+#pragma unroll
+      for (int i = 0; i < LAYER2_F2; i += 2) cp16(r + 32 * i, f + (size_t)i * npt);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  static_assert(LAYER2_F2 % 2 == 0, "two rows a round");
+  for (int k = 0; k < RTE_STAGES - 1; ++k) fetch(k);
+  for (int k = lane; k < nz; k += 32) flag[k] = sl[(size_t)k * sw + 1];
+  auto load = [&](int k, Layer2& L) {
+    const F2* x = ring + (k % RTE_STAGES) * LAYER2_F2 * 32 + lane;
+    F2* l = reinterpret_cast<F2*>(&L);
+#pragma unroll
+    for (int i = 0; i < LAYER2_F2; ++i) l[i] = x[32 * i];
+  };
+  F2 I[4] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
+  // heights up to k + 1 in place, k's layer in L: fetch, load k + 1, apply k
+  auto step = [&](int k, const Layer2& L, Layer2& nxt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(RTE_STAGES - 3) : "memory");
+    __syncwarp();   // for every lane; and height k - 1 read by all
+    fetch(k + RTE_STAGES - 1);
+    if (k + 1 < nz) load(k + 1, nxt);
+    if (k == 0 || flag[k] != 0.0f) {
+      I[0] = L.S;
+      I[1] = I[2] = I[3] = f2(0.f);
+    } else {
+      layer_apply(L, I);
+    }
+  };
+  Layer2 A, B;
+  asm volatile("cp.async.wait_group %0;" ::"n"(RTE_STAGES - 2) : "memory");
+  __syncwarp();
+  load(0, A);
+  for (int k = 0; k < nz; k += 2) {
+    step(k, A, B);
+    if (k + 1 < nz) step(k + 1, B, A);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  const bool bad = pr.n > 0 && synth_store(pr, I, gain, nw, syn + (size_t)col * 4 * nw);
+  if (status && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&status[col], FZ_NAN);
 }
 
 // ------------------------------------------------------ response functions
@@ -2249,6 +2416,9 @@ struct fz_ctx {
   LamP* d_lam = nullptr;
   PairP* d_pairs = nullptr;   // npt entries: k_synth's wavelengths by thread
   int npt = 0;
+  F2* d_lay = nullptr;         // the layers of up to lay_cols columns (k_layers)
+  int lay_cols = 0;
+  int synth_g = 0;             // the numbers of heights at once (4, 2) that k_synth can take
   bool pairs_even = false;     // its warps of equal cost
   bool pairs_vec = false;      // every entry two wavelengths from an even one, NUMW even
   float* d_gain = nullptr;
@@ -2363,6 +2533,15 @@ int saha_chunk_cols(const fz_ctx* c, int ncol) {
   return (int)std::min<size_t>(std::min(ncol, SAHA_CHUNK_SM * c->nsm), cap);
 }
 
+// Batches of at most this many columns run k_layers + k_layers_rte: their layers (160
+// bytes a height and two wavelengths) within SYNTH_LAY_BYTES.
+constexpr int SYNTH_FEW = 64;
+constexpr size_t SYNTH_LAY_BYTES = (size_t)192 << 20;
+int synth_few_cols(const fz_ctx* c) {
+  const size_t per = (size_t)c->nz * LAYER2_F2 * c->npt * sizeof(F2);
+  return (int)std::min<size_t>(SYNTH_FEW, SYNTH_LAY_BYTES / per);
+}
+
 int ensure_scratch(fz_ctx* c, int ncol) {
   if ((size_t)ncol > c->scratch_cols) {
     cudaFree(c->d_slab);
@@ -2373,6 +2552,17 @@ int ensure_scratch(fz_ctx* c, int ncol) {
     FZ_CK(cudaMalloc(&c->d_slab, (size_t)ncol * c->nz * c->sw * sizeof(float)));
     FZ_CK(cudaMalloc(&c->d_chem, (size_t)ncol * c->nz * sizeof(double2)));
     c->scratch_cols = ncol;
+  }
+  // a few columns' layers (launch_synth); without the memory k_synth runs
+  const int few = synth_few_cols(c);
+  if (ncol <= few && ncol > c->lay_cols) {
+    cudaFree(c->d_lay);
+    c->d_lay = nullptr;
+    c->lay_cols = 0;
+    if (cudaMalloc(&c->d_lay, (size_t)ncol * c->nz * LAYER2_F2 * c->npt * sizeof(F2)) == cudaSuccess)
+      c->lay_cols = ncol;
+    else
+      cudaGetLastError();
   }
   const int want = saha_chunk_cols(c, ncol);
   if (want > c->saha_want) {
@@ -2524,14 +2714,42 @@ int launch_lsf(fz_ctx* c, T* d_data, long long nrows, int rows_per_col, cudaStre
 // of 112 wavelengths, 128 heights, ms with 64 and 128: 444 columns 0.40 and
 // 0.36, 592 0.404 and 0.410, 2,048 1.16 and 1.24; one blended region of 500,
 // 504 columns of 256 heights with 64, 128, 256: 2.52, 2.24, 2.10).
+size_t synth_smem(const fz_ctx* c, int g) {
+  return (size_t)c->nz * c->sw * sizeof(float) + (g > 1 ? (size_t)g * LAYER2_F2 * c->npt * sizeof(F2) : 0);
+}
 void launch_synth(fz_ctx* c, int ncol, const float* slab, double* d_syn, float* d_mout, int* d_status, cudaStream_t s,
                   const int* list = nullptr, const int* nlist = nullptr) {
   ProfScope ps(c, 2, s, ncol);
+  // G heights at once for counts in (lo, hi]; a listed batch launches every
+  // form its count may ask for, each gated by it
+  auto go = [&](auto kern, int g, int grid, int threads, int lo, int hi) {
+    kern<<<grid, threads, synth_smem(c, g), s>>>(c->d_params, c->d_pairs, c->npt, c->d_gain, ncol, slab, d_syn, d_mout,
+                                                 d_status, list, nlist, lo, hi);
+  };
+  if (!list && slab == c->d_slab && ncol <= c->lay_cols) {
+    // CTAs of several heights once one height each fills the SMs four times
+    const int hb = std::max(1, std::min(8, ncol * c->nz / (16 * c->nsm)));
+    k_layers<<<dim3((c->nz + hb - 1) / hb, ncol), 128, 0, s>>>(c->d_params, c->d_pairs, c->npt, slab, hb, c->d_lay, d_status);
+    k_layers_rte<<<dim3(c->npt / 32 + 1, ncol), 32, layers_rte_smem(c->nz), s>>>(
+        c->d_params, c->d_pairs, c->npt, c->d_gain, slab, c->d_lay, d_syn, d_mout, d_status);
+    return;
+  }
+  int lo = 0;
+  for (int g = 4; g > 1; g /= 2) {
+    if (!(c->synth_g & g)) continue;
+    const int hi = c->nsm * (4 / g);
+    if (list || (ncol > lo && ncol <= hi)) {
+      if (g == 4)
+        go(k_synth<4>, 4, std::min(ncol, hi), 4 * c->npt, list ? lo : 0, list ? hi : 0);
+      else
+        go(k_synth<2>, 2, std::min(ncol, hi), 2 * c->npt, list ? lo : 0, list ? hi : 0);
+    }
+    if (ncol <= hi) return;
+    lo = hi;
+  }
   const int threads = std::min(c->npt, c->pairs_even ? 256 : (ncol < 4 * c->nsm ? 128 : 64));
   // listed: a grid of 32 CTAs per SM walks the list
-  const int grid = list ? std::min(ncol, c->nsm * 32) : ncol;
-  k_synth<<<grid, threads, (size_t)c->nz * c->sw * sizeof(float), s>>>(c->d_params, c->d_pairs, c->npt, c->d_gain, ncol,
-                                                                      slab, d_syn, d_mout, d_status, list, nlist);
+  go(k_synth<1>, 1, list ? std::min(ncol, c->nsm * 32) : ncol, threads, list ? lo : 0, 0);
 }
 
 // The synthesis of ncol columns, or with a list of the columns list[0,
@@ -4158,8 +4376,27 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
   // opt in to large dynamic shared memory for the slab staging
   const int sms = nz * c->sw * (int)sizeof(float);
   if (sms > 48 * 1024 - (int)sizeof(SynthP) - 16 &&
-      (rc = cuda_fail(cudaFuncSetAttribute(k_synth, cudaFuncAttributeMaxDynamicSharedMemorySize, sms))))
+      (rc = cuda_fail(cudaFuncSetAttribute(k_synth<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sms))))
     return fail(rc);
+  const size_t rsm = layers_rte_smem(nz);
+  if (rsm > 48 * 1024 &&
+      (rc = cuda_fail(cudaFuncSetAttribute(k_layers_rte, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm))))
+    return fail(rc);
+  // several heights at once: blocks of at most 512 threads (two heights: below
+  // that, so that two CTAs share an SM; a table of 256 threads gains nothing),
+  // room for their layers beside the slab
+  if (4 * c->npt <= 512 && synth_smem(c, 4) <= 200 * 1024) {
+    if ((rc = cuda_fail(cudaFuncSetAttribute(k_synth<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)synth_smem(c, 4)))))
+      return fail(rc);
+    c->synth_g |= 4;
+  }
+  if (2 * c->npt < 512 && synth_smem(c, 2) <= 200 * 1024) {
+    if ((rc = cuda_fail(cudaFuncSetAttribute(k_synth<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)synth_smem(c, 2)))))
+      return fail(rc);
+    c->synth_g |= 2;
+  }
   *out = c;
   return 0;
 }
@@ -4249,6 +4486,7 @@ int fz_destroy(fz_ctx* c) {
     cudaFree(p);
   cudaFree(c->d_lam);
   cudaFree(c->d_pairs);
+  cudaFree(c->d_lay);
   cudaFree(c->d_gain);
   cudaFree(c->d_slab);
   cudaFree(c->d_chem);

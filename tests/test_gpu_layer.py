@@ -87,3 +87,23 @@ def test_wavelength_pairs_of_any_region_sizes(fz, orc, n1, n2):
     assert np.all(st == 0)
     assert np.max(np.abs(syn[:, 0] / ref[:, 0] - 1)) < 1e-5
     assert np.max(np.abs(syn[:, 1:] - ref[:, 1:])) < 1e-6
+
+
+@pytest.mark.parametrize("section", ["1 112 -1193.25 21.5\n2 112 -1193.25 21.5\n", "1,2 75 -700.0 33.0\n",
+                                     "1 96 -1021.25 21.5\n2 96 -1021.25 21.5\n3 96 -1021.25 21.5\n4 96 -1021.25 21.5\n",
+                                     "2 5 -43.0 21.5\n"])
+@pytest.mark.parametrize("nz", [2, 5, 8, 9, 33])
+def test_every_batch_size_takes_the_same_steps(fz, section, nz):
+    """Layers of several heights at once (two launches up to 64 columns, groups of
+    a CTA up to two columns per SM) against one height after the other: the same
+    bits, at the sizes where a form begins or ends."""
+    lines = fz.lines_parse(fz.atmos.line_database_text())
+    ctx = fz.Synthesis(lines, fz.regions_from_lines_section(section, lines), nz=nz)
+    m = fz.atmos.make_columns(640, nz, seed=nz)
+    syn, mo, st = ctx.forward(m, hydrostatic=False)
+    assert np.all(st == 0)
+    for n in (1, 3, 64, 65, 148, 149, 296, 297):
+        s, o, t = ctx.forward(m[:n], hydrostatic=False)
+        np.testing.assert_array_equal(s, syn[:n])
+        np.testing.assert_array_equal(o, mo[:n])
+        np.testing.assert_array_equal(t, st[:n])

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(128, PRE ? CHAIN_PRE_CTAS : 4) k_chain(const C
         saha_prepare(w, (double)mget(m, nz, 0, k), K, tb, lane);
       }
       const double pg = (double)mget(m, nz, 1, k), ipg = rcp_d(pg);
-      const RhoOut r = get_rho_warp(w, ab, pg, nelec, K, lane);
+      const RhoOut r = get_rho_warp<false>(w, ab, [&] { return pg; }, nelec, K, lane);
       st |= r.status;
       if (lane == 0) {
         mo[2 * nz + k] = (float)r.dens;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(128, PRE ? CHAIN_PRE_CTAS : 4) k_chain(const C
     // the previous step's last stage
     double pg0 = exp_any(u0, K.exp2_32), ipg0 = rcp_d(pg0);
     {
-      const RhoOut r = get_rho_warp(w, ab, pg0, nelec, K, lane);
+      const RhoOut r = get_rho_warp<false>(w, ab, [&] { return pg0; }, nelec, K, lane);
       st |= r.status;
       if (lane == 0) {
         const float pel = (float)r.pelec;
@@ -251,10 +251,6 @@ __global__ void __launch_bounds__(128, PRE ? CHAIN_PRE_CTAS : 4) k_chain(const C
       double u1 = 0.0, ksum = 0.0, y = u0, pg = pg0, ipg = ipg0;
 #pragma unroll 1
       for (int stg = 0; stg < 5; ++stg) {
-        if (stg > 0) {
-          pg = exp_any(y, K.exp2_32);
-          ipg = rcp_d(pg);
-        }
         if (stg == 1 || stg == 3) {
           if (PRE) {
             // sample 2 (nz-2-k) + 1 is this step's midpoint, the next one T(k)
@@ -265,7 +261,13 @@ __global__ void __launch_bounds__(128, PRE ? CHAIN_PRE_CTAS : 4) k_chain(const C
             saha_prepare(w, stg == 1 ? tmid : tm1, K, tb, lane);
           }
         }
-        const RhoOut q = get_rho_warp(w, ab, pg, nelec, K, lane);
+        // Pg = exp(y); the first stage's is the last step's
+        const RhoOut q = get_rho_warp<L == 32>(w, ab, [&] {
+          const double e = exp_any(y, K.exp2_32);
+          pg = stg > 0 ? e : pg;
+          return pg;
+        }, nelec, K, lane);
+        ipg = rcp_d(pg);
         st |= q.status;
         if (stg < 4) {
           const double d = (q.dens * mgdz) * ipg;
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(128) k_chain_med(const Consts* __restrict__ Kg
   double nelec_down;
   {
     const double pg = exp_any(ua, K.exp2_32);
-    const RhoOut r = get_rho_warp(w, ab, pg, nelec, K, lane);
+    const RhoOut r = get_rho_warp<false>(w, ab, [&] { return pg; }, nelec, K, lane);
     st |= r.status;
     nelec_down = r.pelec / KBOL / tz;
     __syncwarp();
@@ -501,7 +503,7 @@ __global__ void __launch_bounds__(128) k_chain_med(const Consts* __restrict__ Kg
       if (stg == 1 || stg == 3) saha_prepare(w, stg == 1 ? tmid : tm1, K, tb, lane);
       const double y = stg == 0 ? u0 : (stg == 1 ? u0 + kk[0] / 2.0 : (stg == 2 ? u0 + kk[1] / 2.0 : (stg == 3 ? u0 + kk[2] : u1)));
       const double pg = exp_any(y, K.exp2_32), ipg = rcp_d(pg);
-      const RhoOut q = get_rho_warp(w, ab, pg, nelec, K, lane);
+      const RhoOut q = get_rho_warp<false>(w, ab, [&] { return pg; }, nelec, K, lane);
       st |= q.status;
       if (stg < 4) {
         const double d = (q.dens * (-GRAV * dz)) * ipg;   // as k_chain
@@ -2033,7 +2035,7 @@ __global__ void k_gain(const DevParams* __restrict__ Pg, const Consts* __restric
     for (int k = 0; k < N; ++k) {
       const double T = (double)fz_tab_hsra_tem[k];
       saha_prepare(w, T, K, tb, lane);
-      const RhoOut r = get_rho_warp(w, ab, (double)fz_tab_hsra_pg[k], nelec, K, lane);
+      const RhoOut r = get_rho_warp<false>(w, ab, [&] { return (double)fz_tab_hsra_pg[k]; }, nelec, K, lane);
       st |= r.status;
       if (lane < P.nreg) sm_gain[k * P.nreg + lane] = opac_continuum(T, nelec, r.nhyd, P.cont[lane]);
     }

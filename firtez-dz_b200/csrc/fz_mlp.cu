@@ -44,208 +44,148 @@ __device__ __forceinline__ float gelu_d(float z) {
 //   EPI_FWD_LIN : z = C + bias[n] -> fout (fp32)
 //   EPI_BWD_GELU: out = bf16(C * gelu'(zin[m][n]))
 //   EPI_F32     : fout = C (fp32)
-// on the fifth-generation tensor cores (tcgen05): a 128 x 128
-// output tile per CTA of 256 threads, K in blocks of 64 staged into shared
-// memory in the canonical K-major layout (fz_tc.cuh) through three buffers,
-// one elected thread issuing tcgen05.mma (bf16 x bf16 -> FP32 in tensor
-// memory) and committing each block to the buffer's mbarrier, the epilogue
-// read back with tcgen05.ld (warps w and w + 4 share TMEM lanes 32 (w % 4)..,
-// columns 0-63 and 64-127).  Operands whose leading dimension allows it move
-// in 16-byte vectors, the others element by element.
-constexpr int TC_BK = 64, TC_NKC = TC_BK / 8, TC_STAGES = 3;
-constexpr int TC_TILE = 128 * TC_BK * 2;                      // one 128 x 64 bf16 tile
-constexpr size_t TC_SMEM = (size_t)TC_STAGES * 2 * TC_TILE;   // A and B per stage: 96 KB
+// on the fifth-generation tensor cores (tcgen05), fed by the tensor memory
+// accelerator.  An operand is K-major (AMN / BMN false: K contiguous, the
+// forward's X and W) or MN-major (true: MN contiguous, the backward's dZ^T,
+// X^T and W^T), the tensor core reading either layout; what a box holds
+// beyond the operand's edge the copy fills with zeros, so any M, N and K run
+// here as long as the row strides are multiples of 16 bytes (the widths are
+// multiples of 8; dL/dz of the last layer is kept at a padded stride).
+//
+// Persistent CTAs of 320 threads, two per SM, walk the 128 x BN output tiles
+// (n fastest: neighbours share the rows of A in L2).  K runs in blocks of 64
+// through ST shared-memory stages of one ring that goes on from tile to
+// tile.  Warp 8's lane 0 issues the bulk tensor copies of a stage, 128-byte
+// swizzled, and arms the stage's "full" mbarrier with their byte count; warp
+// 9's lane 0 waits for it, issues the block's four tcgen05.mma into one of
+// two accumulators in tensor memory and commits them to the stage's "empty"
+// mbarrier, the tile's last block also to the accumulator's "tfull"; warps
+// 0-7 read that accumulator back (tcgen05.ld; warp w: TMEM lanes 32 (w % 4),
+// half of the columns), hand it back through "tempty" and apply the epilogue
+// while the other accumulator fills.  The epilogue is what bounds the wide
+// layers (erff on every output costs about as much issue time as the MMAs
+// take), hence the second accumulator.  Every sum runs over K in the same order at each
+// BN, so the tile width does not change a result.
+// BN: 16 where N <= 16 (the output layer: an eighth of the columns of a 128
+// tile would be in use), 64 where 128-wide tiles would leave CTAs of the
+// chip without one (a training batch), else 128.  Against one tile per CTA with
+// the epilogue after its MMAs, and threads staging the operands of the 13
+// outputs (896-1024-1024-512-13): 16,384 rows forward 59 / 62 / 35 / 31 us
+// per layer -> 42 / 45 / 30 / 9; of a batch of 1,024, the output layer 30 -> 8,
+// its dW 102 -> 10 and dX 39 -> 8, the others 12-18 -> 9-13.  At 16,384 rows
+// the tensor pipe is then busy 40 %, the issue slots 53 %: neither full, the
+// rest is the L2's latency against 192 KB of tiles in flight per SM.
+// Every wait is bounded (2 s): one that runs out sets the error flag and the
+// CTA frees its tensor memory.
+constexpr int TM_BM = 128, TM_BK = 64;
+constexpr int TM_TILE_A = TM_BM * TM_BK * 2;
+constexpr int TM_EPI_WARPS = 8, TM_THREADS = (TM_EPI_WARPS + 2) * 32;
 constexpr unsigned long long TC_WAIT_NS = 2000000000ull;
+__host__ __device__ constexpr int tm_tile_b(int bn) { return bn * TM_BK * 2; }
+__host__ __device__ constexpr int tm_stages(int bn) { return bn == 128 ? 3 : bn == 64 ? 4 : 5; }
+__host__ __device__ constexpr int tm_smem(int bn) {   // + the 1 KB alignment
+  return tm_stages(bn) * (TM_TILE_A + tm_tile_b(bn)) + 1024;
+}
 
-// Rows [row0, row0 + 128) x K [k0, k0 + 64) of a logical operand X (R x K)
-// stored K-contiguous (X[r * ld + k], kcont) or row-contiguous (X[k * ld +
-// r]) into the K-major tile dst; out-of-range elements are zero.
-__device__ __forceinline__ void tc_stage(const __nv_bfloat16* __restrict__ X, int ld, bool kcont, bool vec, int row0,
-                                         int k0, int R, int K, unsigned char* dst) {
-  const unsigned short* x = reinterpret_cast<const unsigned short*>(X);
-  if (kcont) {
-    for (int i = threadIdx.x; i < 128 * (TC_BK / 8); i += blockDim.x) {
-      const int r = i / (TC_BK / 8), c = i % (TC_BK / 8);
-      const int gr = row0 + r, gk = k0 + 8 * c;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (gr < R) {
-        const unsigned short* src = x + (size_t)gr * ld + gk;
-        if (vec && gk + 8 <= K) {
-          v = *reinterpret_cast<const uint4*>(src);
-        } else {
-          unsigned short e[8];
+// 16 columns nb.. of row m of the accumulator through the epilogue; vec: the
+// row stride and the bases allow 16-byte accesses.
+template <int EPI>
+__device__ __forceinline__ void epi_cols(float v[16], size_t o, int nb, int N, bool vec,
+                                         const float* __restrict__ bias, const float* __restrict__ zin,
+                                         float* __restrict__ zout, float* __restrict__ fout,
+                                         __nv_bfloat16* __restrict__ out) {
+  if (vec && nb + 16 <= N) {
+    if (EPI == EPI_FWD_GELU || EPI == EPI_FWD_LIN)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) e[j] = gk + j < K ? src[j] : (unsigned short)0;
-          v = make_uint4(e[0] | ((unsigned)e[1] << 16), e[2] | ((unsigned)e[3] << 16), e[4] | ((unsigned)e[5] << 16),
-                         e[6] | ((unsigned)e[7] << 16));
-        }
+      for (int i = 0; i < 16; i += 4) {
+        const float4 b = __ldg(reinterpret_cast<const float4*>(bias + nb + i));
+        v[i] += b.x;
+        v[i + 1] += b.y;
+        v[i + 2] += b.z;
+        v[i + 3] += b.w;
       }
-      *reinterpret_cast<uint4*>(dst + fztc::kmajor_offset(r, 8 * c, TC_NKC)) = v;
+    if (EPI == EPI_BWD_GELU || EPI == EPI_FWD_GELU) {
+      if (EPI == EPI_FWD_GELU && zout)
+#pragma unroll
+        for (int i = 0; i < 16; i += 4)
+          *reinterpret_cast<float4*>(zout + o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      if (EPI == EPI_BWD_GELU)
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+          const float4 z = __ldg(reinterpret_cast<const float4*>(zin + o + i));
+          v[i] *= gelu_d(z.x);
+          v[i + 1] *= gelu_d(z.y);
+          v[i + 2] *= gelu_d(z.z);
+          v[i + 3] *= gelu_d(z.w);
+        }
+      uint32_t h[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const __nv_bfloat162 t = EPI == EPI_FWD_GELU ? __floats2bfloat162_rn(gelu(v[2 * i]), gelu(v[2 * i + 1]))
+                                                     : __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        h[i] = *reinterpret_cast<const uint32_t*>(&t);
+      }
+      *reinterpret_cast<uint4*>(out + o) = make_uint4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<uint4*>(out + o + 8) = make_uint4(h[4], h[5], h[6], h[7]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4)
+        *reinterpret_cast<float4*>(fout + o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
     }
-  } else {
-    for (int i = threadIdx.x; i < TC_BK * 16; i += blockDim.x) {
-      const int kk = i / 16, c = i % 16;   // eight consecutive rows 8c.. at one k
-      const int gk = k0 + kk, gr = row0 + 8 * c;
-      unsigned short e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (gk < K) {
-        const unsigned short* src = x + (size_t)gk * ld + gr;
-        if (vec && gr + 8 <= R) {
-          const uint4 v = *reinterpret_cast<const uint4*>(src);
-          e[0] = v.x & 0xffff; e[1] = v.x >> 16; e[2] = v.y & 0xffff; e[3] = v.y >> 16;
-          e[4] = v.z & 0xffff; e[5] = v.z >> 16; e[6] = v.w & 0xffff; e[7] = v.w >> 16;
-        } else {
+    return;
+  }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) e[j] = gr + j < R ? src[j] : (unsigned short)0;
-        }
+  for (int i = 0; i < 16; ++i) {
+    const int n = nb + i;
+    if (n >= N) continue;
+    if (EPI == EPI_BWD_GELU) {
+      out[o + i] = __float2bfloat16_rn(v[i] * gelu_d(zin[o + i]));
+    } else if (EPI == EPI_F32) {
+      fout[o + i] = v[i];
+    } else {
+      const float z = v[i] + bias[n];
+      if (EPI == EPI_FWD_GELU) {
+        if (zout) zout[o + i] = z;
+        out[o + i] = __float2bfloat16_rn(gelu(z));
+      } else {
+        fout[o + i] = z;
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        *reinterpret_cast<unsigned short*>(dst + fztc::kmajor_offset(8 * c + j, kk, TC_NKC)) = e[j];
     }
   }
 }
 
-template <int MODE, int EPI>
-__global__ void __launch_bounds__(256, 1) k_gemm_tc(int M, int N, int K, const __nv_bfloat16* __restrict__ A, int lda,
-                                                    const __nv_bfloat16* __restrict__ B, int ldb,
-                                                    const float* __restrict__ bias, const float* __restrict__ zin,
-                                                    float* __restrict__ zout, float* __restrict__ fout,
-                                                    __nv_bfloat16* __restrict__ out, int ldc, int* __restrict__ err) {
-  extern __shared__ __align__(1024) unsigned char tsm[];
-  __shared__ __align__(8) uint64_t mbar[TC_STAGES];
-  __shared__ uint32_t tbase;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * 128, n0 = blockIdx.x * 128;
-  // A: NT, NN K-contiguous rows of a (M x K); TN the transpose.  B: NT
-  // K-contiguous rows of b (N x K); NN, TN the transpose.
-  const bool akc = MODE != TN, bkc = MODE == NT;
-  const bool avec = (lda % 8) == 0 && (((uintptr_t)A) & 15) == 0;
-  const bool bvec = (ldb % 8) == 0 && (((uintptr_t)B) & 15) == 0;
-  if (warp == 0) {
-    fztc::tmem_alloc(&tbase, 128);
-    fztc::tmem_relinquish();
-  }
-  if (tid == 0) {
-    for (int i = 0; i < TC_STAGES; ++i) fztc::mbar_init(&mbar[i], 1);
-    fztc::fence_mbar_init();
-  }
-  fztc::fence_before_sync();
-  __syncthreads();
-  fztc::fence_after_sync();
-  const uint32_t tmem = tbase;
-  const uint32_t idesc = fztc::idesc_bf16(128, 128);
-  const int nkb = (K + TC_BK - 1) / TC_BK;
-  bool ok = true;
-  for (int kb = 0; kb < nkb && ok; ++kb) {
-    const int buf = kb % TC_STAGES;
-    unsigned char* as = tsm + (size_t)buf * 2 * TC_TILE;
-    unsigned char* bs = as + TC_TILE;
-    if (kb >= TC_STAGES) ok = fztc::mbar_wait(&mbar[buf], ((kb - TC_STAGES) / TC_STAGES) & 1, TC_WAIT_NS);
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    tc_stage(A, lda, akc, avec, m0, kb * TC_BK, M, K, as);
-    tc_stage(B, ldb, bkc, bvec, n0, kb * TC_BK, N, K, bs);
-    fztc::fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      const uint32_t sa = fztc::smem_addr(as), sb = fztc::smem_addr(bs);
-#pragma unroll
-      for (int ks = 0; ks < TC_BK / 16; ++ks) {
-        const uint64_t da = fztc::desc_kmajor(sa + ks * 256, 128, TC_NKC * 128);
-        const uint64_t db = fztc::desc_kmajor(sb + ks * 256, 128, TC_NKC * 128);
-        fztc::mma_bf16(tmem, da, db, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
-      }
-      fztc::commit(&mbar[buf]);
-    }
-  }
-  if (ok && nkb > 0) {
-    const int last = nkb - 1;
-    ok = fztc::mbar_wait(&mbar[last % TC_STAGES], (last / TC_STAGES) & 1, TC_WAIT_NS);
-  }
-  ok = __syncthreads_and(ok);
-  fztc::fence_after_sync();
-  if (ok) {
-    const int q = warp & 3, half = warp >> 2;
-    const int m = m0 + 32 * q + lane;
-#pragma unroll 1
-    for (int cc = 0; cc < 64; cc += 16) {
-      float v[16];
-      fztc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * half + cc), v);
-      if (m >= M) continue;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int n = n0 + 64 * half + cc + i;
-        if (n >= N) continue;
-        const float c = v[i];
-        const size_t o = (size_t)m * ldc + n;
-        if (EPI == EPI_FWD_GELU) {
-          const float z = c + bias[n];
-          if (zout) zout[o] = z;
-          out[o] = __float2bfloat16_rn(gelu(z));
-        } else if (EPI == EPI_FWD_LIN) {
-          fout[o] = c + bias[n];
-        } else if (EPI == EPI_BWD_GELU) {
-          out[o] = __float2bfloat16_rn(c * gelu_d(zin[o]));
-        } else {
-          fout[o] = c;
-        }
-      }
-    }
-  } else if (tid == 0) {
-    atomicExch(err, 1);
-  }
-  fztc::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) fztc::tmem_dealloc(tmem, 128);
-}
-
-// The GEMMs whose bf16 operands sit in device memory with a 16-byte row
-// stride, fed by the tensor memory accelerator: a 128 x 128 output tile per
-// CTA of 256 threads, two CTAs per SM, K in blocks of 64 through three
-// shared-memory stages.  An operand is K-major (AMN / BMN false: K
-// contiguous, the forward's X and W) or MN-major (true: MN contiguous, the
-// backward's dZ^T, X^T and W^T), the tensor core reading either layout.
-// Warp 0's lane 0 issues the bulk tensor copies of A (128 x 64) and B
-// (128 x 64) into a stage, 128-byte swizzled, and arms the stage's "full"
-// mbarrier with their byte count; warp 1's lane 0 waits for it, issues the
-// four tcgen05.mma of the block (FP32 accumulator in 128 TMEM columns) and
-// commits them to the stage's "empty" mbarrier, which hands the stage back
-// to the copies; the last commit arrives on "done".  Then all eight warps
-// read the accumulator back (tcgen05.ld; warp w: TMEM lanes 32 (w % 4), 64
-// columns from 64 (w / 4)) and apply the epilogue, 16-byte stores where the
-// row stride allows.  Every wait is bounded (2 s): one that runs out sets
-// the error flag and the CTA frees its tensor memory.
-constexpr int TM_BM = 128, TM_BN = 128, TM_BK = 64, TM_ST = 3;
-constexpr int TM_TILE_A = TM_BM * TM_BK * 2, TM_TILE_B = TM_BN * TM_BK * 2;   // 16 KB each
-constexpr size_t TM_SMEM = (size_t)TM_ST * (TM_TILE_A + TM_TILE_B) + 1024;    // + the 1 KB alignment
-
-template <int EPI, bool AMN, bool BMN>
-__global__ void __launch_bounds__(256, 2) k_gemm_tma(const __grid_constant__ CUtensorMap ta,
-                                                     const __grid_constant__ CUtensorMap tb, int M, int N, int K,
-                                                     const float* __restrict__ bias, const float* __restrict__ zin,
-                                                     float* __restrict__ zout, float* __restrict__ fout,
-                                                     __nv_bfloat16* __restrict__ out, int ldc,
-                                                     int* __restrict__ err) {
+template <int EPI, bool AMN, bool BMN, int BN>
+__global__ void __launch_bounds__(TM_THREADS, 2)
+    k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int M, int N, int K,
+           const float* __restrict__ bias, const float* __restrict__ zin, float* __restrict__ zout,
+           float* __restrict__ fout, __nv_bfloat16* __restrict__ out, int ldc, int* __restrict__ err) {
+  static_assert(!BMN || BN >= 64, "an MN-major box is 64 wide");
+  constexpr int ST = tm_stages(BN), TILE_B = tm_tile_b(BN), STAGE = TM_TILE_A + TILE_B;
+  constexpr uint32_t TCOLS = 2 * BN;   // two accumulators: 256, 128 or 32 columns
   extern __shared__ unsigned char tm_raw[];
-  __shared__ __align__(8) uint64_t full[TM_ST], empty[TM_ST], done;
+  __shared__ __align__(8) uint64_t full[ST], empty[ST], tfull[2], tempty[2];
   __shared__ uint32_t tbase;
   __shared__ int bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * TM_BM, n0 = blockIdx.x * TM_BN;
   // the swizzled tiles start on a 1 KB boundary
   const uint32_t raw = fztc::smem_addr(tm_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* tiles = tm_raw + (base - raw);
   if (warp == 0) {
-    fztc::tmem_alloc(&tbase, TM_BN);
+    fztc::tmem_alloc(&tbase, TCOLS);
     fztc::tmem_relinquish();
   }
-  if (tid == 0) {
-    for (int i = 0; i < TM_ST; ++i) {
+  if (tid == TM_EPI_WARPS * 32) {
+    fztc::tma_prefetch(&ta);
+    fztc::tma_prefetch(&tb);
+    for (int i = 0; i < ST; ++i) {
       fztc::mbar_init(&full[i], 1);
       fztc::mbar_init(&empty[i], 1);
     }
-    fztc::mbar_init(&done, 1);
+    for (int i = 0; i < 2; ++i) {
+      fztc::mbar_init(&tfull[i], 1);
+      fztc::mbar_init(&tempty[i], TM_EPI_WARPS);
+    }
     bad = 0;
     fztc::fence_mbar_init();
   }
@@ -254,132 +194,117 @@ __global__ void __launch_bounds__(256, 2) k_gemm_tma(const __grid_constant__ CUt
   fztc::fence_after_sync();
   const uint32_t tmem = tbase;
   const int nkb = (K + TM_BK - 1) / TM_BK;
-  if (warp == 0) {
+  const int ntn = (N + BN - 1) / BN, tiles_mn = ntn * ((M + TM_BM - 1) / TM_BM);
+  if (warp == TM_EPI_WARPS) {
     if (lane == 0) {
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int st = kb % TM_ST;
-        // the stage's previous use (block kb - TM_ST) must have been consumed
-        if (kb >= TM_ST && !fztc::mbar_wait(&empty[st], ((kb / TM_ST) - 1) & 1, TC_WAIT_NS)) {
-          atomicExch(&bad, 1);
-          break;
-        }
-        unsigned char* sa = tiles + (size_t)st * (TM_TILE_A + TM_TILE_B);
-        unsigned char* sb = sa + TM_TILE_A;
-        fztc::mbar_arrive_expect_tx(&full[st], TM_TILE_A + TM_TILE_B);
-        // K-major: one 64 (K) x 128 box; MN-major: two 64 (MN) x 64 (K)
-        // boxes, the second 64 MN elements 8 KB on
-        if (AMN) {
-          fztc::tma_load_2d(sa, &ta, m0, kb * TM_BK, &full[st]);
-          fztc::tma_load_2d(sa + TM_TILE_A / 2, &ta, m0 + 64, kb * TM_BK, &full[st]);
-        } else {
-          fztc::tma_load_2d(sa, &ta, kb * TM_BK, m0, &full[st]);
-        }
-        if (BMN) {
-          fztc::tma_load_2d(sb, &tb, n0, kb * TM_BK, &full[st]);
-          fztc::tma_load_2d(sb + TM_TILE_B / 2, &tb, n0 + 64, kb * TM_BK, &full[st]);
-        } else {
-          fztc::tma_load_2d(sb, &tb, kb * TM_BK, n0, &full[st]);
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = fztc::idesc_bf16_major(TM_BM, TM_BN, AMN, BMN);
-      int kb = 0;
-      for (; kb < nkb; ++kb) {
-        const int st = kb % TM_ST;
-        if (!fztc::mbar_wait(&full[st], (kb / TM_ST) & 1, TC_WAIT_NS)) {
-          atomicExch(&bad, 1);
-          break;
-        }
-        fztc::fence_after_sync();
-        const uint32_t sa = base + (uint32_t)st * (TM_TILE_A + TM_TILE_B), sb = sa + TM_TILE_A;
-#pragma unroll
-        for (int ks = 0; ks < TM_BK / 16; ++ks) {
-          const uint64_t da = AMN ? fztc::desc_sw128_mn(sa + 2048 * ks, TM_TILE_A / 2) : fztc::desc_sw128(sa + 32 * ks);
-          const uint64_t db = BMN ? fztc::desc_sw128_mn(sb + 2048 * ks, TM_TILE_B / 2) : fztc::desc_sw128(sb + 32 * ks);
-          fztc::mma_bf16(tmem, da, db, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
-        }
-        fztc::commit(&empty[st]);
-      }
-      if (kb == nkb) fztc::commit(&done);
-    }
-    __syncwarp();
-  }
-  bool ok = fztc::mbar_wait(&done, 0, TC_WAIT_NS);
-  ok = __syncthreads_and(ok) && !*(volatile int*)&bad;
-  fztc::fence_after_sync();
-  if (ok) {
-    const int q = warp & 3, half = warp >> 2;
-    const int m = m0 + 32 * q + lane;
-    const bool vec = (ldc & 7) == 0;
-#pragma unroll 1
-    for (int cc = 0; cc < 64; cc += 16) {
-      float v[16];
-      fztc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * half + cc), v);
-      if (m >= M) continue;
-      const int nb = n0 + 64 * half + cc;
-      const size_t o = (size_t)m * ldc + nb;
-      if (vec && nb + 16 <= N) {
-        if (EPI == EPI_FWD_GELU || EPI == EPI_FWD_LIN)
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] += __ldg(&bias[nb + i]);
-        if (EPI == EPI_BWD_GELU) {
-          uint32_t h[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float2 z = __ldg(reinterpret_cast<const float2*>(zin + o) + i);
-            const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i] * gelu_d(z.x), v[2 * i + 1] * gelu_d(z.y));
-            h[i] = *reinterpret_cast<const uint32_t*>(&t);
+      int st = 0;
+      uint32_t round = 0;   // of the ring; a stage's use of round r frees on its "empty" phase r
+      bool ok = true;
+      for (int t = blockIdx.x; t < tiles_mn && ok; t += gridDim.x) {
+        const int m0 = (t / ntn) * TM_BM, n0 = (t % ntn) * BN;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (round > 0 && !fztc::mbar_wait(&empty[st], (round - 1) & 1, TC_WAIT_NS)) {
+            ok = false;
+            break;
           }
-          *reinterpret_cast<uint4*>(out + o) = make_uint4(h[0], h[1], h[2], h[3]);
-          *reinterpret_cast<uint4*>(out + o + 8) = make_uint4(h[4], h[5], h[6], h[7]);
-        } else if (EPI == EPI_FWD_GELU) {
-          if (zout)
-#pragma unroll
-            for (int i = 0; i < 16; i += 4)
-              *reinterpret_cast<float4*>(zout + o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-          uint32_t h[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const __nv_bfloat162 t = __floats2bfloat162_rn(gelu(v[2 * i]), gelu(v[2 * i + 1]));
-            h[i] = *reinterpret_cast<const uint32_t*>(&t);
-          }
-          *reinterpret_cast<uint4*>(out + o) = make_uint4(h[0], h[1], h[2], h[3]);
-          *reinterpret_cast<uint4*>(out + o + 8) = make_uint4(h[4], h[5], h[6], h[7]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; i += 4)
-            *reinterpret_cast<float4*>(fout + o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int n = nb + i;
-          if (n >= N) continue;
-          if (EPI == EPI_BWD_GELU) {
-            out[o + i] = __float2bfloat16_rn(v[i] * gelu_d(zin[o + i]));
-          } else if (EPI == EPI_F32) {
-            fout[o + i] = v[i];
+          unsigned char* sa = tiles + (size_t)st * STAGE;
+          unsigned char* sb = sa + TM_TILE_A;
+          fztc::mbar_arrive_expect_tx(&full[st], STAGE);
+          // K-major: one 64 (K) x rows box; MN-major: 64 (MN) x 64 (K)
+          // boxes, the next 64 MN elements 8 KB on
+          if (AMN) {
+            fztc::tma_load_2d(sa, &ta, m0, kb * TM_BK, &full[st]);
+            fztc::tma_load_2d(sa + TM_TILE_A / 2, &ta, m0 + 64, kb * TM_BK, &full[st]);
           } else {
-            const float z = v[i] + bias[n];
-            if (EPI == EPI_FWD_GELU) {
-              if (zout) zout[o + i] = z;
-              out[o + i] = __float2bfloat16_rn(gelu(z));
-            } else {
-              fout[o + i] = z;
-            }
+            fztc::tma_load_2d(sa, &ta, kb * TM_BK, m0, &full[st]);
+          }
+          if (BMN) {
+            fztc::tma_load_2d(sb, &tb, n0, kb * TM_BK, &full[st]);
+            if (BN == 128) fztc::tma_load_2d(sb + TILE_B / 2, &tb, n0 + 64, kb * TM_BK, &full[st]);
+          } else {
+            fztc::tma_load_2d(sb, &tb, kb * TM_BK, n0, &full[st]);
+          }
+          if (++st == ST) {
+            st = 0;
+            ++round;
           }
         }
       }
+      if (!ok) {   // the copies in flight: the ST uses before this one
+        atomicExch(&bad, 1);
+        for (int i = 0; i < ST; ++i) fztc::mbar_wait(&full[i], (i < st ? round : round - 1) & 1, TC_WAIT_NS);
+      }
     }
-  } else if (tid == 0) {
-    atomicExch(err, 1);
+    __syncwarp();
+  } else if (warp == TM_EPI_WARPS + 1) {
+    if (lane == 0) {
+      const uint32_t idesc = fztc::idesc_bf16_major(TM_BM, BN, AMN, BMN);
+      int st = 0, i = 0;
+      uint32_t round = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < tiles_mn && ok; t += gridDim.x, ++i) {
+        const uint32_t acc = tmem + (uint32_t)((i & 1) * BN);
+        if (i >= 2) {   // the accumulator's tile i - 2 has been read
+          ok = fztc::mbar_wait(&tempty[i & 1], ((i >> 1) - 1) & 1, TC_WAIT_NS);
+          if (!ok) break;
+          fztc::fence_after_sync();
+        }
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!fztc::mbar_wait(&full[st], round & 1, TC_WAIT_NS)) {
+            ok = false;
+            break;
+          }
+          fztc::fence_after_sync();
+          const uint32_t sa = base + (uint32_t)st * STAGE, sb = sa + TM_TILE_A;
+#pragma unroll
+          for (int ks = 0; ks < TM_BK / 16; ++ks) {
+            const uint64_t da =
+                AMN ? fztc::desc_sw128_mn(sa + 2048 * ks, TM_TILE_A / 2) : fztc::desc_sw128(sa + 32 * ks);
+            const uint64_t db = BMN ? fztc::desc_sw128_mn(sb + 2048 * ks, TILE_B / 2) : fztc::desc_sw128(sb + 32 * ks);
+            fztc::mma_bf16(acc, da, db, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+          }
+          fztc::commit(&empty[st]);
+          if (++st == ST) {
+            st = 0;
+            ++round;
+          }
+        }
+        if (ok) fztc::commit(&tfull[i & 1]);
+      }
+      if (!ok) atomicExch(&bad, 1);
+    }
+    __syncwarp();
+  } else {
+    constexpr int COLS = BN >= 32 ? BN / 2 : BN;   // per warp; at BN = 16 warps 4-7 only hand back
+    const int q = warp & 3, half = warp >> 2;
+    const bool mine = half * COLS < BN;
+    const bool vec = (ldc & 7) == 0 && (((uintptr_t)fout | (uintptr_t)zout | (uintptr_t)out | (uintptr_t)zin) & 15) == 0;
+    int i = 0;
+    for (int t = blockIdx.x; t < tiles_mn; t += gridDim.x, ++i) {
+      const int m = (t / ntn) * TM_BM + 32 * q + lane, n0 = (t % ntn) * BN + half * COLS;
+      if (!fztc::mbar_wait(&tfull[i & 1], (i >> 1) & 1, TC_WAIT_NS)) {
+        atomicExch(&bad, 1);
+        break;
+      }
+      fztc::fence_after_sync();
+      const uint32_t acc = tmem + (uint32_t)((i & 1) * BN) + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * COLS);
+#pragma unroll 1
+      for (int cc = 0; cc < COLS && mine; cc += 16) {
+        float v[16];
+        __syncwarp();
+        fztc::tmem_ld16(acc + (uint32_t)cc, v);
+        if (m < M && n0 + cc < N)
+          epi_cols<EPI>(v, (size_t)m * ldc + n0 + cc, n0 + cc, N, vec, bias, zin, zout, fout, out);
+      }
+      __syncwarp();
+      fztc::fence_before_sync();
+      if (lane == 0) fztc::mbar_arrive(&tempty[i & 1]);
+    }
   }
   fztc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) fztc::tmem_dealloc(tmem, TM_BN);
+  if (tid == 0 && *(volatile int*)&bad) atomicExch(err, 1);
+  if (warp == 0) fztc::tmem_dealloc(tmem, TCOLS);
 }
 
 // Training-step state on the device, so that one captured step replays for
@@ -395,9 +320,9 @@ __device__ __forceinline__ size_t batch_row(const int* order, const TrainState* 
 }
 
 // MSE loss 1/(n*nout) sum lw_j (y - t)^2 (lw: per-output weights, null =
-// all 1) and dL/dy in bf16
+// all 1) and dL/dy in bf16, rows at stride ldd
 __global__ void k_mse(int n, int nout, const float* __restrict__ y, const float* __restrict__ t,
-                      __nv_bfloat16* __restrict__ dy, float* __restrict__ loss, const int* __restrict__ order,
+                      __nv_bfloat16* __restrict__ dy, int ldd, float* __restrict__ loss, const int* __restrict__ order,
                       const TrainState* __restrict__ st, const float* __restrict__ lw = nullptr) {
   __shared__ float red[8];
   t += batch_row(order, st, n) * nout;
@@ -408,7 +333,7 @@ __global__ void k_mse(int n, int nout, const float* __restrict__ y, const float*
     const float d = y[i] - t[i];
     const float wd = lw ? lw[i % nout] * d : d;
     s += wd * d;
-    dy[i] = __float2bfloat16_rn(sc * wd);
+    dy[i / nout * ldd + i % nout] = __float2bfloat16_rn(sc * wd);
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -420,18 +345,76 @@ __global__ void k_mse(int n, int nout, const float* __restrict__ y, const float*
   }
 }
 
-// bias gradient: column sums of dZ (bf16, n x m)
-__global__ void k_colsum(int n, int m, const __nv_bfloat16* __restrict__ dz, float* __restrict__ db) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
+// bias gradient: column sums of dZ (bf16, n x m at row stride ld, a multiple
+// of 8), each in row order.  A block of 128 threads takes 32 columns: tiles
+// of CS_ROWS rows stream into two shared-memory buffers (16-byte async
+// copies) while the first warp adds the previous tile, a lane per column.
+// The sum is one chain of FP32 additions (n x 4 cycles: 2.2 us at 1024
+// rows), which the copies keep fed; reading the rows straight from memory
+// the chain waited for every load (67 us at 1024 x 1024, now 8).  With `st` (the
+// last layer's sums of a training step) it also advances the step state:
+// after the loss has read the batch's position and before any Adam update.
+constexpr int CS_COLS = 32, CS_ROWS = 256;
+__global__ void __launch_bounds__(128) k_colsum(int n, int m, const __nv_bfloat16* __restrict__ dz, int ld,
+                                                float* __restrict__ db, TrainState* __restrict__ st) {
+  __shared__ __align__(16) __nv_bfloat16 buf[2][CS_ROWS][CS_COLS];
+  const int tid = threadIdx.x, c0 = blockIdx.x * CS_COLS;
+  if (st && blockIdx.x == 0 && tid == 0) {
+    st->bi += 1;
+    st->step += 1;
+  }
+  auto fetch = [&](int r0, int b) {
+    for (int i = tid; i < CS_ROWS * (CS_COLS / 8); i += 128) {
+      const int r = i / (CS_COLS / 8), c = 8 * (i % (CS_COLS / 8));
+      if (r0 + r < n && c0 + c < ld)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(fztc::smem_addr(&buf[b][r][c])),
+                     "l"(dz + (size_t)(r0 + r) * ld + c0 + c)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
   float s = 0.0f;
-  for (int i = 0; i < n; ++i) s += __bfloat162float(dz[(size_t)i * m + j]);
-  db[j] = s;
+  fetch(0, 0);
+  for (int r0 = 0, b = 0; r0 < n; r0 += CS_ROWS, b ^= 1) {
+    fetch(r0 + CS_ROWS, b ^ 1);   // empty past the last row
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    if (tid < 32) {
+      const int nr = min(CS_ROWS, n - r0);
+#pragma unroll 16
+      for (int r = 0; r < nr; ++r) s += __bfloat162float(buf[b][r][tid]);
+    }
+    __syncthreads();
+  }
+  if (tid < 32 && c0 + tid < m) db[c0 + tid] = s;
 }
 
-__global__ void k_to_bf16(size_t n, const float* __restrict__ x, __nv_bfloat16* __restrict__ y) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = __float2bfloat16_rn(x[i]);
+// Eight FP32 values at x (vec: 16-byte aligned) as bf16 in one 16-byte word.
+__device__ __forceinline__ uint4 pack8(const float* __restrict__ x, bool vec) {
+  float v[8];
+  if (vec) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(x)), b = __ldg(reinterpret_cast<const float4*>(x) + 1);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = x[i];
+  }
+  uint32_t h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    h[i] = *reinterpret_cast<const uint32_t*>(&t);
+  }
+  return make_uint4(h[0], h[1], h[2], h[3]);
+}
+
+// x (n8 groups of eight FP32 values) as bf16; y is 16-byte aligned.  Bound by
+// its 6 bytes per value: a thread moves 32 bytes in, 16 out (14.7 M values:
+// 28 -> 14 us against one value at a time).
+__global__ void k_to_bf16(size_t n8, const float* __restrict__ x, __nv_bfloat16* __restrict__ y) {
+  const bool vec = ((uintptr_t)x & 15) == 0;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x)
+    reinterpret_cast<uint4*>(y)[i] = pack8(x + 8 * i, vec);
 }
 
 // Observed Stokes rows (n x d, FP64, GAIN-normalised) standardised with the
@@ -444,37 +427,62 @@ __global__ void k_obs_bf16(size_t n, int d, const double* __restrict__ x, const 
   }
 }
 
-// the current batch's rows (n x d) of x as bf16
+// the current batch's rows (n x d, d a multiple of 8) of x as bf16
 __global__ void k_batch_bf16(int n, int d, const float* __restrict__ x, const int* __restrict__ order,
                              const TrainState* __restrict__ st, __nv_bfloat16* __restrict__ y) {
   x += batch_row(order, st, n) * d;
-  const size_t total = (size_t)n * d;
+  const bool vec = ((uintptr_t)x & 15) == 0;
+  const size_t total = (size_t)n * d / 8;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = __float2bfloat16_rn(x[i]);
+    reinterpret_cast<uint4*>(y)[i] = pack8(x + 8 * i, vec);
 }
 
-__global__ void k_train_advance(TrainState* st) {
-  st->bi += 1;
-  st->step += 1;
+// Adam (Kingma & Ba 2015) of one value: FP32 master w, moments m1, m2
+struct AdamK {
+  float lr, b1, b2, eps;
+};
+__device__ __forceinline__ void adam1(const AdamK& k, float c1, float c2, float gi, float& w, float& m1, float& m2) {
+  const float a = k.b1 * m1 + (1.0f - k.b1) * gi;
+  const float b = k.b2 * m2 + (1.0f - k.b2) * gi * gi;
+  m1 = a;
+  m2 = b;
+  w = w - k.lr * (a * c1) / (sqrtf(b * c2) + k.eps);
 }
 
-// Adam (Kingma & Ba 2015) on FP32 masters, refreshing the bf16 copy; the
-// bias corrections 1/(1 - b^t) of step t = st->step + 1
-__global__ void k_adam(size_t n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
-                       float* __restrict__ m2, __nv_bfloat16* __restrict__ wb, float lr, float b1, float b2,
-                       const TrainState* __restrict__ st, float eps) {
-  const float t = (float)(st->step + 1);
-  const float c1 = 1.0f / (1.0f - powf(b1, t)), c2 = 1.0f / (1.0f - powf(b2, t));
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float a = b1 * m1[i] + (1.0f - b1) * gi;
-    const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    const float wi = w[i] - lr * (a * c1) / (sqrtf(b * c2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16_rn(wi);
+// Adam of one layer's weights (n4 groups of four) and biases (nb), the bf16
+// copy of the weights refreshed; the bias corrections 1/(1 - b^t) of step
+// t = st->step (already advanced).  Bound by its 30 bytes per weight; the
+// two powers per thread are paid once for four weights and the biases need
+// no launch of their own (eight launches, 49 us -> four, 26 us, for 2.5 M
+// parameters).
+struct AdamP {
+  size_t n4;
+  int nb;
+  float *w, *m, *v, *b, *mb, *vb;
+  const float *g, *gb;
+  __nv_bfloat16* wb;
+};
+__global__ void __launch_bounds__(256) k_adam(AdamP p, AdamK k, const TrainState* __restrict__ st) {
+  const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const float t = (float)st->step;
+  const float c1 = 1.0f / (1.0f - powf(k.b1, t)), c2 = 1.0f / (1.0f - powf(k.b2, t));
+  for (size_t i = i0; i < p.n4; i += (size_t)gridDim.x * blockDim.x) {
+    const float4 g = __ldg(reinterpret_cast<const float4*>(p.g) + i);
+    float4 w = reinterpret_cast<float4*>(p.w)[i], m = reinterpret_cast<float4*>(p.m)[i],
+           v = reinterpret_cast<float4*>(p.v)[i];
+    adam1(k, c1, c2, g.x, w.x, m.x, v.x);
+    adam1(k, c1, c2, g.y, w.y, m.y, v.y);
+    adam1(k, c1, c2, g.z, w.z, m.z, v.z);
+    adam1(k, c1, c2, g.w, w.w, m.w, v.w);
+    reinterpret_cast<float4*>(p.w)[i] = w;
+    reinterpret_cast<float4*>(p.m)[i] = m;
+    reinterpret_cast<float4*>(p.v)[i] = v;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(w.x, w.y), hi = __floats2bfloat162_rn(w.z, w.w);
+    reinterpret_cast<uint2*>(p.wb)[i] =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
   }
+  for (size_t i = i0; i < (size_t)p.nb; i += (size_t)gridDim.x * blockDim.x)
+    adam1(k, c1, c2, p.gb[i], p.b[i], p.mb[i], p.vb[i]);
 }
 
 // deterministic initial weights: uniform(-1,1)*sqrt(6/(fan_in+fan_out)) from a
@@ -504,15 +512,20 @@ struct fz_mlp {
   int cap = 0;
   __nv_bfloat16* act[MLP_MAXL + 1] = {};   // act[0] = input (bf16), act[l] = gelu(z_l)
   float* z[MLP_MAXL] = {};                 // pre-activations
-  float* yout = nullptr;                    // last layer output (fp32)
-  __nv_bfloat16* dz[MLP_MAXL] = {};        // dL/dz per layer
+  float* yout = nullptr;                    // last layer output (fp32), for the loss
+  __nv_bfloat16* dz[MLP_MAXL] = {};        // dL/dz per layer, rows at stride ldz
   float* loss = nullptr;
   long long step = 0;
   cudaStream_t stream = nullptr;
+  // the backward pass's branches: weight gradients and bias sums beside the
+  // chain of dL/dz
+  cudaStream_t sw = nullptr, sb = nullptr;
+  cudaEvent_t ez[MLP_MAXL] = {}, eb[MLP_MAXL] = {}, ew = nullptr;
   TrainState* tstate = nullptr;   // device
   int* order = nullptr;           // device batch order of one epoch
   int order_cap = 0;
   int* d_err = nullptr;           // set by a tensor-core GEMM that gave up waiting for its MMAs
+  int nsm = 148;
   float* d_lw = nullptr;          // per-output loss weights (null: all 1)
 };
 
@@ -531,6 +544,10 @@ int mlp_fail(cudaError_t e) {
     if (_rc) return _rc;          \
   } while (0)
 
+// Row stride of dL/dz: 16-byte rows for the tensor maps (the hidden widths
+// are multiples of 8 already).
+int ldz(const fz_mlp* p, int l) { return (p->dim[l + 1] + 7) & ~7; }
+
 int grid1(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 16); }
 
 int mlp_reserve(fz_mlp* p, int n) {
@@ -546,7 +563,7 @@ int mlp_reserve(fz_mlp* p, int n) {
   for (int l = 0; l <= p->nl; ++l) MLP_CK(cudaMalloc(&p->act[l], (size_t)n * p->dim[l] * sizeof(__nv_bfloat16)));
   for (int l = 0; l < p->nl; ++l) {
     MLP_CK(cudaMalloc(&p->z[l], (size_t)n * p->dim[l + 1] * sizeof(float)));
-    MLP_CK(cudaMalloc(&p->dz[l], (size_t)n * p->dim[l + 1] * sizeof(__nv_bfloat16)));
+    MLP_CK(cudaMalloc(&p->dz[l], (size_t)n * ldz(p, l) * sizeof(__nv_bfloat16)));
   }
   MLP_CK(cudaMalloc(&p->yout, (size_t)n * p->dim[p->nl] * sizeof(float)));
   p->cap = n;
@@ -570,118 +587,132 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// A K-contiguous bf16 operand (rows x K, row stride ld elements) as a 2-D
-// tensor map of 64 x 128 boxes with 128-byte swizzling.  False (the caller
-// then stages the operand itself) when the operand has fewer rows than a
-// box, or its base or row stride is not 16-byte aligned.
-bool tmap_kmajor(CUtensorMap* m, const __nv_bfloat16* p, int rows, int K, int ld) {
+// A bf16 operand as a 2-D tensor map with 128-byte swizzling: `inner`
+// contiguous elements by `outer` rows at stride ld, in boxes of 64 x box
+// (a box may reach over the operand's edges: zeros).  K-contiguous operands
+// are inner K, outer rows; MN-contiguous ones inner MN, outer K.
+bool tmap(CUtensorMap* m, const __nv_bfloat16* p, int inner, int outer, int ld, int box) {
   const EncodeTiledFn fn = encode_tiled();
-  if (!fn || rows < TM_BM || K < TM_BK || (reinterpret_cast<uintptr_t>(p) & 15) || ((size_t)ld * 2) % 16) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+  if (!fn) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)TM_BK, (cuuint32_t)TM_BM};
+  const cuuint32_t boxes[2] = {64, (cuuint32_t)box};
   const cuuint32_t es[2] = {1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p), dims, strides, box, es,
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p), dims, strides, boxes, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// An MN-contiguous bf16 operand (K rows of mn elements, row stride ld) as a
-// 2-D tensor map of 64 x 64 boxes (MN inner) with 128-byte swizzling.
-bool tmap_mnmajor(CUtensorMap* m, const __nv_bfloat16* p, int K, int mn, int ld) {
-  const EncodeTiledFn fn = encode_tiled();
-  if (!fn || mn < 64 || K < TM_BK || (reinterpret_cast<uintptr_t>(p) & 15) || ((size_t)ld * 2) % 16) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)mn, (cuuint64_t)K};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)TM_BK};
-  const cuuint32_t es[2] = {1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p), dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+template <int MODE, int EPI, int BN>
+int gemm_bn(const fz_mlp* p, cudaStream_t s, int M, int N, int K, const __nv_bfloat16* A, int lda,
+            const __nv_bfloat16* B, int ldb, const float* bias, const float* zin, float* zout, float* fout,
+            __nv_bfloat16* out, int ldc) {
+  constexpr bool AMN = MODE == TN, BMN = MODE != NT;
+  CUtensorMap ma, mb;
+  if (!(AMN ? tmap(&ma, A, M, K, lda, TM_BK) : tmap(&ma, A, K, M, lda, TM_BM)) ||
+      !(BMN ? tmap(&mb, B, N, K, ldb, TM_BK) : tmap(&mb, B, K, N, ldb, BN))) {
+    std::fprintf(stderr, "fz_b200 mlp: no tensor map for a GEMM operand\n");
+    return FZ_ERR_CUDA;
+  }
+  const long long tiles = (long long)((N + BN - 1) / BN) * ((M + TM_BM - 1) / TM_BM);
+  const int grid = (int)std::min<long long>(tiles, 2 * p->nsm);
+  k_gemm<EPI, AMN, BMN, BN><<<grid, TM_THREADS, tm_smem(BN), s>>>(ma, mb, M, N, K, bias, zin, zout, fout, out, ldc,
+                                                                  p->d_err);
+  return 0;
 }
 
 template <int MODE, int EPI>
-void gemm(cudaStream_t s, int* err, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B,
-          int ldb, const float* bias, const float* zin, float* zout, float* fout, __nv_bfloat16* out, int ldc) {
-  const dim3 gtm((N + TM_BN - 1) / TM_BN, (M + TM_BM - 1) / TM_BM);
-  CUtensorMap ma, mb;
-  if constexpr (MODE == NT && (EPI == EPI_FWD_GELU || EPI == EPI_FWD_LIN)) {
-    if (tmap_kmajor(&ma, A, M, K, lda) && tmap_kmajor(&mb, B, N, K, ldb)) {
-      k_gemm_tma<EPI, false, false><<<gtm, 256, TM_SMEM, s>>>(ma, mb, M, N, K, bias, zin, zout, fout, out, ldc, err);
-      return;
-    }
-  } else if constexpr (MODE == NN && EPI == EPI_BWD_GELU) {
-    // A = dZ (M x K, K contiguous); B[n][k] = W[k][n]: W's rows are K
-    if (tmap_kmajor(&ma, A, M, K, lda) && tmap_mnmajor(&mb, B, K, N, ldb) && (ldc & 7) == 0) {
-      k_gemm_tma<EPI, false, true><<<gtm, 256, TM_SMEM, s>>>(ma, mb, M, N, K, bias, zin, zout, fout, out, ldc, err);
-      return;
-    }
-  } else if constexpr (MODE == TN && EPI == EPI_F32) {
-    // A[m][k] = dZ[k][m], B[n][k] = X[k][n]: both with K as the row index
-    if (tmap_mnmajor(&ma, A, K, M, lda) && tmap_mnmajor(&mb, B, K, N, ldb)) {
-      k_gemm_tma<EPI, true, true><<<gtm, 256, TM_SMEM, s>>>(ma, mb, M, N, K, bias, zin, zout, fout, out, ldc, err);
-      return;
-    }
+int gemm(const fz_mlp* p, cudaStream_t s, int M, int N, int K, const __nv_bfloat16* A, int lda,
+         const __nv_bfloat16* B, int ldb, const float* bias, const float* zin, float* zout, float* fout,
+         __nv_bfloat16* out, int ldc) {
+  if constexpr (MODE == NT) {
+    if (N <= 16) return gemm_bn<MODE, EPI, 16>(p, s, M, N, K, A, lda, B, ldb, bias, zin, zout, fout, out, ldc);
   }
-  const dim3 grid((N + 127) / 128, (M + 127) / 128);
-  k_gemm_tc<MODE, EPI><<<grid, 256, TC_SMEM, s>>>(M, N, K, A, lda, B, ldb, bias, zin, zout, fout, out, ldc, err);
+  const long long wide = (long long)((N + 127) / 128) * ((M + TM_BM - 1) / TM_BM);
+  if (wide < 2 * p->nsm) return gemm_bn<MODE, EPI, 64>(p, s, M, N, K, A, lda, B, ldb, bias, zin, zout, fout, out, ldc);
+  return gemm_bn<MODE, EPI, 128>(p, s, M, N, K, A, lda, B, ldb, bias, zin, zout, fout, out, ldc);
 }
 
-template <typename F>
-cudaError_t tma_attrs(F* kernel) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TM_SMEM);
-  return e == cudaSuccess ? cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100) : e;
+template <int EPI, bool AMN, bool BMN, int BN>
+cudaError_t gemm_attr() {
+  auto* k = &k_gemm<EPI, AMN, BMN, BN>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tm_smem(BN));
+  return e == cudaSuccess ? cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) : e;
 }
 
-// The tensor-core GEMMs' shared memory above the default 48 KB (set once,
-// before any stream capture).
-int gemm_tc_attrs() {
-  cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<NT, EPI_FWD_GELU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)TC_SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_gemm_tc<NT, EPI_FWD_LIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_gemm_tc<TN, EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_gemm_tc<NN, EPI_BWD_GELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-  // two CTAs per SM (97 KB each): one CTA's epilogue overlaps the other's MMAs
-  if (e == cudaSuccess) e = tma_attrs(k_gemm_tma<EPI_FWD_GELU, false, false>);
-  if (e == cudaSuccess) e = tma_attrs(k_gemm_tma<EPI_FWD_LIN, false, false>);
-  if (e == cudaSuccess) e = tma_attrs(k_gemm_tma<EPI_BWD_GELU, false, true>);
-  if (e == cudaSuccess) e = tma_attrs(k_gemm_tma<EPI_F32, true, true>);
-  if (e != cudaSuccess) {
-    std::fprintf(stderr, "fz_b200 mlp: CUDA error %s\n", cudaGetErrorString(e));
-    return FZ_ERR_CUDA;
+// The GEMMs' shared memory above the default 48 KB (set once, before any
+// stream capture).
+int gemm_attrs() {
+  const cudaError_t es[] = {gemm_attr<EPI_FWD_GELU, false, false, 16>(), gemm_attr<EPI_FWD_GELU, false, false, 64>(),
+                            gemm_attr<EPI_FWD_GELU, false, false, 128>(), gemm_attr<EPI_FWD_LIN, false, false, 16>(),
+                            gemm_attr<EPI_FWD_LIN, false, false, 64>(), gemm_attr<EPI_FWD_LIN, false, false, 128>(),
+                            gemm_attr<EPI_BWD_GELU, false, true, 64>(), gemm_attr<EPI_BWD_GELU, false, true, 128>(),
+                            gemm_attr<EPI_F32, true, true, 64>(), gemm_attr<EPI_F32, true, true, 128>()};
+  for (cudaError_t e : es)
+    if (e != cudaSuccess) {
+      std::fprintf(stderr, "fz_b200 mlp: CUDA error %s\n", cudaGetErrorString(e));
+      return FZ_ERR_CUDA;
+    }
+  return 0;
+}
+
+// forward of n rows already in act[0] into y; the pre-activations are kept
+// for a backward pass only when keep_z
+int mlp_fwd(fz_mlp* p, int n, float* y, bool keep_z = true) {
+  for (int l = 0; l < p->nl; ++l) {
+    const int in = p->dim[l], out = p->dim[l + 1];
+    const int rc = l + 1 < p->nl
+                       ? gemm<NT, EPI_FWD_GELU>(p, p->stream, n, out, in, p->act[l], in, p->Wb[l], in, p->b[l], nullptr,
+                                                keep_z ? p->z[l] : nullptr, nullptr, p->act[l + 1], out)
+                       : gemm<NT, EPI_FWD_LIN>(p, p->stream, n, out, in, p->act[l], in, p->Wb[l], in, p->b[l], nullptr,
+                                               nullptr, y, nullptr, out);
+    if (rc) return rc;
   }
   return 0;
 }
 
-// forward of n rows already in act[0]; output in yout; the pre-activations
-// are kept for a backward pass only when keep_z
-void mlp_fwd(fz_mlp* p, int n, bool keep_z = true) {
-  for (int l = 0; l < p->nl; ++l) {
-    const int in = p->dim[l], out = p->dim[l + 1];
-    if (l + 1 < p->nl)
-      gemm<NT, EPI_FWD_GELU>(p->stream, p->d_err, n, out, in, p->act[l], in, p->Wb[l], in, p->b[l], nullptr,
-                             keep_z ? p->z[l] : nullptr, nullptr, p->act[l + 1], out);
-    else
-      gemm<NT, EPI_FWD_LIN>(p->stream, p->d_err, n, out, in, p->act[l], in, p->Wb[l], in, p->b[l], nullptr, nullptr, p->yout,
-                            nullptr, out);
-  }
-}
-
-// backward from dz[nl-1]; fills gW, gb
-void mlp_bwd(fz_mlp* p, int n) {
+// backward from dz[nl-1]; fills gW, gb and, with `k`, updates the parameters
+// (Adam).  dL/dz runs down the layers on the caller's stream; beside it, as
+// soon as a layer's dL/dz is there, its weight gradient on sw and its bias
+// sums on sb (a training batch fills less than the chip with any one of
+// them; a step of 1,024 rows took 460 us in one chain of the former kernels, 104
+// now).  A layer's update follows its gradients and the product that still
+// reads its weights: on sw, the first layer's on the stream itself.
+int mlp_bwd(fz_mlp* p, int n, const AdamK* k) {
+  cudaStream_t s = p->stream;
+  auto adam = [&](int l, cudaStream_t t) {
+    const size_t n4 = (size_t)p->dim[l] * p->dim[l + 1] / 4;
+    const AdamP a{n4,       p->dim[l + 1], p->W[l],  p->mW[l], p->vW[l], p->b[l],
+                  p->mb[l], p->vb[l],      p->gW[l], p->gb[l], p->Wb[l]};
+    k_adam<<<grid1(n4), 256, 0, t>>>(a, *k, p->tstate);
+  };
   for (int l = p->nl - 1; l >= 0; --l) {
-    const int in = p->dim[l], out = p->dim[l + 1];
-    // dW (out x in) = dZ^T (out x n) X (n x in)
-    gemm<TN, EPI_F32>(p->stream, p->d_err, out, in, n, p->dz[l], out, p->act[l], in, nullptr, nullptr, nullptr, p->gW[l],
-                      nullptr, in);
-    k_colsum<<<(out + 255) / 256, 256, 0, p->stream>>>(n, out, p->dz[l], p->gb[l]);
+    const int in = p->dim[l], out = p->dim[l + 1], ld = ldz(p, l);
+    int rc = 0;
+    MLP_CK(cudaEventRecord(p->ez[l], s));   // dL/dz of layer l (and the last reader of W of layer l + 1)
+    MLP_CK(cudaStreamWaitEvent(p->sw, p->ez[l], 0));
+    MLP_CK(cudaStreamWaitEvent(p->sb, p->ez[l], 0));
+    k_colsum<<<(out + CS_COLS - 1) / CS_COLS, 128, 0, p->sb>>>(n, out, p->dz[l], ld, p->gb[l],
+                                                               k && l == p->nl - 1 ? p->tstate : nullptr);
+    MLP_CK(cudaEventRecord(p->eb[l], p->sb));
     if (l > 0)   // dZ_{l-1} = (dZ_l W_l) * gelu'(z_{l-1})
-      gemm<NN, EPI_BWD_GELU>(p->stream, p->d_err, n, in, out, p->dz[l], out, p->Wb[l], in, nullptr, p->z[l - 1], nullptr,
-                             nullptr, p->dz[l - 1], in);
+      rc = gemm<NN, EPI_BWD_GELU>(p, s, n, in, out, p->dz[l], ld, p->Wb[l], in, nullptr, p->z[l - 1], nullptr, nullptr,
+                                  p->dz[l - 1], in);
+    // dW (out x in) = dZ^T (out x n) X (n x in)
+    if (!rc)
+      rc = gemm<TN, EPI_F32>(p, l > 0 ? p->sw : s, out, in, n, p->dz[l], ld, p->act[l], in, nullptr, nullptr, nullptr,
+                             p->gW[l], nullptr, in);
+    if (rc) return rc;
+    if (k && l + 1 < p->nl) {
+      MLP_CK(cudaStreamWaitEvent(p->sw, p->eb[l + 1], 0));
+      adam(l + 1, p->sw);
+    }
   }
+  MLP_CK(cudaStreamWaitEvent(s, p->eb[0], 0));
+  if (k) adam(0, s);
+  MLP_CK(cudaEventRecord(p->ew, p->sw));
+  MLP_CK(cudaStreamWaitEvent(s, p->ew, 0));
+  return 0;
 }
 
 }  // namespace
@@ -703,7 +734,13 @@ int fz_mlp_create(fz_mlp** out, int nlayers, const int* dims, unsigned long long
     return code;
   };
   if ((rc = mlp_fail(cudaSetDevice(device)))) return fail(rc);
-  if ((rc = mlp_fail(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking)))) return fail(rc);
+  if ((rc = mlp_fail(cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, device)))) return fail(rc);
+  for (cudaStream_t* q : {&p->stream, &p->sw, &p->sb})
+    if ((rc = mlp_fail(cudaStreamCreateWithFlags(q, cudaStreamNonBlocking)))) return fail(rc);
+  if ((rc = mlp_fail(cudaEventCreateWithFlags(&p->ew, cudaEventDisableTiming)))) return fail(rc);
+  for (int l = 0; l < nlayers; ++l)
+    for (cudaEvent_t* q : {&p->ez[l], &p->eb[l]})
+      if ((rc = mlp_fail(cudaEventCreateWithFlags(q, cudaEventDisableTiming)))) return fail(rc);
   for (int l = 0; l < nlayers; ++l) {
     const size_t nw = (size_t)dims[l] * dims[l + 1];
     float** f32[] = {&p->W[l], &p->gW[l], &p->mW[l], &p->vW[l]};
@@ -715,7 +752,7 @@ int fz_mlp_create(fz_mlp** out, int nlayers, const int* dims, unsigned long long
     if ((rc = mlp_fail(cudaMalloc(&p->Wb[l], nw * sizeof(__nv_bfloat16))))) return fail(rc);
     const float sc = std::sqrt(6.0f / (float)(dims[l] + dims[l + 1]));
     k_init<<<grid1(nw), 256, 0, p->stream>>>(nw, p->W[l], seed + 1000003ull * l, sc);
-    k_to_bf16<<<grid1(nw), 256, 0, p->stream>>>(nw, p->W[l], p->Wb[l]);
+    k_to_bf16<<<grid1(nw / 8), 256, 0, p->stream>>>(nw / 8, p->W[l], p->Wb[l]);
     cudaMemsetAsync(p->b[l], 0, dims[l + 1] * sizeof(float), p->stream);
     cudaMemsetAsync(p->mW[l], 0, nw * sizeof(float), p->stream);
     cudaMemsetAsync(p->vW[l], 0, nw * sizeof(float), p->stream);
@@ -725,7 +762,7 @@ int fz_mlp_create(fz_mlp** out, int nlayers, const int* dims, unsigned long long
   if ((rc = mlp_fail(cudaMalloc(&p->loss, sizeof(float))))) return fail(rc);
   if ((rc = mlp_fail(cudaMalloc(&p->d_err, sizeof(int))))) return fail(rc);
   if ((rc = mlp_fail(cudaMemsetAsync(p->d_err, 0, sizeof(int), p->stream)))) return fail(rc);
-  if ((rc = gemm_tc_attrs())) return fail(rc);
+  if ((rc = gemm_attrs())) return fail(rc);
   if ((rc = mlp_fail(cudaStreamSynchronize(p->stream)))) return fail(rc);
   *out = p;
   return 0;
@@ -768,7 +805,13 @@ int fz_mlp_destroy(fz_mlp* p) {
   cudaFree(p->d_lw);
   cudaFree(p->tstate);
   cudaFree(p->order);
-  if (p->stream) cudaStreamDestroy(p->stream);
+  for (cudaStream_t q : {p->stream, p->sw, p->sb})
+    if (q) cudaStreamDestroy(q);
+  for (int l = 0; l < MLP_MAXL; ++l) {
+    if (p->ez[l]) cudaEventDestroy(p->ez[l]);
+    if (p->eb[l]) cudaEventDestroy(p->eb[l]);
+  }
+  if (p->ew) cudaEventDestroy(p->ew);
   delete p;
   return 0;
 }
@@ -806,7 +849,7 @@ int fz_mlp_set_params(fz_mlp* p, const float* host) {
     o += nw;
     MLP_CK(cudaMemcpyAsync(p->b[l], host + o, p->dim[l + 1] * sizeof(float), cudaMemcpyHostToDevice, p->stream));
     o += p->dim[l + 1];
-    k_to_bf16<<<grid1(nw), 256, 0, p->stream>>>(nw, p->W[l], p->Wb[l]);
+    k_to_bf16<<<grid1(nw / 8), 256, 0, p->stream>>>(nw / 8, p->W[l], p->Wb[l]);
   }
   MLP_CK(cudaGetLastError());
   MLP_CK(cudaStreamSynchronize(p->stream));
@@ -828,15 +871,16 @@ int fz_mlp_forward_device(fz_mlp* p, int n, const float* d_x, float* d_y, void* 
     cudaStreamWaitEvent(s, ev, 0);
   }
   const int d0 = p->dim[0], dl = p->dim[p->nl];
-  for (int i = 0; i < n; i += chunk) {
+  for (int i = 0; i < n && !rc; i += chunk) {
     const int m = std::min(chunk, n - i);
-    k_to_bf16<<<grid1((size_t)m * d0), 256, 0, s>>>((size_t)m * d0, d_x + (size_t)i * d0, p->act[0]);
-    mlp_fwd(p, m, false);
-    cudaMemcpyAsync(d_y + (size_t)i * dl, p->yout, (size_t)m * dl * sizeof(float), cudaMemcpyDeviceToDevice, s);
+    const size_t n8 = (size_t)m * d0 / 8;
+    k_to_bf16<<<grid1(n8), 256, 0, s>>>(n8, d_x + (size_t)i * d0, p->act[0]);
+    rc = mlp_fwd(p, m, d_y + (size_t)i * dl, false);
   }
   cudaEventRecord(ev, s);
   if (stream) cudaStreamWaitEvent((cudaStream_t)stream, ev, 0);
   int r2 = mlp_fail(cudaGetLastError());
+  if (rc) r2 = rc;
   if (!stream) {
     cudaStreamSynchronize(s);
     if (!r2) r2 = mlp_tc_status(p);
@@ -861,18 +905,17 @@ int fz_mlp_forward_obs_device(fz_mlp* p, int n, const double* d_obs, const float
   cudaEventRecord(ev, (cudaStream_t)stream);
   cudaStreamWaitEvent(s, ev, 0);
   const int d0 = p->dim[0], dl = p->dim[p->nl];
-  for (int i = 0; i < n; i += chunk) {
+  for (int i = 0; i < n && !rc; i += chunk) {
     const int m = std::min(chunk, n - i);
     k_obs_bf16<<<grid1((size_t)m * d0), 256, 0, s>>>((size_t)m * d0, d0, d_obs + (size_t)i * d0, d_mu, d_sd,
                                                       p->act[0]);
-    mlp_fwd(p, m, false);
-    cudaMemcpyAsync(d_y + (size_t)i * dl, p->yout, (size_t)m * dl * sizeof(float), cudaMemcpyDeviceToDevice, s);
+    rc = mlp_fwd(p, m, d_y + (size_t)i * dl, false);
   }
   cudaEventRecord(ev, s);
   cudaStreamWaitEvent((cudaStream_t)stream, ev, 0);
   const int r2 = mlp_fail(cudaGetLastError());
   cudaEventDestroy(ev);
-  return r2;
+  return rc ? rc : r2;
 }
 
 // Per-output weights of the training loss (host, nout values), or none
@@ -910,16 +953,19 @@ int fz_mlp_grad_device(fz_mlp* p, int n, const float* d_x, const float* d_t, flo
   if (rc) return rc;
   cudaStream_t s = p->stream;
   const int d0 = p->dim[0], dl = p->dim[p->nl];
-  k_to_bf16<<<grid1((size_t)n * d0), 256, 0, s>>>((size_t)n * d0, d_x, p->act[0]);
-  mlp_fwd(p, n);
-  MLP_CK(cudaMemsetAsync(p->loss, 0, sizeof(float), s));
-  k_mse<<<grid1((size_t)n * dl), 256, 0, s>>>(n, dl, p->yout, d_t, p->dz[p->nl - 1], p->loss, nullptr, nullptr,
-                                              p->d_lw);
-  mlp_bwd(p, n);
-  MLP_CK(cudaGetLastError());
-  if (loss) MLP_CK(cudaMemcpyAsync(loss, p->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-  MLP_CK(cudaStreamSynchronize(s));
-  return mlp_tc_status(p);
+  const size_t n8 = (size_t)n * d0 / 8;
+  k_to_bf16<<<grid1(n8), 256, 0, s>>>(n8, d_x, p->act[0]);
+  rc = mlp_fwd(p, n, p->yout);
+  if (!rc) rc = mlp_fail(cudaMemsetAsync(p->loss, 0, sizeof(float), s));
+  if (!rc) {
+    k_mse<<<grid1((size_t)n * dl), 256, 0, s>>>(n, dl, p->yout, d_t, p->dz[p->nl - 1], ldz(p, p->nl - 1), p->loss,
+                                                nullptr, nullptr, p->d_lw);
+    rc = mlp_bwd(p, n, nullptr);
+  }
+  if (!rc) rc = mlp_fail(cudaGetLastError());
+  if (!rc && loss) rc = mlp_fail(cudaMemcpyAsync(loss, p->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
+  const int r2 = mlp_fail(cudaStreamSynchronize(s));
+  return rc ? rc : r2 ? r2 : mlp_tc_status(p);
 }
 
 // Mini-batch Adam training over n device rows for `epochs` passes (rows
@@ -950,22 +996,17 @@ int fz_mlp_train_device(fz_mlp* p, int n, const float* d_x, const float* d_t, in
   cudaGraphExec_t exec = nullptr;
   if ((rc = mlp_fail(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)))) return rc;
   {
-    k_batch_bf16<<<grid1((size_t)batch * d0), 256, 0, s>>>(batch, d0, d_x, p->order, p->tstate, p->act[0]);
-    mlp_fwd(p, batch);
-    k_mse<<<grid1((size_t)batch * dl), 256, 0, s>>>(batch, dl, p->yout, d_t, p->dz[p->nl - 1], p->loss, p->order,
-                                                   p->tstate, p->d_lw);
-    mlp_bwd(p, batch);
-    const float b1 = 0.9f, b2 = 0.999f;
-    for (int l = 0; l < p->nl; ++l) {
-      const size_t nw = (size_t)p->dim[l] * p->dim[l + 1];
-      k_adam<<<grid1(nw), 256, 0, s>>>(nw, p->W[l], p->gW[l], p->mW[l], p->vW[l], p->Wb[l], lr, b1, b2, p->tstate,
-                                       1e-8f);
-      k_adam<<<grid1(p->dim[l + 1]), 256, 0, s>>>(p->dim[l + 1], p->b[l], p->gb[l], p->mb[l], p->vb[l], nullptr, lr,
-                                                  b1, b2, p->tstate, 1e-8f);
+    const AdamK k{lr, 0.9f, 0.999f, 1e-8f};
+    k_batch_bf16<<<grid1((size_t)batch * d0 / 8), 256, 0, s>>>(batch, d0, d_x, p->order, p->tstate, p->act[0]);
+    rc = mlp_fwd(p, batch, p->yout);
+    if (!rc) {
+      k_mse<<<grid1((size_t)batch * dl), 256, 0, s>>>(batch, dl, p->yout, d_t, p->dz[p->nl - 1], ldz(p, p->nl - 1),
+                                                      p->loss, p->order, p->tstate, p->d_lw);
+      rc = mlp_bwd(p, batch, &k);
     }
-    k_train_advance<<<1, 1, 0, s>>>(p->tstate);
   }
-  rc = mlp_fail(cudaStreamEndCapture(s, &graph));
+  const int r2 = mlp_fail(cudaStreamEndCapture(s, &graph));
+  if (!rc) rc = r2;
   if (!rc) rc = mlp_fail(cudaGraphInstantiate(&exec, graph, 0));
   // batch order: a fixed random permutation of the batch indices per epoch
   std::vector<int> order(nb);

@@ -91,7 +91,7 @@ __device__ __forceinline__ uint64_t globaltimer() {
 // limit_ns; false when the time runs out.
 __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint64_t limit_ns) {
   const uint32_t a = smem_addr(mbar);
-  const uint64_t t0 = globaltimer();
+  uint64_t t0 = 0;   // read only when the first try fails
   while (true) {
     uint32_t done;
     asm volatile(
@@ -101,14 +101,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint6
         : "r"(a), "r"(parity)
         : "memory");
     if (done) return true;
-    if (globaltimer() - t0 > limit_ns) return false;
+    const uint64_t t = globaltimer();
+    if (t0 == 0) t0 = t;
+    if (t - t0 > limit_ns) return false;
   }
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(mbar)) : "memory");
 }
 
 // Arrive on the mbarrier and add tx bytes to the phase's expected count.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mbar)), "r"(bytes)
                : "memory");
+}
+
+__device__ __forceinline__ void tma_prefetch(const void* tmap) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
 // One box of a 2-D tiled tensor map (x = innermost coordinate, in elements)

@@ -31,6 +31,7 @@
 #include "fz_host.h"
 #include "fz_physics.cuh"
 #include "fz_layer2.cuh"
+#include "fz_stage.cuh"
 #include "fz_rf.cuh"
 
 using namespace fzd;
@@ -2387,6 +2388,12 @@ constexpr int NKERN = 15;   // k_chain, k_opac, k_synth, k_opac_rf, k_synth_rf, 
 
 struct fz_ctx {
   int device = 0;
+  // fz_lm_perturbation's copies and its workspace, kept up to LMP_KEEP bytes;
+  // one call at a time
+  fzstage::HostStage stage;
+  std::mutex lmp_mu;
+  unsigned char* d_lmp = nullptr;
+  size_t lmp_len = 0;
   int nz = 0, numw = 0, nreg = 0, nlu = 0, sw = 0;
   std::vector<fz_line> lines;
   std::vector<fz_region> regs;
@@ -4471,6 +4478,7 @@ int fz_destroy(fz_ctx* c) {
   if (!c) return 0;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
+  cudaFree(c->d_lmp);
   cudaFree(c->d_params);
   cudaFree(c->d_consts);
   cudaFree(c->d_pf);
@@ -5008,6 +5016,11 @@ int fz_invert(fz_ctx* c, int npix, const double* obs, const float* init, const d
   return 0;
 }
 
+// The largest workspace fz_lm_perturbation keeps for its next call (4,500
+// pixels of 13 parameters and 896 frequencies in REAL*4); a larger one is
+// allocated for its call and freed.
+constexpr size_t LMP_KEEP = (size_t)256 << 20;
+
 // Batched GET_PERTURBATION on host buffers; the Jacobian comes as REAL*8
 // (jac64) or REAL*4 (jac32), exactly one of them given.  A REAL*8 Jacobian is
 // rounded to FP32 on the device before the split-bf16 normal equations.
@@ -5027,104 +5040,101 @@ static int lm_perturbation_host(fz_ctx* c, int npix, int np, int nfreq, const do
   C.solver = dtype == 2 ? 2 : 1;
   const bool big = np > LM_MAXNP;
   for (int j = 0; j < np && !big; ++j) C.norm[j] = 1.0;
-  double* d_ones = nullptr;   // PARAM_NORMS of a large layout: the Jacobian comes normalised
-  int* d_err = nullptr;
-  double* d_svd = nullptr;
+  // every buffer of the call in one allocation, sized for this call
+  const size_t n = npix, nj = n * np * nfreq;
+  size_t need = 0;
+  auto room = [&](size_t bytes) {
+    const size_t o = need;
+    need += (bytes + 255) & ~(size_t)255;
+    return o;
+  };
+  const size_t o_pix = room(n * sizeof(int)), o_skip = room(n * sizeof(int)), o_st = room(5 * n * sizeof(double));
+  const size_t o_jac = room(nj * sizeof(float)), o_diff = room(n * nfreq * sizeof(double));
+  const size_t o_H = room(n * np * np * sizeof(double)), o_g = room(n * np * sizeof(double));
+  const size_t o_delta = room(n * np * sizeof(double)), o_w = room(nfreq * sizeof(double));
+  const size_t o_ones = room(big ? np * sizeof(double) : 0), o_err = room(big ? sizeof(int) : 0);
+  const size_t o_svd = room(big && C.solver != 2 ? n * 2 * np * np * sizeof(double) : 0);
+  const size_t o_pen = room(reg_pen ? n * np * sizeof(double) : 0);
+  const size_t o_hss = room(reg_hss ? n * np * np * sizeof(double) : 0);
+  const size_t o_j64 = room(jac64 ? nj * sizeof(double) : 0);   // REAL*8 IJACOBIAN, rounded into L.jacb
+  std::vector<double> st(5 * n, 0.0), ones(std::max(nfreq, np), 1.0);
+  for (int i = 0; i < npix; ++i) st[5 * (size_t)i + 2] = lambda[i];
+  std::lock_guard<std::mutex> lock(c->lmp_mu);
+  unsigned char* base = c->d_lmp;
+  if (need > c->lmp_len) {
+    cudaFree(c->d_lmp);
+    c->d_lmp = nullptr;
+    c->lmp_len = 0;
+    FZ_CK(cudaMalloc(&base, need));
+    if (need <= LMP_KEEP) {
+      c->d_lmp = base;
+      c->lmp_len = need;
+    }
+  }
   LMSlots L{};
   L.S = npix;
-  std::vector<int> zeros(npix, 0);
-  std::vector<double> st(5 * (size_t)npix, 0.0);
-  for (int i = 0; i < npix; ++i) st[5 * (size_t)i + 2] = lambda[i];
-  std::vector<double> ones(nfreq, 1.0);
-  double* d_w = nullptr;
+  L.pix = (int*)(base + o_pix);
+  L.skip = (int*)(base + o_skip);
+  L.st = (double*)(base + o_st);
+  L.jacb = (float*)(base + o_jac);
+  L.diff = (double*)(base + o_diff);
+  L.H = (double*)(base + o_H);
+  L.g = (double*)(base + o_g);
+  L.delta = (double*)(base + o_delta);
+  double* d_w = (double*)(base + o_w);
+  double* d_ones = (double*)(base + o_ones);   // PARAM_NORMS of a large layout: the Jacobian comes normalised
+  int* d_err = (int*)(base + o_err);
+  double* d_j64 = (double*)(base + o_j64);
+  if (reg_pen) L.pen = (double*)(base + o_pen);
+  if (reg_hss) L.hss = (double*)(base + o_hss);
+  if (big) C.d_norm = d_ones;
+  const cudaStream_t s = c->stream;
   int rc = 0;
   do {
-    if ((rc = cuda_fail(cudaMalloc(&L.pix, npix * sizeof(int))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&L.skip, npix * sizeof(int))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&L.st, st.size() * sizeof(double))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&L.jacb, (size_t)npix * np * nfreq * sizeof(float))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&L.diff, (size_t)npix * nfreq * sizeof(double))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&L.H, (size_t)npix * np * np * sizeof(double))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&L.g, (size_t)npix * np * sizeof(double))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&L.delta, (size_t)npix * np * sizeof(double))))) break;
-    if ((rc = cuda_fail(cudaMalloc(&d_w, nfreq * sizeof(double))))) break;
-    if (big) {
-      std::vector<double> ones(np, 1.0);
-      if ((rc = cuda_fail(cudaMalloc(&d_ones, np * sizeof(double))))) break;
-      if ((rc = cuda_fail(cudaMalloc(&d_err, sizeof(int))))) break;
-      if (C.solver != 2 && (rc = cuda_fail(cudaMalloc(&d_svd, (size_t)npix * 2 * np * np * sizeof(double))))) break;
-      cudaMemcpy(d_ones, ones.data(), np * sizeof(double), cudaMemcpyHostToDevice);
-      cudaMemset(d_err, 0, sizeof(int));
-      C.d_norm = d_ones;
-    }
-    if (reg_pen) {
-      if ((rc = cuda_fail(cudaMalloc(&L.pen, (size_t)npix * np * sizeof(double))))) break;
-      cudaMemcpy(L.pen, reg_pen, (size_t)npix * np * sizeof(double), cudaMemcpyHostToDevice);
-    }
-    if (reg_hss) {
-      if ((rc = cuda_fail(cudaMalloc(&L.hss, (size_t)npix * np * np * sizeof(double))))) break;
-      cudaMemcpy(L.hss, reg_hss, (size_t)npix * np * np * sizeof(double), cudaMemcpyHostToDevice);
-    }
-    cudaMemcpy(L.pix, zeros.data(), npix * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.skip, zeros.data(), npix * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(L.st, st.data(), st.size() * sizeof(double), cudaMemcpyHostToDevice);
-    if (jac32) {
-      cudaMemcpy(L.jacb, jac32, (size_t)npix * np * nfreq * sizeof(float), cudaMemcpyHostToDevice);
-    } else {
-      // the REAL*8 IJACOBIAN in a buffer of its own, rounded into L.jacb
-      double* d_j64 = nullptr;
-      const size_t nj = (size_t)npix * np * nfreq;
-      if ((rc = cuda_fail(cudaMalloc(&d_j64, nj * sizeof(double))))) break;
-      rc = cuda_fail(cudaMemcpy(d_j64, jac64, nj * sizeof(double), cudaMemcpyHostToDevice));
-      if (!rc) rc = copies_done();
-      if (!rc) {
-        k_f64_to_f32<<<(int)std::min<size_t>((nj + 255) / 256, (size_t)c->nsm * 16), 256, 0, c->stream>>>(
-            nj, d_j64, L.jacb);
-        rc = cuda_fail(cudaStreamSynchronize(c->stream));
-      }
-      cudaFree(d_j64);
-      if (rc) break;
-    }
-    cudaMemcpy(L.diff, diff, (size_t)npix * nfreq * sizeof(double), cudaMemcpyHostToDevice);
-    cudaMemcpy(d_w, ones.data(), nfreq * sizeof(double), cudaMemcpyHostToDevice);
-    if ((rc = copies_done())) break;
+    if ((rc = cuda_fail(cudaMemsetAsync(L.pix, 0, n * sizeof(int), s)))) break;
+    if ((rc = cuda_fail(cudaMemsetAsync(L.skip, 0, n * sizeof(int), s)))) break;
+    if (big && (rc = cuda_fail(cudaMemsetAsync(d_err, 0, sizeof(int), s)))) break;
+    using fzstage::Seg;
+    Seg seg[7];
+    int ns = 0;
+    if (jac32)
+      seg[ns++] = Seg{L.jacb, jac32, nj * sizeof(float)};
+    else
+      seg[ns++] = Seg{d_j64, jac64, nj * sizeof(double)};
+    seg[ns++] = Seg{L.diff, diff, n * nfreq * sizeof(double)};
+    seg[ns++] = Seg{L.st, st.data(), st.size() * sizeof(double)};
+    seg[ns++] = Seg{d_w, ones.data(), nfreq * sizeof(double)};
+    if (big) seg[ns++] = Seg{d_ones, ones.data(), np * sizeof(double)};
+    if (reg_pen) seg[ns++] = Seg{L.pen, reg_pen, n * np * sizeof(double)};
+    if (reg_hss) seg[ns++] = Seg{L.hss, reg_hss, n * np * np * sizeof(double)};
+    if ((rc = cuda_fail(c->stage.upload(s, seg, ns)))) break;
+    if (jac64)
+      k_f64_to_f32<<<(int)std::min<size_t>((nj + 255) / 256, (size_t)c->nsm * 16), 256, 0, s>>>(nj, d_j64, L.jacb);
     if (big) {
       const int nb = (np + GT_M - 1) / GT_M;
       if ((rc = cuda_fail(cudaFuncSetAttribute(k_lm_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)GT_SMEM)))) break;
-      k_lm_gram_tc<<<dim3(nb * (nb + 1) / 2, npix), 128, GT_SMEM, c->stream>>>(C, L, d_w, d_err);
-      k_lm_grad<<<dim3((np + 7) / 8, npix), 256, 0, c->stream>>>(C, L, d_w);
+      k_lm_gram_tc<<<dim3(nb * (nb + 1) / 2, npix), 128, GT_SMEM, s>>>(C, L, d_w, d_err);
+      k_lm_grad<<<dim3((np + 7) / 8, npix), 256, 0, s>>>(C, L, d_w);
       if (C.solver == 2)
-        k_lm_cg_big<<<npix, 256, 6 * np * sizeof(double), c->stream>>>(C, L);
+        k_lm_cg_big<<<npix, 256, 6 * np * sizeof(double), s>>>(C, L);
       else
-        k_lm_svd_big<<<npix, 256, 2 * np * sizeof(double), c->stream>>>(C, L, d_svd);
+        k_lm_svd_big<<<npix, 256, 2 * np * sizeof(double), s>>>(C, L, (double*)(base + o_svd));
     } else {
-      k_lm_normal<<<(npix + 3) / 4, 128, 0, c->stream>>>(C, L, d_w);
-      k_lm_solve<<<(npix + 3) / 4, 128, 0, c->stream>>>(C, L);
+      k_lm_normal<<<(npix + 3) / 4, 128, 0, s>>>(C, L, d_w);
+      k_lm_solve<<<(npix + 3) / 4, 128, 0, s>>>(C, L);
     }
     if ((rc = cuda_fail(cudaGetLastError()))) break;
-    if ((rc = cuda_fail(cudaStreamSynchronize(c->stream)))) break;
-    rc = cuda_fail(cudaMemcpy(delta, L.delta, (size_t)npix * np * sizeof(double), cudaMemcpyDeviceToHost));
-    if (!rc && d_err) {
-      int e = 0;
-      rc = cuda_fail(cudaMemcpy(&e, d_err, sizeof(int), cudaMemcpyDeviceToHost));
-      if (!rc && e) rc = FZ_ERR_CUDA;
-    }
+    if ((rc = cuda_fail(cudaMemcpyAsync(delta, L.delta, n * np * sizeof(double), cudaMemcpyDeviceToHost, s)))) break;
+    int e = 0;
+    if (big && (rc = cuda_fail(cudaMemcpyAsync(&e, d_err, sizeof(int), cudaMemcpyDeviceToHost, s)))) break;
+    rc = cuda_fail(cudaStreamSynchronize(s));
+    if (!rc && e) rc = FZ_ERR_CUDA;
   } while (false);
-  cudaFree(L.pix);
-  cudaFree(L.skip);
-  cudaFree(L.st);
-  cudaFree(L.jacb);
-  cudaFree(L.diff);
-  cudaFree(L.H);
-  cudaFree(L.g);
-  cudaFree(L.delta);
-  cudaFree(L.pen);
-  cudaFree(L.hss);
-  cudaFree(d_w);
-  cudaFree(d_ones);
-  cudaFree(d_err);
-  cudaFree(d_svd);
+  if (base != c->d_lmp) {
+    cudaStreamSynchronize(s);
+    cudaFree(base);
+  }
   return rc;
 }
 

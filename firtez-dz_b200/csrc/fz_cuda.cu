@@ -4776,7 +4776,7 @@ int fz_invert_device(fz_ctx* c, int npix, const double* d_obs, const float* d_in
     } else {
       {
         ProfScope ps(c, 7, s, n);
-        k_lm_normal<<<(n + 3) / 4, 128, 0, s>>>(C, L, d_w, L.rf_list, &c->d_q->rf_count);
+        k_lm_normal<<<n, 128, 0, s>>>(C, L, d_w, L.rf_list, &c->d_q->rf_count);
       }
       {
         ProfScope ps(c, 8, s, n);
@@ -4850,7 +4850,7 @@ int fz_invert_device(fz_ctx* c, int npix, const double* d_obs, const float* d_in
       r = launch_rf_stage(c, S, hydrostatic, L.syn, L.jacb, L.mcur, L.status, s, L.rf_list, &c->d_q->rf_count);
     }
     if (!r) {
-      k_lm_normal<<<(S + 3) / 4, 128, 0, s>>>(C, L, d_w, L.rf_list, &c->d_q->rf_count);
+      k_lm_normal<<<S, 128, 0, s>>>(C, L, d_w, L.rf_list, &c->d_q->rf_count);
       k_lm_solve<<<(S + 3) / 4, 128, 0, s>>>(C, L);
       k_lm_update<<<S, 128, usm, s>>>(C, L, c->d_coef64);
       k_lm_scan<<<1, 1024, 0, s>>>(S, L.pix, c->d_dest, c->d_q, c->d_act);
@@ -5121,7 +5121,7 @@ static int lm_perturbation_host(fz_ctx* c, int npix, int np, int nfreq, const do
       else
         k_lm_svd_big<<<npix, 256, 2 * np * sizeof(double), s>>>(C, L, (double*)(base + o_svd));
     } else {
-      k_lm_normal<<<(npix + 3) / 4, 128, 0, s>>>(C, L, d_w);
+      k_lm_normal<<<npix, 128, 0, s>>>(C, L, d_w);
       k_lm_solve<<<(npix + 3) / 4, 128, 0, s>>>(C, L);
     }
     if ((rc = cuda_fail(cudaGetLastError()))) break;

@@ -403,12 +403,17 @@ __device__ __forceinline__ void mma_bf16(float c[4], const unsigned a[4], const 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// One warp per slot: H = Jn^T Jn (np <= 16) on the tensor cores and
-// g = Jn^T r in FP64.  Jn(r, c) = J(r, c) sqrt(w_r / INU) PARAM_NORM(c).
-// Per k-step of 16 frequencies a thread holds rows {grp, grp+8} x
-// frequencies {2t, 2t+1, 2t+8, 2t+9} of Jn^T: exactly its A fragment, and
-// (column grp of tile 0, column grp+8 of tile 1) its B fragments.
-// With list, warp i serves slot list[i] for i < *nlist: the inversion passes
+// One CTA per slot: H = Jn^T Jn (np <= 16) on the tensor cores by its first
+// warp and g = Jn^T r in FP64 by the other three, a third of the columns
+// each.  Jn(r, c) = J(r, c) sqrt(w_r / INU) PARAM_NORM(c).
+// Per k-step of 16 frequencies a thread of the first warp holds rows {grp,
+// grp+8} x frequencies {2t, 2t+1, 2t+8, 2t+9} of Jn^T: exactly its A
+// fragment, and (column grp of tile 0, column grp+8 of tile 1) its B
+// fragments; four k-steps' loads (8 bytes each) are in flight together.
+// It is bound by the Jacobian's bytes: 1,024 slots of 13 x 896 took 211 us
+// with one warp per slot doing g after H, a square root of the weight per
+// element, and take 46 us now (8 us of bytes).
+// With list, CTA i serves slot list[i] for i < *nlist: the inversion passes
 // the accepted slots (rf_list).  H and g depend only on the best model's
 // Jacobian, synthesis and penalties, which change only on an accepted step;
 // a rejected trial leaves them as the last accepted step computed them, bit
@@ -416,8 +421,8 @@ __device__ __forceinline__ void mma_bf16(float c[4], const unsigned a[4], const 
 __global__ void __launch_bounds__(128) k_lm_normal(LMConf C, LMSlots Sl, const double* __restrict__ w,
                                                    const int* __restrict__ list = nullptr,
                                                    const int* __restrict__ nlist = nullptr) {
-  const int lane = threadIdx.x & 31;
-  int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  int s = blockIdx.x;
   if (list) {
     if (s >= *nlist) return;
     s = list[s];
@@ -426,6 +431,33 @@ __global__ void __launch_bounds__(128) k_lm_normal(LMConf C, LMSlots Sl, const d
   if (Sl.pix[s] < 0 || Sl.skip[s]) return;
   const int nf = C.nfreq, np = C.np;
   const float* J = Sl.jacb + (size_t)s * np * nf;
+  if (wi > 0) {
+    // g = Jn^T r (FP64): columns wi - 1, wi + 2, ...
+    constexpr int NC = (LM_MAXNP + 2) / 3;
+    const double* df = Sl.diff + (size_t)s * nf;
+    double acc[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) acc[i] = 0.0;
+#pragma unroll 2
+    for (int k = lane; k < nf; k += 32) {
+      const double sw = sqrt(w[k]), d = df[k];
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        const int c = wi - 1 + 3 * i;
+        if (c < np) acc[i] += (double)J[(size_t)c * nf + k] * sw * d;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int c = wi - 1 + 3 * i;
+      if (c >= np) continue;
+      for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+      // GET_PERTURBATION subtracts REG_PEN from J^T r (src/lm.f90:169-170)
+      if (lane == 0)
+        Sl.g[(size_t)s * np + c] = acc[i] * C.norm[c] / sqrt(C.inu) - (Sl.pen ? Sl.pen[(size_t)s * np + c] : 0.0);
+    }
+    return;
+  }
   const int grp = lane >> 2, t = lane & 3;
   const int m0 = grp, m1 = grp + 8;
   const float n0 = m0 < np ? (float)C.norm[m0] : 0.0f, n1 = m1 < np ? (float)C.norm[m1] : 0.0f;
@@ -433,15 +465,23 @@ __global__ void __launch_bounds__(128) k_lm_normal(LMConf C, LMSlots Sl, const d
   const float* r1 = J + (size_t)(m1 < np ? m1 : 0) * nf;
   const float rin = (float)(1.0 / sqrt(C.inu));
   float c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
+#pragma unroll 4
   for (int k0 = 0; k0 < nf; k0 += 16) {
     float v[2][4];   // [row m0/m1][freq 2t, 2t+1, 2t+8, 2t+9]
-    const int ks[4] = {k0 + 2 * t, k0 + 2 * t + 1, k0 + 2 * t + 8, k0 + 2 * t + 9};
+    // nf is a multiple of 4 and so is every row's start: pairs of
+    // frequencies are whole and 8-byte aligned
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const bool in = ks[i] < nf;
-      const float sw = in ? sqrtf((float)w[ks[i]]) * rin : 0.0f;
-      v[0][i] = (in && m0 < np) ? r0[ks[i]] * sw * n0 : 0.0f;
-      v[1][i] = (in && m1 < np) ? r1[ks[i]] * sw * n1 : 0.0f;
+    for (int h = 0; h < 2; ++h) {
+      const int k = k0 + 2 * t + 8 * h;
+      const bool in = k < nf;
+      const float2 z = make_float2(0.0f, 0.0f);
+      const float2 x0 = in && m0 < np ? __ldg(reinterpret_cast<const float2*>(r0 + k)) : z;
+      const float2 x1 = in && m1 < np ? __ldg(reinterpret_cast<const float2*>(r1 + k)) : z;
+      const float sa = in ? sqrtf((float)w[k]) * rin : 0.0f, sb = in ? sqrtf((float)w[k + 1]) * rin : 0.0f;
+      v[0][2 * h] = x0.x * sa * n0;
+      v[0][2 * h + 1] = x0.y * sb * n0;
+      v[1][2 * h] = x1.x * sa * n1;
+      v[1][2 * h + 1] = x1.y * sb * n1;
     }
     unsigned short hi[2][4], lo[2][4];
 #pragma unroll
@@ -476,23 +516,16 @@ __global__ void __launch_bounds__(128) k_lm_normal(LMConf C, LMSlots Sl, const d
     if (row < np && colA < np) H[row * np + colA] = (double)c0[i] + (rh ? rh[row * np + colA] : 0.0);
     if (row < np && colB < np) H[row * np + colB] = (double)c1[i] + (rh ? rh[row * np + colB] : 0.0);
   }
-  // g = Jn^T r (FP64)
-  const double* df = Sl.diff + (size_t)s * nf;
-  for (int c = 0; c < np; ++c) {
-    const float* rc = J + (size_t)c * nf;
-    double acc = 0.0;
-    for (int k = lane; k < nf; k += 32) acc += (double)rc[k] * sqrt(w[k]) * df[k];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    // ... and subtracts REG_PEN from J^T r (:169-170)
-    if (lane == 0)
-      Sl.g[(size_t)s * np + c] = acc * C.norm[c] / sqrt(C.inu) - (Sl.pen ? Sl.pen[(size_t)s * np + c] : 0.0);
-  }
 }
 
 // One warp per slot, FP64: delta = (H + lambda diag H)^+ g by one-sided
 // Jacobi (Hestenes) on the columns of the symmetric matrix, singular values
 // below svdtol * max dropped (GET_INVERSE, src/lm.f90:61-133); NaN entries
 // of delta are zeroed (NEW_SOLVE_PERTURBATION, src/get_dmodel.f90:806-820).
+// Bound by the latency of its rotations (sums, two square roots, three
+// divisions, one after the other): 1,024 slots of 13 nodes took 444 us with
+// the 78 pairs of a sweep one by one, and take 151 us with the pairs of a
+// round side by side.
 __global__ void __launch_bounds__(128) k_lm_solve(LMConf C, LMSlots Sl) {
   __shared__ double smA[4][LM_MAXNP][LM_MAXNP + 1], smV[4][LM_MAXNP][LM_MAXNP + 1];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -566,39 +599,54 @@ __global__ void __launch_bounds__(128) k_lm_solve(LMConf C, LMSlots Sl) {
     if (lane < np) Sl.delta[(size_t)s * np + lane] = (d == d) ? d : 0.0;
     return;
   }
+  // A round rotates all columns once, in disjoint pairs (a round-robin
+  // tournament of m players, m = np rounded up to even: m - 1 rounds meet
+  // every pair, an odd np leaves one column out per round).  Four lanes take
+  // a pair, rows r4, r4 + 4, ... each.
+  const int m = (np + 1) & ~1, pr = lane >> 2, r4 = lane & 3;
   for (int sweep = 0; sweep < 40; ++sweep) {
     int rot = 0;
-    for (int p = 0; p < np - 1; ++p)
-      for (int q = p + 1; q < np; ++q) {
-        double a = 0.0, b = 0.0, c = 0.0;
-        if (lane < np) {
-          const double xp = A[lane][p], xq = A[lane][q];
-          a = xp * xp;
-          b = xq * xq;
-          c = xp * xq;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          a += __shfl_xor_sync(0xffffffffu, a, o);
-          b += __shfl_xor_sync(0xffffffffu, b, o);
-          c += __shfl_xor_sync(0xffffffffu, c, o);
-        }
-        if (fabs(c) > 1e-15 * sqrt(a * b) && c != 0.0) {
-          ++rot;
-          const double zeta = (b - a) / (2.0 * c);
-          const double tt = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-          const double cs = 1.0 / sqrt(1.0 + tt * tt), sn = cs * tt;
-          if (lane < np) {
-            const double xp = A[lane][p], xq = A[lane][q];
-            A[lane][p] = cs * xp - sn * xq;
-            A[lane][q] = sn * xp + cs * xq;
-            const double vp = V[lane][p], vq = V[lane][q];
-            V[lane][p] = cs * vp - sn * vq;
-            V[lane][q] = sn * vp + cs * vq;
+    for (int rd = 0; rd < m - 1; ++rd) {
+      const int u = pr == 0 ? m - 1 : (rd + pr) % (m - 1), v = pr == 0 ? rd : (rd - pr + m - 1) % (m - 1);
+      const int p = min(u, v), q = max(u, v);
+      const bool on = pr < m / 2 && q < np;
+      double xp[LM_MAXNP / 4], xq[LM_MAXNP / 4];
+      double a = 0.0, b = 0.0, c = 0.0;
+#pragma unroll
+      for (int k = 0; k < LM_MAXNP / 4; ++k) {
+        const int i = r4 + 4 * k;
+        const bool in = on && i < np;
+        xp[k] = in ? A[i][p] : 0.0;
+        xq[k] = in ? A[i][q] : 0.0;
+        a += xp[k] * xp[k];
+        b += xq[k] * xq[k];
+        c += xp[k] * xq[k];
+      }
+      for (int o = 2; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+      }
+      if (fabs(c) > 1e-15 * sqrt(a * b) && c != 0.0) {
+        rot = 1;
+        const double zeta = (b - a) / (2.0 * c);
+        const double tt = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+        const double cs = 1.0 / sqrt(1.0 + tt * tt), sn = cs * tt;
+#pragma unroll
+        for (int k = 0; k < LM_MAXNP / 4; ++k) {
+          const int i = r4 + 4 * k;
+          if (i < np) {
+            A[i][p] = cs * xp[k] - sn * xq[k];
+            A[i][q] = sn * xp[k] + cs * xq[k];
+            const double vp = V[i][p], vq = V[i][q];
+            V[i][p] = cs * vp - sn * vq;
+            V[i][q] = sn * vp + cs * vq;
           }
         }
-        __syncwarp();
       }
-    if (rot == 0) break;
+      __syncwarp();
+    }
+    if (!__any_sync(0xffffffffu, rot)) break;
   }
   // sigma_j = |A_j|, u_j = A_j / sigma_j; t_j = u_j.g / sigma_j above the cut
   double sig = 0.0, smax = 0.0;

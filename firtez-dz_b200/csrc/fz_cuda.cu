@@ -1,19 +1,25 @@
 // firtez-dz B200: kernels and C-ABI of the Stokes synthesis path.
 //
 // Data flow of one fz_forward call (all on one stream):
-//   k_chain  one warp per column, FP64, lanes over the 92 elements: the
+//   k_saha   a warp per 64 temperature samples of a column and a third of the
+//            elements, FP64: the Saha factors of every sample the chain will
+//            need.
+//   k_chain  32 or 16 lanes per column, FP64, lanes over the 92 elements: the
 //            sequential part of FORWARD1D -- the GET_RHO warm-start chain along
 //            z and, in hydrostatic mode, the RK4 integration of ln Pg from the
 //            top.  Writes (nH, ne) per height to scratch and rho, Pe, mu, Pg
 //            into the output model.
-//   k_opac   one thread per (column, height), FP64: continuum/line opacity,
-//            damping, Doppler width, velocity shift and field geometry ->
-//            the per-column "opacity slab" (nz rows of SW floats) in scratch.
-//   k_synth  one CTA per column, one thread per wavelength, FP32: stages the
-//            slab in shared memory, walks the heights bottom -> top evaluating
-//            the Zeeman-split Voigt/Faraday profiles, the 4x4 evolution
-//            operator and the formal-solution recurrence, writes RSYN1D; one
-//            thread integrates log tau5.
+//   k_opac   one thread per (column, height), or per part of a row in small
+//            batches, FP64: continuum/line opacity, damping, Doppler width,
+//            velocity shift and field geometry -> the per-column "opacity
+//            slab" (nz rows of SW floats) in scratch.
+//   k_synth  one CTA per column, two wavelengths per thread, packed FP32:
+//            stages the slab in shared memory, walks the heights bottom ->
+//            top evaluating the Zeeman-split Voigt/Faraday profiles, the 4x4
+//            evolution operator and the formal-solution recurrence, writes
+//            RSYN1D; one warp forms log tau5.  Few columns take several
+//            heights at once, one to 64 columns k_layers (all heights) and
+//            k_layers_rte (the recurrence).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -109,7 +109,8 @@ __device__ __forceinline__ ExpF2 exp_parts2(F2 x) {
   return e;
 }
 
-// planck at two wavelengths (T and 1/T approximate in both halves).
+// c1 / (e^(c2/T) - 1) at two wavelengths, each quotient corrected by its
+// remainder (rt approximately 1/T).
 __device__ __forceinline__ F2 planck2(F2 c1, F2 c2, F2 T, F2 rt) {
   const F2 q0 = c2 * rt;
   const F2 m = exp_parts2(fma2(fma2(-q0, T, c2), rt, q0)).expm1();

@@ -5,9 +5,10 @@
 //    fixed point GET_RHO (src/chemical_equilibrium.f90:165-278, :1601-1701),
 //    continuum opacity (src/cont_opacity.f90:48-357), line opacity
 //    (src/line_opacity.f90:34-108) and damping (src/damping.f90:842-1012).
-//  * FP32, one thread per wavelength: Hui-Armstrong-Wray Voigt/Faraday
+//  * FP32, one wavelength: Hui-Armstrong-Wray Voigt/Faraday
 //    (src/voigt.f:17-98) and the Landi Degl'Innocenti evolution operator
-//    (src/rtesolver.f90:269-473) written on per-layer optical depths.
+//    (src/rtesolver.f90:269-473) written on per-layer optical depths
+//    (fz_layer2.cuh has the forms of two wavelengths a thread).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -41,7 +42,6 @@ constexpr double HPLA = 6.62606957e-27;
 constexpr double GRAV = 2.7414e4;
 constexpr double KC5THRESHOLD = 2.0e10;   // src/forward.f90:884
 
-__device__ __forceinline__ double spd(float x) { return (double)x; }
 
 // ------------------------------------------------------- partition functions
 __device__ __forceinline__ double horner_exact(const double* c, int n, double x) {
@@ -263,12 +263,6 @@ __device__ __forceinline__ void saha_prepare(WarpSahaT<L>& w, double T, const Co
     w.a2[j] = f.x;
     w.c[j] = f.y;
   }
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;   // xor butterfly: bit-identical in every lane
 }
 
 // One FP64 tensor-core product D = A B (8x4 by 4x8): a lane holds A(lane/4,
@@ -568,16 +562,6 @@ __device__ __forceinline__ float rsqrt_a(float y) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   return r;
-}
-
-// c1 / (e^(c2/T) - 1), each quotient corrected by its remainder.
-__device__ __forceinline__ float planck(float c1, float c2, float T) {
-  const float rt = rcp_a(T);
-  const float q0 = c2 * rt;
-  const float m = exp_parts(fmaf(fmaf(-q0, T, c2), rt, q0)).expm1();
-  const float rm = rcp_a(m);
-  const float s0 = c1 * rm;
-  return fmaf(fmaf(-s0, m, c1), rm, s0);
 }
 
 // The evolution operator of one layer (src/rtesolver.f90:269-473) from its

@@ -7,7 +7,8 @@
 //    and damping (src/damping.f90:878-1008).
 //  * FP32, one thread per wavelength: directional derivatives of the
 //    evolution operator (src/rtesolver.f90:476-1002) written on per-layer
-//    optical depths, in vector form.
+//    optical depths, in vector form, for regions of blended lines
+//    (fz_layer2.cuh has those of single lines).
 #pragma once
 #include "fz_physics.cuh"
 

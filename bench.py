@@ -254,9 +254,6 @@ CALIB_SEED = 909090
 C5_SEED = 5050
 
 
-SAHA_MAX_COLS = 1024   # batches up to this size run the chain on k_saha's precomputed Saha factors
-
-
 def probe_kernels(fz, lines, reg, nz, n):
     """One synthesis and one node-Jacobian call (fz_forward_device,
     fz_forward_rf_device) on n seeded columns of the workload, twice: every
@@ -277,10 +274,13 @@ def probe_kernels(fz, lines, reg, nz, n):
 
 def flops_table(csv_path, ncol, nz, numw, out_path):
     """FLOP per column of each kernel from an ncu CSV of --probe-kernels
-    (metrics smsp__sass_thread_inst_executed_op_{ffma,fadd,fmul,dfma,dadd,
-    dmul}_pred_on.sum): FP32 = 2 ffma + fadd + fmul, FP64 likewise, per
+    (metrics smsp__sass_thread_inst_executed_op_{ffma,ffma2,fadd,fadd2,fmul,
+    fmul2,dfma,dadd,dmul}_pred_on.sum): FP32 = 2 ffma + fadd + fmul, the
+    packed forms (two values an instruction) twice that, FP64 likewise, per
     launch over its ncol columns; the median over a kernel's launches.  A
-    kernel is bound by the pipe with more FLOP."""
+    kernel is bound by the pipe with more FLOP.  A CSV with k_saha holds the
+    chain on its precomputed factors: it adds k_saha and k_chain_pre to the
+    table of the other kernels (two CSVs, one without the chain)."""
     import csv
     import re
     rows = [r for r in csv.reader(open(csv_path)) if r]
@@ -289,13 +289,13 @@ def flops_table(csv_path, ncol, nz, numw, out_path):
     per = {}
     for r in rows[h + 1:]:
         rec = dict(zip(hdr, r))
-        name = re.search(r"(k_\w+)", rec["Kernel Name"]).group(1)
+        name = re.search(r"(k_\w+)", rec["Kernel Name"]).group(1).replace("k_synth_rf2", "k_synth_rf")
         v = float(rec["Metric Value"].replace(",", ""))
         per.setdefault((rec["ID"], name), {})[rec["Metric Name"]] = v
     acc = {}
     for (_, name), m in per.items():
         g = lambda op: m.get("smsp__sass_thread_inst_executed_op_%s_pred_on.sum" % op, 0.0)  # noqa: E731
-        f32 = 2 * g("ffma") + g("fadd") + g("fmul")
+        f32 = 2 * (g("ffma") + 2 * g("ffma2")) + g("fadd") + 2 * g("fadd2") + g("fmul") + 2 * g("fmul2")
         f64 = 2 * g("dfma") + g("dadd") + g("dmul")
         acc.setdefault(name, []).append((f32 / ncol, f64 / ncol, m.get("gpu__time_duration.sum", 0.0)))
     kern = {}
@@ -313,15 +313,14 @@ def flops_table(csv_path, ncol, nz, numw, out_path):
            "kernels": kern}
     old = json.load(open(out_path)) if os.path.exists(out_path) else {"_comment": "", "kernels": {}}
     if "k_saha" in kern:
-        # a small batch (at most SAHA_MAX_COLS columns) runs the chain on
-        # precomputed Saha factors: its two kernels join the table of the
-        # full-batch probe
+        # the chain on precomputed Saha factors: its two kernels join the
+        # table of the others
         doc = old
         doc["kernels"].update({"k_saha": kern["k_saha"], "k_chain_pre": kern["k_chain"]})
-        doc["_comment_small"] = ("k_saha and k_chain_pre (the chain of a batch of at most %d columns on precomputed "
-                                 "Saha factors) from --probe-kernels %d" % (SAHA_MAX_COLS, ncol))
+        doc["_comment_small"] = ("k_saha and k_chain_pre (the chain on precomputed Saha factors) from "
+                                 "--probe-kernels %d" % ncol)
     else:
-        # a full-batch table keeps the small-batch kernels of an earlier probe
+        # a table without the chain keeps the chain of an earlier probe
         for k in ("k_saha", "k_chain_pre"):
             if k in old.get("kernels", {}):
                 doc["kernels"][k] = old["kernels"][k]
@@ -1074,7 +1073,7 @@ def main():
         alg_col = a.nz * 6 * 4 + nf * 8 + np_ * nf * 4      # model in, RSYN1D + EQVDSYN out
     elif kname in ("k_opac_rf", "k_chemder"):
         alg_col = a.nz * 7 * 4                               # T, Pg, rho, Bx, By, Bz, vz in
-    elif kname == "k_chain":
+    elif kname in ("k_chain", "k_chain_pre"):
         alg_col = a.nz * (3 * 4 + 4 * 4 + 16)                # T, Pg, z in; Pg, rho, Pe, mu, (nH, ne) out
     elif kname == "k_synth":
         alg_col = nf * 8 + a.nz * 4                          # RSYN1D and log tau5 out

@@ -12,11 +12,12 @@
 // ms), and pieces of 512 KB cost half the calls of 256 KB ones (1.4 against
 // 1.9 ms).
 //
-// The ring (4 MB) belongs to one object, is allocated by its first copy of
-// STAGE_MIN or more (2 ms, less than that copy saves; 8 MB took up to 9) and
-// freed with it; the threads live for one call.  Below STAGE_MIN, starting
-// them (0.1 ms) and a first piece (0.1 ms) take most of what they save, and
-// where the ring cannot be had the plain copy does the work.
+// The ring (4 MB) belongs to one object and is freed with it; the threads live
+// for one call.  Pinning it takes 2 to 5 ms (8 MB up to 9), so an object gets
+// it once its copies have added up to STAGE_BUY, which by themselves cost as
+// much: a few small copies never pay for a ring.  Below STAGE_MIN, starting
+// the threads (0.1 ms) and a first piece (0.1 ms) take most of what they save,
+// and where the ring cannot be had the plain copy does the work.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -35,7 +36,7 @@
 namespace fzstage {
 
 constexpr int STAGE_THREADS = 4, STAGE_SLOTS = 8;
-constexpr size_t STAGE_PIECE = (size_t)512 << 10, STAGE_MIN = (size_t)4 << 20;
+constexpr size_t STAGE_PIECE = (size_t)512 << 10, STAGE_MIN = (size_t)4 << 20, STAGE_BUY = (size_t)32 << 20;
 
 struct Seg {   // one array
   void* dev;
@@ -71,7 +72,8 @@ class HostStage {
     size_t total = 0;
     for (int i = 0; i < nseg; ++i) total += segs[i].bytes;
     std::vector<Piece> pieces;
-    bool staged = total >= STAGE_MIN && reserve();
+    if (!buf_) moved_ += total;
+    bool staged = total >= STAGE_MIN && (buf_ || moved_ >= STAGE_BUY) && reserve();
     if (staged) {
       try {
         pieces.reserve(total / STAGE_PIECE + nseg);
@@ -101,6 +103,7 @@ class HostStage {
   };
   std::mutex mu_;   // one copy at a time: the ring is the object's
   unsigned char* buf_ = nullptr;
+  size_t moved_ = 0;   // bytes copied before the ring was there
   cudaEvent_t ev_[STAGE_SLOTS] = {};   // a slot's last copy
 
   void release() {

@@ -180,6 +180,7 @@ class HostStage {
     }
     stop.store(true);
     for (int k = 0; k < nt; ++k) th[k].join();
+    if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();   // of the queries, not an error
     return e;
   }
 };

@@ -3782,26 +3782,35 @@ __global__ void k_syn_to_v3(int npix, int nw, const double* __restrict__ syn, fl
 }
 
 // The RF payload of WRITE_RFS3D_V3 from fz_forward_rf_full's output: one
-// thread per (pixel, height, wavelength, Stokes) gathers the six parameters'
-// responses (for a warp: four Stokes rows, 8 consecutive wavelengths each)
-// and stores them as one run of six floats (a warp: 768 contiguous bytes).
-__global__ void k_rf_to_v3(int npix, int nz, int nw, const float* __restrict__ rf, float* __restrict__ out) {
-  const int nf = 4 * nw;
-  const size_t total = (size_t)npix * nz * nf;
+// thread per (pixel, height, wavelength) gathers the six parameters' responses
+// of the four Stokes components -- a warp reads 24 runs of 32 values -- and
+// stores them as one run of 24 floats, in 16-byte words where the payload's
+// base allows them.  Bound by its bytes (in once, out once): 256 pixels of 96
+// heights and 224 wavelengths 206 us (164 at the copy rate).  With a thread
+// per Stokes component the runs were of 8 values and the stores of 8 bytes:
+// 225 us; turning whole rows in shared memory took 363.
+__global__ void __launch_bounds__(256) k_rf_to_v3(int npix, int nz, int nw, const float* __restrict__ rf,
+                                                  float* __restrict__ out) {
+  const size_t nf = 4 * (size_t)nw, total = (size_t)npix * nz * nw;
+  const bool vec = ((uintptr_t)out & 15) == 0;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i % nf);   // w * 4 + s
-    const size_t pk = i / nf;      // p * nz + k
-    const size_t p = pk / nz;
-    const int k = (int)(pk % nz);
-    const int w = r >> 2, s = r & 3;
-    const float* src = rf + (p * 6 * nz + k) * nf + s * nw + w;
-    float v[6];
+    const size_t pk = i / nw;      // p * nz + k
+    const int w = (int)(i % nw);
+    const size_t p = pk / nz, k = pk % nz;
+    const float* src = rf + (p * 6 * nz + k) * nf + w;
+    float v[24];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) v[q] = src[(size_t)q * nz * nf];
-    float2* d = reinterpret_cast<float2*>(out + i * 6);
-    d[0] = make_float2(v[0], v[1]);
-    d[1] = make_float2(v[2], v[3]);
-    d[2] = make_float2(v[4], v[5]);
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) v[6 * s + q] = __ldcs(src + (size_t)q * nz * nf + (size_t)s * nw);
+    float* d = out + i * 24;
+    if (vec) {
+#pragma unroll
+      for (int s = 0; s < 24; s += 4) __stcs(reinterpret_cast<float4*>(d + s), make_float4(v[s], v[s + 1], v[s + 2], v[s + 3]));
+    } else {
+#pragma unroll
+      for (int s = 0; s < 24; s += 2) *reinterpret_cast<float2*>(d + s) = make_float2(v[s], v[s + 1]);
+    }
   }
 }
 
@@ -3952,7 +3961,7 @@ int fz_syn_to_v3_device(int npix, int nw, const double* d_syn, float* d_stokes, 
 int fz_rf_to_v3_device(int npix, int nz, int nw, const float* d_rf, float* d_out, void* stream) {
   if (npix <= 0 || nz <= 0 || nw <= 0 || !d_rf || !d_out) return FZ_ERR_ARG;
   if (((uintptr_t)d_out & 7) != 0) return FZ_ERR_ARG;   // float2 stores
-  k_rf_to_v3<<<grid_for((size_t)npix * nz * 4 * nw, 256), 256, 0, (cudaStream_t)stream>>>(npix, nz, nw, d_rf, d_out);
+  k_rf_to_v3<<<grid_for((size_t)npix * nz * nw, 256), 256, 0, (cudaStream_t)stream>>>(npix, nz, nw, d_rf, d_out);
   return cuda_fail(cudaGetLastError());
 }
 

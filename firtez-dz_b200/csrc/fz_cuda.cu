@@ -157,8 +157,7 @@ __global__ void __launch_bounds__(128, PRE ? CHAIN_PRE_CTAS : 4) k_chain(const C
   // of the list leaves before any work
   const int count = list ? *nlist : ncol;
   if ((gate > 0 && count > gate) || (gate < 0 && count <= -gate)) return;
-  const int end = PRE ? min(count, c0 + cn) : count;
-  const int first = PRE ? c0 : 0;
+  const int end = min(count, c0 + cn), first = c0;
   if (first + (int)((blockIdx.x * (size_t)blockDim.x) / L) >= end) return;
   __shared__ Consts K;
   copy_to_shared(&K, Kg);
@@ -2641,9 +2640,6 @@ int copies_done() { return cuda_fail(cudaStreamSynchronize(cudaStreamLegacy)); }
 // two columns) whose rows stay within SAHA_MAX_BYTES.
 constexpr int SAHA_CHUNK_SM = 40;
 constexpr size_t SAHA_MAX_BYTES = (size_t)5 << 29;
-// Listed batches (an inversion pool's occupied slots, counted on the device)
-// of at most this many columns take a warp per column.
-constexpr int CHAIN_LIST_32 = 1024;
 // Parts of a slab row that k_opac / k_opac_rf run in CTAs of their own: all of
 // them while `cells` threads do not give every SM two CTAs of 256 (129,000 cells: 45 us
 // in one thread each, 52 apart).
@@ -2742,10 +2738,15 @@ struct ProfScope {
 };
 
 // k_chain with wpb warps per block and lanes (32 or 16) lanes per column;
-// lanes = 0 picks 16 when the batch fills 8 warps per SM with two columns a
-// warp (throughput: half the warp instructions per column) and 32 below
-// (latency: every column's chain gets a warp of its own).  chem: the (nH, ne)
-// scratch of the batch, the context's own buffer when null.
+// lanes = 0 picks 16 for chunks that fill 8 warps per SM with two columns a
+// warp (throughput: half the warp instructions per column; 3,100 columns of 128
+// heights 1.03 ms against 1.19, 5,920 1.34 and 1.83) and 32 below (latency:
+// every column's chain gets a warp of its own; 2,048 columns 0.80 ms against
+// 0.96).  A batch's last chunk takes its own size's form: the 580 columns that
+// 6,500 leave over the first chunk cost as much as a full chunk with 16 lanes
+// (6,500 columns 2.24 -> 1.78 ms, 12,000 3.54 -> 3.10).  A listed batch launches
+// both forms for its first chunk, each gated by the count on the device.
+// chem: the (nH, ne) scratch of the batch, the context's own buffer when null.
 void launch_k_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, int* d_status, int hydrostatic, int wpb,
                     int lanes, cudaStream_t s, double2* chem = nullptr, const int* list = nullptr,
                     const int* nlist = nullptr, bool pre = true) {
@@ -2756,10 +2757,11 @@ void launch_k_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, in
     k_chain_med<<<g, 128, 0, s>>>(c->d_consts, c->d_pf, ncol, c->nz, d_model, d_mout, chem, d_status);
     return;
   }
-  const bool autol = lanes != 16 && lanes != 32;
-  if (autol) lanes = ncol >= 16 * c->nsm ? 16 : 32;
   const int nsamp = hydrostatic ? 2 * c->nz - 1 : c->nz;
   pre = pre && c->saha_cols > 0;
+  const bool autol = lanes != 16 && lanes != 32;
+  const int few = 16 * c->nsm - 1;   // columns that take a warp each
+  if (autol) lanes = ncol > few ? 16 : 32;
   auto chain = [&](auto he, auto lc, auto pc, int c0, int cn, int gate) {
     constexpr bool HE = decltype(he)::value, PRE = decltype(pc)::value;
     constexpr int L = decltype(lc)::value;
@@ -2776,13 +2778,16 @@ void launch_k_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, in
     else
       l == 16 ? chain(std::false_type{}, C16{}, pc, c0, cn, gate) : chain(std::false_type{}, C32{}, pc, c0, cn, gate);
   };
-  if (!pre) {
-    chain_l(std::false_type{}, lanes, 0, ncol, 0);
+  if (!pre) {   // the same chunks, so that a column takes the same form
+    const int per = list ? ncol : saha_chunk_cols(c, ncol);
+    for (int c0 = 0; c0 < ncol; c0 += per) {
+      const int cn = std::min(per, ncol - c0);
+      chain_l(std::false_type{}, autol && !list && cn <= few ? 32 : lanes, c0, cn, 0);
+    }
     return;
   }
-  // a listed batch's first chunk launches both forms, each gated by the count
-  const int gate = list && autol && lanes == 16 ? CHAIN_LIST_32 : 0;
   const int per = std::min(c->saha_cols, ncol);
+  const int gate = list && autol && lanes == 16 ? std::min(few, per) : 0;
   for (int c0 = 0; c0 < ncol; c0 += per) {
     const int cn = std::min(per, ncol - c0);
     {
@@ -2801,7 +2806,7 @@ void launch_k_chain(fz_ctx* c, int ncol, const float* d_model, float* d_mout, in
                                          nlist);
     }
     if (gate && c0 == 0) chain_l(std::true_type{}, 32, 0, std::min(cn, gate), gate);
-    chain_l(std::true_type{}, lanes, c0, cn, -gate);
+    chain_l(std::true_type{}, autol && !list && cn <= few ? 32 : lanes, c0, cn, -gate);
   }
 }
 

@@ -2635,6 +2635,24 @@ int cuda_fail(cudaError_t e) {
 // travels on.  To be called between such copies and a launch that reads them.
 int copies_done() { return cuda_fail(cudaStreamSynchronize(cudaStreamLegacy)); }
 
+// Opt kernel K in to launches with up to `bytes` of dynamic shared memory.  The
+// limit is the kernel's on its device, not a context's: it goes to the most
+// that the device has beside K's static arrays, once and for all sizes, so
+// that no context (or thread) lowers it under the launches of another.
+template <auto K>
+int allow_smem(size_t bytes) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a{};
+  FZ_CK(cudaGetDevice(&dev));
+  FZ_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  FZ_CK(cudaFuncGetAttributes(&a, K));
+  const int most = optin - (int)a.sharedSizeBytes;
+  if (most < 0 || bytes > (size_t)most) return cuda_fail(cudaErrorInvalidValue);
+  return a.maxDynamicSharedSizeBytes == most
+             ? 0
+             : cuda_fail(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+}
+
 // k_chain runs on precomputed Saha factors (k_saha's rows), in chunks of at
 // most SAHA_CHUNK_SM columns per SM (a full wave of 16-lane chains: 20 warps of
 // two columns) whose rows stay within SAHA_MAX_BYTES.
@@ -2826,7 +2844,7 @@ int launch_lsf(fz_ctx* c, T* d_data, long long nrows, int rows_per_col, cudaStre
   for (int r = 0; r < c->nreg; ++r)
     if (L.valid[r]) nmax = std::max(nmax, c->regs[r].numwave);
   const size_t smem = lsf_smem(nmax);
-  if (smem > 48 * 1024) FZ_CK(cudaFuncSetAttribute(k_lsf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) FZ_CK_RC(allow_smem<k_lsf<T>>(smem));
   const int threads = 32 * std::min(8, (nmax + LSF_TILE - 1) / LSF_TILE);
   const long long ncol = nrows / rows_per_col, work = ncol * ((rows_per_col + 3) / 4);
   const dim3 grid((unsigned)std::min<long long>(work, (long long)c->nsm * 32), c->nreg);
@@ -2967,27 +2985,29 @@ void launch_synth_rf(fz_ctx* c, int ncol, int hydrostatic, double* d_syn, float*
     launch_synth_rf_t<false, FULL>(c, ncol, d_syn, d_jac, d_oscr, d_mout, d_status, s, list, nlist);
 }
 
+// allow_smem with all of the SM's unified storage as shared memory.
+template <auto K>
+int allow_carveout(size_t bytes) {
+  FZ_CK_RC(allow_smem<K>(bytes));
+  return cuda_fail(cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+}
+
 // Opt in to the dynamic shared memory that launch_synth_rf<FULL> uses (to be
 // called before any stream capture), all of the SM's unified storage as shared
 // memory so that two CTAs can be resident.
 template <bool FULL>
 int prepare_synth_rf(fz_ctx* c) {
-  auto set = [&](auto kern, size_t sms) -> int {
-    FZ_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms));
-    FZ_CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    return 0;
-  };
   const int w = has_blends(c) ? 0 : rf2_warps(c, FULL);
   if (w > 0) {
     const size_t sms = rf2_smem(c, FULL, w);
-    FZ_CK_RC(set(k_synth_rf2<true, FULL>, sms));
-    return set(k_synth_rf2<false, FULL>, sms);
+    FZ_CK_RC((allow_carveout<k_synth_rf2<true, FULL>>(sms)));
+    return allow_carveout<k_synth_rf2<false, FULL>>(sms);
   }
   const size_t sms = FULL ? rf_smem_full(c) : rf_smem(c);
-  FZ_CK_RC(set(k_synth_rf<true, FULL, 256>, sms));
-  FZ_CK_RC(set(k_synth_rf<false, FULL, 256>, sms));
-  FZ_CK_RC(set(k_synth_rf<true, FULL, 512>, sms));
-  return set(k_synth_rf<false, FULL, 512>, sms);
+  FZ_CK_RC((allow_carveout<k_synth_rf<true, FULL, 256>>(sms)));
+  FZ_CK_RC((allow_carveout<k_synth_rf<false, FULL, 256>>(sms)));
+  FZ_CK_RC((allow_carveout<k_synth_rf<true, FULL, 512>>(sms)));
+  return allow_carveout<k_synth_rf<false, FULL, 512>>(sms);
 }
 
 // The response-function kernels run one thread per wavelength in blocks of
@@ -4515,28 +4535,18 @@ int fz_create(fz_ctx** out, const fz_line* lines, int nlines, const fz_region* r
     cudaFree(d_st);
     if (rc) return fail(rc);
   }
-  // opt in to large dynamic shared memory for the slab staging
-  const int sms = nz * c->sw * (int)sizeof(float);
-  if (sms > 48 * 1024 - (int)sizeof(SynthP) - 16 &&
-      (rc = cuda_fail(cudaFuncSetAttribute(k_synth<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sms))))
-    return fail(rc);
-  const size_t rsm = layers_rte_smem(nz);
-  if (rsm > 48 * 1024 &&
-      (rc = cuda_fail(cudaFuncSetAttribute(k_layers_rte, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm))))
-    return fail(rc);
+  // large dynamic shared memory for the slab staging
+  if ((rc = allow_smem<k_synth<1>>(synth_smem(c, 1)))) return fail(rc);
+  if ((rc = allow_smem<k_layers_rte>(layers_rte_smem(nz)))) return fail(rc);
   // several heights at once: blocks of at most 512 threads (two heights: below
   // that, so that two CTAs share an SM; a table of 256 threads gains nothing),
   // room for their layers beside the slab
   if (4 * c->npt <= 512 && synth_smem(c, 4) <= 200 * 1024) {
-    if ((rc = cuda_fail(cudaFuncSetAttribute(k_synth<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)synth_smem(c, 4)))))
-      return fail(rc);
+    if ((rc = allow_smem<k_synth<4>>(synth_smem(c, 4)))) return fail(rc);
     c->synth_g |= 4;
   }
   if (2 * c->npt < 512 && synth_smem(c, 2) <= 200 * 1024) {
-    if ((rc = cuda_fail(cudaFuncSetAttribute(k_synth<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)synth_smem(c, 2)))))
-      return fail(rc);
+    if ((rc = allow_smem<k_synth<2>>(synth_smem(c, 2)))) return fail(rc);
     c->synth_g |= 2;
   }
   *out = c;

@@ -2533,7 +2533,8 @@ struct fz_ctx {
   PairP* d_pairs = nullptr;   // npt entries: k_synth's wavelengths by thread
   int npt = 0;
   F2* d_lay = nullptr;         // the layers of up to lay_cols columns (k_layers)
-  int lay_cols = 0;
+  int lay_cols = 0, lay_want = 0, lay_nold = 0;
+  F2* lay_old[8] = {};         // smaller ones before it (SYNTH_FEW doublings at most)
   int synth_g = 0;             // the numbers of heights at once (4, 2) that k_synth can take
   bool pairs_even = false;     // its warps of equal cost
   bool pairs_vec = false;      // every entry two wavelengths from an even one, NUMW even
@@ -2677,6 +2678,34 @@ int synth_few_cols(const fz_ctx* c) {
   return (int)std::min<size_t>(SYNTH_FEW, SYNTH_LAY_BYTES / per);
 }
 
+// The layers of a few columns (launch_synth; without them k_synth runs, the
+// same bits).  Batches smaller than the scratch ask for them too, so what they
+// had before stays until the context ends -- a graph that a caller captured
+// keeps its pointer -- and the capacity at least doubles (all of it within 2
+// SYNTH_LAY_BYTES).  Never to be called while a stream is captured.
+void ensure_layers(fz_ctx* c, int ncol) {
+  const int few = synth_few_cols(c);
+  if (ncol > few || ncol <= c->lay_want) return;
+  const int n = std::min(few, std::max(ncol, 2 * c->lay_cols));
+  c->lay_want = ncol;   // memory that is not to be had is asked for once
+  F2* p = nullptr;
+  if (cudaMalloc(&p, (size_t)n * c->nz * LAYER2_F2 * c->npt * sizeof(F2)) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (c->d_lay) c->lay_old[c->lay_nold++] = c->d_lay;
+  c->d_lay = p;
+  c->lay_cols = c->lay_want = n;
+}
+
+// True while s is being captured (or may not be asked, for another's capture).
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 int ensure_scratch(fz_ctx* c, int ncol) {
   if ((size_t)ncol > c->scratch_cols) {
     cudaFree(c->d_slab);
@@ -2687,17 +2716,6 @@ int ensure_scratch(fz_ctx* c, int ncol) {
     FZ_CK(cudaMalloc(&c->d_slab, (size_t)ncol * c->nz * c->sw * sizeof(float)));
     FZ_CK(cudaMalloc(&c->d_chem, (size_t)ncol * c->nz * sizeof(double2)));
     c->scratch_cols = ncol;
-  }
-  // a few columns' layers (launch_synth); without the memory k_synth runs
-  const int few = synth_few_cols(c);
-  if (ncol <= few && ncol > c->lay_cols) {
-    cudaFree(c->d_lay);
-    c->d_lay = nullptr;
-    c->lay_cols = 0;
-    if (cudaMalloc(&c->d_lay, (size_t)ncol * c->nz * LAYER2_F2 * c->npt * sizeof(F2)) == cudaSuccess)
-      c->lay_cols = ncol;
-    else
-      cudaGetLastError();
   }
   const int want = saha_chunk_cols(c, ncol);
   if (want > c->saha_want) {
@@ -2907,6 +2925,7 @@ int launch_forward(fz_ctx* c, int ncol, const float* d_model, int hydrostatic, d
                    int* d_status, cudaStream_t s, const int* list = nullptr, const int* nlist = nullptr) {
   int rc = ensure_scratch(c, ncol);
   if (rc) return rc;
+  if (!list && !capturing(s)) ensure_layers(c, ncol);
   if (d_status) FZ_CK(cudaMemsetAsync(d_status, 0, ncol * sizeof(int), s));
   launch_k_chain(c, ncol, d_model, d_mout, d_status, hydrostatic, c->tune.chain_warps, c->tune.chain_lanes, s,
                  nullptr, list, nlist);
@@ -4640,6 +4659,7 @@ int fz_destroy(fz_ctx* c) {
   cudaFree(c->d_lam);
   cudaFree(c->d_pairs);
   cudaFree(c->d_lay);
+  for (F2* p : c->lay_old) cudaFree(p);
   cudaFree(c->d_gain);
   cudaFree(c->d_slab);
   cudaFree(c->d_chem);
@@ -5020,6 +5040,7 @@ int fz_invert_device(fz_ctx* c, int npix, const double* d_obs, const float* d_in
     }
     return hq.done >= npix ? 0 : FZ_ERR_STATE;
   }
+  ensure_layers(c, std::min(S, synth_few_cols(c)));   // of the tail's pools, before their captures
   int graph_n = -1;
   const float* graph_pool = nullptr;
   for (long long it = 0; it < cap; ++it) {

@@ -741,7 +741,8 @@ __device__ __forceinline__ bool synth_layer(const SynthP& P, const PairP& pr, co
 }
 
 __device__ __forceinline__ F2 synth_planck(const PairP& pr, float T) {
-  return planck2(f2(pr.c1[0], pr.c1[1]), f2(pr.c2[0], pr.c2[1]), f2(T), f2(rcp_a(T)));
+  const F2 em1 = exp_parts2(planck_q2(f2(pr.c2[0], pr.c2[1]), T, rcp_a(T))).expm1();
+  return planck_s2(f2(pr.c1[0], pr.c1[1]), em1, rcp2(em1));
 }
 
 // CALCULATE_EQUIVALENT_SYN1D: x GAIN, Stokes-major.  Returns true if a value is
@@ -771,9 +772,9 @@ __device__ __forceinline__ bool synth_store(const PairP& pr, const F2 I[4], cons
 // loop reaches 89 %) -- 38 operations a component and some 130 for the Planck
 // function, the operator and the formal-solution step of a layer, at each
 // wavelength.  65,536 columns of 128 heights, two lines of 112 wavelengths: 61.1
-// ms with the operator's 16 elements formed from CUDA's sinh, sin and exp, 37.9
-// with rte_layer one wavelength a thread, 34.4 with two; four lines on 4,087
-// columns of 160 heights 12.3, 7.4, 6.3.  The error against 64 bits halved
+// ms with the operator's 16 elements formed from CUDA's sinh, sin and exp, 37.9 on
+// the three scalar functions one wavelength a thread, 34.4 with two; four lines on
+// 4,087 columns of 160 heights 12.3, 7.4, 6.3.  The error against 64 bits halved
 // (relative 6.4e-7 -> 2.9e-7).
 //
 // G > 1, for batches that leave the SMs waiting on a few columns' chains: G
@@ -1741,10 +1742,9 @@ __global__ void __launch_bounds__(128, 2) k_synth_rf2(
         const float2 tf = *reinterpret_cast<const float2*>(row);
         const float rt = rcp_a(tf.x);
         // c1 / (e^q - 1), q = c2 / T, and its T derivative S (q / T) e^q / (e^q - 1)
-        const F2 c1 = f2(pr.c1[0], pr.c1[1]), c2 = f2(pr.c2[0], pr.c2[1]);
-        const F2 q0 = c2 * f2(rt), q = fma2(fma2(-q0, f2(tf.x), c2), f2(rt), q0);
+        const F2 q = planck_q2(f2(pr.c2[0], pr.c2[1]), tf.x, rt);
         const F2 em1 = exp_parts2(q).expm1(), rm = rcp2(em1);
-        const F2 S0 = c1 * rm, S = fma2(fma2(-S0, em1, c1), rm, S0);
+        const F2 S = planck_s2(f2(pr.c1[0], pr.c1[1]), em1, rm);
         if (k == 0 || tf.y != 0.0f) {   // SET_BOUNDARY
           I[0] = S;
           I[1] = I[2] = I[3] = ZERO;
@@ -1827,8 +1827,6 @@ __global__ void __launch_bounds__(128, 2) k_synth_rf2(
 #pragma unroll
         for (int i = 1; i < 4; ++i)
           n[i] = fma2(O[4 * i + 3], win[3], fma2(O[4 * i + 2], win[2], fma2(O[4 * i + 1], win[1], O[4 * i] * win[0])));
-        Resp2 R;
-        resp_w(L, win, R);
         const float* ckr = FULL ? nullptr : coef + k * np;
         // the response of parameter slot p into its nodes (or out, FULL)
         auto put = [&](int p, const F2 rf[4]) {
@@ -1849,6 +1847,8 @@ __global__ void __launch_bounds__(128, 2) k_synth_rf2(
             }
           }
         };
+        Resp2 R;
+        resp_w(L, win, R);
         // optical-depth derivatives of the form a (h0, f0) + b (th, tf)
         auto dir = [&](F2 a, F2 b, const Tri& th, const Tri& tf_, F2 c0, F2 rf[4]) {
           const F2 l = fma2(a, h0.l, b * th.l), m = fma2(a, f0.l, b * tf_.l);
@@ -3501,47 +3501,63 @@ __global__ void __launch_bounds__(128) k_ws_expand(int npix, int nz, RFConf R, c
 }
 
 // The formal solution alone on given absorption matrices (SET_BOUNDARY +
-// OLD_ANALYTICAL_SOLVER): one thread per (column, wavelength), the height
-// recursion of the synthesis kernel with the layer optical depths
-// eta * dz (dz from the reference's rule: z_{k+1} - z_k, the top height's
+// OLD_ANALYTICAL_SOLVER), on the synthesis kernels' layers: one thread per
+// column and two wavelengths, their height recursion with the layer optical
+// depths eta * dz (dz from the reference's rule: z_{k+1} - z_k, the top height's
 // backward difference).  eta (nw, 7, nz, ncol), src (nw, nz, ncol), bnd
 // (nz, ncol) or null, out (4, nw, ncol).
 __global__ void k_rte(int ncol, int nz, int nw, const float* __restrict__ eta, const float* __restrict__ src,
                       const double* __restrict__ zz, const int* __restrict__ bnd, double* __restrict__ out) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)ncol * nw) return;
-  const int col = (int)(idx / nw), l = (int)(idx % nw);
-  float I0 = 0.f, I1 = 0.f, I2 = 0.f, I3 = 0.f;
+  const int npair = (nw + 1) / 2;
+  if (idx >= (long long)ncol * npair) return;
+  const int col = (int)(idx / npair), l = 2 * (int)(idx % npair), m = min(l + 1, nw - 1);
+  F2 I[4] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
   for (int k = 0; k < nz; ++k) {
-    const float S = src[((size_t)col * nz + k) * nw + l];
+    const float* sk = src + ((size_t)col * nz + k) * nw;
+    Layer2 L;
+    L.S = f2(sk[l], sk[m]);
     if (k == 0 || (bnd && bnd[(size_t)col * nz + k])) {
-      I0 = S;
-      I1 = I2 = I3 = 0.f;
+      I[0] = L.S;
+      I[1] = I[2] = I[3] = f2(0.f);
       continue;
     }
     const double dz = 1e5 * fabs(k == nz - 1 ? zz[k] - zz[k - 1] : zz[k + 1] - zz[k]);
-    const float* e = eta + ((size_t)col * nz + k) * 7 * nw + l;
-    float t[7];
+    const float* e = eta + ((size_t)col * nz + k) * 7 * nw;
+    auto depth = [&](int i) {
+      const float* q = e + (size_t)i * nw;
+      return f2((float)((double)q[l] * dz), (float)((double)q[m] * dz));
+    };
 #pragma unroll
-    for (int i = 0; i < 7; ++i) t[i] = (float)((double)e[(size_t)i * nw] * dz);
-    rte_layer(t[0], t[1], t[2], t[3], t[4], t[5], t[6], S, I0, I1, I2, I3);
+    for (int i = 0; i < 3; ++i) {
+      L.t[i] = depth(1 + i);
+      L.r[i] = depth(4 + i);
+    }
+    layer_set(L, depth(0));
+    layer_apply(L, I);
   }
   double* o = out + ((size_t)col * nw + l) * 4;
-  o[0] = I0;
-  o[1] = I1;
-  o[2] = I2;
-  o[3] = I3;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a, b;
+    f2_get(I[i], a, b);
+    o[i] = a;
+    if (m > l) o[4 + i] = b;
+  }
 }
 
-// VOIGT on arrays: the FP32 Voigt/Faraday-Voigt pair of the synthesis kernels.
+// VOIGT on arrays: the FP32 Voigt/Faraday-Voigt pair of the synthesis kernels,
+// two arguments a thread.
 __global__ void k_voigt(int n, const float* __restrict__ a, const float* __restrict__ v, float* __restrict__ h,
                         float* __restrict__ f) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= n) return;
-  float hh, ff;
-  voigt_f32(a[i], v[i], hh, ff);
-  h[i] = hh;
-  f[i] = ff;
+  const int j = min(i + 1, n - 1);
+  const F2 aa = f2(a[i], a[j]);
+  F2 wh, wf, id;
+  voigt_w2(VoigtA{aa, aa + aa, aa * aa}, f2(v[i], v[j]), wh, wf, id);
+  f2_get(wh * id, h[i], h[j]);
+  f2_get(wf * id, f[i], f[j]);
 }
 
 __global__ void k_tau5(int ncol, int nz, int sw, const float* __restrict__ slab, float* __restrict__ mout) {
@@ -5487,7 +5503,7 @@ int fz_lm_rearange(fz_ctx* c, int npix, float* models, const double* delta, int 
 int fz_rte_solve_device(int ncol, int nz, int nw, const float* d_eta, const float* d_src, const double* d_zz,
                         const int* d_bnd, double* d_out, void* stream) {
   if (ncol <= 0 || nz <= 1 || nw <= 0 || !d_eta || !d_src || !d_zz || !d_out) return FZ_ERR_ARG;
-  const long long n = (long long)ncol * nw;
+  const long long n = (long long)ncol * ((nw + 1) / 2);
   k_rte<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(ncol, nz, nw, d_eta, d_src, d_zz, d_bnd,
                                                                           d_out);
   return cuda_fail(cudaGetLastError());
@@ -5527,7 +5543,7 @@ int fz_voigt(int n, const float* a, const float* v, float* h, float* f) {
   int rc = cuda_fail(cudaMemcpy(d, a, b, cudaMemcpyHostToDevice));
   if (!rc) rc = cuda_fail(cudaMemcpy(d + n, v, b, cudaMemcpyHostToDevice));
   if (!rc) {
-    k_voigt<<<(n + 255) / 256, 256>>>(n, d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n);
+    k_voigt<<<(n + 511) / 512, 256>>>(n, d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n);
     rc = cuda_fail(cudaGetLastError());
   }
   if (!rc) rc = cuda_fail(cudaMemcpy(h, d + 2 * (size_t)n, b, cudaMemcpyDeviceToHost));

@@ -83,7 +83,11 @@ __device__ __forceinline__ void voigt_w2(const VoigtA& A, F2 u, F2& h, F2& f, F2
   f = u * fma2(p0, q1, -(p1 * q0));
 }
 
-// exp_parts at two arguments.
+// e^x = S (1 + p) with S a power of two: the reduction by ln 2 in two parts
+// (Cody & Waite, Software Manual for the Elementary Functions, 1980, ch. 6)
+// and p = e^r - 1 on |r| <= ln2/2 (weighted least-maximum fit of degree 6,
+// relative error 1.7e-8), so that e^x and e^x - 1 both come without
+// cancellation.  S is cut to 2^-126 .. 2^127; NaN gives NaN.
 struct ExpF2 {
   F2 S, p;
   __device__ __forceinline__ F2 exp() const { return fma2(S, p, S); }
@@ -109,33 +113,52 @@ __device__ __forceinline__ ExpF2 exp_parts2(F2 x) {
   return e;
 }
 
-// c1 / (e^(c2/T) - 1) at two wavelengths, each quotient corrected by its
-// remainder (rt approximately 1/T).
-__device__ __forceinline__ F2 planck2(F2 c1, F2 c2, F2 T, F2 rt) {
-  const F2 q0 = c2 * rt;
-  const F2 m = exp_parts2(fma2(fma2(-q0, T, c2), rt, q0)).expm1();
-  const F2 rm = rcp2(m);
+// c2 / T at two wavelengths, the quotient corrected by its remainder (rt
+// approximately 1/T).
+__device__ __forceinline__ F2 planck_q2(F2 c2, float T, float rt) {
+  const F2 q0 = c2 * f2(rt);
+  return fma2(fma2(-q0, f2(T), c2), f2(rt), q0);
+}
+// c1 / em1 with em1 = e^(c2/T) - 1 and rm approximately its reciprocal.
+__device__ __forceinline__ F2 planck_s2(F2 c1, F2 em1, F2 rm) {
   const F2 s0 = c1 * rm;
-  return fma2(fma2(-s0, m, c1), rm, s0);
+  return fma2(fma2(-s0, em1, c1), rm, s0);
 }
 
-// The functions of evol_abg from the roots, at two arguments of which one at
-// least is above the series' limit, with what their derivatives need: x, y,
-// 1/theta, sinh x, cosh x, sin y, cos y.
+// The evolution operator of one layer (src/rtesolver.f90:269-473) from its
+// optical-depth increments t = eta dz, written on three scalar functions of
+// d = |eta|^2 - |rho|^2 and e = eta.rho (x = lambda_1 dz, y = lambda_2 dz with
+// sign(x y) = sign(e), x^2 - y^2 = d, x y = e, theta = x^2 + y^2):
+//   O = e^-tI { (1 + am) 1 - al X - be Y + ga M }
+//   am = (cosh x + cos y) / 2 - 1,  al = (x sinh x + y sin y) / theta,
+//   be = (x sin y - y sinh x) / theta,  ga = (cosh x - cos y) / theta,
+// where X has the elements of (eta, rho), Y those of (-rho, eta) and M is the
+// reference's M4 before its factor 2/theta.  The functions are entire in d
+// and e^2: where both are below 1/4 (a layer of optical depth up to about 1/2:
+// most of an atmosphere) their series have no quotient by theta and no root;
+// above, from the roots, with the reference's clamp of cosh and sinh at 2^53
+// (-> 1e15, :464-465).  A half far below the limit beside one above takes the
+// series too: the quotients lose its digits as theta goes to 0 (a derivative
+// some 1e-7 / theta, at 0 everything); one little below it takes the roots,
+// whose code is running.
+
+// From the roots, with what the derivatives need: x, y, 1/theta, sinh x, cosh
+// x, sin y, cos y.
 struct Roots2 {
   F2 am, al, be, ga, x, y, it, sh, ch, sy, cy;
 };
 __device__ __forceinline__ Roots2 roots2(F2 d, F2 e) {
-  // the guards keep a half whose matrix vanishes finite beside one above the limit
+  // R = theta / 2 and 1/R, then the larger root and its reciprocal (one Newton
+  // step each: about 1 ulp)
   float d0, d1;
   f2_get(d, d0, d1);
   Roots2 o;
-  const F2 TINY = f2(1.0e-37f), HALF = f2(0.5f);
-  const F2 z = fma2(f2(0.25f) * d, d, fma2(e, e, TINY));
+  const F2 HALF = f2(0.5f);
+  const F2 z = fma2(f2(0.25f) * d, d, e * e);
   F2 g = rsqrt2(z);
   g = fma2(HALF * g, fma2(-z * g, g, f2(1.0f)), g);
   const F2 ad = f2(fabsf(d0), fabsf(d1));
-  const F2 w = fma2(z, g, fma2(HALF, ad, TINY));
+  const F2 w = fma2(z, g, HALF * ad);
   F2 k = rsqrt2(w);
   k = fma2(HALF * k, fma2(-w * k, k, f2(1.0f)), k);
   const F2 big = w * k, small = e * k;
@@ -205,35 +228,67 @@ __device__ __forceinline__ Roots2 roots2(F2 d, F2 e) {
   return o;
 }
 
-// evol_abg at two arguments: the series where it holds for both.
-struct EvolABG2 {
-  F2 am, al, be, ga;
-};
-__device__ __forceinline__ EvolABG2 evol_abg2(F2 d, F2 e) {
-  EvolABG2 o;
+// Whether both halves are below the series' limit, and which of them is far
+// enough below it to take the series beside one above.
+constexpr float EVOL_TINY = 1.0f / 64.0f;
+__device__ __forceinline__ bool evol_low(F2 d, F2 e) {
   float d0, d1, e0, e1;
   f2_get(d, d0, d1);
   f2_get(e, e0, e1);
-  if (fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(e0), fabsf(e1))) <= 0.25f) {
-    const F2 ee = e * e, dd = d * d;
-    const F2 g1 = dd + ee, g2 = fma2(f2(2.0f), ee, dd), g3 = d * g2;
-    const F2 g4 = d * fma2(f2(3.0f), ee, dd), g5 = fma2(g2, g2, f2(-2.0f) * (ee * ee));
-    o.al = fma2(g3, f2(1.0f / 5040.0f), fma2(g1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
-    o.be = -e * fma2(g3, f2(1.0f / 362880.0f), fma2(g1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
-    o.ga = fma2(g3, f2(1.0f / 40320.0f), fma2(g1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
-    o.am = fma2(g5, f2(1.0f / 80640.0f), fma2(g4, f2(1.0f / 1440.0f), fma2(g2, f2(1.0f / 48.0f), f2(0.25f) * d)));
-    return o;
-  }
+  return fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(e0), fabsf(e1))) <= 0.25f;
+}
+struct Low2 {
+  bool a, b;
+};
+__device__ __forceinline__ Low2 evol_low2(F2 d, F2 e) {
+  float d0, d1, e0, e1;
+  f2_get(d, d0, d1);
+  f2_get(e, e0, e1);
+  return Low2{fmaxf(fabsf(d0), fabsf(e0)) <= EVOL_TINY, fmaxf(fabsf(d1), fabsf(e1)) <= EVOL_TINY};
+}
+__device__ __forceinline__ void low_put(const Low2& w, F2& x, F2 y) {   // y in the halves w
+  float x0, x1, y0, y1;
+  f2_get(x, x0, x1);
+  f2_get(y, y0, y1);
+  x = f2(w.a ? y0 : x0, w.b ? y1 : x1);
+}
+
+// The four functions at two arguments.
+struct EvolABG2 {
+  F2 am, al, be, ga;
+};
+__device__ __forceinline__ EvolABG2 evol_series2(F2 d, F2 e) {
+  EvolABG2 o;
+  const F2 ee = e * e, dd = d * d;
+  const F2 g1 = dd + ee, g2 = fma2(f2(2.0f), ee, dd), g3 = d * g2;
+  const F2 g4 = d * fma2(f2(3.0f), ee, dd), g5 = fma2(g2, g2, f2(-2.0f) * (ee * ee));
+  o.al = fma2(g3, f2(1.0f / 5040.0f), fma2(g1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
+  o.be = -e * fma2(g3, f2(1.0f / 362880.0f), fma2(g1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
+  o.ga = fma2(g3, f2(1.0f / 40320.0f), fma2(g1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
+  o.am = fma2(g5, f2(1.0f / 80640.0f), fma2(g4, f2(1.0f / 1440.0f), fma2(g2, f2(1.0f / 48.0f), f2(0.25f) * d)));
+  return o;
+}
+__device__ __forceinline__ EvolABG2 evol_abg2(F2 d, F2 e) {
+  if (evol_low(d, e)) return evol_series2(d, e);
+  const Low2 w = evol_low2(d, e);
   const Roots2 R = roots2(d, e);
-  o.am = R.am;
-  o.al = R.al;
-  o.be = R.be;
-  o.ga = R.ga;
+  EvolABG2 o{R.am, R.al, R.be, R.ga};
+  if (__builtin_expect(w.a || w.b, 0)) {
+    const EvolABG2 q = evol_series2(d, e);
+    low_put(w, o.am, q.am);
+    low_put(w, o.al, q.al);
+    low_put(w, o.be, q.be);
+    low_put(w, o.ga, q.ga);
+  }
   return o;
 }
 
-// What the formal solution needs of one layer at two wavelengths (rte_layer,
-// fz_physics.cuh): I <- I - om0 w0 - E um.I, ... with w0 = I0 - S.
+// What the formal solution needs of one layer at two wavelengths: one height of
+// OLD_ANALYTICAL_SOLVER (src/rtesolver.f90:163-187), I <- (1 - O) S e0 + O I,
+// applied as I + O (I - S e0) + S e0 row by row without forming O.  The
+// operator's vectors are u = al eta - be rho and v = al rho + be eta, and 1 - O(1,1)
+// = om0 comes without cancellation from e^-tI - 1: I <- I - om0 w0 - E um.I, ...
+// with w0 = I0 - S.
 struct Layer2 {
   F2 S, om0, E, dg, ga, t[3], r[3], um[3], up[3], v[3];
 };
@@ -283,8 +338,9 @@ __device__ __forceinline__ bool layer_set(Layer2& L, F2 tI) {
       put(L.up[i], 0.0f);
       put(L.v[i], 0.0f);
     }
+    return true;
   }
-  return b0 || b1;
+  return false;
 }
 
 __device__ __forceinline__ void layer_apply(const Layer2& L, F2 I[4]) {
@@ -310,31 +366,29 @@ __device__ __forceinline__ void layer_apply(const Layer2& L, F2 I[4]) {
 struct EvolD2 {
   F2 am, al, be, ga, al_d, al_e, be_d, be_e, ga_d, ga_e;
 };
-__device__ __forceinline__ EvolD2 evol_d2(F2 d, F2 e) {
+__device__ __forceinline__ EvolD2 evol_series_d2(F2 d, F2 e) {
   EvolD2 o;
-  float d0, d1, e0, e1;
-  f2_get(d, d0, d1);
-  f2_get(e, e0, e1);
-  if (fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(e0), fabsf(e1))) <= 0.25f) {
-    const F2 ee = e * e, dd = d * d;
-    const F2 s1 = dd + ee, s2 = fma2(f2(2.0f), ee, dd), s3 = d * s2;
-    const F2 s4 = d * fma2(f2(3.0f), ee, dd), s5 = fma2(s2, s2, f2(-2.0f) * (ee * ee));
-    const F2 u2 = fma2(f2(3.0f), dd, f2(2.0f) * ee);                        // d s3 / d d
-    const F2 u3 = d * fma2(f2(4.0f), dd, f2(6.0f) * ee);                    // d (d^4 + 3 d^2 e^2 + e^4) / d d
-    const F2 u4 = fma2(f2(6.0f), dd, f2(4.0f) * ee);                        // ... / d e, over e
-    o.al = fma2(s3, f2(1.0f / 5040.0f), fma2(s1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
-    o.al_d = fma2(u3, f2(1.0f / 362880.0f), fma2(u2, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 60.0f), f2(1.0f / 6.0f))));
-    o.al_e = e * fma2(u4, f2(1.0f / 362880.0f), fma2(d, f2(1.0f / 1260.0f), f2(1.0f / 60.0f)));
-    o.be = -e * fma2(s3, f2(1.0f / 362880.0f), fma2(s1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
-    o.be_d = -e * fma2(u2, f2(1.0f / 362880.0f), fma2(d, f2(1.0f / 2520.0f), f2(1.0f / 120.0f)));
-    o.be_e = -fma2(d * fma2(f2(6.0f), ee, dd), f2(1.0f / 362880.0f),
-                   fma2(fma2(f2(3.0f), ee, dd), f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
-    o.ga = fma2(s3, f2(1.0f / 40320.0f), fma2(s1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
-    o.ga_d = fma2(u3, f2(1.0f / 3628800.0f), fma2(u2, f2(1.0f / 40320.0f), fma2(d, f2(1.0f / 360.0f), f2(1.0f / 24.0f))));
-    o.ga_e = e * fma2(u4, f2(1.0f / 3628800.0f), fma2(d, f2(1.0f / 10080.0f), f2(1.0f / 360.0f)));
-    o.am = fma2(s5, f2(1.0f / 80640.0f), fma2(s4, f2(1.0f / 1440.0f), fma2(s2, f2(1.0f / 48.0f), f2(0.25f) * d)));
-    return o;
-  }
+  const F2 ee = e * e, dd = d * d;
+  const F2 s1 = dd + ee, s2 = fma2(f2(2.0f), ee, dd), s3 = d * s2;
+  const F2 s4 = d * fma2(f2(3.0f), ee, dd), s5 = fma2(s2, s2, f2(-2.0f) * (ee * ee));
+  const F2 u2 = fma2(f2(3.0f), dd, f2(2.0f) * ee);                        // d s3 / d d
+  const F2 u3 = d * fma2(f2(4.0f), dd, f2(6.0f) * ee);                    // d (d^4 + 3 d^2 e^2 + e^4) / d d
+  const F2 u4 = fma2(f2(6.0f), dd, f2(4.0f) * ee);                        // ... / d e, over e
+  o.al = fma2(s3, f2(1.0f / 5040.0f), fma2(s1, f2(1.0f / 120.0f), fma2(d, f2(1.0f / 6.0f), f2(1.0f))));
+  o.al_d = fma2(u3, f2(1.0f / 362880.0f), fma2(u2, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 60.0f), f2(1.0f / 6.0f))));
+  o.al_e = e * fma2(u4, f2(1.0f / 362880.0f), fma2(d, f2(1.0f / 1260.0f), f2(1.0f / 60.0f)));
+  o.be = -e * fma2(s3, f2(1.0f / 362880.0f), fma2(s1, f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
+  o.be_d = -e * fma2(u2, f2(1.0f / 362880.0f), fma2(d, f2(1.0f / 2520.0f), f2(1.0f / 120.0f)));
+  o.be_e = -fma2(d * fma2(f2(6.0f), ee, dd), f2(1.0f / 362880.0f),
+                 fma2(fma2(f2(3.0f), ee, dd), f2(1.0f / 5040.0f), fma2(d, f2(1.0f / 120.0f), f2(1.0f / 6.0f))));
+  o.ga = fma2(s3, f2(1.0f / 40320.0f), fma2(s1, f2(1.0f / 720.0f), fma2(d, f2(1.0f / 24.0f), f2(0.5f))));
+  o.ga_d = fma2(u3, f2(1.0f / 3628800.0f), fma2(u2, f2(1.0f / 40320.0f), fma2(d, f2(1.0f / 360.0f), f2(1.0f / 24.0f))));
+  o.ga_e = e * fma2(u4, f2(1.0f / 3628800.0f), fma2(d, f2(1.0f / 10080.0f), f2(1.0f / 360.0f)));
+  o.am = fma2(s5, f2(1.0f / 80640.0f), fma2(s4, f2(1.0f / 1440.0f), fma2(s2, f2(1.0f / 48.0f), f2(0.25f) * d)));
+  return o;
+}
+__device__ __forceinline__ EvolD2 evol_roots_d2(F2 d, F2 e) {
+  EvolD2 o;
   const Roots2 R = roots2(d, e);
   o.am = R.am;
   o.al = R.al;
@@ -355,6 +409,25 @@ __device__ __forceinline__ EvolD2 evol_d2(F2 d, F2 e) {
   o.ga_e = it * fma2(it, xy, -(o.ga * e4));
   return o;
 }
+__device__ __forceinline__ EvolD2 evol_d2(F2 d, F2 e) {
+  if (evol_low(d, e)) return evol_series_d2(d, e);
+  const Low2 w = evol_low2(d, e);
+  EvolD2 o = evol_roots_d2(d, e);
+  if (__builtin_expect(w.a || w.b, 0)) {
+    const EvolD2 q = evol_series_d2(d, e);
+    low_put(w, o.am, q.am);
+    low_put(w, o.al, q.al);
+    low_put(w, o.be, q.be);
+    low_put(w, o.ga, q.ga);
+    low_put(w, o.al_d, q.al_d);
+    low_put(w, o.al_e, q.al_e);
+    low_put(w, o.be_d, q.be_d);
+    low_put(w, o.be_e, q.be_e);
+    low_put(w, o.ga_d, q.ga_d);
+    low_put(w, o.ga_e, q.ga_e);
+  }
+  return o;
+}
 
 // A layer of the response-function kernel: its operator O and what the
 // derivatives need.
@@ -371,9 +444,11 @@ __device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
   F2 er = fma2(L.t[2], L.r[2], fma2(L.t[1], L.r[1], L.t[0] * L.r[0]));
   float c0, c1;
   f2_get(tI + (eta2 + rho2), c0, c1);
-  const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
+  bool gap = false;
   L.on = f2(1.0f);
+  const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
   if (b0 || b1) {
+    gap = true;
     auto zero = [&](F2& x) {
       float a, b;
       f2_get(x, a, b);
@@ -413,7 +488,7 @@ __device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
     L.O[4 * (1 + j) + 1 + k] = s + v;
     L.O[4 * (1 + k) + 1 + j] = s - v;
   }
-  return b0 || b1;
+  return gap;
 }
 
 __device__ __forceinline__ F2 dot3(const F2 a[3], const F2 b[3]) { return fma2(a[2], b[2], fma2(a[1], b[1], a[0] * b[0])); }

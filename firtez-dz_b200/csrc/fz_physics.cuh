@@ -533,143 +533,11 @@ constexpr float SIN_Q0 = -0.166666597f, SIN_Q1 = 0.00833306648f, SIN_Q2 = -0.000
 constexpr float COS_Q0 = -0.5f, COS_Q1 = 0.0416666418f, COS_Q2 = -0.00138884038f, COS_Q3 = 2.47618755e-05f, COS_Q4 = -2.60769184e-07f;
 constexpr float PI_F_HI = 3.140625f, PI_F_MID = 0.000967502594f, PI_F_LO = 1.50995803e-07f;
 
-// e^x = S (1 + p) with S a power of two: the reduction by ln 2 in two parts
-// and p = e^r - 1 on |r| <= ln2/2 (weighted least-maximum fit of degree 6,
-// relative error 1.7e-8), so that e^x and e^x - 1 both come without
-// cancellation.  S is cut to 2^-126 .. 2^127; NaN gives NaN.
-struct ExpF {
-  float S, p;
-  __device__ __forceinline__ float exp() const { return fmaf(S, p, S); }
-  __device__ __forceinline__ float expm1() const { return fmaf(S, p, S - 1.0f); }
-};
-__device__ __forceinline__ ExpF exp_parts(float x) {
-  const float MAGIC = 12582912.0f;   // 1.5 * 2^23
-  const float t = fmaf(x, 1.4426950408889634f, MAGIC), n = t - MAGIC;
-  const float r = fmaf(n, -1.428606765330187e-06f, fmaf(n, -0.693145751953125f, x));
-  float q = fmaf(r, EXP_Q4, EXP_Q3);
-  q = fmaf(r, q, EXP_Q2);
-  q = fmaf(r, q, EXP_Q1);
-  q = fmaf(r, q, EXP_Q0);
-  ExpF e;
-  e.p = fmaf(r * r, q, r);
-  const int i = min(max(__float_as_int(t) - 0x4b400000, -126), 127);
-  e.S = __int_as_float((i + 127) << 23);
-  return e;
-}
-
 // 1/sqrt(y), approximate.
 __device__ __forceinline__ float rsqrt_a(float y) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   return r;
-}
-
-// The evolution operator of one layer (src/rtesolver.f90:269-473) from its
-// optical-depth increments t = eta dz, written on three scalar functions of
-// d = |eta|^2 - |rho|^2 and e = eta.rho (x = lambda_1 dz, y = lambda_2 dz with
-// sign(x y) = sign(e), x^2 - y^2 = d, x y = e, theta = x^2 + y^2):
-//   O = e^-tI { (1 + am) 1 - al X - be Y + ga M }
-//   am = (cosh x + cos y) / 2 - 1,  al = (x sinh x + y sin y) / theta,
-//   be = (x sin y - y sinh x) / theta,  ga = (cosh x - cos y) / theta,
-// where X has the elements of (eta, rho), Y those of (-rho, eta) and M is the
-// reference's M4 before its factor 2/theta.
-struct EvolABG {
-  float am, al, be, ga;
-};
-
-// The four functions.  They are entire in d and e^2: where both are below
-// 1/4 (a layer of optical depth up to about 1/2: most of an atmosphere) their
-// series have no quotient by theta and no root; above, from the roots, with
-// the reference's clamp of cosh and sinh at 2^53 (-> 1e15, :464-465).
-__device__ __forceinline__ EvolABG evol_abg(float d, float e) {
-  EvolABG o;
-  if (fmaxf(fabsf(d), fabsf(e)) <= 0.25f) {
-    const float e2 = e * e, d2 = d * d;
-    const float f1 = d2 + e2, f2 = fmaf(2.0f, e2, d2), f3 = d * f2;
-    const float g3 = d * fmaf(3.0f, e2, d2), h4 = fmaf(f2, f2, -2.0f * (e2 * e2));
-    o.al = fmaf(f3, 1.0f / 5040.0f, fmaf(f1, 1.0f / 120.0f, fmaf(d, 1.0f / 6.0f, 1.0f)));
-    o.be = -e * fmaf(f3, 1.0f / 362880.0f, fmaf(f1, 1.0f / 5040.0f, fmaf(d, 1.0f / 120.0f, 1.0f / 6.0f)));
-    o.ga = fmaf(f3, 1.0f / 40320.0f, fmaf(f1, 1.0f / 720.0f, fmaf(d, 1.0f / 24.0f, 0.5f)));
-    o.am = fmaf(h4, 1.0f / 80640.0f, fmaf(g3, 1.0f / 1440.0f, fmaf(f2, 1.0f / 48.0f, 0.25f * d)));
-    return o;
-  }
-  // R = theta / 2 and 1/R, then the larger root and its reciprocal (one
-  // Newton step each: about 1 ulp)
-  const float z = fmaf(0.25f * d, d, e * e);
-  float g = rsqrt_a(z);
-  g = fmaf(0.5f * g, fmaf(-z * g, g, 1.0f), g);
-  const float w = fmaf(z, g, 0.5f * fabsf(d));
-  float k = rsqrt_a(w);
-  k = fmaf(0.5f * k, fmaf(-w * k, k, 1.0f), k);
-  const float big = w * k, small = e * k;
-  const float x = d >= 0.0f ? big : small, y = d >= 0.0f ? small : big;
-  // sinh x and sinh^2(x/2) from e^(x/2) - 1
-  const ExpF ex = exp_parts(0.5f * x);
-  const float t = ex.expm1(), v = ex.exp();
-  float ri = rcp_a(v);
-  ri = fmaf(ri, fmaf(-v, ri, 1.0f), ri);
-  const float tr = t * ri, s2 = t + tr;   // 2 sinh(x/2)
-  float a = 0.25f * (s2 * s2), sh = s2 * fmaf(0.5f * t, tr, 1.0f);
-  // sin y and sin^2(y/2) from the half angle modulo pi (either sign of both
-  // factors gives the same products)
-  const float hy = 0.5f * y;
-  float sn, cs;
-  if (fabsf(hy) < 3.0e4f) {
-    const float n = rintf(hy * 0.3183098861837907f);
-    const float r = fmaf(n, -PI_F_LO, fmaf(n, -PI_F_MID, fmaf(n, -PI_F_HI, hy)));
-    const float ss = r * r;
-    sn = fmaf(r * ss, fmaf(ss, fmaf(ss, fmaf(ss, SIN_Q3, SIN_Q2), SIN_Q1), SIN_Q0), r);
-    cs = fmaf(ss, fmaf(ss, fmaf(ss, fmaf(ss, fmaf(ss, COS_Q4, COS_Q3), COS_Q2), COS_Q1), COS_Q0), 1.0f);
-  } else {
-    sn = sinf(hy);
-    cs = cosf(hy);
-  }
-  const float b = sn * sn, sy = 2.0f * (sn * cs);
-  float q = a + b;
-  o.am = a - b;
-  if (fabsf(x) >= 37.42994775f) {   // cosh, sinh >= 2^53 in float64
-    const float c2 = fmaf(-2.0f, b, 1.0f);
-    sh = copysignf(1e15f, x);
-    o.am = 0.5f * (1e15f + c2) - 1.0f;
-    q = 0.5f * (1e15f - c2);
-  }
-  const float it = 0.5f * g;
-  o.al = fmaf(x, sh, y * sy) * it;
-  o.be = fmaf(x, sy, -(y * sh)) * it;
-  o.ga = q * g;
-  return o;
-}
-
-// One height of OLD_ANALYTICAL_SOLVER (src/rtesolver.f90:163-187), I <- (1 - O)
-// S e0 + O I, applied as I + O (I - S e0) + S e0 row by row without forming O:
-// the operator's vectors are al eta - be rho and al rho + be eta, and 1 - O(1,1)
-// comes without cancellation from e^-tI - 1.  A non-finite matrix counts as
-// the identity (returns true), as in the reference.
-__device__ __forceinline__ bool rte_layer(float tI, float tQ, float tU, float tV, float rQ, float rU, float rV,
-                                          float S, float& I0, float& I1, float& I2, float& I3) {
-  const float eta2 = fmaf(tV, tV, fmaf(tU, tU, tQ * tQ)), rho2 = fmaf(rV, rV, fmaf(rU, rU, rQ * rQ));
-  if (!(fabsf(tI + (eta2 + rho2)) < 3.0e38f)) return true;
-  const float e = fmaf(tV, rV, fmaf(tU, rU, tQ * rQ));
-  const EvolABG f = evol_abg(eta2 - rho2, e);
-  const ExpF ex = exp_parts(-tI);
-  const float E = ex.exp(), gh = f.ga * (0.5f * (eta2 + rho2));
-  const float om0 = -fmaf(E, f.am + gh, ex.expm1());
-  const float uQ = fmaf(f.al, tQ, -(f.be * rQ)), uU = fmaf(f.al, tU, -(f.be * rU)), uV = fmaf(f.al, tV, -(f.be * rV));
-  const float vQ = fmaf(f.al, rQ, f.be * tQ), vU = fmaf(f.al, rU, f.be * tU), vV = fmaf(f.al, rV, f.be * tV);
-  const float cQ = f.ga * fmaf(tU, rV, -(tV * rU)), cU = f.ga * fmaf(tV, rQ, -(tQ * rV)),
-              cV = f.ga * fmaf(tQ, rU, -(tU * rQ));
-  const float w0 = I0 - S;
-  const float ge = f.ga * fmaf(tV, I3, fmaf(tU, I2, tQ * I1)), gr = f.ga * fmaf(rV, I3, fmaf(rU, I2, rQ * I1));
-  const float dg = (1.0f - gh) + f.am;
-  const float n0 = fmaf(uV - cV, I3, fmaf(uU - cU, I2, (uQ - cQ) * I1));
-  const float n1 = fmaf(rQ, gr, fmaf(tQ, ge, fmaf(vV, I2, fmaf(-vU, I3, fmaf(dg, I1, -((uQ + cQ) * w0))))));
-  const float n2 = fmaf(rU, gr, fmaf(tU, ge, fmaf(vQ, I3, fmaf(-vV, I1, fmaf(dg, I2, -((uU + cU) * w0))))));
-  const float n3 = fmaf(rV, gr, fmaf(tV, ge, fmaf(vU, I1, fmaf(-vQ, I2, fmaf(dg, I3, -((uV + cV) * w0))))));
-  I0 = fmaf(-E, n0, fmaf(-om0, w0, I0));
-  I1 = E * n1;
-  I2 = E * n2;
-  I3 = E * n3;
-  return false;
 }
 
 // Evolution operator O of one layer from its optical-depth increments

@@ -87,15 +87,24 @@ __device__ __forceinline__ void voigt_w2(const VoigtA& A, F2 u, F2& h, F2& f, F2
 // (Cody & Waite, Software Manual for the Elementary Functions, 1980, ch. 6)
 // and p = e^r - 1 on |r| <= ln2/2 (weighted least-maximum fit of degree 6,
 // relative error 1.7e-8), so that e^x and e^x - 1 both come without
-// cancellation.  S is cut to 2^-126 .. 2^127; NaN gives NaN.
+// cancellation; NaN gives NaN.  S is 0 below 2^-126 and 2^127 at most, which
+// serves arguments up to 2^22 ln 2 above; further down r leaves its interval
+// and p its range, so depths from DEPTH_RARE on are cut to 104 first.
+constexpr float DEPTH_RARE = 1.0e12f;
 struct ExpF2 {
   F2 S, p;
   __device__ __forceinline__ F2 exp() const { return fma2(S, p, S); }
   __device__ __forceinline__ F2 expm1() const { return fma2(S, p, S + f2(-1.0f)); }
 };
 __device__ __forceinline__ float exp_scale(float t) {
-  const int i = min(max(__float_as_int(t) - 0x4b400000, -126), 127);
+  const int i = min(max(__float_as_int(t) - 0x4b400000, -127), 127);
   return __int_as_float((i + 127) << 23);
+}
+// An optical depth, or 104 above it, where e^-x is 0.
+__device__ __forceinline__ F2 depth_cut2(F2 x) {
+  float a, b;
+  f2_get(x, a, b);
+  return f2(min_nan(a, 104.0f), min_nan(b, 104.0f));
 }
 __device__ __forceinline__ ExpF2 exp_parts2(F2 x) {
   const float MAGIC = 12582912.0f;
@@ -303,6 +312,8 @@ __device__ __forceinline__ bool layer_set(Layer2& L, F2 tI) {
   const F2 sum = eta2 + rho2;
   float c0, c1;
   f2_get(tI + sum, c0, c1);
+  const bool rare = !(fabsf(c0) < DEPTH_RARE) || !(fabsf(c1) < DEPTH_RARE);
+  if (__builtin_expect(rare, 0)) tI = depth_cut2(tI);
   const EvolABG2 f = evol_abg2(eta2 - rho2, er);
   const ExpF2 ex = exp_parts2(-tI);
   const F2 gh = f.ga * (f2(0.5f) * sum);
@@ -320,7 +331,7 @@ __device__ __forceinline__ bool layer_set(Layer2& L, F2 tI) {
     L.v[i] = fma2(f.al, L.r[i], f.be * L.t[i]);
   }
   const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
-  if (b0 || b1) {
+  if (__builtin_expect(rare && (b0 || b1), 0)) {
     auto put = [&](F2& x, float v) {
       float a, b;
       f2_get(x, a, b);
@@ -446,9 +457,10 @@ __device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
   f2_get(tI + (eta2 + rho2), c0, c1);
   bool gap = false;
   L.on = f2(1.0f);
-  const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
-  if (b0 || b1) {
-    gap = true;
+  if (__builtin_expect(!(fabsf(c0) < DEPTH_RARE) || !(fabsf(c1) < DEPTH_RARE), 0)) {
+    const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
+    gap = b0 || b1;
+    tI = depth_cut2(tI);
     auto zero = [&](F2& x) {
       float a, b;
       f2_get(x, a, b);

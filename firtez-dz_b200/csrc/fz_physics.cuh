@@ -533,6 +533,13 @@ constexpr float SIN_Q0 = -0.166666597f, SIN_Q1 = 0.00833306648f, SIN_Q2 = -0.000
 constexpr float COS_Q0 = -0.5f, COS_Q1 = 0.0416666418f, COS_Q2 = -0.00138884038f, COS_Q3 = 2.47618755e-05f, COS_Q4 = -2.60769184e-07f;
 constexpr float PI_F_HI = 3.140625f, PI_F_MID = 0.000967502594f, PI_F_LO = 1.50995803e-07f;
 
+// The smaller of two values; NaN if either is.
+__device__ __forceinline__ float min_nan(float x, float y) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+  return r;
+}
+
 // 1/sqrt(y), approximate.
 __device__ __forceinline__ float rsqrt_a(float y) {
   float r;

@@ -86,6 +86,11 @@ __host__ __device__ inline int slab_w(int nreg, int nlu) {
   return (w + 3) & ~3;
 }
 constexpr int SLAB_LINE = 4;
+// The T of a row, for the Planck function: T = 0 (a masked column) and what is
+// next to it count as 0.1 K, where the function is 0 from 500 A to 1 mm and its
+// argument c2/T still exact for exp_parts2.  NaN stays NaN.
+constexpr float SLAB_TMIN = 0.1f;
+__device__ __forceinline__ float slab_t(float T) { return fabsf(T) < SLAB_TMIN ? SLAB_TMIN : T; }
 __host__ __device__ inline int slab_geo(int nlu) { return 4 + 4 * nlu; }
 __host__ __device__ inline int slab_kc(int nlu) { return 4 + 4 * nlu + 6; }
 
@@ -585,7 +590,7 @@ __global__ void __launch_bounds__(256) k_opac(const DevParams* __restrict__ Pg, 
       if (opac_mine<SPLIT>(1 + r)) row[slab_kc(P.nlu) + r] = (float)(opac_continuum(T, nelec, nhyd, P.cont[r]) * dz);
     if (opac_mine<SPLIT>(0)) {
       const double kc5 = opac_continuum(T, nelec, nhyd, P.cont[P.nreg]) / nhyd * (1.0 / MAMU);
-      row[0] = Tf;
+      row[0] = slab_t(Tf);
       row[1] = (kc5 < KC5THRESHOLD) ? 0.0f : 1.0f;
       row[2] = (float)kc5;
       row[3] = mget(m, nz, 2, k);
@@ -1207,7 +1212,7 @@ __global__ void __launch_bounds__(256) k_opac_rf(const DevParams* __restrict__ P
     float* row = slab + i * sw;
     if (opac_mine<SPLIT>(0)) {
       const double kc5 = opac_continuum(T, nelec, nhyd, P.cont[P.nreg]) / nhyd * (1.0 / MAMU);
-      row[0] = Tf;
+      row[0] = slab_t(Tf);
       row[1] = (kc5 < KC5THRESHOLD) ? 0.0f : 1.0f;
       row[2] = (float)kc5;
       row[3] = mget(m, nz, 2, k);

@@ -123,7 +123,7 @@ __device__ __forceinline__ ExpF2 exp_parts2(F2 x) {
 }
 
 // c2 / T at two wavelengths, the quotient corrected by its remainder (rt
-// approximately 1/T).
+// approximately 1/T; T of a slab row, so at least SLAB_TMIN or below 0).
 __device__ __forceinline__ F2 planck_q2(F2 c2, float T, float rt) {
   const F2 q0 = c2 * f2(rt);
   return fma2(fma2(-q0, f2(T), c2), f2(rt), q0);

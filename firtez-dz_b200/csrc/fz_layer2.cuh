@@ -446,7 +446,7 @@ struct LayerD2 {
   F2 t[3], r[3], c[3], h, E, om0;   // c = eta x rho, h = (|eta|^2 + |rho|^2) / 2
   EvolD2 f;
   F2 O[16];
-  F2 on;   // 1; 0 in a half whose matrix is not finite (the identity there, without response)
+  unsigned long long on;   // all bits, but none of a half whose matrix is not finite: the identity, without response
 };
 
 __device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
@@ -456,10 +456,11 @@ __device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
   float c0, c1;
   f2_get(tI + (eta2 + rho2), c0, c1);
   bool gap = false;
-  L.on = f2(1.0f);
+  L.on = ~0ull;
   if (__builtin_expect(!(fabsf(c0) < DEPTH_RARE) || !(fabsf(c1) < DEPTH_RARE), 0)) {
     const bool b0 = !(fabsf(c0) < 3.0e38f), b1 = !(fabsf(c1) < 3.0e38f);
     gap = b0 || b1;
+    L.on = (b0 ? 0ull : 0xffffffffull) | (b1 ? 0ull : 0xffffffff00000000ull);
     tI = depth_cut2(tI);
     auto zero = [&](F2& x) {
       float a, b;
@@ -470,7 +471,6 @@ __device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
     zero(eta2);
     zero(rho2);
     zero(er);
-    zero(L.on);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       zero(L.t[i]);
@@ -531,14 +531,13 @@ __device__ __forceinline__ void resp_w(const LayerD2& L, const F2 w[4], Resp2& R
     M[1 + i] = fma2(L.t[i], ew, fma2(L.r[i], rw, -fma2(L.c[i], w[0], L.h * wv[i])));
   }
   mat4(L.O, w, R.Ow);
-  const F2 E = L.E * L.on;
+  const F2 E = L.E;
   const F2 md = E * (f2(0.25f) * f.al), me = E * (f2(-0.5f) * f.be);
   const F2 ad = E * f.al_d, ae = E * f.al_e, bd = E * f.be_d, be = E * f.be_e, gd = E * f.ga_d, ge = E * f.ga_e;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     R.Ad[i] = fma2(gd, M[i], fma2(-bd, Y[i], fma2(-ad, X[i], md * w[i])));
     R.Ae[i] = fma2(ge, M[i], fma2(-be, Y[i], fma2(-ae, X[i], me * w[i])));
-    R.Ow[i] = R.Ow[i] * L.on;
   }
   const F2 al = E * f.al, bt = E * f.be, ga = E * f.ga;
 #pragma unroll
@@ -553,6 +552,7 @@ __device__ __forceinline__ void resp_w(const LayerD2& L, const F2 w[4], Resp2& R
 __device__ __forceinline__ void resp_dir(const LayerD2& L, const Resp2& R, F2 dI, const F2 dt[3], const F2 dr[3], F2 o[4]) {
   const F2 dd = f2(2.0f) * (dot3(L.t, dt) - dot3(L.r, dr)), de = dot3(L.r, dt) + dot3(L.t, dr);
   o[0] = fma2(R.Ad[0], dd, fma2(R.Ae[0], de, fma2(-dI, R.Ow[0], dot3(R.r, dt) - dot3(R.q, dr))));
+  o[0].v &= L.on;   // where the matrix is not finite neither are the changes of its depths
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const int j = (i + 1) % 3, k = (i + 2) % 3;
@@ -560,6 +560,7 @@ __device__ __forceinline__ void resp_dir(const LayerD2& L, const Resp2& R, F2 dI
     v = fma2(dt[j], R.q[k], fma2(-dt[k], R.q[j], v));
     v = fma2(dr[j], R.r[k], fma2(-dr[k], R.r[j], v));
     o[1 + i] = fma2(R.Ad[1 + i], dd, fma2(R.Ae[1 + i], de, fma2(-dI, R.Ow[1 + i], v)));
+    o[1 + i].v &= L.on;
   }
 }
 

@@ -1904,9 +1904,14 @@ __global__ void __launch_bounds__(128, 2) k_synth_rf2(
         dir(f2(dl[1]), f2(ln.x * (2.0f * dl[3])), tri(ca[0], ca[1], ca[2], ga.x, ga.y), tri(av[0], av[1], av[2], ga.x, ga.y),
             f2(dkc[k * sw + 1]), rf);
         if (HE) {
-          const F2 pg2 = f2(p0 ? pgk : 0.0f, p1 ? pgk : 0.0f);   // where skipped H stays (OH = H there)
+          // where skipped H stays (OH = H there), whatever the response
 #pragma unroll
-          for (int i = 0; i < 4; ++i) H[i] = fma2(rf[i], pg2, OH[i]);
+          for (int i = 0; i < 4; ++i) {
+            float a, b, ha, hb;
+            f2_get(fma2(rf[i], f2(pgk), OH[i]), a, b);
+            f2_get(OH[i], ha, hb);
+            H[i] = f2(p0 ? a : ha, p1 ? b : hb);
+          }
         }
         put(1, rf);
         if (HE) {

@@ -483,9 +483,17 @@ __device__ __forceinline__ bool layer_d2(LayerD2& L, F2 tI) {
   L.E = ex.exp();
   L.h = f2(0.5f) * (eta2 + rho2);
   const F2 gh = f.ga * L.h;
-  L.om0 = -fma2(L.E, f.am + gh, ex.expm1());
+  const F2 ag = f.am + gh;
+  L.om0 = -fma2(L.E, ag, ex.expm1());
   const F2 dg = L.E * ((f2(1.0f) - gh) + f.am), ga = L.E * f.ga;
-  L.O[0] = f2(1.0f) - L.om0;
+  {
+    // O(1,1) = E (1 + am + gh): as 1 - om0 where that holds more digits, in thin layers
+    float m0, m1, a0, a1, e0, e1;
+    f2_get(L.om0, m0, m1);
+    f2_get(f2(1.0f) - L.om0, a0, a1);
+    f2_get(fma2(L.E, ag, L.E), e0, e1);
+    L.O[0] = f2(m0 < 0.5f ? a0 : e0, m1 < 0.5f ? a1 : e1);
+  }
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const int j = (i + 1) % 3, k = (i + 2) % 3;

@@ -96,9 +96,11 @@ struct ExpF2 {
   __device__ __forceinline__ F2 exp() const { return fma2(S, p, S); }
   __device__ __forceinline__ F2 expm1() const { return fma2(S, p, S + f2(-1.0f)); }
 };
+// 2^n from t = n + 1.5 * 2^23, cut on the bits of t itself: any float may come
+// here, and the difference of its bits to that constant's may leave an int.
 __device__ __forceinline__ float exp_scale(float t) {
-  const int i = min(max(__float_as_int(t) - 0x4b400000, -127), 127);
-  return __int_as_float((i + 127) << 23);
+  const int i = min(max(__float_as_int(t), 0x4b400000 - 127), 0x4b400000 + 127);
+  return __int_as_float((i - 0x4b400000 + 127) << 23);
 }
 // An optical depth, or 104 above it, where e^-x is 0.
 __device__ __forceinline__ F2 depth_cut2(F2 x) {

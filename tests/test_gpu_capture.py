@@ -68,3 +68,35 @@ def test_a_captured_small_batch_after_a_large_one(fz):
     run(7)      # outside a capture the layers are there again
     torch.cuda.synchronize()
     assert torch.equal(syn[:7], want[0]) and torch.equal(out[:7], want[1])
+
+
+def test_a_captured_batch_keeps_its_layers(fz):
+    """A graph captured while the context holds layers for 7 columns, replayed after
+    batches that needed more of them."""
+    import torch
+    nz, n = 32, 60
+    lines = fz.lines_parse(fz.atmos.line_database_text())
+    ctx = fz.Synthesis(lines, fz.regions_from_lines_section("1 48 -505.25 21.5\n2 48 -505.25 21.5\n", lines), nz=nz)
+    m = torch.from_numpy(fz.atmos.make_columns(100, nz, seed=2)).cuda()
+    syn = torch.empty((100, 4, ctx.numw), dtype=torch.float64, device="cuda")
+    out = torch.empty_like(m)
+
+    def run(k):
+        s = torch.cuda.current_stream().cuda_stream
+        ctx.forward_device(m.data_ptr(), k, syn.data_ptr(), out.data_ptr(), stream=s, hydrostatic=True)
+
+    run(100)
+    run(7)
+    torch.cuda.synchronize()
+    want = syn[:7].clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        run(7)
+    for k in (9, 30, n):
+        run(k)
+    torch.cuda.synchronize()
+    big = syn[:n].clone()
+    syn.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(syn[:7], want) and torch.equal(big[:7], want)

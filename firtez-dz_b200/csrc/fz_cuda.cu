@@ -1668,7 +1668,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT <= 256 ? 2 : 1)) k_synth_rf(const 
 //
 // What bounds it: the FP32 pipe -- per height and wavelength some 52 operations a
 // Zeeman component, 100 for each Stokes vector's products, 46 a direction, 20 a
-// node -- at 8 warps per SM (two CTAs of 4 warps; 247 registers hold the sums, the
+// node -- at 8 warps per SM (two CTAs of 4 warps; 255 registers hold the sums, the
 // operator and the products, and the two wavelengths give the independent work
 // that more warps would).  2,048 columns of 128 heights, two lines of 112
 // wavelengths, 13 nodes: 11.5 ms with a directional derivative of some 250
